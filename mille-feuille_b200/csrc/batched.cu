@@ -12,29 +12,32 @@
 //
 // Random column patterns make the SpMV gather-bound when the gathered vector
 // comes from L1/L2: every lane's element is its own cache line, about one
-// line per cycle per SM.  The matrix is therefore stored in column panels of
-// PW = 32768 columns (16-bit column offsets within the panel, rows of each
-// panel in CSR), and the mixed-precision kernel copies the panel's slice of p
-// (FP32, 128 KB) into shared memory before it streams the panel's chunks:
-// the gathers hit shared memory (about 8 lanes per cycle for random
-// addresses).  A chunk is a range of rows with at most BCE entries in every
-// panel; for each (chunk, panel) pair its row pointers, columns and values
-// arrive by bulk copies in one of NS = 3 shared-memory stages, produced by
-// warp 0 and consumed, in the mixed kernel, by a group of five warps per
-// stage (the FP64 kernel's fifteen consumer warps all take every pass).  A
-// mixed pass sums its rows in two phases: the products of consecutive
-// entries on consecutive lanes, written over the staged values, then one
-// lane per row adding its products in entry order.  The row sums of the
-// panels are added in panel order (partial sums kept in q).  The FP64 kernel
-// (the FP64 policy and trace collection) gathers p from global memory.
+// line per cycle per SM.  The mixed-precision kernel therefore keeps a window
+// of p (FP32, up to 55,296 columns, 216 KB) in shared memory and streams the
+// matrix in sorted slices of 32 rows (batch_sell.cuh): a lane owns a row, its
+// words come as 16-byte loads straight from L2/HBM into registers, the
+// gathers hit shared memory.  What bounds it: shared-memory wavefronts (the
+// gather of 32 random banks takes ~3.5) and the L2 latency of the words, then
+// the three cluster barriers of an iteration.  The earlier form -- bulk
+// copies into three shared-memory stages, products written back to shared
+// memory, one lane per row adding them -- moved every entry through shared
+// memory four times.  Measured, to a 1e-14 residual on one B200: 256 systems
+// of 1,000-32,000 rows, learned classes, 648 -> 370 ms; 24 systems of
+// 1,000-4,000 rows, static classes, 51.7 -> 37.6 ms.
 //
-// Values are held three times: FP64 (reliable updates, FP64 policy), FP32,
-// and FP16 scaled per row by a power of two (the row's largest
-// off-diagonal magnitude maps into [2^14, 2^15)) with the diagonal taken out
-// and kept in FP32 beside the row scale.  A mixed-precision solve reads each
-// chunk in its working class -- FP32 (4 + 2 bytes per entry) or FP16 (one
-// 4-byte word per entry: the value bits and the column offset) -- and
-// accumulates in FP32; FP64 dot products, FP64 reliable updates
+// The panel storage (column panels of PW = 32768 columns, 16-bit column
+// offsets within the panel, rows of each panel in CSR) is what the chunks,
+// the exports and the FP64 kernel use.  A chunk is a range of rows with at
+// most BCE entries in every panel.  The FP64 kernel (the FP64 policy and trace
+// collection) stages (chunk, panel) passes in shared memory by bulk copies
+// and gathers p from global memory.
+//
+// Values of the slices are held in FP64 (reliable updates), FP32, and FP16
+// scaled per row by a power of two (the row's largest off-diagonal magnitude
+// maps into [2^14, 2^15)), the diagonal kept apart.  A mixed-precision solve
+// reads each chunk's rows in its working class -- FP32 (4 + 2 bytes per entry)
+// or FP16 (one 4-byte word per entry: the value bits and the column offset) --
+// and accumulates in FP32; FP64 dot products, FP64 reliable updates
 // r = b - A x from the FP64 values, convergence judged on that FP64
 // residual.
 //
@@ -72,6 +75,7 @@
 #include <type_traits>
 
 #include "mf_internal.h"
+#include "batch_sell.cuh"
 #include "policy_net.cuh"
 #include "tma.cuh"
 
@@ -106,9 +110,7 @@ struct mf_batch_s {
     int *d_prow = nullptr;        // panel row pointers, relative to the panel's first entry
     uint16_t *d_col = nullptr;    // column offset within the panel
     double *d_val = nullptr;
-    float *d_val32 = nullptr;
     __half *d_val16 = nullptr;    // row-scaled, diagonal entries 0
-    uint32_t *d_cv16 = nullptr;   // FP16 value bits << 16 | column offset (one word per entry)
     float *d_rscale = nullptr;    // per row: scale of the FP16 values
     float *d_diag32 = nullptr;    // per row: diagonal (sum of the row's diagonal entries)
     // row chunks of every system
@@ -126,6 +128,14 @@ struct mf_batch_s {
     void *work = nullptr;
     size_t work_bytes = 0;
     int *d_queue = nullptr;
+    // sorted slices of the mixed solves (batch_sell.cuh)
+    int *d_sfirst = nullptr, *d_win0 = nullptr;
+    int2 *d_sdesc = nullptr;
+    int4 *d_srec = nullptr;
+    uint32_t *d_scv = nullptr;
+    float *d_sv32 = nullptr;
+    double *d_sv64 = nullptr, *d_diag64 = nullptr;  // diag64: per row (sum of the row's diagonal entries)
+    uint16_t *d_sc16 = nullptr;
     // CUDA graph of the last solve configuration
     cudaGraphExec_t graph = nullptr;
     const void *graph_b = nullptr;
@@ -147,6 +157,11 @@ namespace {
 
 constexpr int BNT = 512;
 constexpr int BNW = BNT / 32;
+#ifndef MF_BATCH_MNT
+#define MF_BATCH_MNT 512
+#endif
+constexpr int MNT = MF_BATCH_MNT;  // threads of a mixed-kernel CTA
+constexpr int MNW = MNT / 32;
 constexpr int NCSTAT = 6;   // static chunk features 0-4, and max |a| of the chunk
 constexpr int NCDYN = 10;   // [0..3] raw maxima |r|, |p|, |dp|, |q|; [4..7] previous features 6..9; [8] label ratio
 constexpr float LEARN_CONF = 0.9f;   // FP16 when P(label <= FP16) >= this
@@ -160,10 +175,9 @@ struct BatchArgs {
     const int *prow;
     const uint16_t *col;
     const double *val;
-    const float *val32;
     const __half *val16;
-    const uint32_t *cv16;
     const float *rscale, *diag32;
+    SellView sell;                 // mixed solves: the sorted slices
     const double *b;
     double *x;
     void *r, *p0, *p1, *q, *xlo;  // workspace vectors (rows_total each)
@@ -181,7 +195,6 @@ struct BatchArgs {
     double delta;
     unsigned long long budget_ns;  // bound of every shared-memory stage wait
     unsigned backoff_ns;           // sleep between retries of a stage wait
-    int rowsum;                    // mixed passes: 0 two-phase row sums, 1 lane groups per row
     int policy;
     const __nv_bfloat16 *mlp_w;    // LEARNED: the network's BF16 weights
     // trace collection (FP64 solves): samples every collect_every iterations
@@ -212,9 +225,10 @@ __device__ __forceinline__ SysView sys_view(const BatchArgs &a, int sys)
 // Deterministic cluster-wide sum: each CTA reduces its threads in a fixed
 // tree, publishes the value in its shared memory, and after the cluster
 // barrier every CTA adds the CTAs' values in rank order.
+template <int NT>
 __device__ __forceinline__ double cluster_sum(cg::cluster_group &cl, double v, double *slot, double *s_warp)
 {
-    const double c = block_sum<BNT>(v, s_warp);
+    const double c = block_sum<NT>(v, s_warp);
     if (threadIdx.x == 0) *slot = c;
     cl.sync();
     double s = 0.0;
@@ -224,6 +238,7 @@ __device__ __forceinline__ double cluster_sum(cg::cluster_group &cl, double v, d
 }
 
 // Cluster-wide maximum of two non-negative values (exact, so any order).
+template <int NT>
 __device__ __forceinline__ void cluster_max2(cg::cluster_group &cl, float &a, float &b, float *slot2, float *s_warp2)
 {
 #pragma unroll
@@ -239,7 +254,7 @@ __device__ __forceinline__ void cluster_max2(cg::cluster_group &cl, float &a, fl
     __syncthreads();
     if (threadIdx.x == 0) {
         float ma = 0.f, mb = 0.f;
-        for (int w = 0; w < BNW; w++) {
+        for (int w = 0; w < NT / 32; w++) {
             ma = fmaxf(ma, s_warp2[2 * w]);
             mb = fmaxf(mb, s_warp2[2 * w + 1]);
         }
@@ -256,63 +271,46 @@ __device__ __forceinline__ void cluster_max2(cg::cluster_group &cl, float &a, fl
     }
 }
 
+// FP64 kernel: the header of a staged (chunk, panel) pair.
 struct BHdr {
     int r0, r1, e0, direct;   // rows [r0, r1), first entry e0 (relative to the panel)
-    int sh_rp, sh_col, sh_val, cls;
-    int panel, sh_rs, sh_dg, pad0;
+    int sh_rp, sh_col, sh_val, panel;
     long long ebase;          // the panel's first entry (global)
 };
 
-// Stages in flight per CTA.  The mixed kernels stage at most 4 + 2 bytes
-// per entry (FP32 values, 16-bit columns); their consumer warps form
-// MF_BATCH_GROUPS groups, group g consuming the stages k with k % groups = g.
-#ifndef MF_BATCH_STAGES_MIX
-#define MF_BATCH_STAGES_MIX 3
-#endif
-#ifndef MF_BATCH_GROUPS
-#define MF_BATCH_GROUPS 3
-#endif
+// FP64 kernel: shared-memory stages of (chunk, panel) pairs (row pointers,
+// columns, values) in flight per CTA.
 #ifndef MF_BATCH_STAGES_FP64
 #define MF_BATCH_STAGES_FP64 3
 #endif
 
-// Shared-memory stage of one (chunk, panel) pair: row pointers, columns,
-// values.
-template <bool MIX>
 struct Stage {
-    static constexpr int NS = MIX ? MF_BATCH_STAGES_MIX : MF_BATCH_STAGES_FP64;
-    static constexpr int VB = MIX ? 4 : 8;  // widest stored value
+    static constexpr int NS = MF_BATCH_STAGES_FP64;
     static constexpr int OFF_RP = 0;
     static constexpr int OFF_COL = ((BCR + 1) * 4 + 32 + 15) & ~15;
     static constexpr int OFF_VAL = OFF_COL + ((BCE * 2 + 32 + 15) & ~15);
-    static constexpr int OFF_RS = OFF_VAL + ((BCE * VB + 32 + 15) & ~15);  // FP16 passes: row scales
-    static constexpr int OFF_DG = OFF_RS + ((BCR * 4 + 32 + 15) & ~15);    // FP16 passes: FP32 diagonals
-    static constexpr int SIZE = OFF_DG + ((BCR * 4 + 32 + 15) & ~15);
+    static constexpr int SIZE = OFF_VAL + ((BCE * 8 + 32 + 15) & ~15);
     static_assert(OFF_COL % 16 == 0 && OFF_VAL % 16 == 0 && SIZE % 16 == 0, "stage regions 16-byte aligned");
     static_assert((BCR + 1) * 4 + 32 <= OFF_COL, "row pointers fit");
     static_assert(NS >= 1 && NS <= 8, "stage phases kept in a byte");
 };
 
-template <bool MIX>
 struct BSmem {
-    unsigned char stage[Stage<MIX>::NS][Stage<MIX>::SIZE];
-    BHdr hdr[Stage<MIX>::NS];
-    uint64_t bar[Stage<MIX>::NS];    // stage full (the producer's copies landed)
-    uint64_t empty[Stage<MIX>::NS];  // stage released by every consumer warp
-    uint64_t pbar;                   // the p window's copy landed
-    uint64_t wempty;                 // the p window released by every consumer warp
+    unsigned char stage[Stage::NS][Stage::SIZE];
+    BHdr hdr[Stage::NS];
+    uint64_t bar[Stage::NS];    // stage full (the producer's copies landed)
+    uint64_t empty[Stage::NS];  // stage released by every consumer warp
 };
+static_assert(sizeof(BSmem) <= 227 * 1024, "one CTA per SM");
 
-// dynamic shared memory: the stages, the p window (mixed kernel: a panel
-// of p in FP32), the MLP weights as float and the per-warp feature rows
-template <bool MIX>
-struct SmemLayout {
-    static constexpr size_t PWIN = (sizeof(BSmem<MIX>) + 15) & ~(size_t)15;
-    static constexpr size_t PWIN_BYTES = MIX ? (size_t)PW * 4 + 32 : 0;
-    static constexpr size_t W = PWIN + PWIN_BYTES;
+// Dynamic shared memory of the mixed kernel: the window of p (its first
+// element at the same 16-byte phase as in global memory), the policy
+// network's weights as float, a feature row per warp.
+struct MixSmem {
+    static constexpr size_t W = ((size_t)SELL_WIN + 4) * 4;
     static constexpr size_t FEAT = W + sizeof(float) * ((PN_NPARAM + 3) & ~3);
-    static constexpr size_t TOTAL = FEAT + sizeof(float) * BNW * PN_NF;
-    static_assert(TOTAL <= 227 * 1024, "one CTA per SM");
+    static constexpr size_t TOTAL = FEAT + sizeof(float) * MNW * PN_NF;
+    static_assert(TOTAL <= 226 * 1024, "one CTA per SM, 1 KB for the static arrays");
 };
 
 __device__ __forceinline__ void b_add_range(unsigned char *dst, const unsigned char *src, long long a0, long long a1,
@@ -329,13 +327,13 @@ __device__ __forceinline__ unsigned b_range_bytes(long long a0, long long a1)
 }
 
 // A (chunk, panel) pair: rows [r0, r1) of the system, entries [e0, e1) of
-// the panel (relative to its first entry ebase), the chunk's class.
+// the panel (relative to its first entry ebase).
 struct BChunk {
-    int r0, r1, e0, e1, cls, panel;
-    long long ebase, rpbase, rowbase;
+    int r0, r1, e0, e1, panel;
+    long long ebase, rpbase;
 };
 
-__device__ __forceinline__ BChunk b_chunk(const BatchArgs &a, int sys, const SysView &v, int c, int k, bool mix)
+__device__ __forceinline__ BChunk b_chunk(const BatchArgs &a, int sys, const SysView &v, int c, int k)
 {
     BChunk ch;
     ch.r0 = a.crow[c + sys];
@@ -345,58 +343,39 @@ __device__ __forceinline__ BChunk b_chunk(const BatchArgs &a, int sys, const Sys
     ch.ebase = a.pent0[v.gp0 + k];
     ch.e0 = a.prow[ch.rpbase + ch.r0];
     ch.e1 = a.prow[ch.rpbase + ch.r1];
-    ch.cls = mix ? (int)a.ccls[c] : 0;
-    ch.rowbase = v.r0;
     return ch;
 }
 
-// Algorithmic bytes of one (chunk, panel) pass in class `cls`.
-template <bool MIX>
-__device__ __forceinline__ unsigned long long chunk_bytes(const BChunk &ch)
+// Algorithmic bytes of nr rows with ne entries over np panels: vb-byte
+// values, 2-byte columns, row pointers, and for FP16 the rows' scales and
+// diagonals.
+__device__ __forceinline__ unsigned long long pass_bytes(long long ne, int nr, int np, int vb)
 {
-    const unsigned long long ne = (unsigned long long)(ch.e1 - ch.e0), nr = (unsigned long long)(ch.r1 - ch.r0);
-    const unsigned vb = MIX ? (ch.cls ? 2u : 4u) : 8u;
-    return ne * (vb + 2) + (nr + 1) * 4 + (ch.cls ? nr * 8 : 0);
+    return (unsigned long long)ne * (vb + 2) + (unsigned long long)np * ((unsigned)(nr + 1) * 4u + (vb == 2 ? nr * 8u : 0u));
 }
 
 // Thread 0: stage pair `ch` into stage k.
-template <bool MIX>
-__device__ void b_issue(const BatchArgs &a, BSmem<MIX> &S, const BChunk &ch, int k)
+__device__ void b_issue(const BatchArgs &a, BSmem &S, const BChunk &ch, int k)
 {
-    using SG = Stage<MIX>;
     BHdr &h = S.hdr[k];
     const int r0 = ch.r0, r1 = ch.r1, e0 = ch.e0, e1 = ch.e1;
     h.r0 = r0;
     h.r1 = r1;
     h.e0 = e0;
     h.direct = (e1 - e0 > BCE) ? 1 : 0;
-    h.cls = ch.cls;
     h.panel = ch.panel;
     h.ebase = ch.ebase;
-    const long long z0 = ch.ebase, rw = ch.rowbase;
-    const bool h16 = MIX && ch.cls == 1;  // FP16 rows: packed (value, column) words, row scales and diagonals
-    const int vb = MIX ? 4 : 8;  // FP16 passes: one 4-byte word per entry
+    const long long z0 = ch.ebase;
     unsigned total = b_range_bytes(4 * (ch.rpbase + r0), 4 * (ch.rpbase + r1 + 1));
-    if (!h.direct) {
-        total += b_range_bytes(vb * (z0 + e0), vb * (z0 + e1));
-        if (!h16) total += b_range_bytes(2 * (z0 + e0), 2 * (z0 + e1));
-    }
-    if (h16) total += 2 * b_range_bytes(4 * (rw + r0), 4 * (rw + r1));
+    if (!h.direct) total += b_range_bytes(8 * (z0 + e0), 8 * (z0 + e1)) + b_range_bytes(2 * (z0 + e0), 2 * (z0 + e1));
     fence_proxy_async_smem();
     mbar_arrive_expect_tx(&S.bar[k], total);
     unsigned char *st = S.stage[k];
-    b_add_range(st + SG::OFF_RP, (const unsigned char *)a.prow, 4 * (ch.rpbase + r0), 4 * (ch.rpbase + r1 + 1),
+    b_add_range(st + Stage::OFF_RP, (const unsigned char *)a.prow, 4 * (ch.rpbase + r0), 4 * (ch.rpbase + r1 + 1),
                 &S.bar[k], h.sh_rp);
-    if (h16) {
-        b_add_range(st + SG::OFF_RS, (const unsigned char *)a.rscale, 4 * (rw + r0), 4 * (rw + r1), &S.bar[k], h.sh_rs);
-        b_add_range(st + SG::OFF_DG, (const unsigned char *)a.diag32, 4 * (rw + r0), 4 * (rw + r1), &S.bar[k], h.sh_dg);
-    }
     if (h.direct) return;
-    if (!h16)
-        b_add_range(st + SG::OFF_COL, (const unsigned char *)a.col, 2 * (z0 + e0), 2 * (z0 + e1), &S.bar[k], h.sh_col);
-    const unsigned char *vsrc = MIX ? (h16 ? (const unsigned char *)a.cv16 : (const unsigned char *)a.val32)
-                                    : (const unsigned char *)a.val;
-    b_add_range(st + SG::OFF_VAL, vsrc, vb * (z0 + e0), vb * (z0 + e1), &S.bar[k], h.sh_val);
+    b_add_range(st + Stage::OFF_COL, (const unsigned char *)a.col, 2 * (z0 + e0), 2 * (z0 + e1), &S.bar[k], h.sh_col);
+    b_add_range(st + Stage::OFF_VAL, (const unsigned char *)a.val, 8 * (z0 + e0), 8 * (z0 + e1), &S.bar[k], h.sh_val);
 }
 
 // L lanes per row: lanes stride over the row's entries (BU entries per lane
@@ -408,133 +387,73 @@ __device__ void b_issue(const BatchArgs &a, BSmem<MIX> &S, const BChunk &ch, int
 #endif
 constexpr int BU = MF_BATCH_BU;
 
-// product loads in flight per lane in the two-phase row sums
-#ifndef MF_BATCH_P1U
-#define MF_BATCH_P1U 8
-#endif
-#define MF_PRAGMA(x) _Pragma(#x)
-#define MF_UNROLL(n) MF_PRAGMA(unroll n)
-
 struct RowPair {
     int a0, e0, a1, e1;
 };
 
-__device__ __forceinline__ float vfma(float a, float b, float c) { return fmaf(a, b, c); }
-__device__ __forceinline__ double vfma(double a, double b, double c) { return fma(a, b, c); }
-
-template <typename V>
-__device__ __forceinline__ V ld_stream(const V *p)
-{
-    return __ldcs(p);
-}
-template <>
-__device__ __forceinline__ __half ld_stream<__half>(const __half *p)
-{
-    return __ushort_as_half(__ldcs((const unsigned short *)p));
-}
-
-// Row sums of two rows; V is the stored value type (double, float, or the
-// row-scaled __half).  FP64 values accumulate in FP64, the others in FP32.
-template <int L, typename V, class Src, bool GLOBAL>
+// FP64 sums of two rows from global memory.
+template <int L, class Src>
 __device__ __forceinline__ void row_dot2(const RowPair &rb, const uint16_t *__restrict__ col,
-                                         const V *__restrict__ val, int lane, Src src, double &y0, double &y1)
+                                         const double *__restrict__ val, int lane, Src src, double &y0, double &y1)
 {
-    using XT = decltype(src(0));
-    constexpr bool D = std::is_same<V, double>::value;
-    using AT = typename std::conditional<D, double, float>::type;
     const int a0 = rb.a0, e0 = rb.e0, a1 = rb.a1, e1 = rb.e1;
-    AT s0 = 0, s1 = 0;
+    double s0 = 0, s1 = 0;
     const int n0 = e0 - a0, n1 = e1 - a1, nmax = n0 > n1 ? n0 : n1;
     for (int k = lane; k < nmax; k += L * BU) {
         int c0[BU], c1[BU];
-        AT v0[BU], v1[BU];
+        double v0[BU], v1[BU];
 #pragma unroll
         for (int u = 0; u < BU; u++) {
             const int kk = k + u * L;
             const bool in0 = kk < n0, in1 = kk < n1;
-            if constexpr (GLOBAL) {
-                c0[u] = in0 ? (int)ld_stream(col + a0 + kk) : -1;
-                c1[u] = in1 ? (int)ld_stream(col + a1 + kk) : -1;
-                v0[u] = in0 ? (AT)ld_stream(val + a0 + kk) : (AT)0;
-                v1[u] = in1 ? (AT)ld_stream(val + a1 + kk) : (AT)0;
-            } else {  // staged in shared memory
-                c0[u] = in0 ? (int)col[a0 + kk] : -1;
-                c1[u] = in1 ? (int)col[a1 + kk] : -1;
-                v0[u] = in0 ? (AT)val[a0 + kk] : (AT)0;
-                v1[u] = in1 ? (AT)val[a1 + kk] : (AT)0;
-            }
+            c0[u] = in0 ? (int)__ldcs(col + a0 + kk) : -1;
+            c1[u] = in1 ? (int)__ldcs(col + a1 + kk) : -1;
+            v0[u] = in0 ? __ldcs(val + a0 + kk) : 0.0;
+            v1[u] = in1 ? __ldcs(val + a1 + kk) : 0.0;
         }
-        XT x0[BU], x1[BU];
+        double x0[BU], x1[BU];
 #pragma unroll
         for (int u = 0; u < BU; u++) {
-            x0[u] = c0[u] >= 0 ? src(c0[u]) : (XT)0;
-            x1[u] = c1[u] >= 0 ? src(c1[u]) : (XT)0;
+            x0[u] = c0[u] >= 0 ? src(c0[u]) : 0.0;
+            x1[u] = c1[u] >= 0 ? src(c1[u]) : 0.0;
         }
 #pragma unroll
         for (int u = 0; u < BU; u++) {
-            s0 = vfma(v0[u], (AT)x0[u], s0);
-            s1 = vfma(v1[u], (AT)x1[u], s1);
+            s0 = fma(v0[u], x0[u], s0);
+            s1 = fma(v1[u], x1[u], s1);
         }
     }
-    double d0 = (double)s0, d1 = (double)s1;
 #pragma unroll
     for (int o = L / 2; o > 0; o >>= 1) {
-        d0 += __shfl_xor_sync(0xffffffffu, d0, o, L);
-        d1 += __shfl_xor_sync(0xffffffffu, d1, o, L);
+        s0 += __shfl_xor_sync(0xffffffffu, s0, o, L);
+        s1 += __shfl_xor_sync(0xffffffffu, s1, o, L);
     }
-    y0 = d0;
-    y1 = d1;
+    y0 = s0;
+    y1 = s1;
 }
 
-// One row's sum from a staged pass: lanes stride over the row's entries, BU
-// per lane per trip, loaded without predicates -- columns past the row's end
-// are read from the stage and masked into the p window (which holds finite
-// values: zeros before its first copy), their weights are zero.  Lane sums
-// combine in a fixed xor tree.
-template <int L, typename V, class Src>
+// One row's FP64 sum from a staged pass: lanes stride over the row's
+// entries, BU per lane per trip, loaded without predicates -- columns past
+// the row's end are read from the stage and masked into the panel, their
+// weights are zero.  Lane sums combine in a fixed xor tree.
+template <int L, class Src>
 __device__ __forceinline__ double row_dot1_smem(int a, int e, const uint16_t *__restrict__ col,
-                                                const V *__restrict__ val, int lane, Src src)
+                                                const double *__restrict__ val, int lane, Src src)
 {
-    constexpr bool D = std::is_same<V, double>::value;
-    using AT = typename std::conditional<D, double, float>::type;
-    AT s = 0;
+    double s = 0;
     const int n = e - a;
     for (int k = lane; k < n; k += L * BU) {
 #pragma unroll
         for (int u = 0; u < BU; u++) {
             const int kk = k + u * L;
             const int c = (int)col[a + kk] & (PW - 1);
-            const AT v = kk < n ? (AT)val[a + kk] : (AT)0;
-            s = vfma(v, (AT)src(c), s);
+            const double v = kk < n ? val[a + kk] : 0.0;
+            s = fma(v, src(c), s);
         }
     }
-    double d = (double)s;
 #pragma unroll
-    for (int o = L / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o, L);
-    return d;
-}
-
-// The same for an FP16 pass: one 32-bit word per entry (FP16 value bits in
-// the high half, the column offset in the low half), so a slot costs one
-// shared-memory load besides its gather.
-template <int L, class Src>
-__device__ __forceinline__ double row_dot1_cv16(int a, int e, const uint32_t *__restrict__ cv, int lane, Src src)
-{
-    float s = 0.f;
-    const int n = e - a;
-    for (int k = lane; k < n; k += L * BU) {
-#pragma unroll
-        for (int u = 0; u < BU; u++) {
-            const int kk = k + u * L;
-            const uint32_t w = cv[a + kk];
-            const float v = kk < n ? __half2float(__ushort_as_half((unsigned short)(w >> 16))) : 0.f;
-            s = fmaf(v, (float)src((int)(w & (uint32_t)(PW - 1))), s);
-        }
-    }
-    double d = (double)s;
-#pragma unroll
-    for (int o = L / 2; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o, L);
-    return d;
+    for (int o = L / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o, L);
+    return s;
 }
 
 // FP64 row sums of rows i0, i1 (-1: none) of a system over all its panels,
@@ -556,7 +475,7 @@ __device__ __forceinline__ void row_dot2_fp64_all(const BatchArgs &a, const SysV
         const double *xk = xs + (long long)k * PW;
         auto src = [=](int c) -> double { return xk[c]; };
         double t0, t1;
-        row_dot2<L, double, decltype(src), true>(rr, a.col + eb, a.val + eb, lane, src, t0, t1);
+        row_dot2<L>(rr, a.col + eb, a.val + eb, lane, src, t0, t1);
         y0 += t0;
         y1 += t1;
     }
@@ -593,7 +512,12 @@ __device__ void chunk_stats_warp(const BatchArgs &a, const SysView &v, int c, in
         mr = fmaxf(mr, (float)fabs((double)r[i]));
         mp = fmaxf(mp, (float)fabs(pv));
         mdp = fmaxf(mdp, (float)fabs(pv - (double)po[i]));
-        mq = fmaxf(mq, (float)fabs((double)__ldcg(q + i)));
+        // FP64 solves: q read past L1 (partial sums arrive by reductions in
+        // L2); mixed solves: q may be in shared memory
+        double qv;
+        if constexpr (std::is_same<VT, double>::value) qv = __ldcg(q + i);
+        else qv = (double)q[i];
+        mq = fmaxf(mq, (float)fabs(qv));
         if (label) {
             const double s = (double)rscale[i];
             double dq = 0.0, qq = 0.0;
@@ -677,79 +601,40 @@ __device__ __forceinline__ int learned_chunk_class(const float *w, const float *
     return (e[0] + e[1] >= LEARN_CONF * z) ? 1 : 0;
 }
 
-// Thread 0: copy panel `k` of p (FP32: p[k PW .. min(n, (k+1) PW))) into the
-// shared-memory window; shift_elems receives the position of p[k PW] in the
-// window (the copy starts at the 16-byte boundary below it).
-__device__ __forceinline__ void issue_pwin(uint64_t *bar, unsigned char *win, const float *p, int n, int k,
-                                           int &shift_elems)
+// The FP64 kernel (the FP64 policy and trace collection): one cluster per
+// system; warp 0 stages (chunk, panel) passes, the other warps sum their
+// rows, p gathered from global memory.
+template <int L>
+__global__ void __launch_bounds__(BNT, 1) k_batched_cg64(const __grid_constant__ BatchArgs a)
 {
-    const long long a0 = (long long)k * PW, a1 = min((long long)n, a0 + PW);
-    const unsigned long long base = (unsigned long long)(p + a0);
-    const unsigned long long c0 = base & ~15ull, c1 = ((unsigned long long)(p + a1) + 15ull) & ~15ull;
-    shift_elems = (int)((base - c0) >> 2);
-    // p was written by the cluster's threads (generic proxy) before the
-    // cluster barrier; the bulk copy reads it through the async proxy
-    asm volatile("fence.proxy.async.global;\n" ::: "memory");
-    fence_proxy_async_smem();
-    mbar_arrive_expect_tx(bar, (unsigned)(c1 - c0));
-    bulk_g2s(win, (const void *)c0, (unsigned)(c1 - c0), bar);
-}
-
-#ifndef MF_BATCH_MINB
-#define MF_BATCH_MINB 1
-#endif
-
-template <int L, bool MIX>
-__global__ void __launch_bounds__(BNT, MF_BATCH_MINB) k_batched_cg(BatchArgs a)
-{
-    using VT = typename std::conditional<MIX, float, double>::type;
-    using SG = Stage<MIX>;
-    using SL = SmemLayout<MIX>;
-    constexpr int NS = SG::NS;
+    constexpr int NS = Stage::NS;
     cg::cluster_group cl = cg::this_cluster();
     __shared__ double s_warp[BNW];
     __shared__ double s_slot[8];
     __shared__ float s_fslot[2];
     __shared__ float s_fwarp[2 * BNW];
+    __shared__ float s_feat[BNW * PN_NF];
     __shared__ int s_sys;
     __shared__ int s_fail;
-    __shared__ int s_pshift;
     extern __shared__ __align__(16) unsigned char b_smem_raw[];
-    BSmem<MIX> &S = *reinterpret_cast<BSmem<MIX> *>(b_smem_raw);
-    unsigned char *s_win = b_smem_raw + SL::PWIN;
-    float *s_w = reinterpret_cast<float *>(b_smem_raw + SL::W);
-    float *s_feat = reinterpret_cast<float *>(b_smem_raw + SL::FEAT);
-    const bool learned = MIX && a.policy == MF_POLICY_LEARNED && a.mlp_w;
-    const bool rule = MIX && a.policy == MF_POLICY_RULE;
-    const bool collect = !MIX && a.collect_every > 0;
+    BSmem &S = *reinterpret_cast<BSmem *>(b_smem_raw);
+    const bool collect = a.collect_every > 0;
     if (threadIdx.x == 0) {
         for (int k = 0; k < NS; k++) {
             mbar_init(&S.bar[k], 1);
-            mbar_init(&S.empty[k], MIX ? (BNW - 1) / MF_BATCH_GROUPS : BNW - 1);  // the stage's consumer warps
+            mbar_init(&S.empty[k], BNW - 1);  // the consumer warps
         }
-        mbar_init(&S.pbar, 1);
-        mbar_init(&S.wempty, BNW - 1);
         mbar_fence_init();
     }
-    if (learned)
-        for (int k = threadIdx.x; k < PN_NPARAM; k += BNT) s_w[k] = __bfloat162float(a.mlp_w[k]);
-    // the p window holds finite values from the start (padded slots of the
-    // row loop read it with zero weight)
-    if (MIX)
-        for (int k = threadIdx.x; k < (int)(SL::PWIN_BYTES / 4); k += BNT) ((float *)s_win)[k] = 0.f;
     __syncthreads();
     // mbarrier phase parities, one bit per stage (registers: an array indexed
     // by the stage number would live in local memory).  Producer (thread 0):
-    // fills of each stage and of the window so far (parity), which stages /
-    // whether the window were filled at all.  Consumers: passes consumed per
-    // stage and windows consumed (parity).
-    unsigned pfill = 0, pstarted = 0, wpar = 0, wstarted = 0;
-    unsigned cfull = 0, cwpar = 0;
+    // fills of each stage so far (parity) and which stages were filled at
+    // all.  Consumers: passes consumed per stage (parity).
+    unsigned pfill = 0, pstarted = 0, cfull = 0;
     const unsigned rank = cl.block_rank(), ncta = cl.num_blocks();
     const int tid = threadIdx.x;
-    const int lane = tid % L, grp = tid / L;
     const int wid = tid >> 5, wl = tid & 31;
-    constexpr int GPB = BNT / L;  // row groups per CTA
     for (;;) {
         // after a wait that gave up (status word set) no cluster takes another
         // system: the stages' barrier phases of the failed CTA are not known
@@ -764,8 +649,8 @@ __global__ void __launch_bounds__(BNT, MF_BATCH_MINB) k_batched_cg(BatchArgs a)
         const double *b = a.b + r0;
         double *x = a.x + r0;
         const float *rscale = a.rscale + r0;
-        VT *r = (VT *)a.r + r0, *q = (VT *)a.q + r0, *xlo = (VT *)a.xlo + r0;
-        VT *pb[2] = {(VT *)a.p0 + r0, (VT *)a.p1 + r0};
+        double *r = (double *)a.r + r0, *q = (double *)a.q + r0;
+        double *pb[2] = {(double *)a.p0 + r0, (double *)a.p1 + r0};
         // this CTA's chunks and rows
         const int sc0 = a.sc[sys], nch = a.sc[sys + 1] - sc0;
         const int cl0 = sc0 + (int)((long long)nch * rank / ncta), cl1 = sc0 + (int)((long long)nch * (rank + 1) / ncta);
@@ -773,57 +658,36 @@ __global__ void __launch_bounds__(BNT, MF_BATCH_MINB) k_batched_cg(BatchArgs a)
         const int ra = a.crow[cl0 + sys], rb = a.crow[cl1 + sys];
         const int npan = V.npan;
         const int J = nchl * npan;  // (chunk, panel) passes per SpMV, panel-major
-        unsigned long long st_bytes = 0, st_lowp = 0, st_pass = 0;  // thread 0: passes issued
-        double lb = 0.0, lr = 0.0;
+        unsigned long long st_bytes = 0, st_pass = 0;  // thread 0: passes issued
+        double lb = 0.0;
         for (int i = ra + tid; i < rb; i += BNT) {
             const double bv = b[i];
-            const VT rv = (VT)bv;
             x[i] = 0.0;
-            r[i] = rv;
-            pb[0][i] = (VT)0;
-            if (MIX) xlo[i] = (VT)0;
+            r[i] = bv;
+            pb[0][i] = 0.0;
             lb += bv * bv;
-            lr += (double)rv * (double)rv;
         }
-        if (MIX)
-            for (int c = cl0 + tid; c < cl1; c += BNT) a.ccls[c] = (a.ccls_static[c] & 1) ? 1 : 0;
-        const double bb = cluster_sum(cl, lb, &s_slot[0], s_warp);
-        double rho = MIX ? cluster_sum(cl, lr, &s_slot[1], s_warp) : bb;
+        const double bb = cluster_sum<BNT>(cl, lb, &s_slot[0], s_warp);
+        double rho = bb;
         const double nb = sqrt(bb) > 0.0 ? sqrt(bb) : 1.0;
-        double beta = 0.0, rmax = sqrt(rho), relres = sqrt(rho) / nb;
-        int it = 0, refs = 0, status = MF_OK;
-        bool lowp_off = false, have_prev = false;
+        double beta = 0.0, relres = sqrt(rho) / nb;
+        int it = 0, status = MF_OK;
+        bool have_prev = false;
         while (true) {
             if (sqrt(rho) <= a.tol * nb) break;
             if (it >= a.maxiter) {
                 status = MF_ERR_NOT_CONVERGED;
                 break;
             }
-            const VT *pold = pb[it & 1];
-            VT *pnew = pb[(it & 1) ^ 1];
-            const VT bt = (VT)beta;
+            const double *pold = pb[it & 1];
+            double *pnew = pb[(it & 1) ^ 1];
             // p = r + beta p over this CTA's rows, then a cluster barrier: the
-            // SpMV needs all of p.  RULE: one warp per chunk, deciding the
-            // chunk's class from its own rows' change.
-            if (rule && !lowp_off) {
-                for (int c = cl0 + wid; c < cl1; c += BNW) {
-                    const int c0 = a.crow[c + sys], c1 = a.crow[c + 1 + sys];
-                    double v = 0.0;
-                    for (int i = c0 + wl; i < c1; i += 32) {
-                        const VT pv = vfma(bt, pold[i], r[i]);
-                        pnew[i] = pv;
-                        if (npan == 2) q[i] = (VT)0;
-                        v = fmax(v, fabs((double)pv - (double)pold[i]));
-                    }
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-                    if (wl == 0) a.ccls[c] = (unsigned char)rule_chunk_class(v, a.ccls_static[c]);
-                }
-            } else {
-                // four rows per thread in flight: loads first, then the stores
+            // SpMV needs all of p.  Four rows per thread in flight: loads
+            // first, then the stores.
+            {
                 int i = ra + tid;
                 for (; i + 3 * BNT < rb; i += 4 * BNT) {
-                    VT po4[4], r4[4];
+                    double po4[4], r4[4];
 #pragma unroll
                     for (int u = 0; u < 4; u++) {
                         po4[u] = pold[i + u * BNT];
@@ -831,13 +695,13 @@ __global__ void __launch_bounds__(BNT, MF_BATCH_MINB) k_batched_cg(BatchArgs a)
                     }
 #pragma unroll
                     for (int u = 0; u < 4; u++) {
-                        pnew[i + u * BNT] = vfma(bt, po4[u], r4[u]);
-                        if (npan == 2) q[i + u * BNT] = (VT)0;
+                        pnew[i + u * BNT] = fma(beta, po4[u], r4[u]);
+                        if (npan == 2) q[i + u * BNT] = 0.0;
                     }
                 }
                 for (; i < rb; i += BNT) {
-                    pnew[i] = vfma(bt, pold[i], r[i]);
-                    if (npan == 2) q[i] = (VT)0;
+                    pnew[i] = fma(beta, pold[i], r[i]);
+                    if (npan == 2) q[i] = 0.0;
                 }
             }
             cl.sync();
@@ -845,10 +709,8 @@ __global__ void __launch_bounds__(BNT, MF_BATCH_MINB) k_batched_cg(BatchArgs a)
             // SpMV.  Warp 0 produces: its lanes load the descriptors of 32
             // (chunk, panel) passes at a time and lane 0 issues their bulk
             // copies into NS shared-memory stages, each stage refilled once
-            // the consumers have released it (empty barrier), and before the
-            // first pass of each panel the copy of p's window for that panel
-            // (mixed kernel) once the previous window is released.  Warps
-            // 1.. consume: wait for a stage (full barrier), compute its rows,
+            // the consumers have released it (empty barrier).  Warps 1..
+            // consume: wait for a stage (full barrier), compute its rows,
             // release it -- no CTA-wide barrier per pass.  Every wait is
             // bounded; a failure is voted CTA-wide and cluster-wide below.
             bool fail = false;
@@ -858,12 +720,11 @@ __global__ void __launch_bounds__(BNT, MF_BATCH_MINB) k_batched_cg(BatchArgs a)
                     // ones are issued
                     BChunk dn;
                     memset(&dn, 0, sizeof(dn));
-                    if (wl < J) dn = b_chunk(a, sys, V, cl0 + wl % nchl, wl / nchl, MIX);
+                    if (wl < J) dn = b_chunk(a, sys, V, cl0 + wl % nchl, wl / nchl);
                     for (int jb = 0; jb < J && !fail; jb += 32) {
                         const BChunk d = dn;
                         memset(&dn, 0, sizeof(dn));
-                        if (jb + 32 + wl < J)
-                            dn = b_chunk(a, sys, V, cl0 + (jb + 32 + wl) % nchl, (jb + 32 + wl) / nchl, MIX);
+                        if (jb + 32 + wl < J) dn = b_chunk(a, sys, V, cl0 + (jb + 32 + wl) % nchl, (jb + 32 + wl) / nchl);
                         const int cnt = min(32, J - jb);
                         for (int t = 0; t < cnt; t++) {
                             BChunk ch;
@@ -871,33 +732,20 @@ __global__ void __launch_bounds__(BNT, MF_BATCH_MINB) k_batched_cg(BatchArgs a)
                             ch.r1 = __shfl_sync(0xffffffffu, d.r1, t);
                             ch.e0 = __shfl_sync(0xffffffffu, d.e0, t);
                             ch.e1 = __shfl_sync(0xffffffffu, d.e1, t);
-                            ch.cls = __shfl_sync(0xffffffffu, d.cls, t);
                             ch.panel = __shfl_sync(0xffffffffu, d.panel, t);
                             ch.ebase = __shfl_sync(0xffffffffu, d.ebase, t);
                             ch.rpbase = __shfl_sync(0xffffffffu, d.rpbase, t);
-                            ch.rowbase = __shfl_sync(0xffffffffu, d.rowbase, t);
-                            const int j = jb + t, k = j % NS;
+                            const int k = (jb + t) % NS;
                             int ok = 1;
                             if (wl == 0) {
-                                if (MIX && j % nchl == 0) {
-                                    if (wstarted)
-                                        ok = mbar_wait_sleep_bounded(&S.wempty, wpar ^ 1u, a.queue + 1, a.budget_ns,
-                                                                     a.backoff_ns);
-                                    if (ok) {
-                                        issue_pwin(&S.pbar, s_win, (const float *)pnew, V.n, j / nchl, s_pshift);
-                                        wpar ^= 1u;
-                                        wstarted = 1;
-                                    }
-                                }
-                                if (ok && ((pstarted >> k) & 1u))
+                                if ((pstarted >> k) & 1u)
                                     ok = mbar_wait_sleep_bounded(&S.empty[k], ((pfill >> k) & 1u) ^ 1u, a.queue + 1,
-                                                           a.budget_ns, a.backoff_ns);
+                                                                 a.budget_ns, a.backoff_ns);
                                 if (ok) {
-                                    b_issue<MIX>(a, S, ch, k);
+                                    b_issue(a, S, ch, k);
                                     pfill ^= 1u << k;
                                     pstarted |= 1u << k;
-                                    st_bytes += chunk_bytes<MIX>(ch);
-                                    st_lowp += ch.cls;
+                                    st_bytes += pass_bytes(ch.e1 - ch.e0, ch.r1 - ch.r0, 1, 8);
                                     st_pass++;
                                 }
                             }
@@ -909,158 +757,58 @@ __global__ void __launch_bounds__(BNT, MF_BATCH_MINB) k_batched_cg(BatchArgs a)
                         }
                     }
                 } else {
-                    // consumer warps in NGRP groups: group g consumes the
-                    // passes j with j % NGRP == g (stages j % NS, two per
-                    // group), its CWS warps splitting each pass's rows;
-                    // every consumer warp waits for each panel's window and
-                    // releases it after its own passes of that panel
-                    // (mixed kernel; the FP64 kernel's consumer warps all
-                    // take every pass, so that a row's panels are added in
-                    // panel order without a window to order them)
+                    // consumer warps: all of them take every pass, so that a
+                    // row's panels are added in panel order
                     constexpr int NCW = BNW - 1;
-                    constexpr int NGRP = MIX ? MF_BATCH_GROUPS : 1;
-                    constexpr int CWS = NCW / NGRP;             // consumer warps per group
-                    static_assert(NCW % NGRP == 0 && NS % NGRP == 0, "groups split the warps and stages evenly");
-                    const int cw = wid - 1;
-                    const int kg = cw / CWS;                    // this warp's group
-                    const int gr = cw % CWS;                    // warp within the stage's group
-                    const int ct = gr * 32 + wl;                // thread within the stage's group
+                    const int ct = (wid - 1) * 32 + wl;         // consumer thread
                     const int clane = ct % L, cgrp = ct / L;
-                    constexpr int GPC = CWS * 32 / L;           // row groups per stage
-                    const int nwin = MIX ? npan : 1;
-                    for (int pw = 0; pw < nwin && !fail; pw++) {
-                        const int j0 = MIX ? pw * nchl : 0, j1 = MIX ? j0 + nchl : J;
-                        if (MIX) {
-                            const bool ww =
-                                mbar_wait_sleep_bounded(&S.pbar, cwpar, a.queue + 1, a.budget_ns, a.backoff_ns);
-                            cwpar ^= 1u;
-                            if (!__all_sync(0xffffffffu, ww)) {
-                                fail = true;
-                                break;
+                    constexpr int GPC = NCW * 32 / L;           // row groups
+                    for (int j = 0; j < J; j++) {
+                        const int k = j % NS;
+                        bool w = mbar_wait_sleep_bounded(&S.bar[k], (cfull >> k) & 1u, a.queue + 1, a.budget_ns,
+                                                         a.backoff_ns);
+                        cfull ^= 1u << k;
+                        if (!__all_sync(0xffffffffu, w)) {
+                            fail = true;
+                            break;
+                        }
+                        const BHdr &h = S.hdr[k];
+                        const unsigned char *st = S.stage[k];
+                        const int *rps = (const int *)(st + Stage::OFF_RP + h.sh_rp);  // panel row pointers of h.r0 ..
+                        const int nr = h.r1 - h.r0;
+                        const bool firstp = h.panel == 0;
+                        const double *pk = pnew + (long long)h.panel * PW;
+                        auto psrc = [=](int c) -> double { return pk[c]; };
+                        const uint16_t *scol = (const uint16_t *)(st + Stage::OFF_COL + h.sh_col);
+                        const double *sval = (const double *)(st + Stage::OFF_VAL + h.sh_val);
+                        // one row per lane group; the trip count is the same
+                        // for every lane of a warp (shuffles inside)
+                        for (int qb = 0; qb < nr; qb += GPC) {
+                            const int q0 = qb + cgrp;
+                            const bool in = q0 < nr;
+                            const int ra0 = in ? rps[q0] : 0, re0 = in ? rps[q0 + 1] : 0;
+                            double y0;
+                            if (h.direct) {
+                                RowPair rr{ra0, re0, 0, 0};
+                                double y1;
+                                row_dot2<L>(rr, a.col + h.ebase, a.val + h.ebase, clane, psrc, y0, y1);
+                            } else {
+                                y0 = row_dot1_smem<L>(ra0 - h.e0, re0 - h.e0, scol, sval, clane, psrc);
+                            }
+                            if (clane == 0 && in) {
+                                // One panel: the row sum is q; two panels: both
+                                // partial sums are added to q (zeroed by the p
+                                // update; two additions onto zero give the same
+                                // bits in either order); more panels: added in
+                                // panel order.
+                                double *qi = q + h.r0 + q0;
+                                if (npan == 1) *qi = y0;
+                                else if (npan == 2) atomicAdd(qi, y0);
+                                else *qi = firstp ? y0 : *qi + y0;
                             }
                         }
-                        const int jfirst = j0 + (kg - j0 % NGRP + NGRP) % NGRP;
-                        for (int j = jfirst; j < j1; j += NGRP) {
-                            const int k = j % NS;
-                            bool w = mbar_wait_sleep_bounded(&S.bar[k], (cfull >> k) & 1u, a.queue + 1, a.budget_ns,
-                                                             a.backoff_ns);
-                            cfull ^= 1u << k;
-                            if (!__all_sync(0xffffffffu, w)) {
-                                fail = true;
-                                break;
-                            }
-                            const BHdr &h = S.hdr[k];
-                            const unsigned char *st = S.stage[k];
-                            const int *rps = (const int *)(st + SG::OFF_RP + h.sh_rp);  // panel row pointers of h.r0 ..
-                            const int nr = h.r1 - h.r0;
-                            const bool h16 = MIX && h.cls == 1;
-                            const bool firstp = h.panel == 0;
-                            const VT *pwin = MIX ? (const VT *)s_win + s_pshift : (const VT *)pnew + (long long)h.panel * PW;
-                            auto psrc = [=](int c) -> VT { return pwin[c]; };
-                            const uint16_t *scol = (const uint16_t *)(st + SG::OFF_COL + h.sh_col);
-                            const unsigned char *sval = st + SG::OFF_VAL + h.sh_val;
-                            // the row sum of row q0 of this pass goes to q (FP16
-                            // rows: scaled, plus the FP32 diagonal times the
-                            // diagonal's p from the window of the panel that
-                            // holds the diagonal column).  One panel: the row
-                            // sum is q; two panels: both partial sums are added
-                            // to q (zeroed by the p update; two additions onto
-                            // zero give the same bits in either order); more
-                            // panels: added in panel order (the mixed kernel's
-                            // window barrier orders the panels; the FP64
-                            // kernel's warps take every pass in order).
-                            auto row_out = [&](int q0, double y0) {
-                                const int i0 = h.r0 + q0;
-                                if (h16) {
-                                    const float *srs = (const float *)(st + SG::OFF_RS + h.sh_rs);
-                                    const float *sdg = (const float *)(st + SG::OFF_DG + h.sh_dg);
-                                    const float dt =
-                                        (i0 / PW == h.panel) ? sdg[q0] * (float)pwin[i0 - h.panel * PW] : 0.f;
-                                    y0 = (double)fmaf(srs[q0], (float)y0, dt);
-                                }
-                                VT *qi = q + i0;
-                                if (npan == 1) *qi = (VT)y0;
-                                else if (npan == 2) atomicAdd(qi, (VT)y0);
-                                else *qi = firstp ? (VT)y0 : (VT)((double)*qi + y0);
-                            };
-                            if (MIX && !h.direct && a.rowsum == 0) {
-                                // two phases over this warp's share of the
-                                // pass's rows: (1) the products of its entries,
-                                // consecutive entries to consecutive lanes,
-                                // written over the staged values in place;
-                                // (2) one lane per row adds its products in
-                                // entry order
-                                const int qa = (int)((long long)nr * gr / CWS);
-                                const int qe = (int)((long long)nr * (gr + 1) / CWS);
-                                uint32_t *pv = (uint32_t *)(st + SG::OFF_VAL + h.sh_val);
-                                if (qa < qe) {
-                                    const int ea = rps[qa] - h.e0, eb = rps[qe] - h.e0;
-                                    if (h16) {
-                                        MF_UNROLL(MF_BATCH_P1U)
-                                        for (int e = ea + wl; e < eb; e += 32) {
-                                            const uint32_t wv = pv[e];
-                                            const float v = __half2float(__ushort_as_half((unsigned short)(wv >> 16)));
-                                            pv[e] = __float_as_uint(v * (float)pwin[wv & (uint32_t)(PW - 1)]);
-                                        }
-                                    } else {
-                                        MF_UNROLL(MF_BATCH_P1U)
-                                        for (int e = ea + wl; e < eb; e += 32)
-                                            pv[e] = __float_as_uint(__uint_as_float(pv[e]) * (float)pwin[scol[e]]);
-                                    }
-                                    __syncwarp();
-                                    for (int q0 = qa + wl; q0 < qe; q0 += 32) {
-                                        const int s0 = rps[q0] - h.e0, s1 = rps[q0 + 1] - h.e0;
-                                        float acc = 0.f;
-                                        for (int e = s0; e < s1; e++) acc += __uint_as_float(pv[e]);
-                                        row_out(q0, (double)acc);
-                                    }
-                                }
-                                // the products written here precede the next
-                                // bulk copy into this stage
-                                fence_proxy_async_smem();
-                            } else
-                            // one row per lane group; the trip count is the same
-                            // for every lane of a warp (shuffles inside)
-                            for (int qb = 0; qb < nr; qb += GPC) {
-                                const int q0 = qb + cgrp;
-                                const bool in = q0 < nr;
-                                const int ra0 = in ? rps[q0] : 0, re0 = in ? rps[q0 + 1] : 0;
-                                double y0;
-                                if (h.direct) {
-                                    RowPair rr{ra0, re0, 0, 0};
-                                    const uint16_t *gcol = a.col + h.ebase;
-                                    double y1;
-                                    if constexpr (MIX) {
-                                        if (h16)
-                                            row_dot2<L, __half, decltype(psrc), true>(rr, gcol, a.val16 + h.ebase, clane,
-                                                                                       psrc, y0, y1);
-                                        else
-                                            row_dot2<L, float, decltype(psrc), true>(rr, gcol, a.val32 + h.ebase, clane,
-                                                                                      psrc, y0, y1);
-                                    } else {
-                                        row_dot2<L, double, decltype(psrc), true>(rr, gcol, a.val + h.ebase, clane, psrc,
-                                                                                   y0, y1);
-                                    }
-                                } else if constexpr (MIX) {
-                                    if (h16)
-                                        y0 = row_dot1_cv16<L>(ra0 - h.e0, re0 - h.e0, (const uint32_t *)sval, clane, psrc);
-                                    else
-                                        y0 = row_dot1_smem<L, float>(ra0 - h.e0, re0 - h.e0, scol, (const float *)sval,
-                                                                     clane, psrc);
-                                } else {
-                                    y0 = row_dot1_smem<L, double>(ra0 - h.e0, re0 - h.e0, scol, (const double *)sval,
-                                                                  clane, psrc);
-                                }
-                                if (clane == 0 && in) row_out(q0, y0);
-                            }
-                            __syncwarp();
-                            if (wl == 0) mbar_arrive(&S.empty[k]);
-                        }
-                        if (fail) break;
-                        if (MIX) {
-                            __syncwarp();
-                            if (wl == 0) mbar_arrive(&S.wempty);
-                        }
+                        __syncwarp();
+                        if (wl == 0) mbar_arrive(&S.empty[k]);
                     }
                 }
             }
@@ -1070,7 +818,6 @@ __global__ void __launch_bounds__(BNT, MF_BATCH_MINB) k_batched_cg(BatchArgs a)
             if (fail && tid == 0) {
                 for (int k = 0; k < NS; k++)
                     if ((pstarted >> k) & 1u) mbar_drain(&S.bar[k], ((pfill >> k) & 1u) ^ 1u, a.queue + 1, a.budget_ns);
-                if (MIX && wstarted) mbar_drain(&S.pbar, wpar ^ 1u, a.queue + 1, a.budget_ns);
             }
             if (tid == 0) s_fail = fail ? 1 : 0;
             // p.q over this CTA's rows (q read past L1: partial sums arrive by
@@ -1078,18 +825,18 @@ __global__ void __launch_bounds__(BNT, MF_BATCH_MINB) k_batched_cg(BatchArgs a)
             if (!fail) {
                 int i = ra + tid;
                 for (; i + 3 * BNT < rb; i += 4 * BNT) {
-                    VT p4[4], q4[4];
+                    double p4[4], q4[4];
 #pragma unroll
                     for (int u = 0; u < 4; u++) {
                         p4[u] = pnew[i + u * BNT];
                         q4[u] = __ldcg(q + i + u * BNT);
                     }
 #pragma unroll
-                    for (int u = 0; u < 4; u++) loc += (double)p4[u] * (double)q4[u];
+                    for (int u = 0; u < 4; u++) loc += p4[u] * q4[u];
                 }
-                for (; i < rb; i += BNT) loc += (double)pnew[i] * (double)__ldcg(q + i);
+                for (; i < rb; i += BNT) loc += pnew[i] * __ldcg(q + i);
             }
-            const double pq = cluster_sum(cl, loc, &s_slot[2], s_warp);
+            const double pq = cluster_sum<BNT>(cl, loc, &s_slot[2], s_warp);
             int any_fail = 0;
             for (unsigned kk = 0; kk < ncta; kk++) any_fail |= *cl.map_shared_rank(&s_fail, kk);
             if (any_fail) {
@@ -1106,104 +853,45 @@ __global__ void __launch_bounds__(BNT, MF_BATCH_MINB) k_batched_cg(BatchArgs a)
                 // four rows per thread in flight (loads first)
                 int i = ra + tid;
                 for (; i + 3 * BNT < rb; i += 4 * BNT) {
-                    VT p4[4], q4[4], r4[4];
-                    double x4[4];
+                    double p4[4], q4[4], r4[4], x4[4];
 #pragma unroll
                     for (int u = 0; u < 4; u++) {
                         p4[u] = pnew[i + u * BNT];
                         q4[u] = __ldcg(q + i + u * BNT);
                         r4[u] = r[i + u * BNT];
-                        x4[u] = MIX ? (double)xlo[i + u * BNT] : x[i + u * BNT];
+                        x4[u] = x[i + u * BNT];
                     }
 #pragma unroll
                     for (int u = 0; u < 4; u++) {
-                        if (MIX) {
-                            xlo[i + u * BNT] = fmaf((float)alpha, (float)p4[u], (float)x4[u]);
-                            const float ri = fmaf(-(float)alpha, (float)q4[u], (float)r4[u]);
-                            r[i + u * BNT] = ri;
-                            loc += (double)ri * (double)ri;
-                        } else {
-                            x[i + u * BNT] = fma(alpha, (double)p4[u], x4[u]);
-                            const double ri = fma(-alpha, (double)q4[u], (double)r4[u]);
-                            r[i + u * BNT] = ri;
-                            loc += ri * ri;
-                        }
-                    }
-                }
-                for (; i < rb; i += BNT) {
-                    if (MIX) {
-                        xlo[i] = fmaf((float)alpha, (float)pnew[i], (float)xlo[i]);
-                        const float ri = fmaf(-(float)alpha, (float)__ldcg(q + i), (float)r[i]);
-                        r[i] = ri;
-                        loc += (double)ri * (double)ri;
-                    } else {
-                        x[i] = fma(alpha, (double)pnew[i], x[i]);
-                        const double ri = fma(-alpha, (double)__ldcg(q + i), (double)r[i]);
-                        r[i] = ri;
+                        x[i + u * BNT] = fma(alpha, p4[u], x4[u]);
+                        const double ri = fma(-alpha, q4[u], r4[u]);
+                        r[i + u * BNT] = ri;
                         loc += ri * ri;
                     }
                 }
+                for (; i < rb; i += BNT) {
+                    x[i] = fma(alpha, pnew[i], x[i]);
+                    const double ri = fma(-alpha, __ldcg(q + i), r[i]);
+                    r[i] = ri;
+                    loc += ri * ri;
+                }
             }
-            double rho_new = cluster_sum(cl, loc, &s_slot[3], s_warp);
+            const double rho_new = cluster_sum<BNT>(cl, loc, &s_slot[3], s_warp);
             it++;
-            bool checkpoint = learned && !lowp_off && it == 1;
-            if (MIX && (sqrt(rho_new) <= a.delta * rmax || sqrt(rho_new) <= a.tol * nb)) {
-                for (int i = ra + tid; i < rb; i += BNT) {
-                    x[i] += (double)xlo[i];
-                    xlo[i] = (VT)0;
-                }
-                cl.sync();
-                loc = 0.0;
-                for (int base = ra; base < rb; base += 2 * GPB) {
-                    const int i0 = base + grp < rb ? base + grp : -1;
-                    const int i1 = base + GPB + grp < rb ? base + GPB + grp : -1;
-                    double y0, y1;
-                    row_dot2_fp64_all<L>(a, V, x, i0, i1, lane, y0, y1);
-                    if (lane == 0) {
-                        if (i0 >= 0) {
-                            const VT rv = (VT)(b[i0] - y0);
-                            r[i0] = rv;
-                            loc += (double)rv * (double)rv;
-                        }
-                        if (i1 >= 0) {
-                            const VT rv = (VT)(b[i1] - y1);
-                            r[i1] = rv;
-                            loc += (double)rv * (double)rv;
-                        }
-                    }
-                }
-                rho_new = cluster_sum(cl, loc, &s_slot[1], s_warp);
-                const double rt = sqrt(rho_new);
-                // the low-precision classes stop where the FP64 residual did
-                // not follow the recurrence (uniform: every CTA holds the same
-                // cluster sums)
-                if ((rule || learned) && !lowp_off && rt > 0.5 * rmax) {
-                    lowp_off = true;
-                    for (int c = cl0 + tid; c < cl1; c += BNT) a.ccls[c] = (a.ccls_static[c] & 1) ? 1 : 0;
-                }
-                rmax = rt;
-                refs++;
-                checkpoint = learned && !lowp_off;
-            }
-            const bool sample = collect && (it % a.collect_every == 1 || a.collect_every == 1);
-            if (checkpoint || sample) {
+            if (collect && (it % a.collect_every == 1 || a.collect_every == 1)) {
                 // checkpoint statistics: one warp per chunk of this CTA, then
                 // the system's maxima of |r| and |p| over the cluster
                 float gr = 0.f, gp = 0.f;
                 for (int c = cl0 + wid; c < cl1; c += BNW)
-                    chunk_stats_warp<VT>(a, V, c, a.crow[c + sys], a.crow[c + 1 + sys], r, pnew, pold, q, rscale,
-                                         sample, gr, gp);
-                cluster_max2(cl, gr, gp, s_fslot, s_fwarp);
+                    chunk_stats_warp<double>(a, V, c, a.crow[c + sys], a.crow[c + 1 + sys], r, pnew, pold, q, rscale,
+                                             true, gr, gp);
+                cluster_max2<BNT>(cl, gr, gp, s_fslot, s_fwarp);
                 const float rel = (float)(sqrt(rho_new) / nb);
                 float *xf = s_feat + wid * PN_NF;
                 for (int c = cl0 + wid; c < cl1; c += BNW) {
-                    if (wl == 0) chunk_features(a, c, rel, gr, gp, refs, have_prev, xf);
-                    __syncwarp();
-                    float *d = a.cdyn + (size_t)c * NCDYN;
-                    if (checkpoint) {
-                        const int cls = learned_chunk_class(s_w, xf, a.ccls_static[c]);
-                        if (wl == 0) a.ccls[c] = (unsigned char)cls;
-                    } else if (wl == 0) {
+                    if (wl == 0) {
+                        chunk_features(a, c, rel, gr, gp, 0, have_prev, xf);
+                        float *d = a.cdyn + (size_t)c * NCDYN;
                         const unsigned h = ((unsigned)c * 2654435761u) ^ (a.collect_salt + (unsigned)it * 0x9E3779B9u);
                         if ((h >> 8) % (unsigned)a.collect_stride == 0u) {
                             const unsigned long long slot = atomicAdd(a.ccount, 1ull);
@@ -1212,22 +900,513 @@ __global__ void __launch_bounds__(BNT, MF_BATCH_MINB) k_batched_cg(BatchArgs a)
                                 a.cy[slot] = (unsigned char)((double)d[8] <= LABEL_TAU ? 1 : 2);
                             }
                         }
-                    }
-                    if (wl == 0)
                         for (int k = 0; k < 4; k++) d[4 + k] = xf[6 + k];
+                    }
                     __syncwarp();
                 }
                 have_prev = true;
-                __syncthreads();  // classes written before thread 0 issues the next passes
             }
             beta = rho_new / rho;
             rho = rho_new;
             relres = sqrt(rho) / nb;
         }
-        if (MIX && status != MF_OK) {
-            for (int i = ra + tid; i < rb; i += BNT) x[i] += (double)xlo[i];
-        }
         if (tid == 0) {
+            atomicAdd(&a.sysstat[3 * sys], st_bytes);
+            atomicAdd(&a.sysstat[3 * sys + 2], st_pass);
+        }
+        if (rank == 0 && tid == 0) {
+            a.iters[sys] = it;
+            a.refs[sys] = 0;
+            a.status[sys] = status;
+            a.relres[sys] = relres;
+        }
+        cl.sync();  // the cluster's last writes land before the next system
+    }
+}
+
+// The mixed kernel's view of the system its cluster is solving.  The CTA's
+// own rows are [ra, rb); r, xlo and q are indexed from ra.  On chip (small
+// systems): the window of p and the three vectors live in shared memory, p
+// and q reach the other CTAs by distributed shared memory; otherwise they
+// are in global memory.
+struct MixSys {
+    int sys, n, ra, rb, npan;
+    bool chip;
+    float *win;             // the window of p (shared memory)
+    float *r, *xlo, *q;     // this CTA's rows (on chip: shared memory)
+    float *pnew, *pold;     // global p buffers, indexed by row (on chip: written for LEARNED only)
+    const int *rab;         // on chip: first row of every CTA (shared memory)
+};
+
+// Sum over the cluster: warp tree, then warp 0 adds the warps' sums in a
+// fixed tree and writes the CTA's value to every CTA's slots (remote
+// stores), then after the cluster barrier all add the slots in rank order.
+// Two barriers; `slots` is reused only after another cluster barrier.
+__device__ __forceinline__ double mix_sum(cg::cluster_group &cl, double v, double *slots, double *s_warp)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    const int wid = threadIdx.x >> 5, wl = threadIdx.x & 31;
+    const int rank = (int)cl.block_rank(), ncta = (int)cl.num_blocks();
+    if (wl == 0) s_warp[wid] = v;
+    __syncthreads();
+    if (wid == 0) {
+        double c = wl < MNW ? s_warp[wl] : 0.0;
+#pragma unroll
+        for (int o = MNW / 2; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+        if (wl < ncta) *cl.map_shared_rank(slots + rank, wl) = c;  // lanes below MNW hold the sum
+    }
+    cl.sync();
+    double s = 0.0;
+    for (int k = 0; k < ncta; k++) s += slots[k];
+    return s;
+}
+static_assert(MNW <= 32 && MNW >= 16, "a lane per warp in the second step, a lane with the sum per CTA of a cluster");
+
+// The CTA that owns row i.
+__device__ __forceinline__ int mix_owner(const int *rab, int ncta, int i)
+{
+    int o = 0;
+    for (int k = 1; k < ncta; k++) o += i >= rab[k];
+    return o;
+}
+
+// q = A p over the sorted slices; returns this thread's part of p.q (one
+// window; 0 for several).  mode: 0 every chunk FP32, 1 every chunk FP16, 2
+// both kinds.
+__device__ __noinline__ double mix_spmv(const BatchArgs &a, MixSys M, int mode)
+{
+    cg::cluster_group cl = cg::this_cluster();
+    const SellView &E = a.sell;
+    const int tid = threadIdx.x, wid = tid >> 5, wl = tid & 31;
+    const int rank = (int)cl.block_rank(), ncta = (int)cl.num_blocks();
+    const int wf = E.win0[M.sys], nwin = sell_windows(M.n), W = sell_width(M.n);
+    double loc = 0.0;
+    for (int k = 0; k < nwin; k++) {
+        const int c0 = k * W, c1 = min(M.n, c0 + W);
+        if (!M.chip) {
+            // window: whole 16-byte words (up to three elements past the
+            // window's end come from the vector's slack)
+            const float4 *src = reinterpret_cast<const float4 *>(M.pnew + c0);
+            float4 *dst = reinterpret_cast<float4 *>(M.win);
+            const int nq4 = (c1 - c0 + 3) >> 2;
+            int i = tid;
+            for (; i + 7 * MNT < nq4; i += 8 * MNT) {
+                float4 v[8];
+#pragma unroll
+                for (int u = 0; u < 8; u++) v[u] = __ldcg(src + i + u * MNT);
+#pragma unroll
+                for (int u = 0; u < 8; u++) dst[i + u * MNT] = v[u];
+            }
+            for (; i < nq4; i += MNT) dst[i] = __ldcg(src + i);
+            __syncthreads();
+        }
+        // slices, longest first, dealt to the cluster's warps in turn
+        const int s1 = E.first[wf + k + 1], step = MNW * ncta;
+        int s = E.first[wf + k] + wid * ncta + rank;
+        int2 sd = make_int2(0, 0);
+        int4 rec = make_int4(-1, 0, 0, 0);
+        if (s < s1) {
+            sd = __ldg(E.desc + s);
+            rec = __ldg(E.rec + (size_t)s * 32 + wl);
+        }
+        while (s < s1) {
+            const int sn = s + step;
+            int2 sdn = sd;
+            int4 recn = rec;
+            if (sn < s1) {  // the next slice's record loads under this one's sums
+                sdn = __ldg(E.desc + sn);
+                recn = __ldg(E.rec + (size_t)sn * 32 + wl);
+            }
+            const size_t at = (size_t)sd.x * 32 + wl;
+            const int nq = sd.y & 0x7fffffff;
+            float acc = 0.f, scale = __int_as_float(rec.z);
+            if (mode == 1) {
+                acc = sell_dot<Quad16, float>(Quad16{E.cv + at}, nq, M.win);
+            } else {
+                const bool h = mode == 2 && rec.x >= 0 && __ldcg(a.ccls + rec.y) != 0;
+                const unsigned m16 = __ballot_sync(0xffffffffu, h);
+                const unsigned m32 = __ballot_sync(0xffffffffu, !h && rec.x >= 0);
+                float a16 = 0.f;
+                if (m16) a16 = sell_dot<Quad16, float>(Quad16{E.cv + at}, nq, M.win);
+                if (m32) acc = sell_dot<Quad32, float>(Quad32{E.v32 + at, E.c16 + at}, nq, M.win);
+                if (h) acc = a16;
+                else scale = 1.f;
+            }
+            if (sd.y < 0) {  // a long row: its lanes' sums in a fixed tree
+                double d = (double)acc;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+                acc = (float)d;
+            }
+            if (rec.x >= 0 && (sd.y >= 0 || wl == 0)) {
+                const int i = rec.x;
+                const bool own = i >= c0 && i < c1;  // the diagonal's window
+                const float pi = own ? M.win[i - c0] : 0.f;
+                const float y = fmaf(scale, acc, own ? __int_as_float(rec.w) * pi : 0.f);
+                if (M.chip) {
+                    const int o = mix_owner(M.rab, ncta, i);
+                    cl.map_shared_rank(M.q, o)[i - M.rab[o]] = y;
+                } else {
+                    float *qi = M.q + (i - M.ra);
+                    *qi = k == 0 ? y : __ldcg(qi) + y;
+                }
+                if (nwin == 1) loc += (double)pi * (double)y;
+            }
+            s = sn;
+            sd = sdn;
+            rec = recn;
+        }
+        // several windows: the next one's sums continue from every warp's
+        // q, and the window is overwritten
+        if (k + 1 < nwin) cl.sync();
+    }
+    return loc;
+}
+
+// The rare steps, out of line so that the iteration keeps its registers.
+// Reliable update: x += xlo, xlo = 0, then (cluster barrier) r = b - A x from
+// the FP64 values; returns this thread's part of ||r||^2.  One window: over
+// the slices (16-byte streams as in the product, x gathered from L2); several
+// windows: lane groups over the rows of the panel storage.
+template <int L>
+__device__ __noinline__ double mix_refine(const BatchArgs &a, SysView V, MixSys M)
+{
+    cg::cluster_group cl = cg::this_cluster();
+    const int tid = threadIdx.x, wid = tid >> 5, wl = tid & 31;
+    const int rank = (int)cl.block_rank(), ncta = (int)cl.num_blocks();
+    const double *b = a.b + V.r0;
+    double *x = a.x + V.r0;
+    for (int i = tid; i < M.rb - M.ra; i += MNT) {
+        x[M.ra + i] += (double)M.xlo[i];
+        M.xlo[i] = 0.f;
+    }
+    cl.sync();
+    double loc = 0.0;
+    if (sell_windows(M.n) == 1) {
+        const SellView &E = a.sell;
+        const int wf = E.win0[M.sys], s1 = E.first[wf + 1];
+        const double *diag = E.diag64 + V.r0;
+        for (int s = E.first[wf] + wid * ncta + rank; s < s1; s += MNW * ncta) {
+            const int2 sd = __ldg(E.desc + s);
+            const int i = __ldg(&E.rec[(size_t)s * 32 + wl].x);
+            const size_t at = (size_t)sd.x * 32 + wl;
+            double y = sell_dot<Quad64, double>(Quad64{E.v64 + 2 * at, E.c16 + at}, sd.y & 0x7fffffff, x);
+            if (sd.y < 0)
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+            if (i >= 0 && (sd.y >= 0 || wl == 0)) {
+                const float rv = (float)(b[i] - fma(diag[i], x[i], y));
+                if (M.chip) {
+                    const int o = mix_owner(M.rab, ncta, i);
+                    cl.map_shared_rank(M.r, o)[i - M.rab[o]] = rv;
+                } else {
+                    M.r[i - M.ra] = rv;
+                }
+                loc += (double)rv * (double)rv;
+            }
+        }
+    } else {
+        const int lane = tid % L, grp = tid / L;
+        constexpr int GPB = MNT / L;  // row groups per CTA
+        for (int base = M.ra; base < M.rb; base += 2 * GPB) {
+            const int i0 = base + grp < M.rb ? base + grp : -1;
+            const int i1 = base + GPB + grp < M.rb ? base + GPB + grp : -1;
+            double y0, y1;
+            row_dot2_fp64_all<L>(a, V, x, i0, i1, lane, y0, y1);
+            if (lane == 0) {
+                if (i0 >= 0) {
+                    const float rv = (float)(b[i0] - y0);
+                    M.r[i0 - M.ra] = rv;
+                    loc += (double)rv * (double)rv;
+                }
+                if (i1 >= 0) {
+                    const float rv = (float)(b[i1] - y1);
+                    M.r[i1 - M.ra] = rv;
+                    loc += (double)rv * (double)rv;
+                }
+            }
+        }
+    }
+    return loc;
+}
+
+// LEARNED checkpoint: one warp per chunk of this CTA gathers its statistics,
+// then, with the system's maxima of |r| and |p| over the cluster, its class.
+__device__ __noinline__ void mix_checkpoint(const BatchArgs &a, SysView V, MixSys M, int cl0, int cl1,
+                                            float relres, int refs, bool have_prev, const float *s_w, float *s_feat,
+                                            float *s_fslot, float *s_fwarp)
+{
+    cg::cluster_group cl = cg::this_cluster();
+    const int wid = threadIdx.x >> 5, wl = threadIdx.x & 31;
+    float gr = 0.f, gp = 0.f;
+    for (int c = cl0 + wid; c < cl1; c += MNW) {
+        // chunk_stats_warp indexes all vectors alike: from the chunk's first row
+        const int r0 = a.crow[c + M.sys], r1 = a.crow[c + 1 + M.sys], at = r0 - M.ra;
+        chunk_stats_warp<float>(a, V, c, 0, r1 - r0, M.r + at, M.pnew + r0, M.pold + r0, M.q + at, nullptr, false, gr, gp);
+    }
+    cluster_max2<MNT>(cl, gr, gp, s_fslot, s_fwarp);
+    float *xf = s_feat + wid * PN_NF;
+    for (int c = cl0 + wid; c < cl1; c += MNW) {
+        if (wl == 0) chunk_features(a, c, relres, gr, gp, refs, have_prev, xf);
+        __syncwarp();
+        const int cls = learned_chunk_class(s_w, xf, a.ccls_static[c]);
+        if (wl == 0) {
+            a.ccls[c] = (unsigned char)cls;
+            float *d = a.cdyn + (size_t)c * NCDYN;
+            for (int k = 0; k < 4; k++) d[4 + k] = xf[6 + k];
+        }
+        __syncwarp();
+    }
+}
+
+// The mixed kernel (STATIC, RULE, LEARNED): one cluster per system, FP32
+// vectors.  The product q = A p runs over the sorted slices: every CTA holds
+// the window of p in shared memory, the slices are dealt to the cluster's
+// warps longest first (so all warps get nearly equal work whatever the row
+// order), a lane sums one row from 16-byte words that stream from L2/HBM
+// straight into registers, the gathers hit shared memory.  A system whose
+// window and vectors fit keeps them on the chip for the whole solve.
+template <int L>
+__global__ void __launch_bounds__(MNT, 1) k_batched_cg(const __grid_constant__ BatchArgs a)
+{
+    cg::cluster_group cl = cg::this_cluster();
+    __shared__ double s_warp[MNW];
+    __shared__ double s_slot[4][16];
+    __shared__ float s_fslot[2];
+    __shared__ float s_fwarp[2 * MNW];
+    __shared__ int s_sys;
+    __shared__ int s_rab[17];
+    extern __shared__ __align__(16) unsigned char b_smem_raw[];
+    float *s_win = reinterpret_cast<float *>(b_smem_raw);
+    float *s_w = reinterpret_cast<float *>(b_smem_raw + MixSmem::W);
+    float *s_feat = reinterpret_cast<float *>(b_smem_raw + MixSmem::FEAT);
+    const bool learned = a.policy == MF_POLICY_LEARNED && a.mlp_w;
+    const bool rule = a.policy == MF_POLICY_RULE;
+    if (learned)
+        for (int k = threadIdx.x; k < PN_NPARAM; k += MNT) s_w[k] = __bfloat162float(a.mlp_w[k]);
+    __syncthreads();
+    const int rank = (int)cl.block_rank(), ncta = (int)cl.num_blocks();
+    const int tid = threadIdx.x;
+    const int wid = tid >> 5, wl = tid & 31;
+    for (;;) {
+        if (rank == 0 && tid == 0) s_sys = atomicAdd(a.queue, 1);
+        cl.sync();
+        const int qi = *cl.map_shared_rank(&s_sys, 0);
+        cl.sync();  // every CTA has read the index before rank 0 writes the next
+        if (qi >= a.count) break;
+        const int sys = a.order[qi];
+        const SysView V = sys_view(a, sys);
+        const double *b = a.b + V.r0;
+        double *x = a.x + V.r0;
+        // this CTA's chunks and rows
+        const int sc0 = a.sc[sys], nch = a.sc[sys + 1] - sc0;
+        const int cl0 = sc0 + (int)((long long)nch * rank / ncta), cl1 = sc0 + (int)((long long)nch * (rank + 1) / ncta);
+        if (tid <= ncta) s_rab[tid] = a.crow[sc0 + (int)((long long)nch * tid / ncta) + sys];
+        __syncthreads();
+        int most = 0;  // rows of the CTA with most
+        for (int k = 0; k < ncta; k++) most = max(most, s_rab[k + 1] - s_rab[k]);
+        most = (most + 3) & ~3;
+        const int nwin = sell_windows(V.n), n4 = (V.n + 3) & ~3;
+        MixSys M;
+        M.sys = sys;
+        M.n = V.n;
+        M.ra = s_rab[rank];
+        M.rb = s_rab[rank + 1];
+        M.npan = V.npan;
+        M.chip = n4 + 3 * most <= SELL_WIN;
+        M.win = s_win;
+        M.rab = s_rab;
+        // global vectors: every system starts on a 16-byte boundary
+        const long long w0 = ((V.r0 + 4ll * sys) >> 2) << 2;
+        M.pnew = (float *)a.p0 + w0;
+        M.pold = (float *)a.p1 + w0;
+        if (M.chip) {
+            M.r = s_win + n4;
+            M.xlo = M.r + most;
+            M.q = M.xlo + most;
+        } else {
+            M.r = (float *)a.r + w0 + M.ra;
+            M.xlo = (float *)a.xlo + w0 + M.ra;
+            M.q = (float *)a.q + w0 + M.ra;
+        }
+        const int rows = M.rb - M.ra;
+        unsigned long long st_bytes = 0, st_lowp = 0, st_pass = 0;  // this thread's chunks
+        unsigned long long it_bytes = 0;                            // the same per iteration, by the current classes
+        unsigned it_lowp = 0, it_pass = 0;
+        double lb = 0.0, lr = 0.0;
+        for (int i = tid; i < rows; i += MNT) {
+            const double bv = b[M.ra + i];
+            const float rv = (float)bv;
+            x[M.ra + i] = 0.0;
+            M.r[i] = rv;
+            M.xlo[i] = 0.f;
+            M.pnew[M.ra + i] = 0.f;  // p before the first iteration
+            if (M.chip) s_win[M.ra + i] = 0.f;
+            lb += bv * bv;
+            lr += (double)rv * (double)rv;
+        }
+        for (int c = cl0 + tid; c < cl1; c += MNT) a.ccls[c] = (a.ccls_static[c] & 1) ? 1 : 0;
+        const double bb = mix_sum(cl, lb, s_slot[0], s_warp);
+        double rho = mix_sum(cl, lr, s_slot[1], s_warp);
+        const double nb = sqrt(bb) > 0.0 ? sqrt(bb) : 1.0;
+        double beta = 0.0, rmax = sqrt(rho), relres = sqrt(rho) / nb;
+        int it = 0, refs = 0, status = MF_OK, mode = 0;
+        bool lowp_off = false, have_prev = false, dirty = true;  // dirty: classes written since `mode` was found
+        while (true) {
+            if (sqrt(rho) <= a.tol * nb) break;
+            if (it >= a.maxiter) {
+                status = MF_ERR_NOT_CONVERGED;
+                break;
+            }
+            {
+                float *t = M.pold;
+                M.pold = M.pnew;
+                M.pnew = t;
+            }
+            const float bt = (float)beta;
+            // p = r + beta p over this CTA's rows, then a cluster barrier: the
+            // SpMV needs all of p.  RULE: one warp per chunk, deciding the
+            // chunk's class from its own rows' change.
+            auto put_p = [&](int i, float pv) {
+                if (M.chip) {
+                    s_win[M.ra + i] = pv;
+                    for (int k = 1; k < ncta; k++) {
+                        const int o = rank + k < ncta ? rank + k : rank + k - ncta;
+                        cl.map_shared_rank(s_win, o)[M.ra + i] = pv;
+                    }
+                    if (learned) M.pnew[M.ra + i] = pv;
+                } else {
+                    M.pnew[M.ra + i] = pv;
+                }
+            };
+            const float *po = M.chip ? s_win + M.ra : M.pold + M.ra;
+            if (rule && !lowp_off) {
+                for (int c = cl0 + wid; c < cl1; c += MNW) {
+                    const int i0 = a.crow[c + sys] - M.ra, i1 = a.crow[c + 1 + sys] - M.ra;
+                    double v = 0.0;
+                    for (int i = i0 + wl; i < i1; i += 32) {
+                        const float old = po[i], pv = fmaf(bt, old, M.r[i]);
+                        put_p(i, pv);
+                        v = fmax(v, fabs((double)pv - (double)old));
+                    }
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+                    if (wl == 0) a.ccls[c] = (unsigned char)rule_chunk_class(v, a.ccls_static[c]);
+                }
+                dirty = true;
+            } else {
+                // four rows per thread in flight: loads first, then the stores
+                int i = tid;
+                for (; i + 3 * MNT < rows; i += 4 * MNT) {
+                    float po4[4], r4[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        po4[u] = po[i + u * MNT];
+                        r4[u] = M.r[i + u * MNT];
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; u++) put_p(i + u * MNT, fmaf(bt, po4[u], r4[u]));
+                }
+                for (; i < rows; i += MNT) put_p(i, fmaf(bt, po[i], M.r[i]));
+            }
+            cl.sync();
+            if (dirty) {
+                // the classes of the system's chunks: all FP16, all FP32 or both
+                bool c16 = true, c32 = true;
+                it_bytes = 0;
+                it_lowp = it_pass = 0;
+                for (int c = sc0 + tid; c < sc0 + nch; c += MNT) {
+                    const bool h = __ldcg(a.ccls + c) != 0;
+                    c16 &= h;
+                    c32 &= !h;
+                    if (c >= cl0 && c < cl1) {
+                        it_bytes += pass_bytes(a.cent[c + 1 + sys] - a.cent[c + sys],
+                                               a.crow[c + 1 + sys] - a.crow[c + sys], M.npan, h ? 2 : 4);
+                        it_lowp += h ? M.npan : 0;
+                        it_pass += M.npan;
+                    }
+                }
+                mode = __syncthreads_and(c16) ? 1 : __syncthreads_and(c32) ? 0 : 2;
+                dirty = false;
+            }
+            st_bytes += it_bytes;
+            st_lowp += it_lowp;
+            st_pass += it_pass;
+            double loc = mix_spmv(a, M, mode);
+            if (nwin > 1) {
+                cl.sync();
+                for (int i = tid; i < rows; i += MNT) loc += (double)M.pnew[M.ra + i] * (double)__ldcg(M.q + i);
+            }
+            const double pq = mix_sum(cl, loc, s_slot[2], s_warp);
+            if (!(pq != 0.0) || !isfinite(pq)) {
+                status = MF_ERR_BREAKDOWN;
+                break;
+            }
+            const double alpha = rho / pq;
+            loc = 0.0;
+            {
+                // four rows per thread in flight (loads first)
+                const float af = (float)alpha;
+                const float *pn = M.chip ? s_win + M.ra : M.pnew + M.ra;
+                int i = tid;
+                for (; i + 3 * MNT < rows; i += 4 * MNT) {
+                    float p4[4], q4[4], r4[4], x4[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        p4[u] = pn[i + u * MNT];
+                        q4[u] = M.q[i + u * MNT];
+                        r4[u] = M.r[i + u * MNT];
+                        x4[u] = M.xlo[i + u * MNT];
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        M.xlo[i + u * MNT] = fmaf(af, p4[u], x4[u]);
+                        const float ri = fmaf(-af, q4[u], r4[u]);
+                        M.r[i + u * MNT] = ri;
+                        loc += (double)ri * (double)ri;
+                    }
+                }
+                for (; i < rows; i += MNT) {
+                    M.xlo[i] = fmaf(af, pn[i], M.xlo[i]);
+                    const float ri = fmaf(-af, M.q[i], M.r[i]);
+                    M.r[i] = ri;
+                    loc += (double)ri * (double)ri;
+                }
+            }
+            double rho_new = mix_sum(cl, loc, s_slot[3], s_warp);
+            it++;
+            bool checkpoint = learned && !lowp_off && it == 1;
+            if (sqrt(rho_new) <= a.delta * rmax || sqrt(rho_new) <= a.tol * nb) {
+                loc = mix_refine<L>(a, V, M);
+                rho_new = mix_sum(cl, loc, s_slot[1], s_warp);
+                const double rt = sqrt(rho_new);
+                // the low-precision classes stop where the FP64 residual did
+                // not follow the recurrence (uniform: every CTA holds the same
+                // cluster sums)
+                if ((rule || learned) && !lowp_off && rt > 0.5 * rmax) {
+                    lowp_off = true;
+                    dirty = true;
+                    for (int c = cl0 + tid; c < cl1; c += MNT) a.ccls[c] = (a.ccls_static[c] & 1) ? 1 : 0;
+                }
+                rmax = rt;
+                refs++;
+                checkpoint = learned && !lowp_off;
+            }
+            if (checkpoint) {
+                mix_checkpoint(a, V, M, cl0, cl1, (float)(sqrt(rho_new) / nb), refs, have_prev, s_w, s_feat, s_fslot,
+                               s_fwarp);
+                have_prev = true;
+                dirty = true;
+            }
+            beta = rho_new / rho;
+            rho = rho_new;
+            relres = sqrt(rho) / nb;
+        }
+        if (status != MF_OK) {
+            for (int i = tid; i < rows; i += MNT) x[M.ra + i] += (double)M.xlo[i];
+        }
+        if (st_pass) {
             atomicAdd(&a.sysstat[3 * sys], st_bytes);
             atomicAdd(&a.sysstat[3 * sys + 1], st_lowp);
             atomicAdd(&a.sysstat[3 * sys + 2], st_pass);
@@ -1298,17 +1477,33 @@ __global__ void __launch_bounds__(BNT) k_batch_classify(BatchArgs a, const doubl
     }
 }
 
-template <int L, bool MIX>
-int batched_ctas(int count, int cluster)
+// The kernel of a policy kind: entry point, threads, dynamic shared memory.
+struct BatchKernel {
+    void (*fn)(const BatchArgs);
+    int threads;
+    size_t smem;
+};
+
+BatchKernel batch_kernel(bool mixed, int lanes)
 {
+    switch (lanes) {
+    case 4: return mixed ? BatchKernel{k_batched_cg<4>, MNT, MixSmem::TOTAL} : BatchKernel{k_batched_cg64<4>, BNT, sizeof(BSmem)};
+    case 8: return mixed ? BatchKernel{k_batched_cg<8>, MNT, MixSmem::TOTAL} : BatchKernel{k_batched_cg64<8>, BNT, sizeof(BSmem)};
+    case 16: return mixed ? BatchKernel{k_batched_cg<16>, MNT, MixSmem::TOTAL} : BatchKernel{k_batched_cg64<16>, BNT, sizeof(BSmem)};
+    default: return mixed ? BatchKernel{k_batched_cg<32>, MNT, MixSmem::TOTAL} : BatchKernel{k_batched_cg64<32>, BNT, sizeof(BSmem)};
+    }
+}
+
+int batched_ctas(bool mixed, int lanes, int count, int cluster)
+{
+    const BatchKernel k = batch_kernel(mixed, lanes);
     int dev = 0, sms = 0, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // clusters of 16 CTAs are above the portable size: allowed explicitly
-    if (cluster > 8) cudaFuncSetAttribute(k_batched_cg<L, MIX>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    constexpr size_t smem = SmemLayout<MIX>::TOTAL;
-    cudaFuncSetAttribute(k_batched_cg<L, MIX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_batched_cg<L, MIX>, BNT, smem);
+    if (cluster > 8) cudaFuncSetAttribute(k.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k.fn, k.threads, k.smem);
     int ctas = sms * (per > 0 ? per : 1);
     ctas = (ctas / cluster) * cluster;
     const int want = count * cluster;
@@ -1318,9 +1513,9 @@ int batched_ctas(int count, int cluster)
 }
 
 // ctas: computed before any stream capture (batched_ctas)
-template <int L, bool MIX>
-mf_status launch_batched(const BatchArgs &a, int cluster, int ctas, cudaStream_t s)
+mf_status launch_batched(bool mixed, int lanes, const BatchArgs &a, int cluster, int ctas, cudaStream_t s)
 {
+    const BatchKernel k = batch_kernel(mixed, lanes);
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cudaLaunchAttribute attr[1];
@@ -1328,39 +1523,17 @@ mf_status launch_batched(const BatchArgs &a, int cluster, int ctas, cudaStream_t
     attr[0].val.clusterDim.x = cluster;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    cfg.blockDim = dim3(BNT);
-    cfg.dynamicSmemBytes = SmemLayout<MIX>::TOTAL;
+    cfg.blockDim = dim3(k.threads);
+    cfg.dynamicSmemBytes = k.smem;
     cfg.stream = s;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     // enough clusters to fill the GPU (the work queue balances them)
     cfg.gridDim = dim3(ctas);
     note_launch();
-    MF_CUDA(cudaLaunchKernelEx(&cfg, k_batched_cg<L, MIX>, a));
+    MF_CUDA(cudaLaunchKernelEx(&cfg, k.fn, a));
     return MF_OK;
 }
-
-template <bool MIX>
-struct Lanes {
-    static int ctas(int lanes, int count, int cluster)
-    {
-        switch (lanes) {
-        case 4: return batched_ctas<4, MIX>(count, cluster);
-        case 8: return batched_ctas<8, MIX>(count, cluster);
-        case 16: return batched_ctas<16, MIX>(count, cluster);
-        default: return batched_ctas<32, MIX>(count, cluster);
-        }
-    }
-    static mf_status launch(int lanes, const BatchArgs &a, int cluster, int ctas, cudaStream_t s)
-    {
-        switch (lanes) {
-        case 4: return launch_batched<4, MIX>(a, cluster, ctas, s);
-        case 8: return launch_batched<8, MIX>(a, cluster, ctas, s);
-        case 16: return launch_batched<16, MIX>(a, cluster, ctas, s);
-        default: return launch_batched<32, MIX>(a, cluster, ctas, s);
-        }
-    }
-};
 
 // One CTA per system: ||b - A x|| / ||b|| in FP64 (panels added in order
 // per row).
@@ -1390,13 +1563,13 @@ __global__ void k_batch_resid(BatchArgs a, const double *b, const double *x, dou
     }
 }
 
-// Per row of every system (one CTA per system): the FP32 copy, the
-// row-scaled FP16 copy with the diagonal taken out, the row scale and the
+// Per row of every system (one CTA per system): the row-scaled FP16 copy with
+// the diagonal taken out, the row scale and the
 // FP32 diagonal, and the row statistics the chunk features use.
 // Row scale: 2^(e - 14) with e the exponent of the largest off-diagonal
 // magnitude; rows whose scale leaves FP32's normal range, or whose diagonal
 // does not fit FP32, are marked not FP16-capable.
-__global__ void k_batch_rows(BatchArgs a, float *val32, __half *val16, uint32_t *cv16, float *rscale, float *diag32,
+__global__ void k_batch_rows(BatchArgs a, __half *val16, float *rscale, float *diag32, double *diag64,
                              float4 *rowstat, unsigned char *rowflag)
 {
     for (int sys = blockIdx.x; sys < a.count; sys += gridDim.x) {
@@ -1407,7 +1580,6 @@ __global__ void k_batch_rows(BatchArgs a, float *val32, __half *val16, uint32_t 
                 const long long rpb = a.prow0[V.gp0 + k], eb = a.pent0[V.gp0 + k];
                 for (int e = a.prow[rpb + i]; e < a.prow[rpb + i + 1]; e++) {
                     const double v = a.val[eb + e], av = fabs(v);
-                    val32[eb + e] = (float)v;
                     if (av > 0.0 && (amin == 0.0 || av < amin)) amin = av;
                     if ((int)a.col[eb + e] + k * PW == i) {
                         d += v;
@@ -1431,11 +1603,11 @@ __global__ void k_batch_rows(BatchArgs a, float *val32, __half *val16, uint32_t 
                         if ((double)__half2float(h) * ldexp(1.0, e) != v) exact = false;
                     }
                     val16[eb + q] = h;
-                    cv16[eb + q] = ((uint32_t)__half_as_ushort(h) << 16) | (uint32_t)a.col[eb + q];
                 }
             }
             rscale[V.r0 + i] = ok ? ldexpf(1.f, e) : 0.f;
             diag32[V.r0 + i] = (float)d;
+            diag64[V.r0 + i] = d;
             const double margin = d - S;
             rowstat[V.r0 + i] = make_float4((float)fmax(offmax, fabs(d)), (float)amin,
                                             (float)(S / fmax(margin, 1e-30 * fmax(S, 1e-300))),
@@ -1443,6 +1615,12 @@ __global__ void k_batch_rows(BatchArgs a, float *val32, __half *val16, uint32_t 
             rowflag[V.r0 + i] = (unsigned char)((exact ? 1 : 0) | (ok ? 2 : 0));
         }
     }
+}
+
+__global__ void k_batch_cast32(long long n, const double *v, float *out)
+{
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
+        out[e] = (float)v[e];
 }
 
 // Per chunk (one warp per chunk, one CTA per system): the static class byte
@@ -1575,6 +1753,96 @@ void parallel_for(int count, F f)
     for (auto &t : th) t.join();
 }
 
+// The sorted slices of every system (after k_batch_rows): row lengths,
+// slices per window, a stable sort, the slices' storage, the entries.
+cudaError_t batch_slices(mf_batch bt)
+{
+    const int count = bt->count;
+    std::vector<int> win0(count);
+    std::vector<long long> len0;
+    long long lens = 0;
+    for (int s = 0; s < count; s++) {
+        win0[s] = (int)len0.size();
+        for (int k = 0; k < sell_windows(bt->n[s]); k++) {
+            len0.push_back(lens);
+            lens += bt->n[s];
+        }
+    }
+    const int windows = (int)len0.size();
+    cudaError_t e = cudaSuccess;
+    // temporaries: len0 | row lengths | slices per window | long rows
+    char *tmp = nullptr;
+    int *quads = nullptr, *quad0 = nullptr;
+    const size_t o_len = sizeof(long long) * windows, o_ns = o_len + sizeof(int) * (size_t)lens,
+                 o_nl = o_ns + sizeof(int) * (windows + 1), bytes = o_nl + sizeof(int) * windows;
+    int nslices = 0, nquads = 0;
+    SellBuild B;
+    memset(&B, 0, sizeof(B));
+    do {
+        if ((e = cudaMalloc((void **)&tmp, bytes)) != cudaSuccess) break;
+        if ((e = cudaMalloc((void **)&bt->d_win0, sizeof(int) * count)) != cudaSuccess) break;
+        if ((e = cudaMalloc((void **)&bt->d_sfirst, sizeof(int) * (windows + 1))) != cudaSuccess) break;
+        if ((e = cudaMemcpy(bt->d_win0, win0.data(), sizeof(int) * count, cudaMemcpyHostToDevice)) != cudaSuccess) break;
+        if ((e = cudaMemcpy(tmp, len0.data(), sizeof(long long) * windows, cudaMemcpyHostToDevice)) != cudaSuccess) break;
+        int *len = (int *)(tmp + o_len), *ns = (int *)(tmp + o_ns), *nl = (int *)(tmp + o_nl);
+        B.count = count;
+        B.pw = PW;
+        B.n = bt->d_n;
+        B.pan0 = bt->d_pan0;
+        B.win0 = bt->d_win0;
+        B.row0 = bt->d_row0;
+        B.prow0 = bt->d_prow0;
+        B.pent0 = bt->d_pent0;
+        B.len0 = (const long long *)tmp;
+        B.sc = bt->d_sc;
+        B.crow = bt->d_crow;
+        B.prow = bt->d_prow;
+        B.col = bt->d_col;
+        B.val = bt->d_val;
+        B.val16 = bt->d_val16;
+        B.rscale = bt->d_rscale;
+        B.diag32 = bt->d_diag32;
+        const int gw = std::min(windows, 4096);
+        k_sell_lengths<<<dim3(gw, 16), SELL_NT>>>(B, windows, len);
+        k_sell_slices<<<gw, SELL_NT>>>(B, windows, len, ns, nl);
+        note_launch(2);
+        if ((e = cudaMemset(ns + windows, 0, sizeof(int))) != cudaSuccess) break;
+        if (exclusive_scan_i32(ns, bt->d_sfirst, windows + 1, 0, &nslices) != MF_OK) {
+            e = cudaErrorUnknown;
+            break;
+        }
+        if ((e = cudaMalloc((void **)&bt->d_sdesc, sizeof(int2) * ((size_t)nslices + 1))) != cudaSuccess) break;
+        if ((e = cudaMalloc((void **)&bt->d_srec, sizeof(int4) * 32 * ((size_t)nslices + 1))) != cudaSuccess) break;
+        if ((e = cudaMalloc((void **)&quads, sizeof(int) * 2 * ((size_t)nslices + 1))) != cudaSuccess) break;
+        quad0 = quads + nslices + 1;
+        k_sell_sort<<<std::min(windows, 148 * 32), 32>>>(B, windows, len, nl, bt->d_sfirst, bt->d_srec, quads);
+        note_launch();
+        if ((e = cudaMemset(quads + nslices, 0, sizeof(int))) != cudaSuccess) break;
+        if (exclusive_scan_i32(quads, quad0, nslices + 1, 0, &nquads) != MF_OK) {
+            e = cudaErrorUnknown;
+            break;
+        }
+        const size_t words = (size_t)(nquads > 0 ? nquads : 1) * 128;
+        if ((e = cudaMalloc((void **)&bt->d_scv, 4 * words)) != cudaSuccess) break;
+        if ((e = cudaMalloc((void **)&bt->d_sv32, 4 * words)) != cudaSuccess) break;
+        if ((e = cudaMalloc((void **)&bt->d_sc16, 2 * words)) != cudaSuccess) break;
+        if ((e = cudaMalloc((void **)&bt->d_sv64, 8 * words)) != cudaSuccess) break;
+        if ((e = cudaMemset(bt->d_scv, 0, 4 * words)) != cudaSuccess) break;
+        if ((e = cudaMemset(bt->d_sv32, 0, 4 * words)) != cudaSuccess) break;
+        if ((e = cudaMemset(bt->d_sc16, 0, 2 * words)) != cudaSuccess) break;
+        if ((e = cudaMemset(bt->d_sv64, 0, 8 * words)) != cudaSuccess) break;
+        k_sell_fill<<<std::min((nslices + 7) / 8, 148 * 32), SELL_NT>>>(B, windows, bt->d_sfirst, nl, bt->d_srec, quads,
+                                                                        quad0, nslices, bt->d_sdesc, bt->d_scv,
+                                                                        bt->d_sv32, bt->d_sc16, bt->d_sv64);
+        note_launch();
+        if ((e = cudaGetLastError()) != cudaSuccess) break;
+        e = cudaDeviceSynchronize();
+    } while (false);
+    if (tmp) cudaFree(tmp);
+    if (quads) cudaFree(quads);
+    return e;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1675,11 +1943,10 @@ mf_status mf_batch_create(int count, const int *n, const int *const *rowptr, con
     BT_ALLOC(bt->d_cent, sizeof(int) * cent.size());
     BT_ALLOC(bt->d_col, sizeof(uint16_t) * (nz + 16));
     BT_ALLOC(bt->d_val, sizeof(double) * (nz + 2));
-    BT_ALLOC(bt->d_val32, sizeof(float) * (nz + 4));
     BT_ALLOC(bt->d_val16, sizeof(__half) * (nz + 16));
-    BT_ALLOC(bt->d_cv16, sizeof(uint32_t) * (nz + 8));
     BT_ALLOC(bt->d_rscale, sizeof(float) * (rows + 4));
     BT_ALLOC(bt->d_diag32, sizeof(float) * (rows + 4));
+    BT_ALLOC(bt->d_diag64, sizeof(double) * (rows + 4));
     BT_ALLOC(bt->d_ccls, (size_t)nch + 16);
     BT_ALLOC(bt->d_ccls_static, (size_t)nch + 16);
     BT_ALLOC(bt->d_cstat, sizeof(float) * NCSTAT * ((size_t)nch + 1));
@@ -1728,8 +1995,7 @@ mf_status mf_batch_create(int count, const int *n, const int *const *rowptr, con
         a.prow = bt->d_prow;
         a.col = bt->d_col;
         a.val = bt->d_val;
-        k_batch_rows<<<grid, 256>>>(a, bt->d_val32, bt->d_val16, bt->d_cv16, bt->d_rscale, bt->d_diag32, rowstat,
-                                    rowflag);
+        k_batch_rows<<<grid, 256>>>(a, bt->d_val16, bt->d_rscale, bt->d_diag32, bt->d_diag64, rowstat, rowflag);
         note_launch();
         e = cudaGetLastError();
         if (e == cudaSuccess) {
@@ -1740,6 +2006,7 @@ mf_status mf_batch_create(int count, const int *n, const int *const *rowptr, con
         }
     }
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = batch_slices(bt);
     if (e == cudaSuccess) {
         std::vector<unsigned char> st((size_t)nch);
         e = cudaMemcpy(st.data(), bt->d_ccls_static, (size_t)nch, cudaMemcpyDeviceToHost);
@@ -1760,9 +2027,10 @@ mf_status mf_batch_destroy(mf_batch bt)
     if (!bt) return MF_OK;
     if (bt->graph) cudaGraphExecDestroy(bt->graph);
     void *bufs[] = {bt->d_order,  bt->d_n,      bt->d_pan0,   bt->d_npan,   bt->d_row0,   bt->d_prow0,
-                    bt->d_pent0,  bt->d_prow,   bt->d_col,    bt->d_val,    bt->d_val32,  bt->d_val16,
+                    bt->d_pent0,  bt->d_prow,   bt->d_col,    bt->d_val,    bt->d_val16,  bt->d_sfirst,
                     bt->d_rscale, bt->d_diag32, bt->d_iters,  bt->d_refs,   bt->d_status, bt->d_relres,
-                    bt->d_cv16,
+                    bt->d_win0,   bt->d_sdesc,  bt->d_srec,   bt->d_scv,    bt->d_sv32,   bt->d_sc16,
+                    bt->d_sv64,   bt->d_diag64,
                     bt->work,     bt->d_queue,  bt->d_sc,     bt->d_crow,   bt->d_cent,   bt->d_ccls,
                     bt->d_ccls_static, bt->d_cstat, bt->d_cdyn, bt->d_sysstat};
     for (void *p : bufs)
@@ -1781,8 +2049,9 @@ mf_status mf_batch_info(mf_batch bt, long long *rows_total, long long *nnz_total
 }
 
 // five vectors of rows_total doubles, each followed by PW + 16 elements of
-// slack (the last system's p window copy rounds up to 16 bytes)
-static size_t batch_vec_len(mf_batch bt) { return (size_t)bt->rows_total + PW + 16; }
+// slack (the FP64 kernel reads masked columns past a short last panel) and 4
+// per system (the mixed kernel starts every system on a 16-byte boundary)
+static size_t batch_vec_len(mf_batch bt) { return ((size_t)bt->rows_total + 4 * (size_t)bt->count + PW + 16 + 3) & ~(size_t)3; }
 
 static mf_status batch_work(mf_batch bt)
 {
@@ -1814,9 +2083,10 @@ static BatchArgs batch_args(mf_batch bt, const double *b, double *x, const mf_so
     a.prow = bt->d_prow;
     a.col = bt->d_col;
     a.val = bt->d_val;
-    a.val32 = bt->d_val32;
     a.val16 = bt->d_val16;
-    a.cv16 = bt->d_cv16;
+    a.sell = SellView{bt->d_sfirst, bt->d_win0, bt->d_sdesc, bt->d_srec, (const uint4 *)bt->d_scv,
+                      (const float4 *)bt->d_sv32, (const uint2 *)bt->d_sc16, (const double2 *)bt->d_sv64,
+                      bt->d_diag64};
     a.rscale = bt->d_rscale;
     a.diag32 = bt->d_diag32;
     a.b = b;
@@ -1846,8 +2116,6 @@ static BatchArgs batch_args(mf_batch bt, const double *b, double *x, const mf_so
     {
         const char *e = getenv("MF_BATCH_BACKOFF_NS");
         a.backoff_ns = e ? (unsigned)atoi(e) : 0u;
-        const char *rs = getenv("MF_BATCH_ROWSUM");
-        a.rowsum = (rs && !strcmp(rs, "lanes")) ? 1 : 0;
     }
     a.policy = o.policy;
     a.mlp_w = (o.policy == MF_POLICY_LEARNED && bt->policy) ? policy_weights(bt->policy) : nullptr;
@@ -1856,7 +2124,7 @@ static BatchArgs batch_args(mf_batch bt, const double *b, double *x, const mf_so
 
 static int batch_ctas(mf_batch bt, bool mixed, int lanes, int cluster)
 {
-    return mixed ? Lanes<true>::ctas(lanes, bt->count, cluster) : Lanes<false>::ctas(lanes, bt->count, cluster);
+    return batched_ctas(mixed, lanes, bt->count, cluster);
 }
 
 // Enqueues one batched solve.  Nothing here allocates or queries the device:
@@ -1866,7 +2134,7 @@ static mf_status batch_enqueue(mf_batch bt, const BatchArgs &a, bool mixed, int 
 {
     MF_CUDA(cudaMemsetAsync(bt->d_queue, 0, sizeof(int) * 2, s));  // queue head, stage-wait status
     MF_CUDA(cudaMemsetAsync(bt->d_sysstat, 0, sizeof(unsigned long long) * 3 * bt->count, s));
-    MF_TRY(mixed ? Lanes<true>::launch(lanes, a, cluster, ctas, s) : Lanes<false>::launch(lanes, a, cluster, ctas, s));
+    MF_TRY(launch_batched(mixed, lanes, a, cluster, ctas, s));
     k_batch_resid<<<std::min(bt->count, 1184), 256, 0, s>>>(a, a.b, a.x, bt->d_relres + bt->count);
     note_launch();
     MF_CUDA(cudaGetLastError());
@@ -2050,7 +2318,7 @@ mf_status mf_batch_export(mf_batch bt, const char *name, void *host_dst, size_t 
     else if (!strcmp(name, "chunk_rows")) src = bt->d_crow, need = sizeof(int) * (nch + bt->count);
     else if (!strcmp(name, "chunk_ends")) src = bt->d_cent, need = sizeof(int) * (nch + bt->count);
     else if (!strcmp(name, "val16")) src = bt->d_val16, need = 2 * nz;
-    else if (!strcmp(name, "val32")) src = bt->d_val32, need = 4 * nz;
+    else if (!strcmp(name, "val32")) need = 4 * nz;  // made from val below
     else if (!strcmp(name, "val")) src = bt->d_val, need = 8 * nz;
     else if (!strcmp(name, "col")) src = bt->d_col, need = 2 * nz;
     else if (!strcmp(name, "row_scale")) src = bt->d_rscale, need = 4 * rows;
@@ -2062,6 +2330,17 @@ mf_status mf_batch_export(mf_batch bt, const char *name, void *host_dst, size_t 
     if (bytes != need) {
         set_last_error("mf_batch_export: %s has %zu bytes, %zu given", name, need, bytes);
         return MF_ERR_INVALID_ARG;
+    }
+    if (need && !src) {
+        float *tmp = nullptr;
+        MF_CUDA(cudaMalloc(&tmp, need));
+        k_batch_cast32<<<(unsigned)std::min<size_t>((nz + 255) / 256, 148 * 32), 256>>>((long long)nz, bt->d_val, tmp);
+        note_launch();
+        cudaError_t e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaMemcpy(host_dst, tmp, need, cudaMemcpyDeviceToHost);
+        cudaFree(tmp);
+        MF_CUDA(e);
+        return MF_OK;
     }
     if (need) MF_CUDA(cudaMemcpy(host_dst, src, need, cudaMemcpyDeviceToHost));
     return MF_OK;
