@@ -6,7 +6,7 @@
 // Per (system, window) the rows are sorted by their number of off-diagonal
 // entries in the window, longest first (equal lengths in row order), and
 // taken 32 at a time: one slice is one warp's work, lane l owns the l-th row
-// of the slice and adds its entries in entry order.  Entries are stored four
+// of the slice and adds its entries one after another.  Entries are stored four
 // slots at a time ("quads"): lane l's entries 4j .. 4j+3 are 16 consecutive
 // bytes, a warp reads 512 consecutive bytes per quad, and no two lanes share
 // a row, so a row sum needs neither shuffles nor a second pass.  Sorting
@@ -195,14 +195,36 @@ __global__ void __launch_bounds__(32) k_sell_sort(SellBuild a, int windows, cons
 
 // One warp per slice: its descriptor and its entries (the arrays are zeroed
 // before).
-__global__ void __launch_bounds__(SELL_NT)
+//
+// The order of a row's entries is free, and it decides the shared-memory bank
+// conflicts of the gathers: slot j of the 32 rows is one gather of 32 window
+// elements, which in storage order falls on random banks (the fullest of 32
+// banks then holds ~3.5 of 32 lanes).  So a slice of up to SELL_ORD slots is
+// filled slot by slot: in rounds every lane without an entry for the slot
+// looks through its remaining entries (at most SELL_SCAN of them) for one
+// whose bank no lane has taken yet, the lowest lane that found a bank keeps
+// it, the others look again; a lane that finds none takes its next entry.
+// Deterministic: it depends on the matrix alone.
+constexpr int SELL_ORD = 96;
+constexpr int SELL_SCAN = 24;
+constexpr int SELL_ROUNDS = 10;
+constexpr int SELL_FNT = 128;
+
+__global__ void __launch_bounds__(SELL_FNT)
 k_sell_fill(SellBuild a, int windows, const int *__restrict__ first, const int *__restrict__ nlong,
             const int4 *__restrict__ rec, const int *__restrict__ quads, const int *__restrict__ quad0, int nslices,
             int2 *__restrict__ desc, uint32_t *__restrict__ cv, float *__restrict__ v32, uint16_t *__restrict__ c16,
             double *__restrict__ v64)
 {
-    const int lane = threadIdx.x & 31;
-    for (int s = blockIdx.x * (SELL_NT / 32) + (threadIdx.x >> 5); s < nslices; s += gridDim.x * (SELL_NT / 32)) {
+    // per warp and lane: banks of the entries still to place, their numbers,
+    // and the slot of every entry
+    __shared__ unsigned char s_bank[SELL_FNT / 32][SELL_ORD][32], s_id[SELL_FNT / 32][SELL_ORD][32],
+        s_slot[SELL_FNT / 32][SELL_ORD][32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    auto bank = s_bank[wid];
+    auto id = s_id[wid];
+    auto slot = s_slot[wid];
+    for (int s = blockIdx.x * (SELL_FNT / 32) + wid; s < nslices; s += gridDim.x * (SELL_FNT / 32)) {
         int lo = 0, hi = windows - 1;  // the slice's window
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
@@ -215,21 +237,68 @@ k_sell_fill(SellBuild a, int windows, const int *__restrict__ first, const int *
         const int i = rec[(size_t)s * 32 + lane].x;
         const size_t base = (size_t)quad0[s] * 128;
         if (lane == 0) desc[s] = make_int2(quad0[s], quads[s] | (lng ? (int)0x80000000 : 0));
-        if (i < 0) continue;
-        int j = 0;
-        sell_entries(a, sys, n, i, c0, c1, [&](long long e, int c) {
-            // long rows: entry j belongs to lane j % 32 (every lane walks the
-            // row and keeps its own), else all entries are this lane's
-            const int mine = lng ? ((j & 31) == lane ? j >> 5 : -1) : j;
-            if (mine >= 0) {
-                const size_t at = base + (size_t)(mine >> 2) * 128 + lane * 4 + (mine & 3);
-                cv[at] = ((uint32_t)__half_as_ushort(a.val16[e]) << 16) | (uint32_t)(c - c0);
-                v64[at] = a.val[e];
-                v32[at] = (float)a.val[e];
-                c16[at] = (uint16_t)(c - c0);
+        const bool ordered = !lng && quads[s] * 4 <= SELL_ORD;
+        if (ordered) {
+            int m = 0;
+            if (i >= 0)
+                sell_entries(a, sys, n, i, c0, c1, [&](long long, int c) {
+                    bank[m][lane] = (unsigned char)((c - c0) & 31);
+                    id[m][lane] = (unsigned char)m;
+                    m++;
+                });
+            const int most = __reduce_max_sync(0xffffffffu, m);
+            for (int j = 0; j < most; j++) {
+                int pick = -1;  // place of the chosen entry among the remaining ones
+                for (int pass = 0; pass < 2; pass++) {  // the second pass lets every bank take one lane more
+                    unsigned taken = 0;
+                    bool open = j < m && pick < 0;  // this lane has no entry for the slot yet
+                    for (int round = 0; round < SELL_ROUNDS && __any_sync(0xffffffffu, open); round++) {
+                        int k = -1, b = 32 + lane;  // a bank of its own for lanes without a candidate
+                        if (open) {
+                            const int end = min(m, j + SELL_SCAN);
+                            for (int t = j; t < end; t++) {
+                                const int bt = bank[t][lane];
+                                if (!((taken >> bt) & 1u)) {
+                                    k = t;
+                                    b = bt;
+                                    break;
+                                }
+                            }
+                        }
+                        const unsigned same = __match_any_sync(0xffffffffu, b);
+                        const bool won = k >= 0 && (same & ((1u << lane) - 1u)) == 0;
+                        if (won) pick = k;
+                        if (won || k < 0) open = false;
+                        taken |= __reduce_or_sync(0xffffffffu, won ? 1u << b : 0u);
+                    }
+                }
+                if (j < m) {
+                    if (pick < 0) pick = j;
+                    const unsigned char e = id[pick][lane];
+                    slot[e][lane] = (unsigned char)j;
+                    id[pick][lane] = id[j][lane];
+                    bank[pick][lane] = bank[j][lane];
+                }
             }
-            j++;
-        });
+            __syncwarp();
+        }
+        if (i >= 0) {
+            int j = 0;
+            sell_entries(a, sys, n, i, c0, c1, [&](long long e, int c) {
+                // long rows: entry j belongs to lane j % 32 (every lane walks
+                // the row and keeps its own), else all entries are this lane's
+                const int mine = lng ? ((j & 31) == lane ? j >> 5 : -1) : ordered ? (int)slot[j][lane] : j;
+                if (mine >= 0) {
+                    const size_t at = base + (size_t)(mine >> 2) * 128 + lane * 4 + (mine & 3);
+                    cv[at] = ((uint32_t)__half_as_ushort(a.val16[e]) << 16) | (uint32_t)(c - c0);
+                    v64[at] = a.val[e];
+                    v32[at] = (float)a.val[e];
+                    c16[at] = (uint16_t)(c - c0);
+                }
+                j++;
+            });
+        }
+        __syncwarp();
     }
 }
 

@@ -1831,7 +1831,7 @@ cudaError_t batch_slices(mf_batch bt)
         if ((e = cudaMemset(bt->d_sv32, 0, 4 * words)) != cudaSuccess) break;
         if ((e = cudaMemset(bt->d_sc16, 0, 2 * words)) != cudaSuccess) break;
         if ((e = cudaMemset(bt->d_sv64, 0, 8 * words)) != cudaSuccess) break;
-        k_sell_fill<<<std::min((nslices + 7) / 8, 148 * 32), SELL_NT>>>(B, windows, bt->d_sfirst, nl, bt->d_srec, quads,
+        k_sell_fill<<<std::min((nslices + SELL_FNT / 32 - 1) / (SELL_FNT / 32), 148 * 64), SELL_FNT>>>(B, windows, bt->d_sfirst, nl, bt->d_srec, quads,
                                                                         quad0, nslices, bt->d_sdesc, bt->d_scv,
                                                                         bt->d_sv32, bt->d_sc16, bt->d_sv64);
         note_launch();
