@@ -14,6 +14,12 @@
 // of SELL_LONG entries or more are slices of their own, their entries dealt
 // to the 32 lanes in turn.
 //
+// The slices of a (system, window) are stored in the order of SELL_BINS bins:
+// dealt longest first, slice t goes to bin bitrev(t mod SELL_BINS).  A warp
+// takes a range of consecutive bins, and any power-of-two number of warps up
+// to SELL_BINS gets equal shares: bit reversal spreads the bins with one slice
+// more evenly over every such split.
+//
 // Four arrays share that geometry: cv (FP16 value bits << 16 | column in the
 // window), v32 and v64 (FP32 and FP64 values) and c16 (column in the window).  Diagonal
 // entries are left out: a row's FP32 diagonal and FP16 scale are part of its
@@ -29,6 +35,24 @@ namespace {
 constexpr int SELL_WIN = 55296;   // columns of a window: 216 KB of FP32 p beside the policy network's weights
 constexpr int SELL_LONG = 256;    // rows from this length on are spread over a warp
 constexpr int SELL_NT = 256;
+constexpr int SELL_BINS = 512;    // most warps of a cluster
+
+// Bit reversal of a bin number, and the place of dealt slice t (of ns) in
+// storage: bins in order, a bin's slices in the order dealt.
+__host__ __device__ inline int sell_bitrev(int v)
+{
+    int r = 0;
+    for (int b = 1; b < SELL_BINS; b <<= 1, v >>= 1) r = (r << 1) | (v & 1);
+    return r;
+}
+// slices in bins [0, b): bin c holds ns / BINS, one more when bitrev(c) < ns % BINS
+__host__ __device__ inline int sell_before(int ns, int b)
+{
+    const int full = ns / SELL_BINS, extra = ns % SELL_BINS;
+    int m = full * b;
+    for (int c = 0; c < b; c++) m += sell_bitrev(c) < extra;
+    return m;
+}
 
 // Windows of a system of n rows and their width (a multiple of 4 when there
 // are several).
@@ -40,9 +64,9 @@ __host__ __device__ inline int sell_width(int n)
 }
 
 struct SellView {
-    const int *first;      // [windows + 1] first slice of each (system, window)
+    const int *first;      // [windows * (SELL_BINS + 1)] first slice of every bin of each (system, window)
     const int *win0;       // [count] first window of each system
-    const int2 *desc;      // per slice: first quad (of 128 words), quads | long << 31
+    const int2 *desc;      // per slice (+1 at the end): first quad (of 128 words), quads | long << 31
     const int4 *rec;       // per slice and lane: row (-1 none), chunk, FP16 scale, FP32 diagonal
     const uint4 *cv;       // per quad and lane
     const float4 *v32;
@@ -132,12 +156,15 @@ __global__ void __launch_bounds__(SELL_NT) k_sell_slices(SellBuild a, int window
 }
 
 // Per window (one warp): a stable counting sort of the rows by length,
-// longest first, and the slices' records and quad counts.
+// longest first, and the slices' records and quad counts (long rows marked
+// in the top bit), in storage order.
 __global__ void __launch_bounds__(32) k_sell_sort(SellBuild a, int windows, const int *__restrict__ len,
                                                   const int *__restrict__ nlong, const int *__restrict__ first,
-                                                  int4 *__restrict__ rec, int *__restrict__ quads)
+                                                  int4 *__restrict__ rec, int *__restrict__ quads,
+                                                  int *__restrict__ bins)
 {
     __shared__ int s_at[SELL_LONG + 1];  // next place of each length (SELL_LONG: all long rows)
+    __shared__ int s_bin[SELL_BINS + 1]; // first slice of every bin
     const int lane = threadIdx.x;
     for (int w = blockIdx.x; w < windows; w += gridDim.x) {
         const int sys = sell_system(a, w), n = a.n[sys];
@@ -156,9 +183,15 @@ __global__ void __launch_bounds__(32) k_sell_sort(SellBuild a, int windows, cons
                 at += c;
             }
         }
-        // empty lanes of the last slice, and its width
-        for (int k = lane; k < 32 * ns; k += 32)
-            if (k >= 32 * nl + (n - nl)) rec[(size_t)f0 * 32 + k] = make_int4(-1, 0, 0, 0);
+        for (int b = lane; b <= SELL_BINS; b += 32) {
+            s_bin[b] = f0 + sell_before(ns, b);
+            bins[w * (SELL_BINS + 1) + b] = s_bin[b];
+        }
+        __syncwarp();
+        // where dealt slice t is stored
+        auto place = [&](int t) { return (size_t)(s_bin[sell_bitrev(t % SELL_BINS)] + t / SELL_BINS); };
+        // empty lanes of the last slice
+        for (int k = 32 * nl + (n - nl) + lane; k < 32 * ns; k += 32) rec[place(ns - 1) * 32 + (k & 31)] = make_int4(-1, 0, 0, 0);
         __syncwarp();
         int c = a.sc[sys];  // chunk of the current rows (rows ascend)
         for (int i0 = 0; i0 < n; i0 += 32) {
@@ -179,18 +212,25 @@ __global__ void __launch_bounds__(32) k_sell_sort(SellBuild a, int windows, cons
                 const int at = base + before;
                 const int4 v = make_int4(i, ci, __float_as_int(a.rscale[r0 + i]), __float_as_int(a.diag32[r0 + i]));
                 if (key == SELL_LONG) {
-                    for (int t = 0; t < 32; t++) rec[((size_t)f0 + at) * 32 + t] = v;
-                    quads[f0 + at] = (m + 127) / 128;
+                    for (int t = 0; t < 32; t++) rec[place(at) * 32 + t] = v;
+                    quads[place(at)] = (int)((unsigned)((m + 127) / 128) | 0x80000000u);
                 } else {
                     const int k = at - nl;  // place among the other rows
-                    rec[((size_t)f0 + nl) * 32 + k] = v;
-                    if ((k & 31) == 0) quads[f0 + nl + (k >> 5)] = (m + 3) / 4;  // the slice's longest row
+                    rec[place(nl + (k >> 5)) * 32 + (k & 31)] = v;
+                    if ((k & 31) == 0) quads[place(nl + (k >> 5))] = (m + 3) / 4;  // the slice's longest row
                 }
             }
             c = __shfl_sync(0xffffffffu, ci, 31);
         }
         __syncwarp();
     }
+}
+
+// Quad counts without the long-row mark (to be scanned).
+__global__ void __launch_bounds__(SELL_NT) k_sell_counts(int nslices, const int *__restrict__ quads, int *__restrict__ cnt)
+{
+    for (int s = blockIdx.x * SELL_NT + threadIdx.x; s <= nslices; s += gridDim.x * SELL_NT)
+        cnt[s] = s < nslices ? (quads[s] & 0x7fffffff) : 0;
 }
 
 // One warp per slice: its descriptor and its entries (the arrays are zeroed
@@ -201,20 +241,20 @@ __global__ void __launch_bounds__(32) k_sell_sort(SellBuild a, int windows, cons
 // elements, which in storage order falls on random banks (the fullest of 32
 // banks then holds ~3.5 of 32 lanes).  So a slice of up to SELL_ORD slots is
 // filled slot by slot: in rounds every lane without an entry for the slot
-// looks through its remaining entries (at most SELL_SCAN of them) for one
-// whose bank no lane has taken yet, the lowest lane that found a bank keeps
-// it, the others look again; a lane that finds none takes its next entry.
+// looks through its remaining entries for one whose bank no lane has taken
+// yet, the lowest lane that found a bank keeps it, the others look again;
+// lanes left over go through a second pass in which every bank takes one
+// more, and then take their next entry.  Rows of ~40 entries: the fullest
+// bank holds 2.0 lanes instead of 3.4 (modelled).
 // Deterministic: it depends on the matrix alone.
 constexpr int SELL_ORD = 96;
-constexpr int SELL_SCAN = 24;
 constexpr int SELL_ROUNDS = 10;
 constexpr int SELL_FNT = 128;
 
 __global__ void __launch_bounds__(SELL_FNT)
-k_sell_fill(SellBuild a, int windows, const int *__restrict__ first, const int *__restrict__ nlong,
-            const int4 *__restrict__ rec, const int *__restrict__ quads, const int *__restrict__ quad0, int nslices,
-            int2 *__restrict__ desc, uint32_t *__restrict__ cv, float *__restrict__ v32, uint16_t *__restrict__ c16,
-            double *__restrict__ v64)
+k_sell_fill(SellBuild a, int windows, const int *__restrict__ first, const int4 *__restrict__ rec,
+            const int *__restrict__ quads, const int *__restrict__ quad0, int nslices, int2 *__restrict__ desc,
+            uint32_t *__restrict__ cv, float *__restrict__ v32, uint16_t *__restrict__ c16, double *__restrict__ v64)
 {
     // per warp and lane: banks of the entries still to place, their numbers,
     // and the slot of every entry
@@ -233,10 +273,11 @@ k_sell_fill(SellBuild a, int windows, const int *__restrict__ first, const int *
         }
         const int w = lo, sys = sell_system(a, w), n = a.n[sys], W = sell_width(n);
         const int c0 = (w - a.win0[sys]) * W, c1 = min(n, c0 + W);
-        const bool lng = s - first[w] < nlong[w];
+        const bool lng = quads[s] < 0;
         const int i = rec[(size_t)s * 32 + lane].x;
         const size_t base = (size_t)quad0[s] * 128;
-        if (lane == 0) desc[s] = make_int2(quad0[s], quads[s] | (lng ? (int)0x80000000 : 0));
+        if (lane == 0) desc[s] = make_int2(quad0[s], quads[s]);
+        if (lane == 0 && s == nslices - 1) desc[nslices] = make_int2(quad0[nslices], 0);
         const bool ordered = !lng && quads[s] * 4 <= SELL_ORD;
         if (ordered) {
             int m = 0;
@@ -255,8 +296,7 @@ k_sell_fill(SellBuild a, int windows, const int *__restrict__ first, const int *
                     for (int round = 0; round < SELL_ROUNDS && __any_sync(0xffffffffu, open); round++) {
                         int k = -1, b = 32 + lane;  // a bank of its own for lanes without a candidate
                         if (open) {
-                            const int end = min(m, j + SELL_SCAN);
-                            for (int t = j; t < end; t++) {
+                            for (int t = j; t < m; t++) {
                                 const int bt = bank[t][lane];
                                 if (!((taken >> bt) & 1u)) {
                                     k = t;
@@ -303,32 +343,33 @@ k_sell_fill(SellBuild a, int windows, const int *__restrict__ first, const int *
 }
 
 // Read-only matrix words: each is used once per product, so they do not
-// take L1 space.
-__device__ __forceinline__ uint4 ld_words(const uint4 *p)
+// take L1 space.  Predicated inside the instruction: a branch around a load
+// makes the compiler wait for it where the paths meet.
+__device__ __forceinline__ void ld_words(uint4 &v, const uint4 *p, bool on)
 {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(p));
-    return v;
+    asm volatile(
+        "{ .reg .pred q; setp.ne.u32 q, %5, 0; @q ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4]; }"
+        : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+        : "l"(p), "r"((unsigned)on));
 }
-__device__ __forceinline__ uint2 ld_words(const uint2 *p)
+__device__ __forceinline__ void ld_words(uint2 &v, const uint2 *p, bool on)
 {
-    uint2 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
-    return v;
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %3, 0; @q ld.global.nc.L1::no_allocate.v2.u32 {%0, %1}, [%2]; }"
+                 : "+r"(v.x), "+r"(v.y)
+                 : "l"(p), "r"((unsigned)on));
 }
-__device__ __forceinline__ float4 ld_words(const float4 *p)
+__device__ __forceinline__ void ld_words(float4 &v, const float4 *p, bool on)
 {
-    const uint4 v = ld_words((const uint4 *)p);
-    return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+    asm volatile(
+        "{ .reg .pred q; setp.ne.u32 q, %5, 0; @q ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4]; }"
+        : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w)
+        : "l"(p), "r"((unsigned)on));
 }
-
-__device__ __forceinline__ double2 ld_words(const double2 *p)
+__device__ __forceinline__ void ld_words(double2 &v, const double2 *p, bool on)
 {
-    double2 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
-    return v;
+    asm volatile("{ .reg .pred q; setp.ne.u32 q, %3, 0; @q ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2]; }"
+                 : "+d"(v.x), "+d"(v.y)
+                 : "l"(p), "r"((unsigned)on));
 }
 
 __device__ __forceinline__ float half_hi(uint32_t w)
@@ -337,13 +378,13 @@ __device__ __forceinline__ float half_hi(uint32_t w)
 }
 
 // The three kinds of quad: its words as loaded, and its four terms added to
-// a sum.  G: quads of a group; a group is loaded while the one before it is
-// added (two groups of registers).
+// a sum.  N: quads loaded at once.
 struct Quad16 {
-    static constexpr int G = 4;
+    static constexpr int N = 3;
     const uint4 *cv;
     using T = uint4;
-    __device__ __forceinline__ T ld(int q) const { return ld_words(cv + q * 32); }
+    __device__ __forceinline__ Quad16 at(int q) const { return Quad16{cv + (size_t)q * 32}; }
+    __device__ __forceinline__ void ld(T &w, int q, bool on) const { ld_words(w, cv + q * 32, on); }
     __device__ __forceinline__ float add(float acc, const T &w, const float *win) const
     {
         acc = fmaf(half_hi(w.x), win[w.x & 0xffffu], acc);
@@ -354,14 +395,19 @@ struct Quad16 {
 };
 
 struct Quad32 {
-    static constexpr int G = 2;
+    static constexpr int N = 3;
     const float4 *v32;
     const uint2 *c16;
     struct T {
         float4 v;
         uint2 c;
     };
-    __device__ __forceinline__ T ld(int q) const { return T{ld_words(v32 + q * 32), ld_words(c16 + q * 32)}; }
+    __device__ __forceinline__ Quad32 at(int q) const { return Quad32{v32 + (size_t)q * 32, c16 + (size_t)q * 32}; }
+    __device__ __forceinline__ void ld(T &w, int q, bool on) const
+    {
+        ld_words(w.v, v32 + q * 32, on);
+        ld_words(w.c, c16 + q * 32, on);
+    }
     __device__ __forceinline__ float add(float acc, const T &w, const float *win) const
     {
         acc = fmaf(w.v.x, win[w.c.x & 0xffffu], acc);
@@ -372,16 +418,19 @@ struct Quad32 {
 };
 
 struct Quad64 {
-    static constexpr int G = 2;
+    static constexpr int N = 2;
     const double2 *v64;  // two per quad and lane
     const uint2 *c16;
     struct T {
         double2 a, b;
         uint2 c;
     };
-    __device__ __forceinline__ T ld(int q) const
+    __device__ __forceinline__ Quad64 at(int q) const { return Quad64{v64 + (size_t)q * 64, c16 + (size_t)q * 32}; }
+    __device__ __forceinline__ void ld(T &w, int q, bool on) const
     {
-        return T{ld_words(v64 + q * 64), ld_words(v64 + q * 64 + 1), ld_words(c16 + q * 32)};
+        ld_words(w.a, v64 + q * 64, on);
+        ld_words(w.b, v64 + q * 64 + 1, on);
+        ld_words(w.c, c16 + q * 32, on);
     }
     __device__ __forceinline__ double add(double acc, const T &w, const double *x) const
     {
@@ -393,40 +442,49 @@ struct Quad64 {
     }
 };
 
-// One lane's sum over nq quads (the same count for the whole warp): the
-// quads beyond a whole number of groups first, then group by group.
-template <class Q, class S, class X>
-__device__ __forceinline__ S sell_dot(const Q &src, int nq, const X *x)
-{
-    constexpr int G = Q::G;
-    const int rem = nq % G, nf = nq / G;
-    typename Q::T t[G], a[G];
-    S acc = 0;
+// One lane's sum over a slice's quads (the same count for the whole warp),
+// N quads loaded at once, the next N after they are added: the latency is
+// covered by the SM's 32 warps (3 quads per warp: 48 KB in flight).  More
+// quads per warp with fewer warps was slower (16 warps, 12 quads: 357 ms
+// against 322 for 256 systems), and so was a ring that reloads each quad as it
+// is added (592 ms: the compiler waits for every load).  first() loads a slice's first quads (the
+// matrix does not change, so it may run before the barrier that p waits
+// for); sum() adds them and loads and adds the rest.
+template <class Q>
+struct SellSum {
+    Q src;
+    typename Q::T b[Q::N];
+
+    __device__ __forceinline__ explicit SellSum(const Q &q) : src(q)
+    {
 #pragma unroll
-    for (int u = 0; u < G - 1; u++)
-        if (u < rem) t[u] = src.ld(u);
-    if (nf > 0)
-#pragma unroll
-        for (int u = 0; u < G; u++) a[u] = src.ld(rem + u);
-#pragma unroll
-    for (int u = 0; u < G - 1; u++)
-        if (u < rem) acc = src.add(acc, t[u], x);
-    if (nf == 0) return acc;
-    int q = rem + G;
-#pragma unroll 2
-    for (int g = 1; g < nf; g++, q += G) {
-        typename Q::T b[G];
-#pragma unroll
-        for (int u = 0; u < G; u++) b[u] = src.ld(q + u);
-#pragma unroll
-        for (int u = 0; u < G; u++) acc = src.add(acc, a[u], x);
-#pragma unroll
-        for (int u = 0; u < G; u++) a[u] = b[u];
+        for (int u = 0; u < Q::N; u++) b[u] = typename Q::T{};
     }
+    __device__ __forceinline__ void first(int q0, int nq)
+    {
+        const Q at = src.at(q0);
 #pragma unroll
-    for (int u = 0; u < G; u++) acc = src.add(acc, a[u], x);
-    return acc;
-}
+        for (int u = 0; u < Q::N; u++) at.ld(b[u], u, u < nq);
+    }
+    template <class S, class X>
+    __device__ __forceinline__ S sum(int q0, int nq, const X *x)
+    {
+        S acc = 0;
+        for (;;) {
+            // two quads at a time: eight gathers in flight
+#pragma unroll
+            for (int u = 0; u + 1 < Q::N; u += 2) {
+                if (u + 1 < nq) acc = src.add(src.add(acc, b[u], x), b[u + 1], x);
+                else if (u < nq) acc = src.add(acc, b[u], x);
+            }
+            if (Q::N % 2 && Q::N - 1 < nq) acc = src.add(acc, b[Q::N - 1], x);
+            nq -= Q::N;
+            if (nq <= 0) return acc;
+            q0 += Q::N;
+            first(q0, nq);
+        }
+    }
+};
 
 }  // namespace
 }  // namespace mf

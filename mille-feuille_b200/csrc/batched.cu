@@ -16,14 +16,19 @@
 // of p (FP32, up to 55,296 columns, 216 KB) in shared memory and streams the
 // matrix in sorted slices of 32 rows (batch_sell.cuh): a lane owns a row, its
 // words come as 16-byte loads straight from L2/HBM into registers, the
-// gathers hit shared memory.  What bounds it: shared-memory wavefronts (the
-// gather of 32 random banks takes ~3.5) and the L2 latency of the words, then
-// the three cluster barriers of an iteration.  The earlier form -- bulk
-// copies into three shared-memory stages, products written back to shared
-// memory, one lane per row adding them -- moved every entry through shared
-// memory four times.  Measured, to a 1e-14 residual on one B200: 256 systems
-// of 1,000-32,000 rows, learned classes, 648 -> 370 ms; 24 systems of
-// 1,000-4,000 rows, static classes, 51.7 -> 37.6 ms.
+// gathers hit shared memory.  Systems whose window and vectors fit (up to
+// ~22,000 rows with 2 CTAs) keep p, r, q and the correction on the chip, p
+// and q going to the cluster's other CTAs by distributed shared memory.
+// What bounds it: the L1 data pipe (a warp's slot of 32 entries takes ~5
+// wavefronts -- 2 for its words, ~2 for the gather, the rest for the row
+// ends; 6.4 cycles measured), then the three cluster barriers of an
+// iteration.  The earlier form -- bulk copies into three shared-memory
+// stages, products written back to shared memory, one lane per row adding
+// them, vectors in global memory -- moved every entry through shared memory
+// four times.  Measured on one B200: the 512-system benchmark batch (1,000 to
+// 64,000 rows, 1e-10) 1,366 -> 665 ms learned, 1,419 -> 838 static; to 1e-14,
+// 256 systems of 1,000-32,000 rows, learned, 630 -> 288 ms; 24 systems of
+// 1,000-4,000 rows, static, 56.1 -> 28.4 ms.
 //
 // The panel storage (column panels of PW = 32768 columns, 16-bit column
 // offsets within the panel, rows of each panel in CSR) is what the chunks,
@@ -125,8 +130,10 @@ struct mf_batch_s {
     int *d_iters = nullptr, *d_refs = nullptr, *d_status = nullptr;
     double *d_relres = nullptr;
     unsigned long long *d_sysstat = nullptr;  // [count][3] matrix bytes streamed, FP16 chunk passes, chunk passes
+    void *arena = nullptr, *slices = nullptr, *words = nullptr;  // allocations the arrays above and below live in
     void *work = nullptr;
     size_t work_bytes = 0;
+    int auto_cluster = 0;         // CTAs per system of untuned mixed solves (0: not found yet)
     int *d_queue = nullptr;
     // sorted slices of the mixed solves (batch_sell.cuh)
     int *d_sfirst = nullptr, *d_win0 = nullptr;
@@ -158,7 +165,7 @@ namespace {
 constexpr int BNT = 512;
 constexpr int BNW = BNT / 32;
 #ifndef MF_BATCH_MNT
-#define MF_BATCH_MNT 512
+#define MF_BATCH_MNT 1024
 #endif
 constexpr int MNT = MF_BATCH_MNT;  // threads of a mixed-kernel CTA
 constexpr int MNW = MNT / 32;
@@ -924,19 +931,60 @@ __global__ void __launch_bounds__(BNT, 1) k_batched_cg64(const __grid_constant__
     }
 }
 
+// The mixed kernel's dynamic shared memory: the window of p and, for a
+// system on the chip, from the window's end the vectors r, q, xlo.
+extern __shared__ __align__(16) unsigned char mix_smem[];
+__device__ __forceinline__ float *mix_win() { return reinterpret_cast<float *>(mix_smem); }
+
+// Distributed shared memory by address: `addr` (of this CTA) in CTA `rank`
+// of the cluster, and plain stores to it.
+__device__ __forceinline__ unsigned mix_remote(const void *p, int rank)
+{
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void mix_put(unsigned addr, float v)
+{
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ void mix_put(unsigned addr, float4 v)
+{
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+                 : "memory");
+}
+
 // The mixed kernel's view of the system its cluster is solving.  The CTA's
-// own rows are [ra, rb); r, xlo and q are indexed from ra.  On chip (small
-// systems): the window of p and the three vectors live in shared memory, p
-// and q reach the other CTAs by distributed shared memory; otherwise they
-// are in global memory.
+// own rows are [ra, rb); r, xlo and q are indexed from ra4, ra rounded down
+// to a multiple of four (16-byte words of the same rows in every vector).  On
+// chip (CHIP below; systems whose window and vectors fit): p is the window
+// itself, r, q and xlo follow from its end, p and q reach the other CTAs by
+// distributed shared memory.  Otherwise the vectors are in global memory.
 struct MixSys {
-    int sys, n, ra, rb, npan;
-    bool chip;
-    float *win;             // the window of p (shared memory)
-    float *r, *xlo, *q;     // this CTA's rows (on chip: shared memory)
+    int sys, n, ra, rb, ra4, npan;
+    int most;               // entries of an on-chip vector (the CTA with most rows)
+    bool xwin;              // on chip, and x fits in FP64 beside r and q (reliable updates)
+    float *r, *xlo, *q;     // global vectors of this CTA's rows
     float *pnew, *pold;     // global p buffers, indexed by row (on chip: written for LEARNED only)
-    const int *rab;         // on chip: first row of every CTA (shared memory)
+    int s0, s1;             // this warp's slices (one window)
 };
+
+template <bool CHIP>
+__device__ __forceinline__ float *mix_r(const MixSys &M) { return CHIP ? mix_win() + SELL_WIN - M.most : M.r; }
+template <bool CHIP>
+__device__ __forceinline__ float *mix_q(const MixSys &M) { return CHIP ? mix_win() + SELL_WIN - 2 * M.most : M.q; }
+template <bool CHIP>
+__device__ __forceinline__ float *mix_xlo(const MixSys &M) { return CHIP ? mix_win() + SELL_WIN - 3 * M.most : M.xlo; }
+
+// This warp's share of a window's slices: consecutive bins.
+__device__ __forceinline__ void mix_share(const BatchArgs &a, int win, int rank, int ncta, MixSys &M)
+{
+    const int per = SELL_BINS / (MNW * ncta), b0 = (rank * MNW + (threadIdx.x >> 5)) * per;
+    const int *first = a.sell.first + win * (SELL_BINS + 1);
+    M.s0 = first[b0];
+    M.s1 = first[b0 + per];
+}
+static_assert(SELL_BINS % (MNW * 16) == 0, "every cluster size deals whole bins");
 
 // Sum over the cluster: warp tree, then warp 0 adds the warps' sums in a
 // fixed tree and writes the CTA's value to every CTA's slots (remote
@@ -957,13 +1005,13 @@ __device__ __forceinline__ double mix_sum(cg::cluster_group &cl, double v, doubl
         if (wl < ncta) *cl.map_shared_rank(slots + rank, wl) = c;  // lanes below MNW hold the sum
     }
     cl.sync();
-    double s = 0.0;
-    for (int k = 0; k < ncta; k++) s += slots[k];
+    double s = slots[0];
+    for (int k = 1; k < ncta; k++) s += slots[k];
     return s;
 }
 static_assert(MNW <= 32 && MNW >= 16, "a lane per warp in the second step, a lane with the sum per CTA of a cluster");
 
-// The CTA that owns row i.
+// The CTA that owns row i (rab: first row of every CTA).
 __device__ __forceinline__ int mix_owner(const int *rab, int ncta, int i)
 {
     int o = 0;
@@ -973,22 +1021,57 @@ __device__ __forceinline__ int mix_owner(const int *rab, int ncta, int i)
 
 // q = A p over the sorted slices; returns this thread's part of p.q (one
 // window; 0 for several).  mode: 0 every chunk FP32, 1 every chunk FP16, 2
-// both kinds.
-__device__ __noinline__ double mix_spmv(const BatchArgs &a, MixSys M, int mode)
+// both kinds.  sync: the cluster barrier that p waits for is still to come
+// (the first matrix words load before it).
+template <int mode, bool CHIP>
+__device__ __noinline__ double mix_spmv(const BatchArgs &a, MixSys M, const int *rab, bool sync)
 {
     cg::cluster_group cl = cg::this_cluster();
-    const SellView &E = a.sell;
-    const int tid = threadIdx.x, wid = tid >> 5, wl = tid & 31;
+    const int tid = threadIdx.x, wl = tid & 31;
     const int rank = (int)cl.block_rank(), ncta = (int)cl.num_blocks();
-    const int wf = E.win0[M.sys], nwin = sell_windows(M.n), W = sell_width(M.n);
+    const int nwin = CHIP ? 1 : sell_windows(M.n), W = sell_width(M.n);
+    const int2 *desc = a.sell.desc;
+    const int4 *recs = a.sell.rec + wl;
+    float *win = mix_win();
+    float *q = mix_q<CHIP>(M);
     double loc = 0.0;
     for (int k = 0; k < nwin; k++) {
         const int c0 = k * W, c1 = min(M.n, c0 + W);
-        if (!M.chip) {
+        if (nwin > 1) mix_share(a, a.sell.win0[M.sys] + k, rank, ncta, M);
+        int4 rec = __ldg(recs + (size_t)M.s0 * 32), recn = rec;
+        int2 sd = __ldg(desc + M.s0), sdn = sd;
+        // a row's sum: scale, diagonal, store
+        auto row = [&](float acc, bool h16, bool lng) {
+            if (lng) {  // a long row: its lanes' sums in a fixed tree
+                double d = (double)acc;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+                acc = (float)d;
+            }
+            if (rec.x >= 0 && (!lng || wl == 0)) {
+                const int i = rec.x;
+                const bool own = i >= c0 && i < c1;  // the diagonal's window
+                const float pi = own ? win[i - c0] : 0.f;
+                const float y = fmaf(h16 ? __int_as_float(rec.z) : 1.f, acc, own ? __int_as_float(rec.w) * pi : 0.f);
+                if (CHIP) {
+                    const int o = mix_owner(rab, ncta, i), at = i - (rab[o] & ~3);
+                    if (o == rank) q[at] = y;
+                    else mix_put(mix_remote(q + at, o), y);
+                } else {
+                    float *qi = q + (i - M.ra4);
+                    *qi = k == 0 ? y : __ldcg(qi) + y;
+                }
+                if (nwin == 1) loc += (double)pi * (double)y;
+            }
+        };
+        auto window = [&]() {
+            if (sync) cl.sync();
+            sync = false;
+            if (CHIP) return;
             // window: whole 16-byte words (up to three elements past the
             // window's end come from the vector's slack)
             const float4 *src = reinterpret_cast<const float4 *>(M.pnew + c0);
-            float4 *dst = reinterpret_cast<float4 *>(M.win);
+            float4 *dst = reinterpret_cast<float4 *>(win);
             const int nq4 = (c1 - c0 + 3) >> 2;
             int i = tid;
             for (; i + 7 * MNT < nq4; i += 8 * MNT) {
@@ -1000,62 +1083,50 @@ __device__ __noinline__ double mix_spmv(const BatchArgs &a, MixSys M, int mode)
             }
             for (; i < nq4; i += MNT) dst[i] = __ldcg(src + i);
             __syncthreads();
-        }
-        // slices, longest first, dealt to the cluster's warps in turn
-        const int s1 = E.first[wf + k + 1], step = MNW * ncta;
-        int s = E.first[wf + k] + wid * ncta + rank;
-        int2 sd = make_int2(0, 0);
-        int4 rec = make_int4(-1, 0, 0, 0);
-        if (s < s1) {
-            sd = __ldg(E.desc + s);
-            rec = __ldg(E.rec + (size_t)s * 32 + wl);
-        }
-        while (s < s1) {
-            const int sn = s + step;
-            int2 sdn = sd;
-            int4 recn = rec;
-            if (sn < s1) {  // the next slice's record loads under this one's sums
-                sdn = __ldg(E.desc + sn);
-                recn = __ldg(E.rec + (size_t)sn * 32 + wl);
+        };
+        // the warp's slices: the next slice's descriptor, record and first
+        // words on their way while a slice is finished
+        auto run = [&](auto sum) {
+            sum.first(sd.x, M.s0 < M.s1 ? sd.y & 0x7fffffff : 0);
+            window();
+            for (int s = M.s0; s < M.s1; s++) {
+                const int sn = min(s + 1, M.s1 - 1);
+                sdn = __ldg(desc + sn);
+                recn = __ldg(recs + (size_t)sn * 32);
+                const float acc = sum.template sum<float>(sd.x, sd.y & 0x7fffffff, win);
+                const bool lng = sd.y < 0;
+                sd = sdn;
+                sum.first(sd.x, s + 1 < M.s1 ? sd.y & 0x7fffffff : 0);
+                row(acc, mode == 1, lng);
+                rec = recn;
             }
-            const size_t at = (size_t)sd.x * 32 + wl;
-            const int nq = sd.y & 0x7fffffff;
-            float acc = 0.f, scale = __int_as_float(rec.z);
-            if (mode == 1) {
-                acc = sell_dot<Quad16, float>(Quad16{E.cv + at}, nq, M.win);
-            } else {
-                const bool h = mode == 2 && rec.x >= 0 && __ldcg(a.ccls + rec.y) != 0;
+        };
+        if constexpr (mode == 1) {
+            run(SellSum<Quad16>(Quad16{a.sell.cv + wl}));
+        } else if constexpr (mode == 0) {
+            run(SellSum<Quad32>(Quad32{a.sell.v32 + wl, a.sell.c16 + wl}));
+        } else {
+            window();
+            SellSum<Quad16> s16(Quad16{a.sell.cv + wl});
+            SellSum<Quad32> s32(Quad32{a.sell.v32 + wl, a.sell.c16 + wl});
+            for (int s = M.s0; s < M.s1; s++) {
+                rec = __ldg(recs + (size_t)s * 32);
+                sd = __ldg(desc + s);
+                const int nq = sd.y & 0x7fffffff;
+                const bool h = rec.x >= 0 && __ldcg(a.ccls + rec.y) != 0;
                 const unsigned m16 = __ballot_sync(0xffffffffu, h);
                 const unsigned m32 = __ballot_sync(0xffffffffu, !h && rec.x >= 0);
-                float a16 = 0.f;
-                if (m16) a16 = sell_dot<Quad16, float>(Quad16{E.cv + at}, nq, M.win);
-                if (m32) acc = sell_dot<Quad32, float>(Quad32{E.v32 + at, E.c16 + at}, nq, M.win);
-                if (h) acc = a16;
-                else scale = 1.f;
-            }
-            if (sd.y < 0) {  // a long row: its lanes' sums in a fixed tree
-                double d = (double)acc;
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-                acc = (float)d;
-            }
-            if (rec.x >= 0 && (sd.y >= 0 || wl == 0)) {
-                const int i = rec.x;
-                const bool own = i >= c0 && i < c1;  // the diagonal's window
-                const float pi = own ? M.win[i - c0] : 0.f;
-                const float y = fmaf(scale, acc, own ? __int_as_float(rec.w) * pi : 0.f);
-                if (M.chip) {
-                    const int o = mix_owner(M.rab, ncta, i);
-                    cl.map_shared_rank(M.q, o)[i - M.rab[o]] = y;
-                } else {
-                    float *qi = M.q + (i - M.ra);
-                    *qi = k == 0 ? y : __ldcg(qi) + y;
+                float a16 = 0.f, a32 = 0.f;
+                if (m16) {
+                    s16.first(sd.x, nq);
+                    a16 = s16.template sum<float>(sd.x, nq, win);
                 }
-                if (nwin == 1) loc += (double)pi * (double)y;
+                if (m32) {
+                    s32.first(sd.x, nq);
+                    a32 = s32.template sum<float>(sd.x, nq, win);
+                }
+                row(h ? a16 : a32, h, sd.y < 0);
             }
-            s = sn;
-            sd = sdn;
-            rec = recn;
         }
         // several windows: the next one's sums continue from every warp's
         // q, and the window is overwritten
@@ -1064,47 +1135,92 @@ __device__ __noinline__ double mix_spmv(const BatchArgs &a, MixSys M, int mode)
     return loc;
 }
 
+// f4(i) for every aligned group of four rows i .. i+3 inside [ra, rb), f1(i)
+// for the rows at the two ends.
+template <class F4, class F1>
+__device__ __forceinline__ void mix_rows(int ra, int rb, F4 f4, F1 f1)
+{
+    const int tid = threadIdx.x, qa = (ra + 3) >> 2, qb = rb >> 2;
+    if (qa < qb) {
+        for (int j = qa + tid; j < qb; j += MNT) f4(4 * j);
+        const int i = tid < 4 ? ra + tid : 4 * qb + tid - 4;
+        if (tid < 4 ? i < 4 * qa : (tid < 8 && i < rb)) f1(i);
+    } else {
+        for (int i = ra + tid; i < rb; i += MNT) f1(i);
+    }
+}
+
 // The rare steps, out of line so that the iteration keeps its registers.
 // Reliable update: x += xlo, xlo = 0, then (cluster barrier) r = b - A x from
 // the FP64 values; returns this thread's part of ||r||^2.  One window: over
-// the slices (16-byte streams as in the product, x gathered from L2); several
-// windows: lane groups over the rows of the panel storage.
-template <int L>
-__device__ __noinline__ double mix_refine(const BatchArgs &a, SysView V, MixSys M)
+// the slices as in the product, x gathered from shared memory where it fits
+// beside r and q (the window of p gives way; this CTA's rows of p are kept in
+// global memory meanwhile), else from L2 -- there every lane's element is a
+// cache line of its own, ~10 times the time.  Several windows: lane groups
+// over the rows of the panel storage.
+template <int L, bool CHIP>
+__device__ __noinline__ double mix_refine(const BatchArgs &a, SysView V, MixSys M, const int *rab, bool psaved)
 {
     cg::cluster_group cl = cg::this_cluster();
-    const int tid = threadIdx.x, wid = tid >> 5, wl = tid & 31;
+    const int tid = threadIdx.x, wl = tid & 31;
     const int rank = (int)cl.block_rank(), ncta = (int)cl.num_blocks();
     const double *b = a.b + V.r0;
     double *x = a.x + V.r0;
-    for (int i = tid; i < M.rb - M.ra; i += MNT) {
-        x[M.ra + i] += (double)M.xlo[i];
-        M.xlo[i] = 0.f;
+    float *win = mix_win(), *r = mix_r<CHIP>(M), *xlo = mix_xlo<CHIP>(M);
+    const bool xwin = CHIP && M.xwin;
+    for (int i = M.ra + tid; i < M.rb; i += MNT) {
+        x[i] += (double)xlo[i - M.ra4];
+        if (xwin && !psaved) M.pnew[i] = win[i];
     }
     cl.sync();
     double loc = 0.0;
-    if (sell_windows(M.n) == 1) {
-        const SellView &E = a.sell;
-        const int wf = E.win0[M.sys], s1 = E.first[wf + 1];
-        const double *diag = E.diag64 + V.r0;
-        for (int s = E.first[wf] + wid * ncta + rank; s < s1; s += MNW * ncta) {
-            const int2 sd = __ldg(E.desc + s);
-            const int i = __ldg(&E.rec[(size_t)s * 32 + wl].x);
-            const size_t at = (size_t)sd.x * 32 + wl;
-            double y = sell_dot<Quad64, double>(Quad64{E.v64 + 2 * at, E.c16 + at}, sd.y & 0x7fffffff, x);
-            if (sd.y < 0)
+    if (CHIP || sell_windows(M.n) == 1) {
+        const double *diag = a.sell.diag64 + V.r0;
+        const int2 *desc = a.sell.desc;
+        const int4 *recs = a.sell.rec + wl;
+        double *xw = reinterpret_cast<double *>(mix_smem);
+        if (xwin) {
+            int i = tid;
+            for (; i + 7 * MNT < M.n; i += 8 * MNT) {
+                double v[8];
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-            if (i >= 0 && (sd.y >= 0 || wl == 0)) {
-                const float rv = (float)(b[i] - fma(diag[i], x[i], y));
-                if (M.chip) {
-                    const int o = mix_owner(M.rab, ncta, i);
-                    cl.map_shared_rank(M.r, o)[i - M.rab[o]] = rv;
-                } else {
-                    M.r[i - M.ra] = rv;
-                }
-                loc += (double)rv * (double)rv;
+                for (int u = 0; u < 8; u++) v[u] = __ldcg(x + i + u * MNT);
+#pragma unroll
+                for (int u = 0; u < 8; u++) xw[i + u * MNT] = v[u];
             }
+            for (; i < M.n; i += MNT) xw[i] = __ldcg(x + i);
+            __syncthreads();
+        }
+        auto rows = [&](const double *xg) {
+            SellSum<Quad64> sum(Quad64{a.sell.v64 + 2 * wl, a.sell.c16 + wl});
+            for (int s = M.s0; s < M.s1; s++) {
+                const int2 sd = __ldg(desc + s);
+                const int i = __ldg(&recs[(size_t)s * 32].x), nq = sd.y & 0x7fffffff;
+                sum.first(sd.x, nq);
+                double y = sum.template sum<double>(sd.x, nq, xg);
+                const bool lng = sd.y < 0;
+                if (lng)
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+                if (i >= 0 && (!lng || wl == 0)) {
+                    const float rv = (float)(b[i] - fma(diag[i], xg[i], y));
+                    if (CHIP) {
+                        const int o = mix_owner(rab, ncta, i), at = i - (rab[o] & ~3);
+                        if (o == rank) r[at] = rv;
+                        else mix_put(mix_remote(r + at, o), rv);
+                    } else {
+                        r[i - M.ra4] = rv;
+                    }
+                    loc += (double)rv * (double)rv;
+                }
+            }
+        };
+        if (xwin) {
+            rows(xw);
+            __syncthreads();  // x read
+            for (int i = M.ra + tid; i < M.rb; i += MNT) win[i] = M.pnew[i];
+        } else {
+            rows(x);
         }
     } else {
         const int lane = tid % L, grp = tid / L;
@@ -1117,33 +1233,36 @@ __device__ __noinline__ double mix_refine(const BatchArgs &a, SysView V, MixSys 
             if (lane == 0) {
                 if (i0 >= 0) {
                     const float rv = (float)(b[i0] - y0);
-                    M.r[i0 - M.ra] = rv;
+                    r[i0 - M.ra4] = rv;
                     loc += (double)rv * (double)rv;
                 }
                 if (i1 >= 0) {
                     const float rv = (float)(b[i1] - y1);
-                    M.r[i1 - M.ra] = rv;
+                    r[i1 - M.ra4] = rv;
                     loc += (double)rv * (double)rv;
                 }
             }
         }
     }
+    for (int i = M.ra + tid; i < M.rb; i += MNT) xlo[i - M.ra4] = 0.f;
     return loc;
 }
 
 // LEARNED checkpoint: one warp per chunk of this CTA gathers its statistics,
 // then, with the system's maxima of |r| and |p| over the cluster, its class.
-__device__ __noinline__ void mix_checkpoint(const BatchArgs &a, SysView V, MixSys M, int cl0, int cl1,
-                                            float relres, int refs, bool have_prev, const float *s_w, float *s_feat,
-                                            float *s_fslot, float *s_fwarp)
+template <bool CHIP>
+__device__ __noinline__ void mix_checkpoint(const BatchArgs &a, SysView V, MixSys M, int cl0, int cl1, float relres,
+                                            int refs, bool have_prev, const float *s_w, float *s_feat, float *s_fslot,
+                                            float *s_fwarp)
 {
     cg::cluster_group cl = cg::this_cluster();
     const int wid = threadIdx.x >> 5, wl = threadIdx.x & 31;
     float gr = 0.f, gp = 0.f;
     for (int c = cl0 + wid; c < cl1; c += MNW) {
         // chunk_stats_warp indexes all vectors alike: from the chunk's first row
-        const int r0 = a.crow[c + M.sys], r1 = a.crow[c + 1 + M.sys], at = r0 - M.ra;
-        chunk_stats_warp<float>(a, V, c, 0, r1 - r0, M.r + at, M.pnew + r0, M.pold + r0, M.q + at, nullptr, false, gr, gp);
+        const int r0 = a.crow[c + M.sys], r1 = a.crow[c + 1 + M.sys], at = r0 - M.ra4;
+        chunk_stats_warp<float>(a, V, c, 0, r1 - r0, mix_r<CHIP>(M) + at, M.pnew + r0, M.pold + r0, mix_q<CHIP>(M) + at,
+                                nullptr, false, gr, gp);
     }
     cluster_max2<MNT>(cl, gr, gp, s_fslot, s_fwarp);
     float *xf = s_feat + wid * PN_NF;
@@ -1160,6 +1279,241 @@ __device__ __noinline__ void mix_checkpoint(const BatchArgs &a, SysView V, MixSy
     }
 }
 
+// p = r + beta p over this CTA's rows, to the window of every CTA (on chip)
+// or to global memory.  RULE: one warp per chunk, deciding the chunk's class
+// from its own rows' change.
+template <bool CHIP>
+__device__ __forceinline__ void mix_direction(const BatchArgs &a, cg::cluster_group &cl, const MixSys &M, float bt,
+                                              bool by_rule, bool keep, int cl0, int cl1)
+{
+    const int wid = threadIdx.x >> 5, wl = threadIdx.x & 31, ra4 = M.ra4;
+    const int rank = (int)cl.block_rank(), ncta = (int)cl.num_blocks();
+    float *win = mix_win();
+    const float *po = CHIP ? win : M.pold, *r = mix_r<CHIP>(M);
+    auto put1 = [&](int i, float pv) {
+        if (CHIP) {
+            win[i] = pv;
+            for (int k = 1; k < ncta; k++)
+                mix_put(mix_remote(win + i, rank + k < ncta ? rank + k : rank + k - ncta), pv);
+            if (keep) M.pnew[i] = pv;
+        } else {
+            M.pnew[i] = pv;
+        }
+    };
+    if (by_rule) {
+        for (int c = cl0 + wid; c < cl1; c += MNW) {
+            const int i0 = a.crow[c + M.sys], i1 = a.crow[c + 1 + M.sys];
+            double v = 0.0;
+            for (int i = i0 + wl; i < i1; i += 32) {
+                const float old = po[i], pv = fmaf(bt, old, r[i - ra4]);
+                put1(i, pv);
+                v = fmax(v, fabs((double)pv - (double)old));
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+            if (wl == 0) a.ccls[c] = (unsigned char)rule_chunk_class(v, a.ccls_static[c]);
+        }
+        return;
+    }
+    mix_rows(
+        M.ra, M.rb,
+        [&](int i) {
+            const float4 o = *(const float4 *)(po + i), rv = *(const float4 *)(r + (i - ra4));
+            const float4 pv = make_float4(fmaf(bt, o.x, rv.x), fmaf(bt, o.y, rv.y), fmaf(bt, o.z, rv.z), fmaf(bt, o.w, rv.w));
+            if (CHIP) {
+                *(float4 *)(win + i) = pv;
+                for (int k = 1; k < ncta; k++)
+                    mix_put(mix_remote(win + i, rank + k < ncta ? rank + k : rank + k - ncta), pv);
+                if (keep) *(float4 *)(M.pnew + i) = pv;
+            } else {
+                *(float4 *)(M.pnew + i) = pv;
+            }
+        },
+        [&](int i) { put1(i, fmaf(bt, po[i], r[i - ra4])); });
+}
+
+// x += alpha p, r -= alpha q over this CTA's rows (x: the FP32 correction);
+// returns this thread's part of ||r||^2.
+template <bool CHIP>
+__device__ __forceinline__ double mix_update(const MixSys &M, float af)
+{
+    const int ra4 = M.ra4;
+    const float *pn = CHIP ? mix_win() : M.pnew, *q = mix_q<CHIP>(M);
+    float *r = mix_r<CHIP>(M), *xlo = mix_xlo<CHIP>(M);
+    double loc = 0.0;
+    mix_rows(
+        M.ra, M.rb,
+        [&](int i) {
+            const int o = i - ra4;
+            const float4 p4 = *(const float4 *)(pn + i), q4 = *(const float4 *)(q + o);
+            float4 r4 = *(const float4 *)(r + o), x4 = *(const float4 *)(xlo + o);
+            x4 = make_float4(fmaf(af, p4.x, x4.x), fmaf(af, p4.y, x4.y), fmaf(af, p4.z, x4.z), fmaf(af, p4.w, x4.w));
+            r4 = make_float4(fmaf(-af, q4.x, r4.x), fmaf(-af, q4.y, r4.y), fmaf(-af, q4.z, r4.z), fmaf(-af, q4.w, r4.w));
+            *(float4 *)(xlo + o) = x4;
+            *(float4 *)(r + o) = r4;
+            loc += (double)r4.x * (double)r4.x;
+            loc += (double)r4.y * (double)r4.y;
+            loc += (double)r4.z * (double)r4.z;
+            loc += (double)r4.w * (double)r4.w;
+        },
+        [&](int i) {
+            const int o = i - ra4;
+            xlo[o] = fmaf(af, pn[i], xlo[o]);
+            const float ri = fmaf(-af, q[o], r[o]);
+            r[o] = ri;
+            loc += (double)ri * (double)ri;
+        });
+    return loc;
+}
+
+// Shared memory of a mixed CTA beside the window.
+struct MixShared {
+    double warp[MNW];
+    double slot[4][16];
+    float fslot[2];
+    float fwarp[2 * MNW];
+    int sys;
+    int rab[17];  // first row of every CTA of the cluster
+};
+
+// One system, by the whole cluster.
+template <int L, bool CHIP>
+__device__ __noinline__ void mix_solve(const BatchArgs &a, MixShared &S, SysView V, MixSys M, int sc0, int nch)
+{
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = (int)cl.block_rank(), ncta = (int)cl.num_blocks(), tid = threadIdx.x;
+    float *s_w = reinterpret_cast<float *>(mix_smem + MixSmem::W), *s_feat = reinterpret_cast<float *>(mix_smem + MixSmem::FEAT);
+    const bool learned = a.policy == MF_POLICY_LEARNED && a.mlp_w;
+    const bool rule = a.policy == MF_POLICY_RULE;
+    const double *b = a.b + V.r0;
+    double *x = a.x + V.r0;
+    const int sys = M.sys, nwin = CHIP ? 1 : sell_windows(V.n);
+    const int ra = M.ra, rb = M.rb, ra4 = M.ra4;
+    const int cl0 = sc0 + (int)((long long)nch * rank / ncta), cl1 = sc0 + (int)((long long)nch * (rank + 1) / ncta);
+    unsigned long long st_bytes = 0, it_bytes = 0;  // this thread's chunks: in all, per iteration by the current classes
+    unsigned it_lowp = 0, it_pass = 0;
+    unsigned long long st_lowp = 0, st_pass = 0;
+    double lb = 0.0, lr = 0.0;
+    {
+        float *r = mix_r<CHIP>(M), *xlo = mix_xlo<CHIP>(M);
+        for (int i = ra + tid; i < rb; i += MNT) {
+            const double bv = b[i];
+            const float rv = (float)bv;
+            x[i] = 0.0;
+            r[i - ra4] = rv;
+            xlo[i - ra4] = 0.f;
+            M.pnew[i] = 0.f;  // p before the first iteration
+            if (CHIP) mix_win()[i] = 0.f;
+            lb += bv * bv;
+            lr += (double)rv * (double)rv;
+        }
+    }
+    for (int c = cl0 + tid; c < cl1; c += MNT) a.ccls[c] = (a.ccls_static[c] & 1) ? 1 : 0;
+    const double bb = mix_sum(cl, lb, S.slot[0], S.warp);
+    double rho = mix_sum(cl, lr, S.slot[1], S.warp);
+    const double nb = sqrt(bb) > 0.0 ? sqrt(bb) : 1.0;
+    double beta = 0.0, rmax = sqrt(rho), relres = sqrt(rho) / nb;
+    int it = 0, refs = 0, status = MF_OK, mode = 0;
+    bool lowp_off = false, have_prev = false, dirty = true;  // dirty: classes written since `mode` was found
+    while (true) {
+        if (sqrt(rho) <= a.tol * nb) break;
+        if (it >= a.maxiter) {
+            status = MF_ERR_NOT_CONVERGED;
+            break;
+        }
+        {
+            float *t = M.pold;
+            M.pold = M.pnew;
+            M.pnew = t;
+        }
+        const bool by_rule = rule && !lowp_off;
+        mix_direction<CHIP>(a, cl, M, (float)beta, by_rule, learned, cl0, cl1);
+        // a cluster barrier: the product needs all of p (mix_spmv has it
+        // where the classes are known)
+        const bool sync = !dirty && !by_rule;
+        if (!sync) {
+            cl.sync();
+            // the classes of the system's chunks: all FP16, all FP32 or both
+            bool c16 = true, c32 = true;
+            it_bytes = 0;
+            it_lowp = it_pass = 0;
+            for (int c = sc0 + tid; c < sc0 + nch; c += MNT) {
+                const bool h = __ldcg(a.ccls + c) != 0;
+                c16 &= h;
+                c32 &= !h;
+                if (c >= cl0 && c < cl1) {
+                    it_bytes += pass_bytes(a.cent[c + 1 + sys] - a.cent[c + sys], a.crow[c + 1 + sys] - a.crow[c + sys],
+                                           M.npan, h ? 2 : 4);
+                    it_lowp += h ? M.npan : 0;
+                    it_pass += M.npan;
+                }
+            }
+            mode = __syncthreads_and(c16) ? 1 : __syncthreads_and(c32) ? 0 : 2;
+            dirty = false;
+        }
+        st_bytes += it_bytes;
+        st_lowp += it_lowp;
+        st_pass += it_pass;
+        double loc = mode == 1   ? mix_spmv<1, CHIP>(a, M, S.rab, sync)
+                     : mode == 0 ? mix_spmv<0, CHIP>(a, M, S.rab, sync)
+                                 : mix_spmv<2, CHIP>(a, M, S.rab, sync);
+        if (nwin > 1) {
+            cl.sync();
+            for (int i = ra + tid; i < rb; i += MNT) loc += (double)M.pnew[i] * (double)__ldcg(M.q + i - ra4);
+        }
+        const double pq = mix_sum(cl, loc, S.slot[2], S.warp);
+        if (!(pq != 0.0) || !isfinite(pq)) {
+            status = MF_ERR_BREAKDOWN;
+            break;
+        }
+        const double alpha = rho / pq;
+        loc = mix_update<CHIP>(M, (float)alpha);
+        double rho_new = mix_sum(cl, loc, S.slot[3], S.warp);
+        it++;
+        bool checkpoint = learned && !lowp_off && it == 1;
+        if (sqrt(rho_new) <= a.delta * rmax || sqrt(rho_new) <= a.tol * nb) {
+            loc = mix_refine<L, CHIP>(a, V, M, S.rab, learned);
+            rho_new = mix_sum(cl, loc, S.slot[1], S.warp);
+            const double rt = sqrt(rho_new);
+            // the low-precision classes stop where the FP64 residual did
+            // not follow the recurrence (uniform: every CTA holds the same
+            // cluster sums)
+            if ((rule || learned) && !lowp_off && rt > 0.5 * rmax) {
+                lowp_off = true;
+                dirty = true;
+                for (int c = cl0 + tid; c < cl1; c += MNT) a.ccls[c] = (a.ccls_static[c] & 1) ? 1 : 0;
+            }
+            rmax = rt;
+            refs++;
+            checkpoint = learned && !lowp_off;
+        }
+        if (checkpoint) {
+            mix_checkpoint<CHIP>(a, V, M, cl0, cl1, (float)(sqrt(rho_new) / nb), refs, have_prev, s_w, s_feat, S.fslot,
+                                 S.fwarp);
+            have_prev = true;
+            dirty = true;
+        }
+        beta = rho_new / rho;
+        rho = rho_new;
+        relres = sqrt(rho) / nb;
+    }
+    if (status != MF_OK) {
+        const float *xlo = mix_xlo<CHIP>(M);
+        for (int i = ra + tid; i < rb; i += MNT) x[i] += (double)xlo[i - ra4];
+    }
+    if (st_pass) {
+        atomicAdd(&a.sysstat[3 * sys], st_bytes);
+        atomicAdd(&a.sysstat[3 * sys + 1], st_lowp);
+        atomicAdd(&a.sysstat[3 * sys + 2], st_pass);
+    }
+    if (rank == 0 && tid == 0) {
+        a.iters[sys] = it;
+        a.refs[sys] = refs;
+        a.status[sys] = status;
+        a.relres[sys] = relres;
+    }
+}
+
 // The mixed kernel (STATIC, RULE, LEARNED): one cluster per system, FP32
 // vectors.  The product q = A p runs over the sorted slices: every CTA holds
 // the window of p in shared memory, the slices are dealt to the cluster's
@@ -1171,252 +1525,49 @@ template <int L>
 __global__ void __launch_bounds__(MNT, 1) k_batched_cg(const __grid_constant__ BatchArgs a)
 {
     cg::cluster_group cl = cg::this_cluster();
-    __shared__ double s_warp[MNW];
-    __shared__ double s_slot[4][16];
-    __shared__ float s_fslot[2];
-    __shared__ float s_fwarp[2 * MNW];
-    __shared__ int s_sys;
-    __shared__ int s_rab[17];
-    extern __shared__ __align__(16) unsigned char b_smem_raw[];
-    float *s_win = reinterpret_cast<float *>(b_smem_raw);
-    float *s_w = reinterpret_cast<float *>(b_smem_raw + MixSmem::W);
-    float *s_feat = reinterpret_cast<float *>(b_smem_raw + MixSmem::FEAT);
-    const bool learned = a.policy == MF_POLICY_LEARNED && a.mlp_w;
-    const bool rule = a.policy == MF_POLICY_RULE;
-    if (learned)
+    __shared__ MixShared S;
+    if (a.policy == MF_POLICY_LEARNED && a.mlp_w) {
+        float *s_w = reinterpret_cast<float *>(mix_smem + MixSmem::W);
         for (int k = threadIdx.x; k < PN_NPARAM; k += MNT) s_w[k] = __bfloat162float(a.mlp_w[k]);
+    }
     __syncthreads();
-    const int rank = (int)cl.block_rank(), ncta = (int)cl.num_blocks();
-    const int tid = threadIdx.x;
-    const int wid = tid >> 5, wl = tid & 31;
+    const int rank = (int)cl.block_rank(), ncta = (int)cl.num_blocks(), tid = threadIdx.x;
     for (;;) {
-        if (rank == 0 && tid == 0) s_sys = atomicAdd(a.queue, 1);
+        if (rank == 0 && tid == 0) S.sys = atomicAdd(a.queue, 1);
         cl.sync();
-        const int qi = *cl.map_shared_rank(&s_sys, 0);
+        const int qi = *cl.map_shared_rank(&S.sys, 0);
         cl.sync();  // every CTA has read the index before rank 0 writes the next
         if (qi >= a.count) break;
         const int sys = a.order[qi];
         const SysView V = sys_view(a, sys);
-        const double *b = a.b + V.r0;
-        double *x = a.x + V.r0;
-        // this CTA's chunks and rows
+        // the CTAs' rows: whole chunks
         const int sc0 = a.sc[sys], nch = a.sc[sys + 1] - sc0;
-        const int cl0 = sc0 + (int)((long long)nch * rank / ncta), cl1 = sc0 + (int)((long long)nch * (rank + 1) / ncta);
-        if (tid <= ncta) s_rab[tid] = a.crow[sc0 + (int)((long long)nch * tid / ncta) + sys];
+        if (tid <= ncta) S.rab[tid] = a.crow[sc0 + (int)((long long)nch * tid / ncta) + sys];
         __syncthreads();
-        int most = 0;  // rows of the CTA with most
-        for (int k = 0; k < ncta; k++) most = max(most, s_rab[k + 1] - s_rab[k]);
-        most = (most + 3) & ~3;
-        const int nwin = sell_windows(V.n), n4 = (V.n + 3) & ~3;
+        int most = 0;
+        for (int k = 0; k < ncta; k++) most = max(most, S.rab[k + 1] - (S.rab[k] & ~3));
         MixSys M;
         M.sys = sys;
         M.n = V.n;
-        M.ra = s_rab[rank];
-        M.rb = s_rab[rank + 1];
+        M.ra = S.rab[rank];
+        M.rb = S.rab[rank + 1];
+        M.ra4 = M.ra & ~3;
         M.npan = V.npan;
-        M.chip = n4 + 3 * most <= SELL_WIN;
-        M.win = s_win;
-        M.rab = s_rab;
+        M.most = (most + 3) & ~3;
+        const int n4 = (V.n + 3) & ~3;
+        const bool chip = n4 + 3 * M.most <= SELL_WIN;
+        M.xwin = 2 * n4 + 2 * M.most <= SELL_WIN;
+        M.s0 = M.s1 = 0;
+        if (sell_windows(V.n) == 1) mix_share(a, a.sell.win0[sys], rank, ncta, M);
         // global vectors: every system starts on a 16-byte boundary
         const long long w0 = ((V.r0 + 4ll * sys) >> 2) << 2;
         M.pnew = (float *)a.p0 + w0;
         M.pold = (float *)a.p1 + w0;
-        if (M.chip) {
-            M.r = s_win + n4;
-            M.xlo = M.r + most;
-            M.q = M.xlo + most;
-        } else {
-            M.r = (float *)a.r + w0 + M.ra;
-            M.xlo = (float *)a.xlo + w0 + M.ra;
-            M.q = (float *)a.q + w0 + M.ra;
-        }
-        const int rows = M.rb - M.ra;
-        unsigned long long st_bytes = 0, st_lowp = 0, st_pass = 0;  // this thread's chunks
-        unsigned long long it_bytes = 0;                            // the same per iteration, by the current classes
-        unsigned it_lowp = 0, it_pass = 0;
-        double lb = 0.0, lr = 0.0;
-        for (int i = tid; i < rows; i += MNT) {
-            const double bv = b[M.ra + i];
-            const float rv = (float)bv;
-            x[M.ra + i] = 0.0;
-            M.r[i] = rv;
-            M.xlo[i] = 0.f;
-            M.pnew[M.ra + i] = 0.f;  // p before the first iteration
-            if (M.chip) s_win[M.ra + i] = 0.f;
-            lb += bv * bv;
-            lr += (double)rv * (double)rv;
-        }
-        for (int c = cl0 + tid; c < cl1; c += MNT) a.ccls[c] = (a.ccls_static[c] & 1) ? 1 : 0;
-        const double bb = mix_sum(cl, lb, s_slot[0], s_warp);
-        double rho = mix_sum(cl, lr, s_slot[1], s_warp);
-        const double nb = sqrt(bb) > 0.0 ? sqrt(bb) : 1.0;
-        double beta = 0.0, rmax = sqrt(rho), relres = sqrt(rho) / nb;
-        int it = 0, refs = 0, status = MF_OK, mode = 0;
-        bool lowp_off = false, have_prev = false, dirty = true;  // dirty: classes written since `mode` was found
-        while (true) {
-            if (sqrt(rho) <= a.tol * nb) break;
-            if (it >= a.maxiter) {
-                status = MF_ERR_NOT_CONVERGED;
-                break;
-            }
-            {
-                float *t = M.pold;
-                M.pold = M.pnew;
-                M.pnew = t;
-            }
-            const float bt = (float)beta;
-            // p = r + beta p over this CTA's rows, then a cluster barrier: the
-            // SpMV needs all of p.  RULE: one warp per chunk, deciding the
-            // chunk's class from its own rows' change.
-            auto put_p = [&](int i, float pv) {
-                if (M.chip) {
-                    s_win[M.ra + i] = pv;
-                    for (int k = 1; k < ncta; k++) {
-                        const int o = rank + k < ncta ? rank + k : rank + k - ncta;
-                        cl.map_shared_rank(s_win, o)[M.ra + i] = pv;
-                    }
-                    if (learned) M.pnew[M.ra + i] = pv;
-                } else {
-                    M.pnew[M.ra + i] = pv;
-                }
-            };
-            const float *po = M.chip ? s_win + M.ra : M.pold + M.ra;
-            if (rule && !lowp_off) {
-                for (int c = cl0 + wid; c < cl1; c += MNW) {
-                    const int i0 = a.crow[c + sys] - M.ra, i1 = a.crow[c + 1 + sys] - M.ra;
-                    double v = 0.0;
-                    for (int i = i0 + wl; i < i1; i += 32) {
-                        const float old = po[i], pv = fmaf(bt, old, M.r[i]);
-                        put_p(i, pv);
-                        v = fmax(v, fabs((double)pv - (double)old));
-                    }
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-                    if (wl == 0) a.ccls[c] = (unsigned char)rule_chunk_class(v, a.ccls_static[c]);
-                }
-                dirty = true;
-            } else {
-                // four rows per thread in flight: loads first, then the stores
-                int i = tid;
-                for (; i + 3 * MNT < rows; i += 4 * MNT) {
-                    float po4[4], r4[4];
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        po4[u] = po[i + u * MNT];
-                        r4[u] = M.r[i + u * MNT];
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; u++) put_p(i + u * MNT, fmaf(bt, po4[u], r4[u]));
-                }
-                for (; i < rows; i += MNT) put_p(i, fmaf(bt, po[i], M.r[i]));
-            }
-            cl.sync();
-            if (dirty) {
-                // the classes of the system's chunks: all FP16, all FP32 or both
-                bool c16 = true, c32 = true;
-                it_bytes = 0;
-                it_lowp = it_pass = 0;
-                for (int c = sc0 + tid; c < sc0 + nch; c += MNT) {
-                    const bool h = __ldcg(a.ccls + c) != 0;
-                    c16 &= h;
-                    c32 &= !h;
-                    if (c >= cl0 && c < cl1) {
-                        it_bytes += pass_bytes(a.cent[c + 1 + sys] - a.cent[c + sys],
-                                               a.crow[c + 1 + sys] - a.crow[c + sys], M.npan, h ? 2 : 4);
-                        it_lowp += h ? M.npan : 0;
-                        it_pass += M.npan;
-                    }
-                }
-                mode = __syncthreads_and(c16) ? 1 : __syncthreads_and(c32) ? 0 : 2;
-                dirty = false;
-            }
-            st_bytes += it_bytes;
-            st_lowp += it_lowp;
-            st_pass += it_pass;
-            double loc = mix_spmv(a, M, mode);
-            if (nwin > 1) {
-                cl.sync();
-                for (int i = tid; i < rows; i += MNT) loc += (double)M.pnew[M.ra + i] * (double)__ldcg(M.q + i);
-            }
-            const double pq = mix_sum(cl, loc, s_slot[2], s_warp);
-            if (!(pq != 0.0) || !isfinite(pq)) {
-                status = MF_ERR_BREAKDOWN;
-                break;
-            }
-            const double alpha = rho / pq;
-            loc = 0.0;
-            {
-                // four rows per thread in flight (loads first)
-                const float af = (float)alpha;
-                const float *pn = M.chip ? s_win + M.ra : M.pnew + M.ra;
-                int i = tid;
-                for (; i + 3 * MNT < rows; i += 4 * MNT) {
-                    float p4[4], q4[4], r4[4], x4[4];
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        p4[u] = pn[i + u * MNT];
-                        q4[u] = M.q[i + u * MNT];
-                        r4[u] = M.r[i + u * MNT];
-                        x4[u] = M.xlo[i + u * MNT];
-                    }
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        M.xlo[i + u * MNT] = fmaf(af, p4[u], x4[u]);
-                        const float ri = fmaf(-af, q4[u], r4[u]);
-                        M.r[i + u * MNT] = ri;
-                        loc += (double)ri * (double)ri;
-                    }
-                }
-                for (; i < rows; i += MNT) {
-                    M.xlo[i] = fmaf(af, pn[i], M.xlo[i]);
-                    const float ri = fmaf(-af, M.q[i], M.r[i]);
-                    M.r[i] = ri;
-                    loc += (double)ri * (double)ri;
-                }
-            }
-            double rho_new = mix_sum(cl, loc, s_slot[3], s_warp);
-            it++;
-            bool checkpoint = learned && !lowp_off && it == 1;
-            if (sqrt(rho_new) <= a.delta * rmax || sqrt(rho_new) <= a.tol * nb) {
-                loc = mix_refine<L>(a, V, M);
-                rho_new = mix_sum(cl, loc, s_slot[1], s_warp);
-                const double rt = sqrt(rho_new);
-                // the low-precision classes stop where the FP64 residual did
-                // not follow the recurrence (uniform: every CTA holds the same
-                // cluster sums)
-                if ((rule || learned) && !lowp_off && rt > 0.5 * rmax) {
-                    lowp_off = true;
-                    dirty = true;
-                    for (int c = cl0 + tid; c < cl1; c += MNT) a.ccls[c] = (a.ccls_static[c] & 1) ? 1 : 0;
-                }
-                rmax = rt;
-                refs++;
-                checkpoint = learned && !lowp_off;
-            }
-            if (checkpoint) {
-                mix_checkpoint(a, V, M, cl0, cl1, (float)(sqrt(rho_new) / nb), refs, have_prev, s_w, s_feat, s_fslot,
-                               s_fwarp);
-                have_prev = true;
-                dirty = true;
-            }
-            beta = rho_new / rho;
-            rho = rho_new;
-            relres = sqrt(rho) / nb;
-        }
-        if (status != MF_OK) {
-            for (int i = tid; i < rows; i += MNT) x[M.ra + i] += (double)M.xlo[i];
-        }
-        if (st_pass) {
-            atomicAdd(&a.sysstat[3 * sys], st_bytes);
-            atomicAdd(&a.sysstat[3 * sys + 1], st_lowp);
-            atomicAdd(&a.sysstat[3 * sys + 2], st_pass);
-        }
-        if (rank == 0 && tid == 0) {
-            a.iters[sys] = it;
-            a.refs[sys] = refs;
-            a.status[sys] = status;
-            a.relres[sys] = relres;
-        }
+        M.r = (float *)a.r + w0 + M.ra4;
+        M.xlo = (float *)a.xlo + w0 + M.ra4;
+        M.q = (float *)a.q + w0 + M.ra4;
+        if (chip) mix_solve<L, true>(a, S, V, M, sc0, nch);
+        else mix_solve<L, false>(a, S, V, M, sc0, nch);
         cl.sync();  // the cluster's last writes land before the next system
     }
 }
@@ -1512,26 +1663,35 @@ int batched_ctas(bool mixed, int lanes, int count, int cluster)
     return ctas;
 }
 
-// ctas: computed before any stream capture (batched_ctas)
+struct BatchConfig {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+};
+
+void batch_config(BatchConfig &c, const BatchKernel &k, int cluster, int ctas, cudaStream_t s)
+{
+    memset(&c, 0, sizeof(c));
+    c.attr[0].id = cudaLaunchAttributeClusterDimension;
+    c.attr[0].val.clusterDim.x = cluster;
+    c.attr[0].val.clusterDim.y = 1;
+    c.attr[0].val.clusterDim.z = 1;
+    c.cfg.blockDim = dim3(k.threads);
+    c.cfg.dynamicSmemBytes = k.smem;
+    c.cfg.stream = s;
+    c.cfg.attrs = c.attr;
+    c.cfg.numAttrs = 1;
+    c.cfg.gridDim = dim3(ctas);
+}
+
+// ctas: computed before any stream capture (batched_ctas); enough clusters to
+// fill the GPU (the work queue balances them)
 mf_status launch_batched(bool mixed, int lanes, const BatchArgs &a, int cluster, int ctas, cudaStream_t s)
 {
     const BatchKernel k = batch_kernel(mixed, lanes);
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = cluster;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.blockDim = dim3(k.threads);
-    cfg.dynamicSmemBytes = k.smem;
-    cfg.stream = s;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    // enough clusters to fill the GPU (the work queue balances them)
-    cfg.gridDim = dim3(ctas);
+    BatchConfig c;
+    batch_config(c, k, cluster, ctas, s);
     note_launch();
-    MF_CUDA(cudaLaunchKernelEx(&cfg, k.fn, a));
+    MF_CUDA(cudaLaunchKernelEx(&c.cfg, k.fn, a));
     return MF_OK;
 }
 
@@ -1758,11 +1918,9 @@ void parallel_for(int count, F f)
 cudaError_t batch_slices(mf_batch bt)
 {
     const int count = bt->count;
-    std::vector<int> win0(count);
     std::vector<long long> len0;
     long long lens = 0;
     for (int s = 0; s < count; s++) {
-        win0[s] = (int)len0.size();
         for (int k = 0; k < sell_windows(bt->n[s]); k++) {
             len0.push_back(lens);
             lens += bt->n[s];
@@ -1770,21 +1928,20 @@ cudaError_t batch_slices(mf_batch bt)
     }
     const int windows = (int)len0.size();
     cudaError_t e = cudaSuccess;
-    // temporaries: len0 | row lengths | slices per window | long rows
+    // temporaries: len0 | row lengths | slices per window | long rows | first slices
     char *tmp = nullptr;
     int *quads = nullptr, *quad0 = nullptr;
     const size_t o_len = sizeof(long long) * windows, o_ns = o_len + sizeof(int) * (size_t)lens,
-                 o_nl = o_ns + sizeof(int) * (windows + 1), bytes = o_nl + sizeof(int) * windows;
+                 o_nl = o_ns + sizeof(int) * (windows + 1), o_f = o_nl + sizeof(int) * windows,
+                 bytes = o_f + sizeof(int) * (windows + 1);
     int nslices = 0, nquads = 0;
     SellBuild B;
     memset(&B, 0, sizeof(B));
+    auto pad = [](size_t v) { return (v + 255) / 256 * 256; };
     do {
-        if ((e = cudaMalloc((void **)&tmp, bytes)) != cudaSuccess) break;
-        if ((e = cudaMalloc((void **)&bt->d_win0, sizeof(int) * count)) != cudaSuccess) break;
-        if ((e = cudaMalloc((void **)&bt->d_sfirst, sizeof(int) * (windows + 1))) != cudaSuccess) break;
-        if ((e = cudaMemcpy(bt->d_win0, win0.data(), sizeof(int) * count, cudaMemcpyHostToDevice)) != cudaSuccess) break;
+        if ((e = pool_malloc_async(&tmp, bytes, 0)) != cudaSuccess) break;
         if ((e = cudaMemcpy(tmp, len0.data(), sizeof(long long) * windows, cudaMemcpyHostToDevice)) != cudaSuccess) break;
-        int *len = (int *)(tmp + o_len), *ns = (int *)(tmp + o_ns), *nl = (int *)(tmp + o_nl);
+        int *len = (int *)(tmp + o_len), *ns = (int *)(tmp + o_ns), *nl = (int *)(tmp + o_nl), *first = (int *)(tmp + o_f);
         B.count = count;
         B.pw = PW;
         B.n = bt->d_n;
@@ -1806,40 +1963,45 @@ cudaError_t batch_slices(mf_batch bt)
         k_sell_lengths<<<dim3(gw, 16), SELL_NT>>>(B, windows, len);
         k_sell_slices<<<gw, SELL_NT>>>(B, windows, len, ns, nl);
         note_launch(2);
-        if ((e = cudaMemset(ns + windows, 0, sizeof(int))) != cudaSuccess) break;
-        if (exclusive_scan_i32(ns, bt->d_sfirst, windows + 1, 0, &nslices) != MF_OK) {
+        if ((e = cudaMemsetAsync(ns + windows, 0, sizeof(int), 0)) != cudaSuccess) break;
+        if (exclusive_scan_i32(ns, first, windows + 1, 0, &nslices) != MF_OK) {
             e = cudaErrorUnknown;
             break;
         }
-        if ((e = cudaMalloc((void **)&bt->d_sdesc, sizeof(int2) * ((size_t)nslices + 1))) != cudaSuccess) break;
-        if ((e = cudaMalloc((void **)&bt->d_srec, sizeof(int4) * 32 * ((size_t)nslices + 1))) != cudaSuccess) break;
-        if ((e = cudaMalloc((void **)&quads, sizeof(int) * 2 * ((size_t)nslices + 1))) != cudaSuccess) break;
+        // bins | descriptors | records
+        const size_t o_desc = pad(sizeof(int) * (size_t)windows * (SELL_BINS + 1)),
+                     o_rec = o_desc + pad(sizeof(int2) * ((size_t)nslices + 1)),
+                     s_bytes = o_rec + sizeof(int4) * 32 * ((size_t)nslices + 2);
+        if ((e = cudaMalloc(&bt->slices, s_bytes)) != cudaSuccess) break;
+        bt->d_sfirst = (int *)bt->slices;
+        bt->d_sdesc = (int2 *)((char *)bt->slices + o_desc);
+        bt->d_srec = (int4 *)((char *)bt->slices + o_rec);
+        if ((e = pool_malloc_async(&quads, sizeof(int) * 2 * ((size_t)nslices + 1), 0)) != cudaSuccess) break;
         quad0 = quads + nslices + 1;
-        k_sell_sort<<<std::min(windows, 148 * 32), 32>>>(B, windows, len, nl, bt->d_sfirst, bt->d_srec, quads);
-        note_launch();
-        if ((e = cudaMemset(quads + nslices, 0, sizeof(int))) != cudaSuccess) break;
-        if (exclusive_scan_i32(quads, quad0, nslices + 1, 0, &nquads) != MF_OK) {
+        k_sell_sort<<<std::min(windows, 148 * 32), 32>>>(B, windows, len, nl, first, bt->d_srec, quads, bt->d_sfirst);
+        k_sell_counts<<<std::min(nslices / SELL_NT + 1, 1184), SELL_NT>>>(nslices, quads, quad0);
+        note_launch(2);
+        if (exclusive_scan_i32(quad0, quad0, nslices + 1, 0, &nquads) != MF_OK) {
             e = cudaErrorUnknown;
             break;
         }
-        const size_t words = (size_t)(nquads > 0 ? nquads : 1) * 128;
-        if ((e = cudaMalloc((void **)&bt->d_scv, 4 * words)) != cudaSuccess) break;
-        if ((e = cudaMalloc((void **)&bt->d_sv32, 4 * words)) != cudaSuccess) break;
-        if ((e = cudaMalloc((void **)&bt->d_sc16, 2 * words)) != cudaSuccess) break;
-        if ((e = cudaMalloc((void **)&bt->d_sv64, 8 * words)) != cudaSuccess) break;
-        if ((e = cudaMemset(bt->d_scv, 0, 4 * words)) != cudaSuccess) break;
-        if ((e = cudaMemset(bt->d_sv32, 0, 4 * words)) != cudaSuccess) break;
-        if ((e = cudaMemset(bt->d_sc16, 0, 2 * words)) != cudaSuccess) break;
-        if ((e = cudaMemset(bt->d_sv64, 0, 8 * words)) != cudaSuccess) break;
-        k_sell_fill<<<std::min((nslices + SELL_FNT / 32 - 1) / (SELL_FNT / 32), 148 * 64), SELL_FNT>>>(B, windows, bt->d_sfirst, nl, bt->d_srec, quads,
-                                                                        quad0, nslices, bt->d_sdesc, bt->d_scv,
-                                                                        bt->d_sv32, bt->d_sc16, bt->d_sv64);
+        // FP64 values | FP32 values | FP16 words | columns
+        const size_t words = ((size_t)nquads + 1) * 128;
+        if ((e = cudaMalloc(&bt->words, 18 * words)) != cudaSuccess) break;
+        bt->d_sv64 = (double *)bt->words;
+        bt->d_sv32 = (float *)(bt->d_sv64 + words);
+        bt->d_scv = (uint32_t *)(bt->d_sv32 + words);
+        bt->d_sc16 = (uint16_t *)(bt->d_scv + words);
+        if ((e = cudaMemsetAsync(bt->words, 0, 18 * words, 0)) != cudaSuccess) break;
+        k_sell_fill<<<std::min((nslices + SELL_FNT / 32 - 1) / (SELL_FNT / 32), 148 * 64), SELL_FNT>>>(
+            B, windows, first, bt->d_srec, quads, quad0, nslices, bt->d_sdesc, bt->d_scv, bt->d_sv32, bt->d_sc16,
+            bt->d_sv64);
         note_launch();
-        if ((e = cudaGetLastError()) != cudaSuccess) break;
-        e = cudaDeviceSynchronize();
+        e = cudaGetLastError();
     } while (false);
-    if (tmp) cudaFree(tmp);
-    if (quads) cudaFree(quads);
+    if (tmp) cudaFreeAsync(tmp, 0);
+    if (quads) cudaFreeAsync(quads, 0);
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
     return e;
 }
 
@@ -1928,41 +2090,56 @@ mf_status mf_batch_create(int count, const int *n, const int *const *rowptr, con
     float4 *rowstat = nullptr;
     unsigned char *rowflag = nullptr;
     cudaError_t e = cudaSuccess;
-#define BT_ALLOC(p, bytes) \
-    if (e == cudaSuccess) e = cudaMalloc((void **)&(p), (bytes))
-    BT_ALLOC(bt->d_order, sizeof(int) * count);
-    BT_ALLOC(bt->d_n, sizeof(int) * count);
-    BT_ALLOC(bt->d_pan0, sizeof(int) * count);
-    BT_ALLOC(bt->d_npan, sizeof(int) * count);
-    BT_ALLOC(bt->d_row0, sizeof(long long) * count);
-    BT_ALLOC(bt->d_prow0, sizeof(long long) * (panels + 1));
-    BT_ALLOC(bt->d_pent0, sizeof(long long) * (panels + 1));
-    BT_ALLOC(bt->d_prow, sizeof(int) * (prows + 8));  // slack: 16-byte bulk-copy rounding
-    BT_ALLOC(bt->d_sc, sizeof(int) * (count + 1));
-    BT_ALLOC(bt->d_crow, sizeof(int) * crow.size());
-    BT_ALLOC(bt->d_cent, sizeof(int) * cent.size());
-    BT_ALLOC(bt->d_col, sizeof(uint16_t) * (nz + 16));
-    BT_ALLOC(bt->d_val, sizeof(double) * (nz + 2));
-    BT_ALLOC(bt->d_val16, sizeof(__half) * (nz + 16));
-    BT_ALLOC(bt->d_rscale, sizeof(float) * (rows + 4));
-    BT_ALLOC(bt->d_diag32, sizeof(float) * (rows + 4));
-    BT_ALLOC(bt->d_diag64, sizeof(double) * (rows + 4));
-    BT_ALLOC(bt->d_ccls, (size_t)nch + 16);
-    BT_ALLOC(bt->d_ccls_static, (size_t)nch + 16);
-    BT_ALLOC(bt->d_cstat, sizeof(float) * NCSTAT * ((size_t)nch + 1));
-    BT_ALLOC(bt->d_cdyn, sizeof(float) * NCDYN * ((size_t)nch + 1));
-    BT_ALLOC(bt->d_iters, sizeof(int) * count);
-    BT_ALLOC(bt->d_refs, sizeof(int) * count);
-    BT_ALLOC(bt->d_status, sizeof(int) * count);
-    BT_ALLOC(bt->d_relres, sizeof(double) * count * 2);
-    BT_ALLOC(bt->d_sysstat, sizeof(unsigned long long) * 3 * count);
-    BT_ALLOC(bt->d_queue, sizeof(int) * 4);
-    BT_ALLOC(rowstat, sizeof(float4) * (rows + 1));
-    BT_ALLOC(rowflag, (size_t)rows + 16);
-#undef BT_ALLOC
+    // one allocation for all of them, every array on a 256-byte boundary (the
+    // first pass adds up the sizes, the second hands out the addresses)
+    auto arrays = [&](auto take) {
+        take(bt->d_order, sizeof(int) * count);
+        take(bt->d_win0, sizeof(int) * count);
+        take(bt->d_n, sizeof(int) * count);
+        take(bt->d_pan0, sizeof(int) * count);
+        take(bt->d_npan, sizeof(int) * count);
+        take(bt->d_row0, sizeof(long long) * count);
+        take(bt->d_prow0, sizeof(long long) * (panels + 1));
+        take(bt->d_pent0, sizeof(long long) * (panels + 1));
+        take(bt->d_prow, sizeof(int) * (prows + 8));
+        take(bt->d_sc, sizeof(int) * (count + 1));
+        take(bt->d_crow, sizeof(int) * crow.size());
+        take(bt->d_cent, sizeof(int) * cent.size());
+        take(bt->d_col, sizeof(uint16_t) * (nz + 16));
+        take(bt->d_val, sizeof(double) * (nz + 2));
+        take(bt->d_val16, sizeof(__half) * (nz + 16));
+        take(bt->d_rscale, sizeof(float) * (rows + 4));
+        take(bt->d_diag32, sizeof(float) * (rows + 4));
+        take(bt->d_diag64, sizeof(double) * (rows + 4));
+        take(bt->d_ccls, (size_t)nch + 16);
+        take(bt->d_ccls_static, (size_t)nch + 16);
+        take(bt->d_cstat, sizeof(float) * NCSTAT * ((size_t)nch + 1));
+        take(bt->d_cdyn, sizeof(float) * NCDYN * ((size_t)nch + 1));
+        take(bt->d_iters, sizeof(int) * count);
+        take(bt->d_refs, sizeof(int) * count);
+        take(bt->d_status, sizeof(int) * count);
+        take(bt->d_relres, sizeof(double) * count * 2);
+        take(bt->d_sysstat, sizeof(unsigned long long) * 3 * count);
+        take(bt->d_queue, sizeof(int) * 4);
+    };
+    size_t arena = 0;
+    arrays([&](auto &, size_t bytes) { arena += (bytes + 255) / 256 * 256; });
+    e = cudaMalloc(&bt->arena, arena);
+    if (e == cudaSuccess) e = pool_malloc_async(&rowstat, sizeof(float4) * ((size_t)rows + 1), 0);
+    if (e == cudaSuccess) e = pool_malloc_async(&rowflag, (size_t)rows + 16, 0);
+    if (e == cudaSuccess) {
+        char *at = (char *)bt->arena;
+        arrays([&](auto &p, size_t bytes) {
+            p = (std::remove_reference_t<decltype(p)>)at;
+            at += (bytes + 255) / 256 * 256;
+        });
+    }
 #define BT_COPY(dst, src, bytes) \
     if (e == cudaSuccess && (bytes) > 0) e = cudaMemcpy((dst), (src), (bytes), cudaMemcpyHostToDevice)
+    std::vector<int> win0(count);
+    for (int s = 1; s < count; s++) win0[s] = win0[s - 1] + sell_windows(n[s - 1]);
     BT_COPY(bt->d_order, order.data(), sizeof(int) * count);
+    BT_COPY(bt->d_win0, win0.data(), sizeof(int) * count);
     BT_COPY(bt->d_n, n, sizeof(int) * count);
     BT_COPY(bt->d_pan0, pan0.data(), sizeof(int) * count);
     BT_COPY(bt->d_npan, npan.data(), sizeof(int) * count);
@@ -2005,7 +2182,6 @@ mf_status mf_batch_create(int count, const int *n, const int *const *rowptr, con
             e = cudaGetLastError();
         }
     }
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
     if (e == cudaSuccess) e = batch_slices(bt);
     if (e == cudaSuccess) {
         std::vector<unsigned char> st((size_t)nch);
@@ -2015,8 +2191,8 @@ mf_status mf_batch_create(int count, const int *n, const int *const *rowptr, con
             bt->fp16_allowed_chunks += (v >> 1) & 1;
         }
     }
-    if (rowstat) cudaFree(rowstat);
-    if (rowflag) cudaFree(rowflag);
+    if (rowstat) cudaFreeAsync(rowstat, 0);
+    if (rowflag) cudaFreeAsync(rowflag, 0);
     if (e != cudaSuccess) return fail(e);
     *out = bt;
     return MF_OK;
@@ -2026,13 +2202,7 @@ mf_status mf_batch_destroy(mf_batch bt)
 {
     if (!bt) return MF_OK;
     if (bt->graph) cudaGraphExecDestroy(bt->graph);
-    void *bufs[] = {bt->d_order,  bt->d_n,      bt->d_pan0,   bt->d_npan,   bt->d_row0,   bt->d_prow0,
-                    bt->d_pent0,  bt->d_prow,   bt->d_col,    bt->d_val,    bt->d_val16,  bt->d_sfirst,
-                    bt->d_rscale, bt->d_diag32, bt->d_iters,  bt->d_refs,   bt->d_status, bt->d_relres,
-                    bt->d_win0,   bt->d_sdesc,  bt->d_srec,   bt->d_scv,    bt->d_sv32,   bt->d_sc16,
-                    bt->d_sv64,   bt->d_diag64,
-                    bt->work,     bt->d_queue,  bt->d_sc,     bt->d_crow,   bt->d_cent,   bt->d_ccls,
-                    bt->d_ccls_static, bt->d_cstat, bt->d_cdyn, bt->d_sysstat};
+    void *bufs[] = {bt->arena, bt->slices, bt->words, bt->work};
     for (void *p : bufs)
         if (p) cudaFree(p);
     delete bt;
@@ -2167,10 +2337,38 @@ static mf_status batch_check_opts(mf_batch bt, const mf_solve_opts &o)
     return MF_OK;
 }
 
-static void batch_schedule(mf_batch bt, int &lanes, int &cluster)
+// CTAs per system of a mixed solve that nobody tuned: 2 where the systems
+// fill the device, else the most (up to 16) at which every system still has a
+// resident cluster and the largest at least 512 rows per CTA.  Measured (us
+// per iteration): 24 systems of 1,000-4,000 rows 17.2 with 2 CTAs, 15.1 with
+// 4, 15.1 with 8; 256 systems of 1,000-32,000 rows (1.7 waves of 2-CTA
+// clusters) 322 ms a solve with 2, 362 with 4.
+static int batch_auto_cluster(mf_batch bt, int lanes)
+{
+    if (bt->auto_cluster) return bt->auto_cluster;
+    const BatchKernel k = batch_kernel(true, lanes);
+    const int nmax = *std::max_element(bt->n.begin(), bt->n.end());
+    int best = 2;
+    for (int c = 4; c <= 16 && c * 512 <= nmax; c *= 2) {
+        batched_ctas(true, lanes, bt->count, c);  // the kernel's attributes
+        BatchConfig cfg;
+        batch_config(cfg, k, c, c * bt->count, nullptr);
+        int fit = 0;
+        if (cudaOccupancyMaxActiveClusters(&fit, k.fn, &cfg.cfg) != cudaSuccess) {
+            cudaGetLastError();
+            break;
+        }
+        if (fit < bt->count) break;
+        best = c;
+    }
+    bt->auto_cluster = best;
+    return best;
+}
+
+static void batch_schedule(mf_batch bt, bool mixed, int &lanes, int &cluster)
 {
     lanes = bt->tuned_lanes ? bt->tuned_lanes : 4;
-    cluster = bt->tuned_cluster ? bt->tuned_cluster : 2;
+    cluster = bt->tuned_cluster ? bt->tuned_cluster : mixed ? batch_auto_cluster(bt, lanes) : 2;
     if (const char *e = getenv("MF_BATCH_LANES")) lanes = atoi(e);
     if (const char *e = getenv("MF_BATCH_CLUSTER")) cluster = atoi(e);
     if (lanes != 4 && lanes != 8 && lanes != 16 && lanes != 32) lanes = 4;
@@ -2187,8 +2385,8 @@ mf_status mf_batch_cg_solve(mf_batch bt, const double *b, double *x, const mf_so
     MF_TRY(batch_check_opts(bt, o));
     cudaStream_t s = (cudaStream_t)stream;
     int lanes, cluster;
-    batch_schedule(bt, lanes, cluster);
     const bool mixed = o.policy != MF_POLICY_FP64;
+    batch_schedule(bt, mixed, lanes, cluster);
     MF_TRY(batch_work(bt));
     const int ctas = batch_ctas(bt, mixed, lanes, cluster);
     const BatchArgs a = batch_args(bt, b, x, o);
