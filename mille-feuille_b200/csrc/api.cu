@@ -171,7 +171,7 @@ mf_status mf_matrix_destroy(mf_matrix m)
                     m->d_val_low, m->d_col, m->d_ptr, m->d_cidx, m->d_f16, m->d_i8, m->d_class, m->d_f16ok,
                     m->d_nonzero_row_new, m->d_tile_rowidx, m->d_block_signal, m->d_blockrowid_new, m->d_blockcsr_ptr_new, m->d_rbb_rowidx,
                     m->d_rbb_colstart, m->d_rbb_colstop, m->d_part, m->d_cta_chunk, m->d_chunks, m->work, m->host_io,
-                    m->d_wcls, m->d_poff, m->d_pay, m->d_resid, m->d_pol, m->d_sslot, m->d_smeta, m->d_sval,
+                    m->d_wcls, m->d_poff, m->d_pay, m->d_resid, m->d_pol, m->d_sslot, m->d_smeta, m->d_sval, m->d_soff,
                     m->d_shdr, m->d_spay, m->d_scta_chunk, m->d_schunks, m->d_spos, m->d_sdesc, m->mr_work,
                     m->mr_io, m->d_tc_index, m->d_tc_dense};
     for (void *p : bufs)
@@ -296,7 +296,7 @@ mf_status mf_encode_column_index(mf_matrix m, void *stream)
 mf_status mf_spmv(mf_matrix m, const double *x, double *y, void *stream)
 {
     if (!m || (m->v.rows > 0 && (!x || !y))) return MF_ERR_INVALID_ARG;
-    return spmv_fp64(m->v, x, y, (cudaStream_t)stream);
+    return spmv(m, x, y, (cudaStream_t)stream);
 }
 
 void mf_solve_opts_default(mf_solve_opts *o)

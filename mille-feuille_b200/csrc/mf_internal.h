@@ -1,8 +1,10 @@
 // mf_internal.h -- internal (C++) view of the device-resident tiled matrix.
 #pragma once
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
+#include <mutex>
 
 #include "mf.h"
 #include "mf_common.cuh"
@@ -73,11 +75,15 @@ struct mf_matrix_s {
     int pol_static_ready = 0, pol_have_prev = 0;
     float pol_prev_relres = 0.f;
     // row-slot execution layout of the persistent solvers (slots.cu)
-    int slots_state = 0;       // 0 not built, 1 built, -1 not describable
+    std::mutex slots_mu;           // held while they are built
+    std::atomic<int> slots_state{0};  // 0 not built, 1 built, -1 not describable
+    std::atomic<int> spmv_calls{0};   // products from the tiles so far (mf_spmv)
     long long nslots = 0;
     int *d_sslot = nullptr;
     uint16_t *d_smeta = nullptr;
     double *d_sval = nullptr;
+    void *d_soff = nullptr;    // column - row of every slot entry, int16 or int32
+    int soff_bytes = 0;        // 2 or 4
     unsigned *d_shdr = nullptr;
     unsigned char *d_spay = nullptr;
     int slot_policy = -1;      // policy whose classes the slot payload holds
@@ -119,6 +125,7 @@ mf_status build_tiles(mf_matrix m, int rowA, int colA, const int *d_rowptr, cons
 mf_status strip_partition(mf_matrix m, int ctas, cudaStream_t s);
 // spmv.cu
 mf_status spmv_fp64(const MfTiles &A, const double *x, double *y, cudaStream_t s);
+mf_status spmv(mf_matrix m, const double *x, double *y, cudaStream_t s);
 mf_status spmv_fp64_cidx(const MfTiles &A, const unsigned char *cidx, const double *x, double *y, cudaStream_t s);
 // residual.cu: per-strip partials (2 doubles per strip) then a fixed-order sum
 mf_status residual_norm(const MfTiles &A, const double *b, const double *x, double *part, double *out,

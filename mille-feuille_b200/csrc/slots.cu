@@ -11,6 +11,11 @@
 //   * per entry a 16-bit word (tile index within the strip << 4 | in-tile
 //     column; 0xFFFF = empty) and the FP64 value; the column is
 //     tile_columnidx[tile_ptr[strip] + tile] * 16 + in-tile column;
+//   * beside that word the distance column - row (SpMV and SpMM: the column
+//     without a look at the strip's tile columns), 16 bits where every entry
+//     lies within 32,767 columns of the diagonal, else 32; the lowest value of
+//     the type marks an empty entry.  Two entries of a row are of one tile
+//     when their columns / 16 agree;
 //   * a row's entries keep the reference's order (tiles in column order,
 //     entries in tile order), and the tile index tells where a tile's
 //     partial sum ends, so the FP64 row sums round exactly as blockspmv_cpu
@@ -50,8 +55,9 @@ __device__ __forceinline__ void row_bounds(const MfTiles &A, int t, int r, int r
     hi = (r == rowlen - 1) ? nz : (int)A.ptr[po + r + 1];
 }
 
-// K of every strip (half-warp per strip); flags strips with too many tiles.
-__global__ void k_slot_count(MfTiles A, int *__restrict__ K, int *__restrict__ too_many)
+// K of every strip (half-warp per strip); flags strips with too many tiles;
+// the most tile columns a strip's tiles lie from its own (16-bit distances).
+__global__ void k_slot_count(MfTiles A, int *__restrict__ K, int *__restrict__ too_many, int *__restrict__ far)
 {
     const int hl = threadIdx.x & 15;
     for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 4; s <= A.tilem; s += (gridDim.x * blockDim.x) >> 4) {
@@ -66,18 +72,22 @@ __global__ void k_slot_count(MfTiles A, int *__restrict__ K, int *__restrict__ t
             for (int t = t0; t < t1; t++) {
                 int lo, hi;
                 row_bounds(A, t, hl, rowlen, A.tile_nnz[t + 1] - A.tile_nnz[t], lo, hi);
-                cnt += hi - lo;
+                cnt += max(hi - lo, 0);  // a tile of 256 entries wraps its last pointers to 0
             }
         for (int o = 8; o > 0; o >>= 1) cnt = max(cnt, __shfl_xor_sync(0xFFFFu << (threadIdx.x & 16), cnt, o, 16));
         if (hl == 0) {
+            // tiles ascend by column: the first and the last lie farthest
+            const int d = t1 > t0 ? max(s - A.tile_columnidx[t0], A.tile_columnidx[t1 - 1] - s) : 0;
+            if (d > *(volatile int *)far) atomicMax(far, d);
             K[s] = cnt;
             if (t1 - t0 > SLOT_MAX_TILES) atomicExch(too_many, 1);
         }
     }
 }
 
+template <typename OT>
 __global__ void k_slot_fill(MfTiles A, const int *__restrict__ sslot, uint16_t *__restrict__ meta,
-                            double *__restrict__ val)
+                            double *__restrict__ val, OT *__restrict__ dist)
 {
     const int hl = threadIdx.x & 15;
     for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 4; s < A.tilem; s += (gridDim.x * blockDim.x) >> 4) {
@@ -94,11 +104,14 @@ __global__ void k_slot_fill(MfTiles A, const int *__restrict__ sslot, uint16_t *
                 for (int q = lo; q < hi; q++, k++) {
                     meta[base + (size_t)k * MF_TILE] = (uint16_t)(((t - t0) << 4) | A.col[off + q]);
                     val[base + (size_t)k * MF_TILE] = A.val[off + q];
+                    dist[base + (size_t)k * MF_TILE] =
+                        (OT)(A.tile_columnidx[t] * MF_TILE + (int)A.col[off + q] - (s * MF_TILE + hl));
                 }
             }
         for (; k < K; k++) {
             meta[base + (size_t)k * MF_TILE] = 0xFFFFu;
             val[base + (size_t)k * MF_TILE] = 0.0;
+            dist[base + (size_t)k * MF_TILE] = (OT)(sizeof(OT) == 2 ? INT16_MIN : INT32_MIN);
         }
     }
 }
@@ -460,39 +473,72 @@ mf_status build_slot_chunks(mf_matrix m, int G, bool staged, cudaStream_t s)
     return MF_OK;
 }
 
-mf_status build_slots(mf_matrix m, cudaStream_t s)
+// Builds the slots once (any thread; they do not change afterwards, and the
+// stream is waited for, so every stream may read them).  most > 0: not built
+// when they would hold more entries than that.
+mf_status build_slots(mf_matrix m, cudaStream_t s, long long most)
 {
-    if (m->slots_state != 0) return MF_OK;
+    if (m->slots_state.load(std::memory_order_acquire) != 0) return MF_OK;
+    std::lock_guard<std::mutex> lk(m->slots_mu);
+    if (m->slots_state.load(std::memory_order_relaxed) != 0) return MF_OK;
     const MfTiles &A = m->v;
     const int tilem = A.tilem;
     int *d_K = nullptr, *d_flag = nullptr;
-    MF_CUDA(cudaMalloc(&m->d_sslot, sizeof(int) * (tilem + 1) + 32));  // slack: 16-byte bulk-copy rounding
-    MF_CUDA(pool_malloc_async(&d_K, sizeof(int) * (tilem + 1) + sizeof(int), s));
+    // one temporary: slots per strip, flag and farthest tile, their scan
+    MF_CUDA(pool_malloc_async(&d_K, sizeof(int) * 2 * ((size_t)tilem + 2), s));
     d_flag = d_K + tilem + 1;
-    MF_CUDA(cudaMemsetAsync(d_flag, 0, sizeof(int), s));
-    k_slot_count<<<grid_for3((long long)(tilem + 1) * 16, 256), 256, 0, s>>>(A, d_K, d_flag);
+    int *d_at = d_flag + 2;
+    MF_CUDA(cudaMemsetAsync(d_flag, 0, 2 * sizeof(int), s));
+    k_slot_count<<<grid_for3((long long)(tilem + 1) * 16, 256), 256, 0, s>>>(A, d_K, d_flag, d_flag + 1);
     note_launch();
     MF_CUDA(cudaGetLastError());
-    int total = 0, flag = 0;
-    MF_TRY(exclusive_scan_i32(d_K, m->d_sslot, tilem + 1, s, &total));
-    MF_CUDA(cudaMemcpyAsync(&flag, d_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
+    int total = 0, h_flag[2] = {0, 0};
+    MF_TRY(exclusive_scan_i32(d_K, d_at, tilem + 1, s, &total));
+    MF_CUDA(cudaMemcpyAsync(h_flag, d_flag, sizeof(h_flag), cudaMemcpyDeviceToHost, s));
     MF_CUDA(cudaStreamSynchronize(s));
-    cudaFreeAsync(d_K, s);
-    if (flag || total < 0 || (long long)total * MF_TILE > (1ll << 40)) {
-        m->slots_state = -1;  // chunked tile path
+    const size_t E = (size_t)total * MF_TILE;
+    // tiles within 2,046 tile columns of the strip: every entry within 32,751 columns
+    const int ob = h_flag[1] <= 2046 ? 2 : 4;
+    if (h_flag[0] || total < 0 || (long long)E > (1ll << 40)) {
+        cudaFreeAsync(d_K, s);
+        m->slots_state.store(-1, std::memory_order_release);  // chunked tile path
         return MF_OK;
     }
-    m->nslots = total;
-    const size_t E = (size_t)total * MF_TILE;
-    MF_CUDA(cudaMalloc(&m->d_smeta, sizeof(uint16_t) * E + 32));
-    MF_CUDA(cudaMalloc(&m->d_sval, sizeof(double) * E + 32));
+    if (most > 0 && (long long)E > most) {
+        cudaFreeAsync(d_K, s);
+        return MF_OK;
+    }
+    // slack: 16-byte bulk-copy rounding
+    if (cudaMalloc(&m->d_sslot, sizeof(int) * (tilem + 1) + 32) != cudaSuccess ||
+        cudaMalloc(&m->d_smeta, sizeof(uint16_t) * E + 32) != cudaSuccess ||
+        cudaMalloc(&m->d_sval, sizeof(double) * E + 32) != cudaSuccess ||
+        cudaMalloc(&m->d_soff, ob * E + 32) != cudaSuccess) {
+        cudaGetLastError();
+        if (m->d_sslot) cudaFree(m->d_sslot);
+        if (m->d_smeta) cudaFree(m->d_smeta);
+        if (m->d_sval) cudaFree(m->d_sval);
+        m->d_sslot = nullptr;
+        m->d_smeta = nullptr;
+        m->d_sval = nullptr;
+        m->d_soff = nullptr;
+        cudaFreeAsync(d_K, s);
+        set_last_error("no device memory for the row slots (%zu entries)", E);
+        return MF_ERR_NO_MEMORY;
+    }
+    MF_CUDA(cudaMemcpyAsync(m->d_sslot, d_at, sizeof(int) * (tilem + 1), cudaMemcpyDeviceToDevice, s));
+    cudaFreeAsync(d_K, s);
     if (tilem > 0) {
-        k_slot_fill<<<grid_for3((long long)tilem * 16, 256), 256, 0, s>>>(A, m->d_sslot, m->d_smeta, m->d_sval);
+        const int grid = grid_for3((long long)tilem * 16, 256);
+        if (ob == 2) k_slot_fill<<<grid, 256, 0, s>>>(A, m->d_sslot, m->d_smeta, m->d_sval, (int16_t *)m->d_soff);
+        else k_slot_fill<<<grid, 256, 0, s>>>(A, m->d_sslot, m->d_smeta, m->d_sval, (int32_t *)m->d_soff);
         note_launch();
         MF_CUDA(cudaGetLastError());
     }
-    m->slots_state = 1;
+    MF_CUDA(cudaStreamSynchronize(s));
+    m->nslots = total;
+    m->soff_bytes = ob;
     m->slot_policy = -1;
+    m->slots_state.store(1, std::memory_order_release);
     return MF_OK;
 }
 

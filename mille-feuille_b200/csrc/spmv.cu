@@ -2,12 +2,20 @@
 // stir_spmv_cuda_kernel_newcsr, src/Mille-feuille-cg.h:97-166, and of
 // blockspmv_cpu, src/blockspmv_cpu.h:2-112).  Thread per row; no atomics;
 // bit-identical to blockspmv_cpu.
+//
+// A handle's first product runs from the tiles; from the second on it runs
+// from the row slots (slots.cu), built then: a strip's slots are read
+// coalesced and a row's entries load eight at a time, where the tiles cost
+// two X#include <climits>
+
+#include "solver.h"
 #include "spmv_core.cuh"
 
 namespace mf {
 namespace {
 
 constexpr int SPMV_NT = 256;
+constexpr int SPMV_MINB = 5;  // 48 registers, 40 warps per SM: 34.8 us (4: 38.9, 6: 35.2; 128^3 Poisson)
 
 __global__ void __launch_bounds__(SPMV_NT) k_spmv_fp64(MfTiles A, const double *__restrict__ x, double *__restrict__ y)
 {
@@ -17,6 +25,67 @@ __global__ void __launch_bounds__(SPMV_NT) k_spmv_fp64(MfTiles A, const double *
         const int rowlen = (bi == A.tilem - 1) ? A.rows - bi * MF_TILE : MF_TILE;
         if (r < rowlen) y[bi * MF_TILE + r] = row_fp64(A, bi, r, rowlen, x);
     }
+}
+
+// The next N entries of a row from the row slots: their columns and values,
+// then their elements of x are in flight together; then the sums in
+// blockspmv_cpu's order (a partial sum per tile, added when the tile column
+// changes).  An empty entry (always after the row's others) adds a zero
+// product: no sum here is ever -0.0, so that changes no bit.
+template <int N, typename OT>
+__device__ __forceinline__ void slot_sums(const OT *__restrict__ d0, const double *__restrict__ v0,
+                                          const double *__restrict__ xi, int lane, int &prev, double &yd, double &part)
+{
+    constexpr OT EMPTY = (OT)(sizeof(OT) == 2 ? INT16_MIN : INT32_MIN);
+    int d[N];
+    double v[N], xv[N];
+#pragma unroll
+    for (int u = 0; u < N; u++) {
+        d[u] = (int)__ldcs(d0 + u * MF_TILE);
+        v[u] = __ldcs(v0 + u * MF_TILE);
+    }
+#pragma unroll
+    for (int u = 0; u < N; u++) xv[u] = d[u] != (int)EMPTY ? xi[d[u]] : 0.0;
+#pragma unroll
+    for (int u = 0; u < N; u++) {
+        const int t = (d[u] + lane) >> 4;  // tile column, counted from the strip's own
+        if (t != (u == 0 ? prev : (d[u - 1] + lane) >> 4)) {
+            yd = __dadd_rn(yd, part);
+            part = 0.0;
+        }
+        part = __dadd_rn(part, __dmul_rn(xv[u], v[u]));
+    }
+    prev = (d[N - 1] + lane) >> 4;
+}
+
+// Thread per row over the row slots (slot k of a strip: the k-th entry of its
+// 16 rows).
+template <typename OT>
+__global__ void __launch_bounds__(SPMV_NT, SPMV_MINB) k_spmv_slots(int rows, const int *__restrict__ sslot,
+                                                           const OT *__restrict__ soff, const double *__restrict__ sval,
+                                                           const double *__restrict__ x, double *__restrict__ y)
+{
+    const int i = blockIdx.x * SPMV_NT + threadIdx.x, s = i >> 4, lane = i & 15;
+    if (i >= rows) return;
+    const int k0 = sslot[s];
+    int K = sslot[s + 1] - k0;
+    const OT *d = soff + (size_t)k0 * MF_TILE + lane;
+    const double *v = sval + (size_t)k0 * MF_TILE + lane, *xi = x + i;
+    double yd = 0.0, part = 0.0;
+    int prev = INT_MIN;
+    for (; K > 8; K -= 8, d += 8 * MF_TILE, v += 8 * MF_TILE) slot_sums<8>(d, v, xi, lane, prev, yd, part);
+    switch (K) {  // straight code for every remainder: no load is predicated
+    case 8: slot_sums<8>(d, v, xi, lane, prev, yd, part); break;
+    case 7: slot_sums<7>(d, v, xi, lane, prev, yd, part); break;
+    case 6: slot_sums<6>(d, v, xi, lane, prev, yd, part); break;
+    case 5: slot_sums<5>(d, v, xi, lane, prev, yd, part); break;
+    case 4: slot_sums<4>(d, v, xi, lane, prev, yd, part); break;
+    case 3: slot_sums<3>(d, v, xi, lane, prev, yd, part); break;
+    case 2: slot_sums<2>(d, v, xi, lane, prev, yd, part); break;
+    case 1: slot_sums<1>(d, v, xi, lane, prev, yd, part); break;
+    default: break;
+    }
+    y[i] = __dadd_rn(yd, part);
 }
 
 // As k_spmv_fp64, with each entry's in-tile column read from the 4-bit
@@ -68,6 +137,50 @@ mf_status spmv_fp64(const MfTiles &A, const double *x, double *y, cudaStream_t s
     if (A.tilem == 0) return MF_OK;
     int grid = ceil_div(A.tilem, SPMV_NT / MF_TILE);
     k_spmv_fp64<<<grid, SPMV_NT, 0, s>>>(A, x, y);
+    note_launch();
+    MF_CUDA(cudaGetLastError());
+    return MF_OK;
+}
+
+// Whether the slots may be built on this call: not while the stream (or, on
+// the legacy stream, any blocking stream) is being captured.
+static bool may_build(cudaStream_t s)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return st == cudaStreamCaptureStatusNone;
+}
+
+// y = A x.  Building the slots costs as much as ~30 products (128^3 Poisson: 1
+// ms, mostly allocation, against 28 us saved by each later one), so the first
+// product of a handle, which may be its only one, does not; a matrix whose slots would be more than half padding, or that they
+// cannot describe, stays with the tiles.
+mf_status spmv(mf_matrix m, const double *x, double *y, cudaStream_t s)
+{
+    const MfTiles &A = m->v;
+    if (A.tilem == 0) return MF_OK;
+    if (m->slots_state.load(std::memory_order_acquire) == 0 && m->spmv_calls.load(std::memory_order_relaxed) >= 0) {
+        const int calls = m->spmv_calls.fetch_add(1, std::memory_order_relaxed);
+        if (calls >= 1 && may_build(s)) {
+            // another thread's capture does not mind the allocations here
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            const mf_status st = build_slots(m, s, 2LL * A.nnz + 4096);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            if (st != MF_OK) cudaGetLastError();  // no memory for them: the tiles serve
+            if (st != MF_OK || m->slots_state.load() != 1) m->spmv_calls.store(-1);  // do not try again
+        }
+    }
+    if (m->slots_state.load(std::memory_order_acquire) != 1 || m->nslots * MF_TILE > 2LL * A.nnz + 4096)
+        return spmv_fp64(A, x, y, s);
+    const int grid = ceil_div(A.rows, SPMV_NT);
+    if (m->soff_bytes == 2)
+        k_spmv_slots<<<grid, SPMV_NT, 0, s>>>(A.rows, m->d_sslot, (const int16_t *)m->d_soff, m->d_sval, x, y);
+    else
+        k_spmv_slots<<<grid, SPMV_NT, 0, s>>>(A.rows, m->d_sslot, (const int32_t *)m->d_soff, m->d_sval, x, y);
     note_launch();
     MF_CUDA(cudaGetLastError());
     return MF_OK;
