@@ -128,7 +128,7 @@ mf_status mf_matrix_create(int rowA, int colA, const int *rowptr, const int *col
         }
         size_t b_rp = sizeof(int) * (rowA + 1), b_ci = sizeof(int) * nnz_end, b_v = sizeof(double) * nnz_end,
                b_vl = val_low ? sizeof(float) * nnz_end : 0;
-        MF_CUDA(cudaMalloc(&tmp, b_rp + b_ci + b_v + b_vl + 64));
+        MF_CUDA(pool_malloc_async(&tmp, b_rp + b_ci + b_v + b_vl + 64, s));
         char *c = (char *)tmp;
         double *dv = (double *)c;
         int *dci = (int *)(c + b_v);
@@ -139,7 +139,7 @@ mf_status mf_matrix_create(int rowA, int colA, const int *rowptr, const int *col
         if (e == cudaSuccess && nnz_end > 0) e = cudaMemcpyAsync(dv, val, b_v, cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess && val_low && nnz_end > 0) e = cudaMemcpyAsync(dvl, val_low, b_vl, cudaMemcpyHostToDevice, s);
         if (e != cudaSuccess) {
-            cudaFree(tmp);
+            cudaFreeAsync(tmp, s);
             set_last_error("H2D copy: %s", cudaGetErrorString(e));
             return MF_ERR_CUDA;
         }
@@ -154,7 +154,7 @@ mf_status mf_matrix_create(int rowA, int colA, const int *rowptr, const int *col
     mf_status st = build_tiles(m, rowA, colA, d_rp, d_ci, d_v, d_vl, s);
     if (tmp) {
         cudaStreamSynchronize(s);
-        cudaFree(tmp);
+        cudaFreeAsync(tmp, s);
     }
     if (st != MF_OK) {
         mf_matrix_destroy(m);
@@ -167,10 +167,16 @@ mf_status mf_matrix_create(int rowA, int colA, const int *rowptr, const int *col
 mf_status mf_matrix_destroy(mf_matrix m)
 {
     if (!m) return MF_OK;
-    void *bufs[] = {m->d_tile_ptr, m->d_tile_columnidx, m->d_tile_nnz, m->d_csrptr_offset, m->d_blknnznnz, m->d_val,
-                    m->d_val_low, m->d_col, m->d_ptr, m->d_cidx, m->d_f16, m->d_i8, m->d_class, m->d_f16ok,
-                    m->d_nonzero_row_new, m->d_tile_rowidx, m->d_block_signal, m->d_blockrowid_new, m->d_blockcsr_ptr_new, m->d_rbb_rowidx,
-                    m->d_rbb_colstart, m->d_rbb_colstop, m->d_part, m->d_cta_chunk, m->d_chunks, m->work, m->host_io,
+    int dev = -1;
+    cudaGetDevice(&dev);
+    if (dev != m->device) cudaSetDevice(m->device);
+    if (m->tiles_mem) {
+        // back to the pool once nothing on the device can still read it
+        cudaDeviceSynchronize();
+        cudaFreeAsync(m->tiles_mem, 0);
+    }
+    if (dev != m->device && dev >= 0) cudaSetDevice(dev);
+    void *bufs[] = {m->d_part, m->d_cta_chunk, m->d_chunks, m->work, m->host_io,
                     m->d_wcls, m->d_poff, m->d_pay, m->d_resid, m->d_pol, m->d_sslot, m->d_smeta, m->d_sval, m->d_soff,
                     m->d_shdr, m->d_spay, m->d_scta_chunk, m->d_schunks, m->d_spos, m->d_sdesc, m->mr_work,
                     m->mr_io, m->d_tc_index, m->d_tc_dense};

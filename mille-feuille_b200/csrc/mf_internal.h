@@ -37,7 +37,8 @@ struct mf_matrix_s {
     int rowblkblock;
     size_t device_bytes;
 
-    // owned device buffers
+    // the tile arrays below live in one allocation of the library's pool
+    void *tiles_mem = nullptr;
     int *d_tile_ptr = nullptr, *d_tile_columnidx = nullptr, *d_tile_nnz = nullptr;
     int *d_csrptr_offset = nullptr;
     unsigned char *d_blknnznnz = nullptr;

@@ -9,14 +9,27 @@
 // (src/blockspmv_cpu.h:35-83), and the per-class payloads
 // (src/main-cg-mixed.cu:2325-2342).
 //
-// Design (not the reference's): one CTA per tile-row sorts the tile-row's
-// entries by (tile column, CSR position) with a bitonic network in shared
-// memory (global memory for tile-rows above SORT_CAP entries).  After one
-// scan of tile counts, a second pass scatters: because tiles are ordered by
-// column and entries keep CSR order, an entry's destination is simply the
-// tile-row's first CSR offset plus its sorted position, so values move in one
-// coalesced pass with no per-entry search.
+// Design (not the reference's): one warp per tile-row of up to 256 entries.
+// It sorts the tile-row's entries by (tile column, CSR position) with a
+// bitonic network on 32-bit keys in registers; after one scan of tile counts
+// a second pass writes everything the tile-row's tiles have: because tiles
+// are ordered by column and entries keep CSR order, an entry's destination is
+// simply the tile-row's first CSR offset plus its sorted position, so the
+// values, columns and payloads move once, coalesced; row counts and class
+// flags of its tiles collect in shared memory, and the row pointers, classes
+// and offsets follow from them.  Longer tile-rows (or more than 2^24 tile
+// columns) take a CTA each: 64-bit keys in shared memory (global memory
+// above SORT_CAP entries), then one pass per array.
+//
+// All arrays live in one allocation of the library's memory pool, sized by
+// bounds known once the tiles are counted, so a build waits for the GPU three
+// times and allocates once.  Measured on a 96^3 Poisson matrix (6.1 M
+// entries), create, one product, destroy: 11.3 -> 0.43 ms (create 6.3 -> 0.40,
+// of which kernels ~0.2; destroy 4.2 -> 0.01).
 #include <cuda_fp16.h>
+
+#include <algorithm>
+#include <type_traits>
 
 #include "mf_internal.h"
 
@@ -26,6 +39,10 @@ namespace {
 constexpr int BUILD_NT = 256;
 constexpr int SORT_CAP = 4096;  // entries sorted in shared memory
 constexpr unsigned long long KEY_PAD = ~0ull;
+constexpr int WARP_CAP = 256;            // entries of a tile-row one warp handles
+constexpr int WARP_TILEN = 1 << 24;      // tile columns its 32-bit keys can hold
+constexpr int WS_NT = 256;               // threads of the warp sort
+constexpr int WF_NT = 128;               // threads of the warp fill
 
 // Ascending bitonic network over P (power of two) keys; only pairs whose
 // partner index is above the lower index are compared, so virtual +inf
@@ -57,10 +74,253 @@ __device__ void bitonic_sort(unsigned long long *keys, int m, int P)
     }
 }
 
-// Pass 1: sort each tile-row's entries by (tile column, CSR position); write
-// the permutation and the number of distinct tile columns.
+// Ascending bitonic sort of 32 R keys of a warp, element r * 32 + lane in
+// key[r].
+template <int R>
+__device__ __forceinline__ void warp_sort(unsigned (&key)[R], int lane)
+{
+#pragma unroll
+    for (int k = 2; k <= 32 * R; k <<= 1) {
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const bool up = ((r * 32 + lane) & k) == 0;
+                if (j >= 32) {
+                    const int o = r ^ (j / 32);
+                    if (o > r) {
+                        const unsigned a = min(key[r], key[o]), b = max(key[r], key[o]);
+                        key[r] = up ? a : b;
+                        key[o] = up ? b : a;
+                    }
+                } else {
+                    const unsigned v = __shfl_xor_sync(0xffffffffu, key[r], j);
+                    key[r] = ((lane & j) == 0) == up ? min(key[r], v) : max(key[r], v);
+                }
+            }
+        }
+    }
+}
+
+template <int R>
+__device__ __forceinline__ int sort_tilerow(int m, const int *__restrict__ colidx, unsigned char *__restrict__ perm,
+                                            int lane)
+{
+    unsigned key[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int k = r * 32 + lane;
+        key[r] = k < m ? ((unsigned)(colidx[k] >> 4) << 8) | (unsigned)k : 0xffffffffu;
+    }
+    warp_sort(key, lane);
+    int cnt = 0;
+    unsigned last = 0xffffffffu;  // tile column before this register's first element
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int k = r * 32 + lane;
+        const unsigned col = key[r] >> 8;
+        unsigned before = __shfl_up_sync(0xffffffffu, col, 1);
+        if (lane == 0) before = last;
+        last = __shfl_sync(0xffffffffu, col, 31);
+        cnt += __popc(__ballot_sync(0xffffffffu, k < m && (k == 0 || col != before)));
+        if (k < m) perm[k] = (unsigned char)(key[r] & 255u);
+    }
+    return cnt;
+}
+
+// Pass 1 for tile-rows of at most `most` entries, a warp each: the entries'
+// order (positions within the tile-row) and the number of distinct tile
+// columns.
+__global__ void __launch_bounds__(WS_NT)
+k_sort_warps(int tilem, int rowA, int most, const int *__restrict__ rowptr, const int *__restrict__ colidx,
+             unsigned char *__restrict__ perm, int *__restrict__ tilecnt)
+{
+    const int lane = threadIdx.x & 31, rp0 = rowptr[0];
+    for (int bi = blockIdx.x * (WS_NT / 32) + (threadIdx.x >> 5); bi < tilem; bi += gridDim.x * (WS_NT / 32)) {
+        const int rs = bi * MF_TILE, re = min(rowA, rs + MF_TILE);
+        const int base = rowptr[rs], m = rowptr[re] - base;
+        if (m > most) continue;
+        const int *c = colidx + base;
+        unsigned char *p = perm + (base - rp0);
+        int cnt;
+        if (m <= 32) cnt = sort_tilerow<1>(m, c, p, lane);
+        else if (m <= 64) cnt = sort_tilerow<2>(m, c, p, lane);
+        else if (m <= 128) cnt = sort_tilerow<4>(m, c, p, lane);
+        else cnt = sort_tilerow<8>(m, c, p, lane);
+        if (lane == 0) tilecnt[bi] = cnt;
+    }
+}
+
+// The bits of a value's flags, and the value's payloads (see k_payloads).
+constexpr unsigned FL_INT8 = 1, FL_IN16 = 2, FL_IN32 = 4, FL_FIN16 = 8, FL_NORM16 = 16, FL_ALL = 31;
+
+__device__ __forceinline__ unsigned value_payload(double v, float low, uint16_t &f16, int8_t &i8)
+{
+    const half h = __float2half_rn(low);
+    f16 = __half_as_ushort(h);
+    const long long w = (fabs(v) < 2147483648.0) ? (long long)__double2int_rz(v) : (long long)INT_MIN;
+    i8 = (int8_t)(unsigned char)(unsigned)(int)w;
+    unsigned f = FL_ALL;
+    if (!(v == trunc(v) && v >= -128.0 && v <= 127.0)) f &= ~FL_INT8;
+    if ((double)(float)v != v) f &= ~FL_IN32;
+    if ((double)__half2float(h) != v) f &= ~FL_IN16;
+    if (__hisinf(h) || __hisnan(h)) f &= ~FL_FIN16;
+    if (v != 0.0 && (f16 & 0x7C00u) == 0) f &= ~FL_NORM16;  // zero or subnormal from a nonzero value
+    return f;
+}
+
+__device__ __forceinline__ unsigned char flags_class(unsigned f)
+{
+    return f & FL_INT8 ? MF_CLASS_INT8 : f & FL_IN16 ? MF_CLASS_FP16 : f & FL_IN32 ? MF_CLASS_FP32 : MF_CLASS_FP64;
+}
+
+__device__ __forceinline__ unsigned char flags_f16ok(unsigned f)
+{
+    return (unsigned char)((f & FL_FIN16 ? 1 : 0) | ((f & FL_FIN16) && (f & FL_NORM16) ? 2 : 0));
+}
+
+// What pass 2 writes.
+struct TileOut {
+    int *tile_columnidx, *tile_nnz, *tile_rowidx, *csrptr_offset, *nz_rows;
+    unsigned char *blkptr, *blknnznnz, *col, *cls, *f16ok;
+    double *val;
+    float *low;
+    uint16_t *f16;
+    int8_t *i8;
+    int *err, *class_count, *max_nz;
+};
+
+// Pass 2 for tile-rows of at most `most` entries, a warp each.
+__global__ void __launch_bounds__(WF_NT)
+k_fill_warps(int tilem, int rowA, int T, int most, const int *__restrict__ rowptr, const int *__restrict__ colidx,
+             const double *__restrict__ val, const float *__restrict__ val_low, const unsigned char *__restrict__ perm,
+             const int *__restrict__ tile_ptr, TileOut o)
+{
+    constexpr int NW = WF_NT / 32;
+    __shared__ int s_rp[NW][MF_TILE + 1];
+    __shared__ unsigned s_cnt[NW][WARP_CAP][MF_TILE / 2];  // entries per tile and row, 16 bits each
+    __shared__ unsigned s_flag[NW][WARP_CAP];
+    __shared__ int s_class[5], s_max;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (threadIdx.x < 5) s_class[threadIdx.x] = 0;
+    if (threadIdx.x == 5) s_max = 0;
+    __syncthreads();
+    const int rp0 = rowptr[0];
+    const int last_begin = tile_ptr[tilem - 1], rowlen_last = rowA - (tilem - 1) * MF_TILE;
+    for (int bi = blockIdx.x * NW + w; bi < tilem; bi += gridDim.x * NW) {
+        const int rs = bi * MF_TILE, rows = min(rowA - rs, MF_TILE);
+        const int base = rowptr[rs], m = rowptr[rs + rows] - base;
+        if (m > most) continue;
+        const int t0 = tile_ptr[bi], nt = tile_ptr[bi + 1] - t0, d0 = base - rp0;
+        if (lane <= rows) s_rp[w][lane] = rowptr[rs + lane] - base;
+        for (int k = lane; k < nt * (MF_TILE / 2); k += 32) s_cnt[w][k / (MF_TILE / 2)][k % (MF_TILE / 2)] = 0;
+        for (int k = lane; k < nt; k += 32) s_flag[w][k] = FL_ALL;
+        __syncwarp();
+        int carry = -1, last = -1;  // tile ordinal and tile column before this group of 32 entries
+        for (int c0 = 0; c0 < m; c0 += 32) {
+            const int k = c0 + lane;
+            const bool in = k < m;
+            const int p = in ? perm[d0 + k] : 0;
+            const int col = in ? colidx[base + p] : -16;
+            const double v = in ? val[base + p] : 0.0;
+            const float low = in ? (val_low ? val_low[base + p] : (float)v) : 0.f;
+            int row = 0;  // last r with s_rp[r] <= p
+#pragma unroll
+            for (int st = 8; st > 0; st >>= 1)
+                if (row + st < rows && s_rp[w][row + st] <= p) row += st;
+            const int jc = col >> 4;
+            int before = __shfl_up_sync(0xffffffffu, jc, 1);
+            if (lane == 0) before = last;
+            last = __shfl_sync(0xffffffffu, jc, 31);
+            const bool head = in && (k == 0 || jc != before);
+            const unsigned heads = __ballot_sync(0xffffffffu, head);
+            const int ord = carry + __popc(heads & (0xffffffffu >> (31 - lane)));
+            carry += __popc(heads);
+            if (in) {
+                const int dst = d0 + k;
+                if (head) {
+                    o.tile_columnidx[t0 + ord] = jc;
+                    o.tile_nnz[t0 + ord] = dst;
+                    o.tile_rowidx[t0 + ord] = bi;
+                }
+                uint16_t f16;
+                int8_t i8;
+                const unsigned f = value_payload(v, low, f16, i8);
+                o.val[dst] = v;
+                o.low[dst] = low;
+                o.col[dst] = (unsigned char)(col & 15);
+                o.f16[dst] = f16;
+                o.i8[dst] = i8;
+                atomicAdd(&s_cnt[w][ord][row >> 1], row & 1 ? 0x10000u : 1u);
+                if (f != FL_ALL) atomicAnd(&s_flag[w][ord], f);
+            }
+        }
+        __syncwarp();
+        for (int k = lane; k < nt; k += 32) {
+            const int t = t0 + k;
+            // row pointers: the counts' exclusive sums, mod 256 as the
+            // reference's unsigned char arithmetic
+            unsigned char p8[MF_TILE];
+            int at = 0;
+#pragma unroll
+            for (int r = 0; r < MF_TILE; r += 2) {
+                const unsigned c = s_cnt[w][k][r >> 1];
+                p8[r] = (unsigned char)at;
+                at += (int)(c & 0xffffu);
+                p8[r + 1] = (unsigned char)at;
+                at += (int)(c >> 16);
+            }
+            const int nz = at;
+            if (nz > 256) atomicExch(o.err, (int)MF_ERR_UNSUPPORTED);
+            const int po = t < last_begin ? t * MF_TILE : last_begin * MF_TILE + (t - last_begin) * rowlen_last;
+            int nonempty = 0;
+            if (rows == MF_TILE) {
+                uint4 q;
+                unsigned *qw = reinterpret_cast<unsigned *>(&q);
+#pragma unroll
+                for (int r = 0; r < MF_TILE; r += 4)
+                    qw[r / 4] = p8[r] | (unsigned)p8[r + 1] << 8 | (unsigned)p8[r + 2] << 16 | (unsigned)p8[r + 3] << 24;
+                *reinterpret_cast<uint4 *>(o.blkptr + po) = q;
+            }
+#pragma unroll
+            for (int r = 0; r < MF_TILE; r++) {
+                if (r < rows) {
+                    if (rows != MF_TILE) o.blkptr[po + r] = p8[r];
+                    const int stop = (r == rows - 1) ? nz : (int)p8[r + 1 < MF_TILE ? r + 1 : r];
+                    if (stop != (int)p8[r]) nonempty++;
+                }
+            }
+            o.csrptr_offset[t] = po;
+            o.blknnznnz[t] = (unsigned char)nz;
+            o.nz_rows[t] = 1 + nonempty;
+            const unsigned f = s_flag[w][k];
+            const unsigned char c = flags_class(f);
+            o.cls[t] = c;
+            o.f16ok[t] = flags_f16ok(f);
+            atomicAdd(&s_class[c], 1);
+            atomicMax(&s_max, nz);
+        }
+        __syncwarp();
+    }
+    __syncthreads();
+    if (threadIdx.x < 5 && s_class[threadIdx.x]) atomicAdd(&o.class_count[threadIdx.x], s_class[threadIdx.x]);
+    if (threadIdx.x == 5 && s_max) atomicMax(o.max_nz, s_max);
+}
+
+// The ends of the arrays with one entry more than tiles.
+__global__ void k_tile_ends(int tilem, int rowA, int T, int nnz, const int *__restrict__ tile_ptr, TileOut o)
+{
+    const int lb = tilem > 0 ? tile_ptr[tilem - 1] : 0, rowlen_last = rowA - (tilem - 1) * MF_TILE;
+    o.tile_nnz[T] = nnz;
+    o.csrptr_offset[T] = (T > lb) ? lb * MF_TILE + (T - lb) * rowlen_last : T * MF_TILE;
+    o.blknnznnz[T] = 0;
+    o.nz_rows[T] = 0;
+}
+
+// Pass 1 for tile-rows above `most` entries: sort by (tile column, CSR
+// position); write the permutation and the number of distinct tile columns.
 __global__ void __launch_bounds__(BUILD_NT)
-k_sort_tilerows(int tilem, int rowA, const int *__restrict__ rowptr, const int *__restrict__ colidx,
+k_sort_tilerows(int tilem, int rowA, int most, const int *__restrict__ rowptr, const int *__restrict__ colidx,
                 int *__restrict__ perm, unsigned long long *__restrict__ big_keys, int *__restrict__ tilecnt)
 {
     __shared__ unsigned long long s_keys[SORT_CAP];
@@ -68,6 +328,7 @@ k_sort_tilerows(int tilem, int rowA, const int *__restrict__ rowptr, const int *
     for (int bi = blockIdx.x; bi < tilem; bi += gridDim.x) {
         const int rs = bi * MF_TILE, re = min(rowA, rs + MF_TILE);
         const int base = rowptr[rs], m = rowptr[re] - base;
+        if (m <= most) continue;  // a warp has it
         int P = 1;
         while (P < m) P <<= 1;
         unsigned long long *keys = (m <= SORT_CAP) ? s_keys : (big_keys + base);
@@ -99,10 +360,11 @@ k_sort_tilerows(int tilem, int rowA, const int *__restrict__ rowptr, const int *
     }
 }
 
-// Pass 2: scatter entries to tile order; tile columns, tile offsets, the
-// first position of each non-empty (tile,row) run, tile row index.
+// Pass 2 for tile-rows above `most` entries: scatter entries to tile order;
+// tile columns, tile offsets, the first position of each non-empty (tile,row)
+// run, tile row index.
 __global__ void __launch_bounds__(BUILD_NT)
-k_fill_tilerows(int tilem, int rowA, int rp0, const int *__restrict__ rowptr, const int *__restrict__ colidx,
+k_fill_tilerows(int tilem, int rowA, int most, int rp0, const int *__restrict__ rowptr, const int *__restrict__ colidx,
                 const double *__restrict__ val, const float *__restrict__ val_low, const int *__restrict__ perm,
                 const int *__restrict__ tile_ptr, int *__restrict__ tile_columnidx, int *__restrict__ tile_nnz,
                 int *__restrict__ tile_rowidx, int *__restrict__ run_start, double *__restrict__ out_val,
@@ -117,6 +379,10 @@ k_fill_tilerows(int tilem, int rowA, int rp0, const int *__restrict__ rowptr, co
         if (threadIdx.x == 0) s_carry = 0;
         __syncthreads();
         const int base = s_rp[0], m = s_rp[rows] - base;
+        if (m <= most) {  // a warp has it
+            __syncthreads();
+            continue;
+        }
         const int t0 = tile_ptr[bi];
         for (int c0 = 0; c0 < m; c0 += BUILD_NT) {
             const int k = c0 + threadIdx.x;
@@ -186,29 +452,27 @@ k_fill_tilerows(int tilem, int rowA, int rp0, const int *__restrict__ rowptr, co
     }
 }
 
-// Per tile: in-tile u8 row pointers from the first position of each
-// non-empty row (empty rows take the start of the next non-empty row, as an
-// exclusive scan of per-row counts does), u8 entry count, row-pointer offset,
-// and the non-empty-row count with the reference's test (stop != start,
-// src/main-cg.cu:1241-1245).
-__global__ void k_tile_finish(int tilem, int rowA, int T, const int *__restrict__ tile_ptr,
-                              const int *__restrict__ tile_rowidx, int *__restrict__ tile_nnz,
-                              const int *__restrict__ run_start, int *__restrict__ csrptr_offset,
-                              unsigned char *__restrict__ blkptr, unsigned char *__restrict__ blknnznnz,
-                              int *__restrict__ nz_rows, int *__restrict__ err, int nnz_total)
+// Per tile of a tile-row above `most` entries: in-tile u8 row pointers from
+// the first position of each non-empty row (empty rows take the start of the
+// next non-empty row, as an exclusive scan of per-row counts does), u8 entry
+// count, row-pointer offset, and the non-empty-row count with the reference's
+// test (stop != start, src/main-cg.cu:1241-1245).
+__global__ void k_tile_finish(int tilem, int rowA, int T, int most, const int *__restrict__ rowptr,
+                              const int *__restrict__ tile_ptr, const int *__restrict__ run_start, TileOut o)
 {
     const int last_row_tiles_begin = (tilem > 0) ? tile_ptr[tilem - 1] : 0;
     const int rowlen_last = rowA - (tilem - 1) * MF_TILE;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
-        const int off = tile_nnz[t];
-        const int nz = ((t + 1 < T) ? tile_nnz[t + 1] : nnz_total) - off;
-        if (nz > 256) atomicExch(err, (int)MF_ERR_UNSUPPORTED);
-        const int bi = tile_rowidx[t];
+        const int bi = o.tile_rowidx[t];
+        if (rowptr[min(rowA, (bi + 1) * MF_TILE)] - rowptr[bi * MF_TILE] <= most) continue;
+        const int off = o.tile_nnz[t];
+        const int nz = o.tile_nnz[t + 1] - off;
+        if (nz > 256) atomicExch(o.err, (int)MF_ERR_UNSUPPORTED);
         const int rowlen = (bi == tilem - 1) ? rowlen_last : MF_TILE;
         const int po = (t < last_row_tiles_begin) ? t * MF_TILE
                                                    : last_row_tiles_begin * MF_TILE + (t - last_row_tiles_begin) * rowlen_last;
-        csrptr_offset[t] = po;
-        blknnznnz[t] = (unsigned char)nz;
+        o.csrptr_offset[t] = po;
+        o.blknnznnz[t] = (unsigned char)nz;
         int next = nz, nonempty = 0;
         unsigned char p8[MF_TILE];
         for (int r = rowlen - 1; r >= 0; r--) {
@@ -218,17 +482,11 @@ __global__ void k_tile_finish(int tilem, int rowA, int T, const int *__restrict_
             p8[r] = (unsigned char)next;
         }
         for (int r = 0; r < rowlen; r++) {
-            blkptr[po + r] = p8[r];
+            o.blkptr[po + r] = p8[r];
             const int stop = (r == rowlen - 1) ? nz : (int)p8[r + 1];
             if (stop != (int)p8[r]) nonempty++;
         }
-        nz_rows[t] = 1 + nonempty;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        tile_nnz[T] = nnz_total;
-        csrptr_offset[T] = (T > last_row_tiles_begin) ? last_row_tiles_begin * MF_TILE + (T - last_row_tiles_begin) * rowlen_last
-                                                      : T * MF_TILE;
-        blknnznnz[T] = 0;
+        o.nz_rows[t] = 1 + nonempty;
     }
 }
 
@@ -308,45 +566,39 @@ __global__ void k_rbb_fill(int tilem, const int *__restrict__ tile_ptr, const in
 // f16ok: bit 0 every FP16 payload value of the tile is finite (|v| within
 // binary16's range), the condition for running an inexact tile in FP16;
 // bit 1 every nonzero one is also normal (|v| >= 2^-14: no subnormal loss).
-__global__ void k_payloads(int T, const int *__restrict__ tile_nnz, const double *__restrict__ val,
-                           const float *__restrict__ low, uint16_t *__restrict__ f16, int8_t *__restrict__ i8,
-                           unsigned char *__restrict__ cls, unsigned char *__restrict__ f16ok,
-                           int *__restrict__ class_count, int *__restrict__ max_nz)
+// (Here: the tiles of tile-rows above `most` entries.)
+__global__ void k_payloads(int T, int rowA, int most, const int *__restrict__ rowptr, TileOut o)
 {
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
-        const int a = tile_nnz[t], b = tile_nnz[t + 1];
-        bool is_int8 = true, in16 = true, in32 = true, fin16 = true, norm16 = true;
+        const int bi = o.tile_rowidx[t];
+        if (rowptr[min(rowA, (bi + 1) * MF_TILE)] - rowptr[bi * MF_TILE] <= most) continue;
+        const int a = o.tile_nnz[t], b = o.tile_nnz[t + 1];
+        unsigned f = FL_ALL;
         for (int k = a; k < b; k++) {
-            const double v = val[k];
-            const double av = fabs(v);
-            const half h = __float2half_rn(low[k]);
-            f16[k] = __half_as_ushort(h);
-            long long w = (av < 2147483648.0) ? (long long)__double2int_rz(v) : (long long)INT_MIN;
-            i8[k] = (int8_t)(unsigned char)(unsigned)(int)w;
-            if (!(v == trunc(v) && v >= -128.0 && v <= 127.0)) is_int8 = false;
-            const float vf = (float)v;
-            if ((double)vf != v) in32 = false;
-            if ((double)__half2float(h) != v) in16 = false;
-            if (__hisinf(h) || __hisnan(h)) fin16 = false;
-            const unsigned short hb = __half_as_ushort(h);
-            if (v != 0.0 && (hb & 0x7C00u) == 0) norm16 = false;  // zero or subnormal from a nonzero value
+            uint16_t f16;
+            int8_t i8;
+            f &= value_payload(o.val[k], o.low[k], f16, i8);
+            o.f16[k] = f16;
+            o.i8[k] = i8;
         }
-        f16ok[t] = (unsigned char)((fin16 ? 1 : 0) | (fin16 && norm16 ? 2 : 0));
-        unsigned char c = is_int8 ? MF_CLASS_INT8 : in16 ? MF_CLASS_FP16 : in32 ? MF_CLASS_FP32 : MF_CLASS_FP64;
-        cls[t] = c;
-        atomicAdd(&class_count[c], 1);
-        atomicMax(max_nz, b - a);
+        o.f16ok[t] = flags_f16ok(f);
+        const unsigned char c = flags_class(f);
+        o.cls[t] = c;
+        atomicAdd(&o.class_count[c], 1);
+        atomicMax(o.max_nz, b - a);
     }
 }
 
-__global__ void k_validate(int rowA, int colA, const int *__restrict__ rowptr, const int *__restrict__ colidx,
-                           int *__restrict__ err)
+// Also counts the tile-rows above `most` entries.
+__global__ void k_validate(int rowA, int colA, int most, const int *__restrict__ rowptr,
+                           const int *__restrict__ colidx, int *__restrict__ err, int *__restrict__ big)
 {
     const int rp0 = rowptr[0], rpn = rowptr[rowA];
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)rowA + (rpn - rp0);
          i += (long long)gridDim.x * blockDim.x) {
         if (i < rowA) {
             if (rowptr[i + 1] < rowptr[i]) atomicExch(err, (int)MF_ERR_INVALID_ARG);
+            if (i % MF_TILE == 0 && rowptr[i + min((long long)MF_TILE, rowA - i)] - rowptr[i] > most) atomicAdd(big, 1);
         } else {
             int c = colidx[rp0 + (i - rowA)];
             if (c < 0 || c >= colA) atomicExch(err, (int)MF_ERR_INVALID_ARG);
@@ -382,15 +634,6 @@ __global__ void k_strip_split(int tilem, int ctas, const int *__restrict__ pref,
     }
 }
 
-template <typename T>
-mf_status dalloc(T **p, size_t n, size_t *acc)
-{
-    size_t bytes = sizeof(T) * (n > 0 ? n : 1) + 16;  // 16 B slack for vector loads at the tail
-    MF_CUDA(cudaMalloc((void **)p, bytes));
-    *acc += bytes;
-    return MF_OK;
-}
-
 int grid_for(long long work, int nt)
 {
     long long g = (work + nt - 1) / nt;
@@ -405,161 +648,170 @@ mf_status build_tiles(mf_matrix m, int rowA, int colA, const int *d_rowptr, cons
                       const double *d_val, const float *d_val_low, cudaStream_t s)
 {
     const int tilem = ceil_div(rowA, MF_TILE), tilen = ceil_div(colA, MF_TILE);
-    int rp0 = 0, rpn = 0;
+    const int most = tilen <= WARP_TILEN ? WARP_CAP : -1;  // entries of the tile-rows that go to warps
+    // temporaries and status words, freed on every way out
+    struct Temps {
+        cudaStream_t s;
+        void *p[8];
+        int n = 0;
+        ~Temps() { for (int k = 0; k < n; k++) cudaFreeAsync(p[k], s); }
+        mf_status take(void **q, size_t bytes)
+        {
+            MF_CUDA(pool_malloc_async(q, bytes, s));
+            p[n++] = *q;
+            return MF_OK;
+        }
+    } tmp;
+    tmp.s = s;
+    // status words: [0] err, [1..5] tiles per class, [6] largest tile, [7] long tile-rows
+    int *d_err = nullptr;
+    MF_TRY(tmp.take((void **)&d_err, sizeof(int) * 8));
+    MF_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int) * 8, s));
+    if (rowA > 0) {
+        k_validate<<<std::min(grid_for(rowA, 64), 148 * 16), 256, 0, s>>>(rowA, colA, most, d_rowptr, d_colidx, d_err,
+                                                                         d_err + 7);
+        note_launch();
+        MF_CUDA(cudaGetLastError());
+    }
+    int h[8] = {0}, rp0 = 0, rpn = 0;
     MF_CUDA(cudaMemcpyAsync(&rp0, d_rowptr, sizeof(int), cudaMemcpyDeviceToHost, s));
     MF_CUDA(cudaMemcpyAsync(&rpn, d_rowptr + rowA, sizeof(int), cudaMemcpyDeviceToHost, s));
+    MF_CUDA(cudaMemcpyAsync(h, d_err, sizeof(h), cudaMemcpyDeviceToHost, s));
     MF_CUDA(cudaStreamSynchronize(s));
     const int nnz = rpn - rp0;
     if (nnz < 0) { set_last_error("rowptr[rowA] < rowptr[0]"); return MF_ERR_INVALID_ARG; }
-
-    size_t acc = 0;
-    int *d_err = nullptr;
-    MF_CUDA(pool_malloc_async(&d_err, sizeof(int) * 8, s));
-    MF_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int) * 8, s));
-    int *d_class_count = d_err + 1;  // [5]
-    int *d_maxnz = d_err + 6;
-    if (rowA > 0) {
-        k_validate<<<grid_for((long long)rowA + nnz, 256), 256, 0, s>>>(rowA, colA, d_rowptr, d_colidx, d_err);
-        note_launch();
-        MF_CUDA(cudaGetLastError());
-    }
-    int h_err = 0;
-    MF_CUDA(cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
-    MF_CUDA(cudaStreamSynchronize(s));
-    if (h_err) {
-        cudaFreeAsync(d_err, s);
+    if (h[0]) {
         set_last_error("CSR input invalid: rowptr not monotone or column outside [0, colA)");
         return MF_ERR_INVALID_ARG;
     }
+    const bool big = h[7] > 0;
 
-    // pass 1: per tile-row sort
-    int *d_perm = nullptr, *d_cnt = nullptr;
+    // pass 1: the entries' order in every tile-row, tiles per tile-row
+    unsigned char *d_perm8 = nullptr;
+    int *d_perm = nullptr, *d_cnt = nullptr, *d_tp = nullptr;
     unsigned long long *d_big = nullptr;
-    MF_CUDA(pool_malloc_async(&d_perm, sizeof(int) * (size_t)(nnz + rp0 + 1), s));
-    MF_CUDA(pool_malloc_async(&d_cnt, sizeof(int) * (size_t)(tilem + 1), s));
-    // global sort space only when some tile-row exceeds the shared-memory cap
-    MF_CUDA(pool_malloc_async(&d_big, sizeof(unsigned long long) * (size_t)(nnz + rp0 + 1), s));
-    MF_TRY(dalloc(&m->d_tile_ptr, tilem + 1, &acc));
+    MF_TRY(tmp.take((void **)&d_perm8, (size_t)nnz + 16));
+    MF_TRY(tmp.take((void **)&d_cnt, sizeof(int) * 2 * (size_t)(tilem + 1)));
+    d_tp = d_cnt + tilem + 1;
+    if (big) {
+        MF_TRY(tmp.take((void **)&d_perm, sizeof(int) * ((size_t)nnz + rp0 + 1)));
+        MF_TRY(tmp.take((void **)&d_big, sizeof(unsigned long long) * ((size_t)nnz + rp0 + 1)));
+    }
     if (tilem > 0) {
-        k_sort_tilerows<<<grid_for(tilem, 1) , BUILD_NT, 0, s>>>(tilem, rowA, d_rowptr, d_colidx, d_perm, d_big, d_cnt);
+        k_sort_warps<<<grid_for((long long)tilem * 32, WS_NT), WS_NT, 0, s>>>(tilem, rowA, most, d_rowptr, d_colidx,
+                                                                               d_perm8, d_cnt);
         note_launch();
+        if (big) {
+            k_sort_tilerows<<<grid_for(tilem, 1), BUILD_NT, 0, s>>>(tilem, rowA, most, d_rowptr, d_colidx, d_perm, d_big,
+                                                                     d_cnt);
+            note_launch();
+        }
         MF_CUDA(cudaGetLastError());
     }
     MF_CUDA(cudaMemsetAsync(d_cnt + tilem, 0, sizeof(int), s));
-    int T = 0;
-    MF_TRY(exclusive_scan_i32(d_cnt, m->d_tile_ptr, tilem + 1, s, &T));
+    MF_TRY(exclusive_scan_i32(d_cnt, d_tp, tilem + 1, s, nullptr));
+    int T = 0, last_begin = 0;
+    MF_CUDA(cudaMemcpyAsync(&T, d_tp + tilem, sizeof(int), cudaMemcpyDeviceToHost, s));
+    if (tilem > 0) MF_CUDA(cudaMemcpyAsync(&last_begin, d_tp + tilem - 1, sizeof(int), cudaMemcpyDeviceToHost, s));
+    MF_CUDA(cudaStreamSynchronize(s));
+    // Blockcsr_Ptr size: T*16 minus the short last tile-row
+    const int rowlen_last = rowA - (tilem - 1) * MF_TILE;
+    const int ptrlen = (tilem > 0) ? last_begin * MF_TILE + (T - last_begin) * rowlen_last : 0;
 
-    MF_TRY(dalloc(&m->d_tile_columnidx, T, &acc));
-    MF_TRY(dalloc(&m->d_tile_nnz, T + 1, &acc));
-    MF_TRY(dalloc(&m->d_csrptr_offset, T + 1, &acc));
-    MF_TRY(dalloc(&m->d_blknnznnz, T + 1, &acc));
-    MF_TRY(dalloc(&m->d_tile_rowidx, T, &acc));
-    MF_TRY(dalloc(&m->d_val, nnz, &acc));
-    MF_TRY(dalloc(&m->d_val_low, nnz, &acc));
-    MF_TRY(dalloc(&m->d_col, nnz, &acc));
-    MF_TRY(dalloc(&m->d_cidx, (nnz + 1) / 2, &acc));
+    // every array: one allocation, each on a 256-byte boundary with 16 bytes of
+    // slack for vector loads at its tail.  Not known yet: the non-empty rows
+    // (at most one per entry, and a sentinel per tile) and the row blocks (at
+    // most one per tile-row and one per four tiles).
+    const size_t non_most = (size_t)T + nnz + 1, rbb_most = (size_t)tilem + T / 4 + 1;
+    auto arrays = [&](auto take) {
+        take(m->d_tile_ptr, tilem + 1);
+        take(m->d_tile_columnidx, T);
+        take(m->d_tile_nnz, T + 1);
+        take(m->d_csrptr_offset, T + 1);
+        take(m->d_blknnznnz, T + 1);
+        take(m->d_tile_rowidx, T);
+        take(m->d_val, nnz);
+        take(m->d_val_low, nnz);
+        take(m->d_col, nnz);
+        take(m->d_cidx, (nnz + 1) / 2);
+        take(m->d_nonzero_row_new, T + 1);
+        take(m->d_ptr, ptrlen);
+        take(m->d_blockrowid_new, non_most);
+        take(m->d_blockcsr_ptr_new, non_most);
+        take(m->d_block_signal, tilem + 1);
+        take(m->d_rbb_rowidx, rbb_most);
+        take(m->d_rbb_colstart, rbb_most);
+        take(m->d_rbb_colstop, rbb_most);
+        take(m->d_f16, nnz);
+        take(m->d_i8, nnz);
+        take(m->d_class, T);
+        take(m->d_f16ok, T);
+    };
+    size_t total = 0;
+    arrays([&](auto &p, size_t n) { total += (sizeof(*p) * (n > 0 ? n : 1) + 16 + 255) / 256 * 256; });
+    MF_CUDA(pool_malloc_async(&m->tiles_mem, total, s));
+    char *at = (char *)m->tiles_mem;
+    arrays([&](auto &p, size_t n) {
+        p = (std::remove_reference_t<decltype(p)>)at;
+        at += (sizeof(*p) * (n > 0 ? n : 1) + 16 + 255) / 256 * 256;
+    });
+    MF_CUDA(cudaMemcpyAsync(m->d_tile_ptr, d_tp, sizeof(int) * (tilem + 1), cudaMemcpyDeviceToDevice, s));
     MF_CUDA(cudaMemsetAsync(m->d_cidx, 0, (size_t)(nnz + 1) / 2 + 1, s));
-    int *d_run = nullptr;
-    MF_CUDA(pool_malloc_async(&d_run, sizeof(int) * (size_t)T * MF_TILE + 16, s));
-    MF_CUDA(cudaMemsetAsync(d_run, 0xff, sizeof(int) * (size_t)T * MF_TILE + 16, s));
+    TileOut o{m->d_tile_columnidx, m->d_tile_nnz, m->d_tile_rowidx, m->d_csrptr_offset, m->d_nonzero_row_new,
+              m->d_ptr, m->d_blknnznnz, m->d_col, m->d_class, m->d_f16ok, m->d_val, m->d_val_low, m->d_f16, m->d_i8,
+              d_err, d_err + 1, d_err + 6};
+    k_tile_ends<<<1, 1, 0, s>>>(tilem, rowA, T, nnz, m->d_tile_ptr, o);
+    note_launch();
     if (tilem > 0) {
-        k_fill_tilerows<<<grid_for(tilem, 1), BUILD_NT, 0, s>>>(tilem, rowA, rp0, d_rowptr, d_colidx, d_val, d_val_low,
-                                                                d_perm, m->d_tile_ptr, m->d_tile_columnidx, m->d_tile_nnz,
-                                                                m->d_tile_rowidx, d_run, m->d_val, m->d_val_low, m->d_col);
+        k_fill_warps<<<grid_for((long long)tilem * 32, WF_NT), WF_NT, 0, s>>>(
+            tilem, rowA, T, most, d_rowptr, d_colidx, d_val, d_val_low, d_perm8, m->d_tile_ptr, o);
+        note_launch();
+        if (big) {
+            int *d_run = nullptr;
+            MF_TRY(tmp.take((void **)&d_run, sizeof(int) * (size_t)T * MF_TILE + 16));
+            MF_CUDA(cudaMemsetAsync(d_run, 0xff, sizeof(int) * (size_t)T * MF_TILE + 16, s));
+            k_fill_tilerows<<<grid_for(tilem, 1), BUILD_NT, 0, s>>>(
+                tilem, rowA, most, rp0, d_rowptr, d_colidx, d_val, d_val_low, d_perm, m->d_tile_ptr, m->d_tile_columnidx,
+                m->d_tile_nnz, m->d_tile_rowidx, d_run, m->d_val, m->d_val_low, m->d_col);
+            k_tile_finish<<<grid_for(T, 256), 256, 0, s>>>(tilem, rowA, T, most, d_rowptr, m->d_tile_ptr, d_run, o);
+            k_payloads<<<grid_for(T, 256), 256, 0, s>>>(T, rowA, most, d_rowptr, o);
+            note_launch(3);
+        }
+    }
+    MF_CUDA(cudaGetLastError());
+
+    // non-empty-row lists
+    MF_CUDA(cudaMemsetAsync(m->d_blockrowid_new, 0, non_most, s));
+    MF_CUDA(cudaMemsetAsync(m->d_blockcsr_ptr_new, 0, non_most, s));
+    MF_TRY(exclusive_scan_i32(m->d_nonzero_row_new, m->d_nonzero_row_new, T + 1, s, nullptr));
+    if (T > 0) {
+        k_nonzero_lists<<<grid_for(T, 256), 256, 0, s>>>(tilem, rowA, T, m->d_tile_rowidx, m->d_tile_nnz,
+                                                         m->d_csrptr_offset, m->d_ptr, m->d_nonzero_row_new,
+                                                         m->d_blockrowid_new, m->d_blockcsr_ptr_new);
         note_launch();
         MF_CUDA(cudaGetLastError());
     }
-    const int csrptrlen = (tilem > 0) ? 0 : 0;  // computed below from csrptr_offset[T]
-    (void)csrptrlen;
-    int *d_nzr = nullptr;
-    MF_TRY(dalloc(&d_nzr, T + 1, &acc));
-    m->d_nonzero_row_new = d_nzr;
-    // Blockcsr_Ptr size: T*16 minus the short last tile-row
-    const int rowlen_last = rowA - (tilem - 1) * MF_TILE;
-    int last_begin = 0;
+
+    // row-block schedule (d_cnt is free again)
+    k_rbb_count<<<grid_for(tilem + 1, 256), 256, 0, s>>>(tilem, m->d_tile_ptr, d_cnt, m->d_block_signal);
+    note_launch();
+    MF_TRY(exclusive_scan_i32(d_cnt, d_cnt, tilem + 1, s, nullptr));
     if (tilem > 0) {
-        MF_CUDA(cudaMemcpyAsync(&last_begin, m->d_tile_ptr + tilem - 1, sizeof(int), cudaMemcpyDeviceToHost, s));
-        MF_CUDA(cudaStreamSynchronize(s));
-    }
-    const int ptrlen = (tilem > 0) ? last_begin * MF_TILE + (T - last_begin) * rowlen_last : 0;
-    MF_TRY(dalloc(&m->d_ptr, ptrlen, &acc));
-    if (T > 0) {
-        k_tile_finish<<<grid_for(T, 256), 256, 0, s>>>(tilem, rowA, T, m->d_tile_ptr, m->d_tile_rowidx, m->d_tile_nnz,
-                                                       d_run, m->d_csrptr_offset, m->d_ptr, m->d_blknnznnz, d_nzr, d_err,
-                                                       nnz);
-        note_launch();
-    } else {
-        k_tile_finish<<<1, 32, 0, s>>>(tilem, rowA, 0, m->d_tile_ptr, m->d_tile_rowidx, m->d_tile_nnz, d_run,
-                                       m->d_csrptr_offset, m->d_ptr, m->d_blknnznnz, d_nzr, d_err, nnz);
+        k_rbb_fill<<<grid_for(tilem, 256), 256, 0, s>>>(tilem, m->d_tile_ptr, d_cnt, m->d_rbb_rowidx, m->d_rbb_colstart,
+                                                        m->d_rbb_colstop);
         note_launch();
     }
     MF_CUDA(cudaGetLastError());
-    MF_CUDA(cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, s));
+
+    int cnt_non = 0, rbb = 0, host_counts[8] = {0};
+    MF_CUDA(cudaMemcpyAsync(&cnt_non, m->d_nonzero_row_new + T, sizeof(int), cudaMemcpyDeviceToHost, s));
+    MF_CUDA(cudaMemcpyAsync(&rbb, d_cnt + tilem, sizeof(int), cudaMemcpyDeviceToHost, s));
+    MF_CUDA(cudaMemcpyAsync(host_counts, d_err, sizeof(int) * 8, cudaMemcpyDeviceToHost, s));
     MF_CUDA(cudaStreamSynchronize(s));
-    cudaFreeAsync(d_run, s);
-    cudaFreeAsync(d_perm, s);
-    cudaFreeAsync(d_big, s);
-    if (h_err) {
-        cudaFreeAsync(d_err, s);
-        cudaFreeAsync(d_cnt, s);
+    if (host_counts[0]) {
         set_last_error("a 16x16 tile holds more than 256 entries (duplicate entries); u8 row pointers cannot describe it");
         return MF_ERR_UNSUPPORTED;
     }
-
-    // non-empty-row lists
-    MF_CUDA(cudaMemsetAsync(d_nzr + T, 0, sizeof(int), s));
-    int cnt_non = 0;
-    MF_TRY(exclusive_scan_i32(d_nzr, d_nzr, T + 1, s, &cnt_non));
-    MF_TRY(dalloc(&m->d_blockrowid_new, cnt_non + 1, &acc));
-    MF_TRY(dalloc(&m->d_blockcsr_ptr_new, cnt_non + 1, &acc));
-    MF_CUDA(cudaMemsetAsync(m->d_blockrowid_new, 0, cnt_non + 1, s));
-    MF_CUDA(cudaMemsetAsync(m->d_blockcsr_ptr_new, 0, cnt_non + 1, s));
-    if (T > 0) {
-        k_nonzero_lists<<<grid_for(T, 256), 256, 0, s>>>(tilem, rowA, T, m->d_tile_rowidx, m->d_tile_nnz,
-                                                         m->d_csrptr_offset, m->d_ptr, d_nzr, m->d_blockrowid_new,
-                                                         m->d_blockcsr_ptr_new);
-        note_launch();
-        MF_CUDA(cudaGetLastError());
-    }
-
-    // row-block schedule
-    MF_TRY(dalloc(&m->d_block_signal, tilem + 1, &acc));
-    int rbb = 0;
-    {
-        int *d_rc = nullptr;
-        MF_CUDA(pool_malloc_async(&d_rc, sizeof(int) * (tilem + 1), s));
-        k_rbb_count<<<grid_for(tilem + 1, 256), 256, 0, s>>>(tilem, m->d_tile_ptr, d_rc, m->d_block_signal);
-        note_launch();
-        MF_CUDA(cudaGetLastError());
-        MF_TRY(exclusive_scan_i32(d_rc, d_rc, tilem + 1, s, &rbb));
-        MF_TRY(dalloc(&m->d_rbb_rowidx, rbb, &acc));
-        MF_TRY(dalloc(&m->d_rbb_colstart, rbb, &acc));
-        MF_TRY(dalloc(&m->d_rbb_colstop, rbb, &acc));
-        if (tilem > 0) {
-            k_rbb_fill<<<grid_for(tilem, 256), 256, 0, s>>>(tilem, m->d_tile_ptr, d_rc, m->d_rbb_rowidx,
-                                                            m->d_rbb_colstart, m->d_rbb_colstop);
-            note_launch();
-            MF_CUDA(cudaGetLastError());
-        }
-        cudaFreeAsync(d_rc, s);
-    }
-
-    // payloads and static classes
-    MF_TRY(dalloc(&m->d_f16, nnz, &acc));
-    MF_TRY(dalloc(&m->d_i8, nnz, &acc));
-    MF_TRY(dalloc(&m->d_class, T, &acc));
-    MF_TRY(dalloc(&m->d_f16ok, T, &acc));
-    if (T > 0) {
-        k_payloads<<<grid_for(T, 256), 256, 0, s>>>(T, m->d_tile_nnz, m->d_val, m->d_val_low, m->d_f16, m->d_i8,
-                                                    m->d_class, m->d_f16ok, d_class_count, d_maxnz);
-        note_launch();
-        MF_CUDA(cudaGetLastError());
-    }
-    int host_counts[8] = {0};
-    MF_CUDA(cudaMemcpyAsync(host_counts, d_err, sizeof(int) * 8, cudaMemcpyDeviceToHost, s));
-    MF_CUDA(cudaStreamSynchronize(s));
-    cudaFreeAsync(d_err, s);
-    cudaFreeAsync(d_cnt, s);
 
     m->v.rows = rowA;
     m->v.cols = colA;
@@ -585,7 +837,7 @@ mf_status build_tiles(mf_matrix m, int rowA, int colA, const int *d_rowptr, cons
     m->nonzero_rows = cnt_non;
     m->last_tile_begin = last_begin;
     m->rowblkblock = rbb;
-    m->device_bytes = acc;
+    m->device_bytes = total;
     return MF_OK;
 }
 
