@@ -14,8 +14,10 @@
 // The CG keeps k independent recurrences (the textbook unpreconditioned CG
 // per column: alpha_j = rho_j / p_j.q_j, beta_j = rho_new_j / rho_j) that
 // share each SpMM.  Per iteration three launches: the SpMM with the p.q
-// partial sums, the x / r update with the r.r partial sums, and p = r + beta
-// p.  Per-column sums are deterministic: every block reduces its columns in
+// partial sums, r -= alpha q with the r.r partial sums, and x += alpha p, p =
+// r + beta p (x with p: one read of p less than with r).  Consecutive launches
+// sweep the rows in opposite directions, so that each starts on the rows the
+// one before left in L2.  Per-column sums are deterministic: every block reduces its columns in
 // a fixed tree and writes one partial per column; the last block to finish
 // (a device-scope counter) adds the partials in block order and updates the
 // per-column state.  A converged column keeps alpha = beta = 0 from then on
@@ -23,10 +25,19 @@
 // column has converged or maxiter is reached, so the host queues batches of
 // iterations and reads the stop flag between batches.
 //
+// The SpMM is bound by latency (an entry's distance and value, then its
+// element of X: 2.6 TB/s), the vector kernels by HBM (5.4 and 6.4 TB/s at
+// 96^3).  Measured against the earlier form (16-bit tile words looked up
+// per entry, x updated with r: 11 vector streams, always swept upwards): 16
+// right-hand sides of the 96^3 Poisson matrix 278 -> 218 ms, mf_spmm with 5
+// columns of a 290,177-row matrix 47.1 -> 28.6 us (its result is written
+// column-major by the SpMM itself).
+//
 // No tensor cores: FP64 has no tcgen05 kind, and the tiles of the stencil
 // systems hold 3-7 entries per row, so a dense-tile MMA would mostly
 // multiply zeros.  The gain is the matrix read once for k right-hand sides.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
 
@@ -40,10 +51,12 @@ constexpr int MR_GRID = 148 * 8;           // fixed grid: the partial sums do no
 constexpr int MR_MAXK = 16;
 constexpr int MR_BATCH = 16;               // iterations queued between stop-flag reads
 constexpr int MR_VEC_MINB = 8;             // streaming kernels: 8 blocks per SM (32 registers)
-#ifndef MF_MR_SPMM_MINB
-#define MF_MR_SPMM_MINB 5
-#endif
-constexpr int MR_SPMM_MINB = MF_MR_SPMM_MINB;  // SpMM blocks per SM (4: 64 registers, 5: 48)
+// SpMM: blocks per SM and entries of a row in flight.  16 right-hand sides on
+// the 96^3 Poisson matrix, whole solve: 4 blocks (64 registers) with 8
+// entries 218 ms, 4 and 4 221, 3 and 8 219, 2 and 8 227, 5 (48 registers) and 4
+// 235, 6 and 2 316.
+constexpr int MR_SPMM_MINB = 4;
+constexpr int MR_U = 8;
 
 // Per-solve device state (one struct, zeroed before the solve).
 struct MrState {
@@ -56,7 +69,7 @@ struct MrState {
     int status[MR_MAXK];     // MF_OK, MF_ERR_BREAKDOWN
     int done[MR_MAXK];
     int it;                  // iterations issued
-    int stop;                // every column done, or maxiter reached
+    int stop;                // 1: every column done, or maxiter reached; 2: and the last x update done too
     unsigned count;          // blocks finished in the current launch (last-block pattern)
 };
 
@@ -183,60 +196,110 @@ __global__ void __launch_bounds__(MR_NT, MR_VEC_MINB) k_mr_init(int n, int k, co
     }
 }
 
-// Y = A X over the row slots (X, Y row-interleaved with KP columns).  With
-// PQ: skipped once the solve stopped; per-column partials of p.q (X = p,
-// Y = q) and, in the last block, alpha per column.
-template <int KP, bool PQ>
-__global__ void __launch_bounds__(MR_NT, MR_SPMM_MINB) k_mr_spmm(MfTiles A, const int *__restrict__ sslot,
-                                                   const uint16_t *__restrict__ smeta,
+// The next N entries of a row against 4 columns of X (xi: the row's own
+// element): columns and values of all N, then their elements of X in flight
+// together, then the sums in blockspmv_cpu's order (a partial sum per tile,
+// added when the tile column changes).  Empty entries add zero products; no
+// sum here is ever -0.0, so that changes no bit.
+template <int KP, int N, typename OT>
+__device__ __forceinline__ void mr_sums(const OT *__restrict__ d0, const double *__restrict__ v0,
+                                        const double *__restrict__ xi, int lane, int &prev, double (&yd)[4],
+                                        double (&part)[4])
+{
+    constexpr OT EMPTY = (OT)(sizeof(OT) == 2 ? INT16_MIN : INT32_MIN);
+    int d[N];
+    double v[N];
+    double2 xa[N], xb[N];
+#pragma unroll
+    for (int u = 0; u < N; u++) {
+        d[u] = (int)d0[u * MF_TILE];
+        v[u] = v0[u * MF_TILE];
+    }
+#pragma unroll
+    for (int u = 0; u < N; u++) {
+        const double2 *x = (const double2 *)(xi + (long long)d[u] * KP);
+        const bool in = d[u] != (int)EMPTY;
+        xa[u] = in ? x[0] : make_double2(0.0, 0.0);
+        xb[u] = in ? x[1] : make_double2(0.0, 0.0);
+    }
+#pragma unroll
+    for (int u = 0; u < N; u++) {
+        const int t = (d[u] + lane) >> 4;  // tile column, counted from the strip's own
+        if (t != (u == 0 ? prev : (d[u - 1] + lane) >> 4)) {
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                yd[q] = __dadd_rn(yd[q], part[q]);
+                part[q] = 0.0;
+            }
+        }
+        part[0] = __dadd_rn(part[0], __dmul_rn(xa[u].x, v[u]));
+        part[1] = __dadd_rn(part[1], __dmul_rn(xa[u].y, v[u]));
+        part[2] = __dadd_rn(part[2], __dmul_rn(xb[u].x, v[u]));
+        part[3] = __dadd_rn(part[3], __dmul_rn(xb[u].y, v[u]));
+    }
+    prev = (d[N - 1] + lane) >> 4;
+}
+
+// Y = A X over the row slots (X row-interleaved with KP columns).  Y is
+// row-interleaved, or (COLS) column-major with leading dimension ldy, its
+// first k columns.  With PQ: skipped once the solve stopped; per-column
+// partials of p.q (X = p, Y = q) and, in the last block, alpha per column.
+template <int KP, bool PQ, bool COLS, typename OT>
+__global__ void __launch_bounds__(MR_NT, MR_SPMM_MINB) k_mr_spmm(int rows, const int *__restrict__ sslot,
+                                                   const OT *__restrict__ soff,
                                                    const double *__restrict__ sval, const double *__restrict__ X,
-                                                   double *__restrict__ Y, double *__restrict__ partials, MrState *st)
+                                                   double *__restrict__ Y, int k, long long ldy, int back,
+                                                   double *__restrict__ partials, MrState *st)
 {
     constexpr int QT = KP / 4;          // threads per row
     constexpr int RPB = MR_NT / QT;     // rows per block and pass
     __shared__ double sw[MR_NT / 32][MR_MAXK];
     __shared__ double tot[MR_MAXK];
-    if (PQ && *(volatile int *)&st->stop) return;
+    if (PQ && *(volatile int *)&st->stop) {
+        // the x update of the last iteration ran before this launch
+        if (blockIdx.x == 0 && threadIdx.x == 0) st->stop = 2;
+        return;
+    }
     const int c0 = (threadIdx.x % QT) * 4;
     double pq[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int i = blockIdx.x * RPB + threadIdx.x / QT; i < A.rows; i += gridDim.x * RPB) {
-        const int s = i >> 4, hl = i & 15;
-        const int k0 = sslot[s], K = sslot[s + 1] - k0;
-        const int *tcol = A.tile_columnidx + A.tile_ptr[s];
+    const int step = gridDim.x * RPB, passes = (rows + step - 1) / step;
+    for (int ps = 0; ps < passes; ps++) {
+        const int i = (back ? passes - 1 - ps : ps) * step + blockIdx.x * RPB + threadIdx.x / QT;
+        if (i >= rows) continue;
+        const int s = i >> 4, lane = i & 15;
+        const int k0 = sslot[s];
+        int K = sslot[s + 1] - k0;
+        const OT *d = soff + (size_t)k0 * MF_TILE + lane;
+        const double *v = sval + (size_t)k0 * MF_TILE + lane;
+        const double *xi = X + (long long)i * KP + c0;
         double yd[4] = {0.0, 0.0, 0.0, 0.0}, part[4] = {0.0, 0.0, 0.0, 0.0};
-        int prevj = -1;
-#pragma unroll 4
-        for (int kk = 0; kk < K; kk++) {
-            const size_t e = (size_t)(k0 + kk) * MF_TILE + hl;
-            const unsigned m = smeta[e];
-            if (m == 0xFFFFu) continue;
-            const double v = sval[e];
-            const int tj = (int)(m >> 4);
-            const long long col = (long long)tcol[tj] * MF_TILE + (m & 15u);
-            const double2 xa = *(const double2 *)(X + col * KP + c0);
-            const double2 xb = *(const double2 *)(X + col * KP + c0 + 2);
-            if (tj != prevj) {
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    yd[q] = __dadd_rn(yd[q], part[q]);
-                    part[q] = 0.0;
-                }
-                prevj = tj;
-            }
-            part[0] = __dadd_rn(part[0], __dmul_rn(xa.x, v));
-            part[1] = __dadd_rn(part[1], __dmul_rn(xa.y, v));
-            part[2] = __dadd_rn(part[2], __dmul_rn(xb.x, v));
-            part[3] = __dadd_rn(part[3], __dmul_rn(xb.y, v));
+        int prev = INT_MIN;
+        for (; K >= MR_U; K -= MR_U, d += MR_U * MF_TILE, v += MR_U * MF_TILE)
+            mr_sums<KP, MR_U>(d, v, xi, lane, prev, yd, part);
+        switch (K) {  // straight code for every remainder: no load is predicated
+        case 7: mr_sums<KP, 7>(d, v, xi, lane, prev, yd, part); break;
+        case 6: mr_sums<KP, 6>(d, v, xi, lane, prev, yd, part); break;
+        case 5: mr_sums<KP, 5>(d, v, xi, lane, prev, yd, part); break;
+        case 4: mr_sums<KP, 4>(d, v, xi, lane, prev, yd, part); break;
+        case 3: mr_sums<KP, 3>(d, v, xi, lane, prev, yd, part); break;
+        case 2: mr_sums<KP, 2>(d, v, xi, lane, prev, yd, part); break;
+        case 1: mr_sums<KP, 1>(d, v, xi, lane, prev, yd, part); break;
+        default: break;
         }
         double y[4];
 #pragma unroll
         for (int q = 0; q < 4; q++) y[q] = __dadd_rn(yd[q], part[q]);
-        double *yo = Y + (long long)i * KP + c0;
-        *(double2 *)yo = make_double2(y[0], y[1]);
-        *(double2 *)(yo + 2) = make_double2(y[2], y[3]);
+        if (COLS) {
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (c0 + q < k) Y[(c0 + q) * ldy + i] = y[q];
+        } else {
+            double *yo = Y + (long long)i * KP + c0;
+            *(double2 *)yo = make_double2(y[0], y[1]);
+            *(double2 *)(yo + 2) = make_double2(y[2], y[3]);
+        }
         if (PQ) {
-            const double *xo = X + (long long)i * KP + c0;
-            const double2 pa = *(const double2 *)xo, pb = *(const double2 *)(xo + 2);
+            const double2 pa = *(const double2 *)xi, pb = *(const double2 *)(xi + 2);
             pq[0] = __dadd_rn(pq[0], __dmul_rn(pa.x, y[0]));
             pq[1] = __dadd_rn(pq[1], __dmul_rn(pa.y, y[1]));
             pq[2] = __dadd_rn(pq[2], __dmul_rn(pb.x, y[2]));
@@ -278,11 +341,25 @@ __global__ void __launch_bounds__(MR_NT, MR_SPMM_MINB) k_mr_spmm(MfTiles A, cons
     }
 }
 
-// x += alpha p, r -= alpha q; per-column r.r; the last block counts the
-// iteration, tests convergence and sets beta and the stop flag.
+// Calls f(e) for this thread's entries of a vector of `total`, e =
+// blockIdx.x * MR_NT + threadIdx.x + j * gridDim.x * MR_NT, j up or (back) down.
+template <class F>
+__device__ __forceinline__ void mr_sweep(long long total, int back, F f)
+{
+    const long long step = (long long)gridDim.x * MR_NT, e0 = (long long)blockIdx.x * MR_NT + threadIdx.x;
+    if (e0 >= total) return;
+    if (!back) {
+        for (long long e = e0; e < total; e += step) f(e);
+    } else {
+        for (long long e = e0 + (total - 1 - e0) / step * step; e >= 0; e -= step) f(e);
+    }
+}
+
+// r -= alpha q; per-column r.r; the last block counts the iteration, tests
+// convergence and sets beta and the stop flag.
 template <int KP>
-__global__ void __launch_bounds__(MR_NT, MR_VEC_MINB) k_mr_update(int n, double *__restrict__ x, double *__restrict__ r,
-                                                     const double *__restrict__ p, const double *__restrict__ q,
+__global__ void __launch_bounds__(MR_NT, MR_VEC_MINB) k_mr_update(int n, int back, double *__restrict__ r,
+                                                     const double *__restrict__ q,
                                                      double *__restrict__ partials, MrState *st, double tol, int fixed,
                                                      int maxiter)
 {
@@ -290,14 +367,12 @@ __global__ void __launch_bounds__(MR_NT, MR_VEC_MINB) k_mr_update(int n, double 
     __shared__ double tot[MR_MAXK];
     if (*(volatile int *)&st->stop) return;
     const double al = st->alpha[threadIdx.x % KP];
-    const long long total = (long long)n * KP;
     double rr = 0.0;
-    for (long long e = (long long)blockIdx.x * MR_NT + threadIdx.x; e < total; e += (long long)gridDim.x * MR_NT) {
-        x[e] = fma(al, p[e], x[e]);
+    mr_sweep((long long)n * KP, back, [&](long long e) {
         const double ri = fma(-al, q[e], r[e]);
         r[e] = ri;
         rr = __dadd_rn(rr, __dmul_rn(ri, ri));
-    }
+    });
     block_cols<KP>(rr, sw, partials + (size_t)blockIdx.x * KP);
     if (!mr_last_block(st)) return;
     sum_partials<KP>(partials, tot);
@@ -321,16 +396,20 @@ __global__ void __launch_bounds__(MR_NT, MR_VEC_MINB) k_mr_update(int n, double 
     }
 }
 
-// p = r + beta p (the same fused multiply-add as the single-vector CG).
+// x += alpha p, then p = r + beta p (the same fused multiply-adds as the
+// single-vector CG).  Runs once more after the stop flag is set: for the x of
+// the last iteration.
 template <int KP>
-__global__ void __launch_bounds__(MR_NT, MR_VEC_MINB) k_mr_pupdate(int n, const double *__restrict__ r, double *__restrict__ p,
-                                                      const MrState *st)
+__global__ void __launch_bounds__(MR_NT, MR_VEC_MINB) k_mr_pupdate(int n, int back, const double *__restrict__ r,
+                                                      double *__restrict__ p, double *__restrict__ x, const MrState *st)
 {
-    if (*(const volatile int *)&st->stop) return;
-    const double bt = st->beta[threadIdx.x % KP];
-    const long long total = (long long)n * KP;
-    for (long long e = (long long)blockIdx.x * MR_NT + threadIdx.x; e < total; e += (long long)gridDim.x * MR_NT)
-        p[e] = fma(bt, p[e], r[e]);
+    if (*(const volatile int *)&st->stop == 2) return;
+    const double al = st->alpha[threadIdx.x % KP], bt = st->beta[threadIdx.x % KP];
+    mr_sweep((long long)n * KP, back, [&](long long e) {
+        const double pv = p[e];
+        x[e] = fma(al, pv, x[e]);
+        p[e] = fma(bt, pv, r[e]);
+    });
 }
 
 // ||b - A x|| per column (q = A x given); the last block stores them.
@@ -369,30 +448,34 @@ int mr_grid(Kern kernel, long long work)
     return (int)std::max(1ll, std::min<long long>(cap, (work + MR_NT - 1) / MR_NT));
 }
 
-template <int KP>
-mf_status spmm_kp(mf_matrix m, const double *xi, double *yi, double *partials, MrState *st, bool pq, cudaStream_t s)
+// The SpMM of a matrix with 16- or 32-bit distances.
+template <int KP, bool PQ, bool COLS>
+void launch_spmm(mf_matrix m, int grid, const double *xi, double *y, int k, long long ldy, int back, double *partials,
+                 MrState *st, cudaStream_t s)
 {
-    const MfTiles &A = m->v;
-    const int grid = mr_grid(k_mr_spmm<KP, true>, (long long)A.rows * (KP / 4));
-    if (pq)
-        k_mr_spmm<KP, true><<<grid, MR_NT, 0, s>>>(A, m->d_sslot, m->d_smeta, m->d_sval, xi, yi, partials, st);
+    if (m->soff_bytes == 2)
+        k_mr_spmm<KP, PQ, COLS><<<grid, MR_NT, 0, s>>>(m->v.rows, m->d_sslot, (const int16_t *)m->d_soff, m->d_sval, xi,
+                                                       y, k, ldy, back, partials, st);
     else
-        k_mr_spmm<KP, false><<<grid, MR_NT, 0, s>>>(A, m->d_sslot, m->d_smeta, m->d_sval, xi, yi, partials, st);
+        k_mr_spmm<KP, PQ, COLS><<<grid, MR_NT, 0, s>>>(m->v.rows, m->d_sslot, (const int32_t *)m->d_soff, m->d_sval, xi,
+                                                       y, k, ldy, back, partials, st);
     note_launch();
-    MF_CUDA(cudaGetLastError());
-    return MF_OK;
+}
+
+template <int KP>
+int spmm_grid(mf_matrix m)
+{
+    const long long work = (long long)m->v.rows * (KP / 4);
+    return m->soff_bytes == 2 ? mr_grid(k_mr_spmm<KP, true, false, int16_t>, work)
+                              : mr_grid(k_mr_spmm<KP, true, false, int32_t>, work);
 }
 
 template <int KP>
 mf_status spmm_cm(mf_matrix m, int k, const double *X, int ldx, double *Y, int ldy, cudaStream_t s)
 {
     const MfTiles &A = m->v;
-    double *xi = nullptr, *yi = nullptr;
-    const cudaError_t ea = pool_malloc_async(&xi, sizeof(double) * ((size_t)A.cols * KP + KP), s);
-    const cudaError_t eb = pool_malloc_async(&yi, sizeof(double) * ((size_t)A.rows * KP + KP), s);
-    if (ea != cudaSuccess || eb != cudaSuccess) {
-        if (xi) cudaFreeAsync(xi, s);
-        if (yi) cudaFreeAsync(yi, s);
+    double *xi = nullptr;
+    if (pool_malloc_async(&xi, sizeof(double) * ((size_t)A.cols * KP + KP), s) != cudaSuccess) {
         set_last_error("multi-vector SpMM: no device memory for %d columns", KP);
         return MF_ERR_NO_MEMORY;
     }
@@ -400,14 +483,12 @@ mf_status spmm_cm(mf_matrix m, int k, const double *X, int ldx, double *Y, int l
     k_mr_pack<KP><<<mr_grid(k_mr_pack<KP>, (long long)A.cols * KP), MR_NT, 0, s>>>(A.cols, k, X, ldx, xi);
     note_launch();
     if (cudaGetLastError() != cudaSuccess) st = MF_ERR_CUDA;
-    if (st == MF_OK) st = spmm_kp<KP>(m, xi, yi, nullptr, nullptr, false, s);
     if (st == MF_OK) {
-        k_mr_unpack<KP><<<mr_grid(k_mr_unpack<KP>, (long long)A.rows * KP), MR_NT, 0, s>>>(A.rows, k, yi, Y, ldy);
-        note_launch();
+        // no partial sums here: as many blocks as there is work for
+        launch_spmm<KP, false, true>(m, ceil_div((long long)A.rows * (KP / 4), MR_NT), xi, Y, k, ldy, 0, nullptr, nullptr, s);
         if (cudaGetLastError() != cudaSuccess) st = MF_ERR_CUDA;
     }
     cudaFreeAsync(xi, s);
-    cudaFreeAsync(yi, s);
     if (st != MF_OK) set_last_error("multi-vector SpMM: kernel launch failed");
     return st;
 }
@@ -420,7 +501,7 @@ mf_status cg_multi_kp(mf_matrix m, int k, const double *B, int ldb, double *X, i
     const int n = A.rows;
     const size_t E = (size_t)n * KP + KP;
     const int gv = mr_grid(k_mr_update<KP>, (long long)n * KP);
-    const int gs = mr_grid(k_mr_spmm<KP, true>, (long long)n * (KP / 4));
+    const int gs = spmm_grid<KP>(m);
     const int fixed = o.tol < 0.0;
     // workspace kept in the matrix handle: 5 interleaved vectors, the
     // partials, the state (each region 256-byte aligned)
@@ -442,14 +523,17 @@ mf_status cg_multi_kp(mf_matrix m, int k, const double *B, int ldb, double *X, i
     double *partials = (double *)((char *)m->mr_work + vec_bytes);
     MrState *st = (MrState *)((char *)m->mr_work + vec_bytes + part_bytes);
     double *bi = buf, *xi = buf + E, *ri = buf + 2 * E, *pi = buf + 3 * E, *qi = buf + 4 * E;
-    auto launched = [&]() -> mf_status {
-        note_launch();
+    auto check = [&]() -> mf_status {
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) {
             set_last_error("multi-RHS CG: %s", cudaGetErrorString(e));
             return MF_ERR_CUDA;
         }
         return MF_OK;
+    };
+    auto launched = [&]() -> mf_status {
+        note_launch();
+        return check();
     };
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     mf_status rc = MF_OK;
@@ -468,7 +552,7 @@ mf_status cg_multi_kp(mf_matrix m, int k, const double *B, int ldb, double *X, i
         k_mr_init<KP><<<gv, MR_NT, 0, s>>>(n, k, bi, xi, ri, pi, partials, st, o.tol, fixed, o.maxiter);
         if ((rc = launched()) != MF_OK) break;
         // batches of iterations; every launch returns at once after the stop
-        int issued = 0, stop = 0;
+        int issued = 0, stop = 0, back = 0;
         while (rc == MF_OK) {
             if (cudaMemcpyAsync(&stop, &st->stop, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
                 cudaStreamSynchronize(s) != cudaSuccess) {
@@ -478,18 +562,20 @@ mf_status cg_multi_kp(mf_matrix m, int k, const double *B, int ldb, double *X, i
             }
             if (stop || issued >= o.maxiter) break;
             for (int t = 0; t < MR_BATCH && rc == MF_OK; t++) {
-                k_mr_spmm<KP, true><<<gs, MR_NT, 0, s>>>(A, m->d_sslot, m->d_smeta, m->d_sval, pi, qi, partials, st);
+                launch_spmm<KP, true, false>(m, gs, pi, qi, k, 0, back, partials, st, s);
+                if ((rc = check()) != MF_OK) break;
+                k_mr_update<KP><<<gv, MR_NT, 0, s>>>(n, !back, ri, qi, partials, st, o.tol, fixed, o.maxiter);
                 if ((rc = launched()) != MF_OK) break;
-                k_mr_update<KP><<<gv, MR_NT, 0, s>>>(n, xi, ri, pi, qi, partials, st, o.tol, fixed, o.maxiter);
+                k_mr_pupdate<KP><<<gv, MR_NT, 0, s>>>(n, back, ri, pi, xi, st);
                 if ((rc = launched()) != MF_OK) break;
-                k_mr_pupdate<KP><<<gv, MR_NT, 0, s>>>(n, ri, pi, st);
-                if ((rc = launched()) != MF_OK) break;
+                back = !back;  // three launches: the next SpMM starts where this one ended
             }
             issued += MR_BATCH;
         }
         if (rc != MF_OK) break;
         // true residuals from the FP64 SpMM of x, then x to the caller
-        if ((rc = spmm_kp<KP>(m, xi, qi, nullptr, nullptr, false, s)) != MF_OK) break;
+        launch_spmm<KP, false, false>(m, gs, xi, qi, k, 0, 0, nullptr, nullptr, s);
+        if ((rc = check()) != MF_OK) break;
         k_mr_resid<KP><<<gv, MR_NT, 0, s>>>(n, bi, qi, partials, st);
         if ((rc = launched()) != MF_OK) break;
         k_mr_unpack<KP><<<gv, MR_NT, 0, s>>>(n, k, xi, X, ldx);
@@ -507,10 +593,10 @@ mf_status cg_multi_kp(mf_matrix m, int k, const double *B, int ldb, double *X, i
     if (e1) cudaEventDestroy(e1);
     if (rc != MF_OK) return rc;
     // algorithmic bytes: per iteration the FP64 matrix stream once for all
-    // columns and 11 vector streams of n x KP (SpMM: p in, q out; update: x,
-    // p, q, r in, x, r out; p update: r, p in, p out)
+    // columns and 10 vector streams of n x KP (SpMM: p in, q out; r update: q, r
+    // in, r out; x and p update: r, p, x in, p, x out)
     const long long T = A.tilenum;
-    const long long per_it = (long long)A.nnz * 9 + 24 * T + 16LL * n + 88LL * n * KP;
+    const long long per_it = (long long)A.nnz * 9 + 24 * T + 16LL * n + 80LL * n * KP;
     mf_status ret = MF_OK;
     for (int j = 0; j < k; j++) {
         mf_solve_report &r = reports[j];
