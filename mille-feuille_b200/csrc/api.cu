@@ -16,35 +16,108 @@ static std::atomic<long long> g_launches{0};
 
 void note_launch(int k) { g_launches.fetch_add(k, std::memory_order_relaxed); }
 
+// The library's memory pool of a device and the stream that allocations kept
+// on handles are ordered on; made at first use.
+struct DevPool {
+    cudaMemPool_t pool = nullptr;
+    cudaStream_t stream = nullptr;
+};
+static std::mutex g_pool_mu;
+static DevPool g_pools[64];
+static std::atomic<int> g_handles[64];
+
+// What the pool keeps across synchronisations: up to 1 GiB while the device
+// has handles, up to 256 MiB otherwise.
+static constexpr uint64_t POOL_KEEP = 1024ull << 20, POOL_KEEP_IDLE = 256ull << 20;
+
+static cudaError_t device_pool(int *dev, DevPool *out)
+{
+    cudaError_t e = cudaGetDevice(dev);
+    if (e != cudaSuccess) return e;
+    if (*dev < 0 || *dev >= 64) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    DevPool &d = g_pools[*dev];
+    if (!d.pool) {
+        cudaMemPoolProps props;
+        memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = *dev;
+        e = cudaMemPoolCreate(&d.pool, &props);
+        if (e != cudaSuccess) {
+            d.pool = nullptr;
+            return e;
+        }
+        uint64_t keep = POOL_KEEP;
+        cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    *out = d;
+    return cudaSuccess;
+}
+
 cudaError_t pool_malloc_async(void **p, size_t bytes, cudaStream_t s)
 {
-    static std::mutex mu;
-    static cudaMemPool_t pools[64] = {};
     int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
+    DevPool d;
+    const cudaError_t e = device_pool(&dev, &d);
+    if (e == cudaErrorInvalidDevice && dev >= 64) return cudaMallocAsync(p, bytes, s);
     if (e != cudaSuccess) return e;
-    if (dev < 0 || dev >= 64) return cudaMallocAsync(p, bytes, s);
-    cudaMemPool_t pool;
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        if (!pools[dev]) {
-            cudaMemPoolProps props;
-            memset(&props, 0, sizeof(props));
-            props.allocType = cudaMemAllocationTypePinned;
-            props.handleTypes = cudaMemHandleTypeNone;
-            props.location.type = cudaMemLocationTypeDevice;
-            props.location.id = dev;
-            e = cudaMemPoolCreate(&pools[dev], &props);
-            if (e != cudaSuccess) {
-                pools[dev] = nullptr;
-                return e;
-            }
-            uint64_t keep = 256ull << 20;  // up to 256 MiB stays in the pool across synchronisations
-            cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep);
+    return cudaMallocFromPoolAsync(p, bytes, d.pool, s);
+}
+
+static cudaError_t handle_stream(cudaStream_t *out)
+{
+    int dev = 0;
+    DevPool d;
+    cudaError_t e = device_pool(&dev, &d);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    if (!g_pools[dev].stream) {
+        e = cudaStreamCreateWithFlags(&g_pools[dev].stream, cudaStreamNonBlocking);
+        if (e != cudaSuccess) {
+            g_pools[dev].stream = nullptr;
+            return e;
         }
-        pool = pools[dev];
     }
-    return cudaMallocFromPoolAsync(p, bytes, pool, s);
+    *out = g_pools[dev].stream;
+    return cudaSuccess;
+}
+
+// Memory kept on a handle, from the pool: ready for every stream when this
+// returns (its own stream is waited for, which holds nothing but these
+// allocations).
+cudaError_t handle_malloc(void **p, size_t bytes)
+{
+    *p = nullptr;
+    cudaStream_t hs = nullptr;
+    if (handle_stream(&hs) != cudaSuccess) return cudaMalloc(p, bytes);
+    cudaError_t e = pool_malloc_async(p, bytes, hs);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(hs);
+    if (e != cudaSuccess) *p = nullptr;
+    return e;
+}
+
+// Back to the pool; the caller has waited for everything that uses it.
+void handle_free(void *p)
+{
+    if (!p) return;
+    cudaStream_t hs = nullptr;
+    if (handle_stream(&hs) != cudaSuccess || cudaFreeAsync(p, hs) != cudaSuccess) {
+        cudaGetLastError();
+        cudaFree(p);
+    }
+}
+
+void handle_count(int device, int d)
+{
+    if (device < 0 || device >= 64) return;
+    if (g_handles[device].fetch_add(d) + d == 0 && d < 0) {
+        cudaStream_t hs = nullptr;
+        if (handle_stream(&hs) == cudaSuccess) cudaStreamSynchronize(hs);
+        std::lock_guard<std::mutex> lk(g_pool_mu);
+        if (g_pools[device].pool) cudaMemPoolTrimTo(g_pools[device].pool, POOL_KEEP_IDLE);
+    }
 }
 
 void set_last_error(const char *fmt, ...)
@@ -61,7 +134,7 @@ mf_status ensure_work(mf_matrix m, size_t bytes)
     if (m->work) cudaFree(m->work);
     m->work = nullptr;
     m->work_bytes = 0;
-    MF_CUDA(cudaMalloc(&m->work, bytes));
+    MF_CUDA(handle_malloc(&m->work, bytes));
     m->work_bytes = bytes;
     return MF_OK;
 }
@@ -151,6 +224,7 @@ mf_status mf_matrix_create(int rowA, int colA, const int *rowptr, const int *col
     mf_matrix m = new mf_matrix_s();
     memset(&m->v, 0, sizeof(m->v));
     cudaGetDevice(&m->device);
+    handle_count(m->device, 1);
     mf_status st = build_tiles(m, rowA, colA, d_rp, d_ci, d_v, d_vl, s);
     if (tmp) {
         cudaStreamSynchronize(s);
@@ -170,18 +244,14 @@ mf_status mf_matrix_destroy(mf_matrix m)
     int dev = -1;
     cudaGetDevice(&dev);
     if (dev != m->device) cudaSetDevice(m->device);
-    if (m->tiles_mem) {
-        // back to the pool once nothing on the device can still read it
-        cudaDeviceSynchronize();
-        cudaFreeAsync(m->tiles_mem, 0);
-    }
-    if (dev != m->device && dev >= 0) cudaSetDevice(dev);
-    void *bufs[] = {m->d_part, m->d_cta_chunk, m->d_chunks, m->work, m->host_io,
-                    m->d_wcls, m->d_poff, m->d_pay, m->d_resid, m->d_pol, m->d_sslot, m->d_smeta, m->d_sval, m->d_soff,
+    cudaDeviceSynchronize();  // nothing on the device can still use the handle's memory
+    void *bufs[] = {m->tiles_mem, m->d_part, m->d_cta_chunk, m->d_chunks, m->work, m->host_io,
+                    m->d_wcls, m->d_poff, m->d_pay, m->d_resid, m->d_pol, m->slots_mem,
                     m->d_shdr, m->d_spay, m->d_scta_chunk, m->d_schunks, m->d_spos, m->d_sdesc, m->mr_work,
                     m->mr_io, m->d_tc_index, m->d_tc_dense};
-    for (void *p : bufs)
-        if (p) cudaFree(p);
+    for (void *p : bufs) handle_free(p);
+    handle_count(m->device, -1);
+    if (dev != m->device && dev >= 0) cudaSetDevice(dev);
     delete m;
     return MF_OK;
 }
@@ -368,7 +438,7 @@ static mf_status solve_host_common(bool bicg, mf_matrix m, const double *b_host,
         if (m->host_io) cudaFree(m->host_io);
         m->host_io = nullptr;
         m->host_io_n = 0;
-        MF_CUDA(cudaMalloc(&m->host_io, sizeof(double) * (2 * n + 2)));
+        MF_CUDA(handle_malloc(&m->host_io, sizeof(double) * (2 * n + 2)));
         m->host_io_n = n;
     }
     double *db = m->host_io, *dx = m->host_io + n + 1;
@@ -474,7 +544,7 @@ mf_status mf_cg_solve_multi_host(mf_matrix m, int k, const double *B_host, doubl
         if (m->mr_io) cudaFree(m->mr_io);
         m->mr_io = nullptr;
         m->mr_io_bytes = 0;
-        MF_CUDA(cudaMalloc(&m->mr_io, 2 * bytes));
+        MF_CUDA(handle_malloc(&m->mr_io, 2 * bytes));
         m->mr_io_bytes = 2 * bytes;
     }
     double *dB = (double *)m->mr_io, *dX = dB + n * (size_t)k;

@@ -104,13 +104,13 @@ mf_status build_chunks(mf_matrix m, cudaStream_t s)
     if (m->d_chunks) cudaFree(m->d_chunks);
     m->d_cta_chunk = nullptr;
     m->d_chunks = nullptr;
-    MF_CUDA(cudaMalloc(&m->d_cta_chunk, sizeof(int) * (G + 1)));
+    MF_CUDA(handle_malloc(&m->d_cta_chunk, sizeof(int) * (G + 1)));
     k_chunk_count<<<grid_for3(G + 1, 128), 128, 0, s>>>(G, m->d_part, m->d_tile_ptr, m->d_tile_nnz, m->d_cta_chunk);
     note_launch();
     MF_CUDA(cudaGetLastError());
     int total = 0;
     MF_TRY(exclusive_scan_i32(m->d_cta_chunk, m->d_cta_chunk, G + 1, s, &total));
-    MF_CUDA(cudaMalloc(&m->d_chunks, sizeof(ChunkRec) * (total > 0 ? total : 1)));
+    MF_CUDA(handle_malloc(&m->d_chunks, sizeof(ChunkRec) * (total > 0 ? total : 1)));
     if (G > 0) {
         k_chunk_fill<<<grid_for3(G, 128), 128, 0, s>>>(G, m->d_part, m->d_tile_ptr, m->d_tile_nnz, m->d_cta_chunk,
                                                        (ChunkRec *)m->d_chunks);

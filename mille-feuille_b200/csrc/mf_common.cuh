@@ -18,11 +18,23 @@ void set_last_error(const char *fmt, ...);
 // Counts kernel launches issued by the library (mf_kernel_launches()).
 void note_launch(int k = 1);
 // Stream-ordered temporary allocation from the library's own memory pool of
-// the current device (created on first use; it keeps up to 256 MiB of freed
-// memory across synchronisations instead of returning it each time, so the
-// temporaries of a solve's checkpoints cost no driver allocation).  Free
-// with cudaFreeAsync.
+// the current device (created on first use; it keeps freed memory across
+// synchronisations instead of returning it each time -- up to 1 GiB while the
+// device has matrix handles, up to 256 MiB otherwise -- so the temporaries of
+// a solve's checkpoints cost no driver allocation).  Free with cudaFreeAsync.
 cudaError_t pool_malloc_async(void **p, size_t bytes, cudaStream_t s);
+// Memory kept on a handle, from the same pool (a driver allocation costs 0.1
+// to 1 ms, a matrix has up to twenty): usable on every stream at once.
+// handle_free returns it; nothing may still use it.  handle_count(device, +1 /
+// -1): a matrix handle was made / destroyed.
+cudaError_t handle_malloc(void **p, size_t bytes);
+void handle_free(void *p);
+void handle_count(int device, int d);
+template <typename T>
+inline cudaError_t handle_malloc(T **p, size_t bytes)
+{
+    return handle_malloc((void **)p, bytes);
+}
 template <typename T>
 inline cudaError_t pool_malloc_async(T **p, size_t bytes, cudaStream_t s)
 {

@@ -80,6 +80,7 @@ struct mf_matrix_s {
     std::atomic<int> slots_state{0};  // 0 not built, 1 built, -1 not describable
     std::atomic<int> spmv_calls{0};   // products from the tiles so far (mf_spmv)
     long long nslots = 0;
+    void *slots_mem = nullptr;     // the four arrays below live in it
     int *d_sslot = nullptr;
     uint16_t *d_smeta = nullptr;
     double *d_sval = nullptr;

@@ -512,7 +512,8 @@ mf_status cg_multi_kp(mf_matrix m, int k, const double *B, int ldb, double *X, i
         if (m->mr_work) cudaFree(m->mr_work);
         m->mr_work = nullptr;
         m->mr_work_bytes = 0;
-        if (cudaMalloc(&m->mr_work, need) != cudaSuccess) {
+        if (handle_malloc(&m->mr_work, need) != cudaSuccess) {
+            cudaGetLastError();
             m->mr_work = nullptr;
             set_last_error("multi-RHS CG: no device memory for 5 x %zu vector entries", E);
             return MF_ERR_NO_MEMORY;

@@ -90,7 +90,7 @@ mf_status static_working_classes(mf_matrix m, unsigned char *d_wcls, cudaStream_
 mf_status pack_payload(mf_matrix m, const unsigned char *d_wcls, cudaStream_t s)
 {
     const int T = m->v.tilenum;
-    if (!m->d_poff) MF_CUDA(cudaMalloc(&m->d_poff, sizeof(unsigned) * (T + 1) + 16));
+    if (!m->d_poff) MF_CUDA(handle_malloc(&m->d_poff, sizeof(unsigned) * (T + 1) + 16));
     int *sizes = nullptr;
     MF_CUDA(pool_malloc_async(&sizes, sizeof(int) * (T + 1), s));
     k_pack_sizes<<<grid_for(T + 1, 256), 256, 0, s>>>(T, m->d_tile_nnz, d_wcls, sizes);
@@ -110,7 +110,7 @@ mf_status pack_payload(mf_matrix m, const unsigned char *d_wcls, cudaStream_t s)
         m->pay_bytes = 0;
         // the largest packing (every tile FP32) bounds all later ones
         const size_t cap = (size_t)m->v.nnz * 4 + (size_t)T * 4 + 32;
-        MF_CUDA(cudaMalloc(&m->d_pay, cap > need ? cap : need));
+        MF_CUDA(handle_malloc(&m->d_pay, cap > need ? cap : need));
         m->pay_bytes = cap > need ? cap : need;
     }
     if (T > 0) {

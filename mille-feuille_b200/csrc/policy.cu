@@ -381,7 +381,7 @@ static mf_status policy_work(mf_matrix m, PolicyWork &pw, cudaStream_t s)
         if (m->d_pol) cudaFree(m->d_pol);
         m->d_pol = nullptr;
         m->pol_bytes = 0;
-        MF_CUDA(cudaMalloc(&m->d_pol, need));
+        MF_CUDA(handle_malloc(&m->d_pol, need));
         m->pol_bytes = need;
         m->pol_static_ready = 0;
         m->pol_have_prev = 0;

@@ -97,7 +97,7 @@ extern "C" mf_status mf_residual_norm(mf_matrix m, const double *b, const double
         if (m->d_resid) cudaFree(m->d_resid);
         m->d_resid = nullptr;
         m->resid_bytes = 0;
-        MF_CUDA(cudaMalloc(&m->d_resid, need));
+        MF_CUDA(handle_malloc(&m->d_resid, need));
         m->resid_bytes = need;
     }
     return residual_norm(m->v, b, x, m->d_resid, out, (cudaStream_t)stream);

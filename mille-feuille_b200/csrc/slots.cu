@@ -428,7 +428,7 @@ mf_status build_slot_chunks(mf_matrix m, int G, bool staged, cudaStream_t s)
     m->schunk_ctas = 0;
     m->schunk_mode = 0;
     m->schunk_staged = 0;
-    MF_CUDA(cudaMalloc(&m->d_scta_chunk, sizeof(int) * (G + 1)));
+    MF_CUDA(handle_malloc(&m->d_scta_chunk, sizeof(int) * (G + 1)));
     int *cnt = nullptr;
     MF_CUDA(pool_malloc_async(&cnt, sizeof(int) * (G + 2), s));
     int *unstaged = cnt + G + 1;
@@ -440,7 +440,7 @@ mf_status build_slot_chunks(mf_matrix m, int G, bool staged, cudaStream_t s)
     MF_CUDA(cudaGetLastError());
     int total = 0;
     MF_TRY(exclusive_scan_i32(cnt, m->d_scta_chunk, G + 1, s, &total));
-    MF_CUDA(cudaMalloc(&m->d_schunks, sizeof(SlotChunk) * (size_t)(total > 0 ? total : 1)));
+    MF_CUDA(handle_malloc(&m->d_schunks, sizeof(SlotChunk) * (size_t)(total > 0 ? total : 1)));
     k_slot_chunk_fill<<<grid_for3(G, WALK_NT), WALK_NT, 0, s>>>(G, m->d_part, m->d_sslot, m->d_tile_ptr, tcol,
                                                         staged ? 1 : 0, m->d_scta_chunk, (SlotChunk *)m->d_schunks,
                                                         unstaged);
@@ -455,8 +455,8 @@ mf_status build_slot_chunks(mf_matrix m, int G, bool staged, cudaStream_t s)
     m->schunk_mode = mode;
     m->schunk_unstaged = h_unstaged;
     if (staged && !h_unstaged) {
-        if (!m->d_spos) MF_CUDA(cudaMalloc(&m->d_spos, sizeof(uint16_t) * (size_t)m->nslots * MF_TILE + 32));
-        if (!m->d_sdesc) MF_CUDA(cudaMalloc(&m->d_sdesc, sizeof(int2) * ((size_t)m->v.tilem + 2)));
+        if (!m->d_spos) MF_CUDA(handle_malloc(&m->d_spos, sizeof(uint16_t) * (size_t)m->nslots * MF_TILE + 32));
+        if (!m->d_sdesc) MF_CUDA(handle_malloc(&m->d_sdesc, sizeof(int2) * ((size_t)m->v.tilem + 2)));
         if (total > 0) {
             k_slot_pos<<<grid_for3((long long)total * 16 * MF_TILE, 256), 256, 0, s>>>(
                 m->v, total, (const SlotChunk *)m->d_schunks, m->d_sslot, m->d_smeta, m->d_spos, m->d_sdesc);
@@ -509,22 +509,19 @@ mf_status build_slots(mf_matrix m, cudaStream_t s, long long most)
         return MF_OK;
     }
     // slack: 16-byte bulk-copy rounding
-    if (cudaMalloc(&m->d_sslot, sizeof(int) * (tilem + 1) + 32) != cudaSuccess ||
-        cudaMalloc(&m->d_smeta, sizeof(uint16_t) * E + 32) != cudaSuccess ||
-        cudaMalloc(&m->d_sval, sizeof(double) * E + 32) != cudaSuccess ||
-        cudaMalloc(&m->d_soff, ob * E + 32) != cudaSuccess) {
+    const size_t o_val = (sizeof(int) * ((size_t)tilem + 1) + 32 + 255) / 256 * 256,
+                 o_off = o_val + (sizeof(double) * E + 32 + 255) / 256 * 256,
+                 o_meta = o_off + (ob * E + 32 + 255) / 256 * 256;
+    if (handle_malloc(&m->slots_mem, o_meta + sizeof(uint16_t) * E + 32) != cudaSuccess) {
         cudaGetLastError();
-        if (m->d_sslot) cudaFree(m->d_sslot);
-        if (m->d_smeta) cudaFree(m->d_smeta);
-        if (m->d_sval) cudaFree(m->d_sval);
-        m->d_sslot = nullptr;
-        m->d_smeta = nullptr;
-        m->d_sval = nullptr;
-        m->d_soff = nullptr;
         cudaFreeAsync(d_K, s);
         set_last_error("no device memory for the row slots (%zu entries)", E);
         return MF_ERR_NO_MEMORY;
     }
+    m->d_sslot = (int *)m->slots_mem;
+    m->d_sval = (double *)((char *)m->slots_mem + o_val);
+    m->d_soff = (char *)m->slots_mem + o_off;
+    m->d_smeta = (uint16_t *)((char *)m->slots_mem + o_meta);
     MF_CUDA(cudaMemcpyAsync(m->d_sslot, d_at, sizeof(int) * (tilem + 1), cudaMemcpyDeviceToDevice, s));
     cudaFreeAsync(d_K, s);
     if (tilem > 0) {
@@ -547,8 +544,8 @@ mf_status pack_slots(mf_matrix m, const unsigned char *d_wcls, cudaStream_t s)
     const MfTiles &A = m->v;
     const int ns = (int)m->nslots;
     if (!m->d_shdr) {
-        MF_CUDA(cudaMalloc(&m->d_shdr, sizeof(unsigned) * ((size_t)ns + 1) + (size_t)ns + 32));
-        MF_CUDA(cudaMalloc(&m->d_spay, (size_t)ns * 64 + 64));
+        MF_CUDA(handle_malloc(&m->d_shdr, sizeof(unsigned) * ((size_t)ns + 1) + (size_t)ns + 32));
+        MF_CUDA(handle_malloc(&m->d_spay, (size_t)ns * 64 + 64));
     }
     unsigned char *srank = (unsigned char *)(m->d_shdr + ns + 1);
     int *sizes = nullptr;

@@ -84,7 +84,7 @@ static mf_status persistent_solve(bool bicg, mf_matrix m, const double *b, doubl
     // other mixed policy
     const int base_policy = o.policy == MF_POLICY_STATIC_FP16 ? MF_POLICY_STATIC_FP16 : MF_POLICY_STATIC;
     if (mixed) {
-        if (!m->d_wcls) MF_CUDA(cudaMalloc(&m->d_wcls, (size_t)T + 16));
+        if (!m->d_wcls) MF_CUDA(handle_malloc(&m->d_wcls, (size_t)T + 16));
         if ((slots ? m->slot_policy : m->packed_policy) != base_policy) {
             MF_TRY(static_working_classes(m, m->d_wcls, s, base_policy == MF_POLICY_STATIC_FP16));
             MF_TRY(repack(base_policy));

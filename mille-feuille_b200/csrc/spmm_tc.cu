@@ -256,7 +256,7 @@ mf_status tc_prepare(mf_matrix m, int fill, cudaStream_t s)
     m->d_tc_dense = nullptr;
     m->tc_fill = 0;
     m->tc_ndense = 0;
-    MF_CUDA(cudaMalloc(&m->d_tc_index, sizeof(int) * (size_t)(T + 1) + 16));
+    MF_CUDA(handle_malloc(&m->d_tc_index, sizeof(int) * (size_t)(T + 1) + 16));
     int *flag = nullptr;
     MF_CUDA(pool_malloc_async(&flag, sizeof(int) * (size_t)(T + 1) + 16, s));
     int nd = 0;
@@ -270,7 +270,7 @@ mf_status tc_prepare(mf_matrix m, int fill, cudaStream_t s)
         MF_CUDA(cudaGetLastError());
     }
     cudaFreeAsync(flag, s);
-    MF_CUDA(cudaMalloc(&m->d_tc_dense, sizeof(__half) * 256 * (size_t)(nd > 0 ? nd : 1)));
+    MF_CUDA(handle_malloc(&m->d_tc_dense, sizeof(__half) * 256 * (size_t)(nd > 0 ? nd : 1)));
     if (nd > 0) {
         k_tc_fill<<<tc_grid((long long)T * 32, TC_NT), TC_NT, 0, s>>>(m->v, T, m->d_tile_rowidx, m->d_tc_index,
                                                                        (__half *)m->d_tc_dense);

@@ -848,7 +848,7 @@ mf_status strip_partition(mf_matrix m, int ctas, cudaStream_t s)
     m->d_part = nullptr;
     m->part_ctas = 0;
     const int tilem = m->v.tilem;
-    MF_CUDA(cudaMalloc(&m->d_part, sizeof(int) * (ctas + 1)));
+    MF_CUDA(handle_malloc(&m->d_part, sizeof(int) * (ctas + 1)));
     int *d_cost = nullptr;
     MF_CUDA(pool_malloc_async(&d_cost, sizeof(int) * (tilem + 1), s));
     k_strip_cost<<<grid_for(tilem + 1, 256), 256, 0, s>>>(tilem, m->d_tile_ptr, m->d_tile_nnz, d_cost);
