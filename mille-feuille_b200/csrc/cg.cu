@@ -395,7 +395,9 @@ __global__ void __launch_bounds__(NT, LAY == 0 ? MINB : SMINB) k_cg1(CgArgs a)
         };
         if (!spmv_any<0, LAY>(a, S, gc, cb, ce, sb0, se0, psrc, aout, nullptr)) gc.ok = false;
         double d[4];
-        grid_sum4(a, l, 4, gc, S, d);
+        // two sets of partials in turn: a CTA that is ahead writes the next
+        // ones while others still read these
+        grid_sum4(a, l, ((it + 1) & 1) ? 0 : 4, gc, S, d);
         if (!gc.ok) break;
         it++;
         rr = d[3];
@@ -429,6 +431,222 @@ __global__ void __launch_bounds__(NT, LAY == 0 ? MINB : SMINB) k_cg1(CgArgs a)
         st[S_RELRES] = sqrt(rr) / nb;
     }
 }
+
+// The same method for small short-row systems: a thread per row that keeps
+// its row's entries (at most ROWS_K), its x, r, q and p in registers for the
+// whole solve.  A neighbour's r, q and p lie in one 32-byte record (double
+// buffered), so a pass is one round of gathers, the row's sum, one record
+// written, and the reduction.  The reduction's scalars (alpha, beta, the stop
+// test) are worked out by warp 0 alone before the CTA barrier that hands them
+// out.  Taken for rows of at most ROWS_K entries and at most as many rows as
+// threads are resident (2 CTAs per SM: 75,776); above, k_cg1 streams the slots
+// (13.7 us per iteration at 216,000 rows).  Bound by latency: gathers from L2,
+// FP64 chains, the grid barrier.  Against k_cg1, us per iteration: 1,024 rows
+// (5-point) 6.9 -> 3.6, 16,384 rows 6.9 -> 4.0, 72,900 rows 8.4 -> 6.2, 74,046
+// rows (7-point) 9.4 -> 7.1.
+constexpr int ROWS_K = 8;
+constexpr int ROWS_MINB = 2;  // CTAs per SM: 128 registers
+
+struct __align__(32) RowRec {
+    double r, q, p, pad;
+};
+
+template <typename OT>
+__global__ void __launch_bounds__(NT, ROWS_MINB) k_cg1_rows(CgArgs a)
+{
+    constexpr OT EMPTY = (OT)(sizeof(OT) == 2 ? INT16_MIN : INT32_MIN);
+    __shared__ double s_w[NT / 32][4];
+    __shared__ double s_out[4];  // alpha, beta, r.r, ||r|| for the history
+    __shared__ int s_exit;       // -1: go on, else the exit reason
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, G = gridDim.x, g = blockIdx.x;
+    const int i = g * NT + tid;
+    const bool row = i < a.A.rows;
+    const size_t npad = (size_t)a.A.tilem * MF_TILE + 16;
+    RowRec *buf[2] = {(RowRec *)a.r, (RowRec *)a.r + npad};
+    // the row's entries: column (-1: none), value, first entry of a tile
+    int col[ROWS_K];
+    double val[ROWS_K];
+    unsigned first = 0;
+    {
+        const int s = i >> 4, k0 = row ? a.sslot[s] : 0, K = row ? a.sslot[s + 1] - k0 : 0;
+        const size_t e0 = (size_t)k0 * MF_TILE + (i & 15);
+        int prev = -1;
+#pragma unroll
+        for (int u = 0; u < ROWS_K; u++) {
+            const OT d = u < K ? ((const OT *)a.soff)[e0 + (size_t)u * MF_TILE] : EMPTY;
+            col[u] = d != EMPTY ? i + (int)d : -1;
+            val[u] = d != EMPTY ? a.sval[e0 + (size_t)u * MF_TILE] : 0.0;
+            if (col[u] >= 0 && (col[u] >> 4) != prev) {
+                first |= 1u << u;
+                prev = col[u] >> 4;
+            }
+            if (col[u] >= a.A.rows) col[u] = -1;  // columns past the rows meet zeros
+        }
+    }
+    double r = row ? a.b[i] : 0.0, q = 0.0, p = 0.0, x = 0.0;
+    auto put = [&](RowRec *to) {
+        if (!row) return;
+        double2 *d = (double2 *)(to + i);
+        d[0] = make_double2(r, q);
+        d[1] = make_double2(p, 0.0);
+    };
+    put(buf[0]);
+    unsigned long long epoch = 0;
+    // sums of l over the grid in v (lanes of warp 0, every CTA the same bits);
+    // false when a wait gave up.  Only warp 0 returns with sums.
+    auto exchange = [&](double (&l)[4], double (&v)[4]) -> bool {
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) l[k] += __shfl_xor_sync(0xffffffffu, l[k], o);
+        if (lane == 0)
+#pragma unroll
+            for (int k = 0; k < 4; k++) s_w[w][k] = l[k];
+        __syncthreads();
+        if (w != 0) return true;
+        // lane k * 8 + warp: the CTA's four sums
+        double c = s_w[lane & 7][lane >> 3];
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+        // two sets of partials in turn: a CTA that is ahead writes the next
+        // ones while others still read these
+        epoch++;
+        double *part = a.partials + (epoch & 1) * 4 * G;
+        if ((lane & 7) == 0) part[(lane >> 3) * G + g] = c;
+        __syncwarp();
+        int ok = 1;
+        if (lane == 0) {
+            // the CTA's stores (before its barrier) and the lanes' partials,
+            // then the arrival
+            fence_acq_rel_gpu();
+            red_add_release_u64(a.bar, 1ull);
+            const unsigned long long target = epoch * (unsigned long long)G;
+            if (ld_relaxed_u64(a.bar) < target) {
+                const unsigned long long t0 = globaltimer_ns();
+                unsigned spins = 0;
+                while (ld_relaxed_u64(a.bar) < target) {
+                    if ((++spins & 15u) == 0u) {
+                        if (ld_volatile_i32(a.status) != DEV_OK) { ok = 0; break; }
+                        if (globaltimer_ns() - t0 > a.budget_ns) {
+                            atomicCAS(a.status, DEV_OK, DEV_TIMEOUT);
+                            ok = 0;
+                            break;
+                        }
+                    }
+                }
+            }
+            fence_acq_rel_gpu();  // with the relaxed load that saw the target: acquire
+        }
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[k] = 0.0;
+        for (int j = lane; j < G; j += 32)
+#pragma unroll
+            for (int k = 0; k < 4; k++) v[k] += __ldcg(part + k * G + j);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+        return ok != 0;
+    };
+    double l[4] = {__dmul_rn(r, r), 0.0, 0.0, 0.0}, v[4] = {0.0, 0.0, 0.0, 0.0};
+    bool ok = exchange(l, v);
+    double nb = 0.0, limit = 0.0;  // warp 0
+    if (w == 0) {
+        const double bb = v[0];
+        nb = sqrt(bb) > 0.0 ? sqrt(bb) : 1.0;
+        limit = a.tol * nb;
+        if (lane == 0) s_exit = ok ? -1 : (int)EXIT_MAXITER;
+        if (a.hist && g == 0 && lane == 0) a.hist[0] = sqrt(bb) / nb;
+    }
+    __syncthreads();
+    double al = 0.0, be = 0.0, rr = 0.0;
+    int it = -1, o = 0;  // updates done; pass 0 makes r_0
+    int reason = s_exit;
+    while (reason < 0) {
+        const RowRec *old = buf[o];
+        // the neighbours' records, all in flight
+        double2 ga[ROWS_K];
+        double gp[ROWS_K];
+#pragma unroll
+        for (int u = 0; u < ROWS_K; u++) {
+            ga[u] = make_double2(0.0, 0.0);
+            gp[u] = 0.0;
+            if (col[u] >= 0) {
+                ga[u] = __ldcg((const double2 *)(old + col[u]));
+                gp[u] = __ldcg((const double *)(old + col[u]) + 2);
+            }
+        }
+        double yd = 0.0, part = 0.0;
+#pragma unroll
+        for (int u = 0; u < ROWS_K; u++) {
+            const double pu = fma(be, gp[u], fma(-al, ga[u].y, ga[u].x));
+            if ((first >> u) & 1u) {
+                yd = __dadd_rn(yd, part);
+                part = 0.0;
+            }
+            part = __dadd_rn(part, __dmul_rn(pu, val[u]));
+        }
+        const double y = __dadd_rn(yd, part);
+        const double pn = fma(be, p, fma(-al, q, r));
+        r = fma(-al, q, r);
+        x = fma(al, p, x);
+        p = pn;
+        q = y;
+        o ^= 1;
+        put(buf[o]);
+        l[0] = __dmul_rn(p, q);
+        l[1] = __dmul_rn(r, q);
+        l[2] = __dmul_rn(q, q);
+        l[3] = __dmul_rn(r, r);
+        ok = exchange(l, v);
+        it++;
+        if (w == 0) {
+            const double s = v[3];
+            int ex = -1;
+            double na = 0.0, nbe = 0.0;
+            const bool done = (!a.fixed && sqrt(s) <= limit) || s == 0.0;
+            if (!ok) {
+                ex = EXIT_MAXITER;  // the status word tells
+            } else if (done) {
+                ex = EXIT_CONVERGED;
+            } else if (it >= a.maxiter) {
+                ex = EXIT_MAXITER;
+            } else if (!(v[0] != 0.0) || !isfinite(v[0])) {
+                if (g == 0 && lane == 0) atomicCAS(a.status, DEV_OK, DEV_BREAKDOWN);
+                ex = EXIT_BREAKDOWN;
+            } else {
+                na = s / v[0];
+                nbe = (s - 2.0 * na * v[1] + na * na * v[2]) / s;
+            }
+            if (lane == 0) {
+                s_out[0] = na;
+                s_out[1] = nbe;
+                s_out[2] = s;
+                s_exit = ex;
+                if (a.hist && g == 0 && ok) a.hist[it] = sqrt(s) / nb;
+            }
+        }
+        __syncthreads();
+        al = s_out[0];
+        be = s_out[1];
+        rr = s_out[2];
+        reason = s_exit;
+    }
+    if (row) a.xhi[i] = x;
+    if (g == 0 && tid == 0) {
+        double *st = a.state;
+        st[S_RHO] = rr;
+        st[S_BETA] = be;
+        st[S_NB] = nb;
+        st[S_RMAX] = sqrt(rr);
+        st[S_ITERS] = (double)(it < 0 ? 0 : it);
+        st[S_REFS] = 0.0;
+        st[S_EXIT] = (double)reason;
+        st[S_RELRES] = sqrt(rr) / nb;
+    }
+}
+static_assert(sizeof(RowRec) == 4 * sizeof(double), "two record buffers fit eight solver vectors");
 
 // Jacobi: 1 / a_ii of every row from the tile format (the diagonal tile of
 // the row's strip, the row's entry in its column), 1 where the diagonal is
@@ -630,17 +848,32 @@ mf_status launch_cg(bool mixed, CgArgs &a, int G, cudaStream_t s)
     if (!mixed && a.one_reduction) {
         // the grid was sized for k_cg; k_cg1 runs when as many of its CTAs
         // are resident (same launch bounds, its own occupancy checked once)
-        static int resident[2] = {-1, -1};
-        const int li = a.sslot ? 1 : 0;
-        dyn = a.sslot ? smem_bytes<1>() : smem_bytes<0>();
-        fn = a.sslot ? (const void *)k_cg1<1> : (const void *)k_cg1<0>;
-        if (resident[li] < 0) {
-            int dev = 0, sms = 0, per = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            MF_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-            MF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, NT, dyn));
-            resident[li] = sms * per;
+        static int resident[4] = {-1, -1, -1, -1};
+        const bool rows = a.sslot && a.slot_kmax <= ROWS_K && G == ceil_div(a.A.rows, NT);
+        int li = rows ? (a.soff_bytes == 2 ? 2 : 3) : a.sslot ? 1 : 0;
+        auto pick = [&]() {
+            dyn = li >= 2 ? 0 : li ? smem_bytes<1>() : smem_bytes<0>();
+            fn = li == 3   ? (const void *)k_cg1_rows<int32_t>
+                 : li == 2 ? (const void *)k_cg1_rows<int16_t>
+                 : li      ? (const void *)k_cg1<1>
+                           : (const void *)k_cg1<0>;
+        };
+        auto fits = [&]() -> mf_status {
+            pick();
+            if (resident[li] < 0) {
+                int dev = 0, sms = 0, per = 0;
+                cudaGetDevice(&dev);
+                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+                MF_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+                MF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, NT, dyn));
+                resident[li] = sms * per;
+            }
+            return MF_OK;
+        };
+        MF_TRY(fits());
+        if (G > resident[li] && li >= 2) {  // more rows than resident threads: the chunked kernel
+            li = 1;
+            MF_TRY(fits());
         }
         if (G <= resident[li]) {
             MF_CUDA(cudaLaunchCooperativeKernel(fn, dim3(G), dim3(NT), args, dyn, s));

@@ -86,6 +86,7 @@ struct mf_matrix_s {
     double *d_sval = nullptr;
     void *d_soff = nullptr;    // column - row of every slot entry, int16 or int32
     int soff_bytes = 0;        // 2 or 4
+    int slot_kmax = 0;         // most slots of a strip (entries of the longest row)
     unsigned *d_shdr = nullptr;
     unsigned char *d_spay = nullptr;
     int slot_policy = -1;      // policy whose classes the slot payload holds

@@ -56,8 +56,10 @@ __device__ __forceinline__ void row_bounds(const MfTiles &A, int t, int r, int r
 }
 
 // K of every strip (half-warp per strip); flags strips with too many tiles;
-// the most tile columns a strip's tiles lie from its own (16-bit distances).
-__global__ void k_slot_count(MfTiles A, int *__restrict__ K, int *__restrict__ too_many, int *__restrict__ far)
+// the most tile columns a strip's tiles lie from its own (16-bit distances) and
+// the largest K.
+__global__ void k_slot_count(MfTiles A, int *__restrict__ K, int *__restrict__ too_many, int *__restrict__ far,
+                             int *__restrict__ kmax)
 {
     const int hl = threadIdx.x & 15;
     for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 4; s <= A.tilem; s += (gridDim.x * blockDim.x) >> 4) {
@@ -79,6 +81,7 @@ __global__ void k_slot_count(MfTiles A, int *__restrict__ K, int *__restrict__ t
             // tiles ascend by column: the first and the last lie farthest
             const int d = t1 > t0 ? max(s - A.tile_columnidx[t0], A.tile_columnidx[t1 - 1] - s) : 0;
             if (d > *(volatile int *)far) atomicMax(far, d);
+            if (cnt > *(volatile int *)kmax) atomicMax(kmax, cnt);
             K[s] = cnt;
             if (t1 - t0 > SLOT_MAX_TILES) atomicExch(too_many, 1);
         }
@@ -484,15 +487,15 @@ mf_status build_slots(mf_matrix m, cudaStream_t s, long long most)
     const MfTiles &A = m->v;
     const int tilem = A.tilem;
     int *d_K = nullptr, *d_flag = nullptr;
-    // one temporary: slots per strip, flag and farthest tile, their scan
-    MF_CUDA(pool_malloc_async(&d_K, sizeof(int) * 2 * ((size_t)tilem + 2), s));
+    // one temporary: slots per strip; flag, farthest tile, largest K; their scan
+    MF_CUDA(pool_malloc_async(&d_K, sizeof(int) * 2 * ((size_t)tilem + 3), s));
     d_flag = d_K + tilem + 1;
-    int *d_at = d_flag + 2;
-    MF_CUDA(cudaMemsetAsync(d_flag, 0, 2 * sizeof(int), s));
-    k_slot_count<<<grid_for3((long long)(tilem + 1) * 16, 256), 256, 0, s>>>(A, d_K, d_flag, d_flag + 1);
+    int *d_at = d_flag + 3;
+    MF_CUDA(cudaMemsetAsync(d_flag, 0, 3 * sizeof(int), s));
+    k_slot_count<<<grid_for3((long long)(tilem + 1) * 16, 256), 256, 0, s>>>(A, d_K, d_flag, d_flag + 1, d_flag + 2);
     note_launch();
     MF_CUDA(cudaGetLastError());
-    int total = 0, h_flag[2] = {0, 0};
+    int total = 0, h_flag[3] = {0, 0, 0};
     MF_TRY(exclusive_scan_i32(d_K, d_at, tilem + 1, s, &total));
     MF_CUDA(cudaMemcpyAsync(h_flag, d_flag, sizeof(h_flag), cudaMemcpyDeviceToHost, s));
     MF_CUDA(cudaStreamSynchronize(s));
@@ -534,6 +537,7 @@ mf_status build_slots(mf_matrix m, cudaStream_t s, long long most)
     MF_CUDA(cudaStreamSynchronize(s));
     m->nslots = total;
     m->soff_bytes = ob;
+    m->slot_kmax = h_flag[2];
     m->slot_policy = -1;
     m->slots_state.store(1, std::memory_order_release);
     return MF_OK;

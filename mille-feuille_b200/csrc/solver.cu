@@ -103,6 +103,9 @@ static mf_status persistent_solve(bool bicg, mf_matrix m, const double *b, doubl
         a.sslot = m->d_sslot;
         a.smeta = m->d_smeta;
         a.sval = m->d_sval;
+        a.soff = m->d_soff;
+        a.soff_bytes = m->soff_bytes;
+        a.slot_kmax = m->slot_kmax;
         a.shdr = m->d_shdr;
         a.spay = m->d_spay;
         a.scta_chunk = m->d_scta_chunk;

@@ -110,6 +110,9 @@ struct CgArgs {
     // Jacobi-preconditioned CG (null otherwise)
     void *z;                       // z = D^-1 r (solver's vector type)
     const double *dinv;            // [rows] 1 / diagonal (1 where the diagonal is 0)
+    // column - row of the slot entries (k_cg1_rows), and their size
+    const void *soff;
+    int soff_bytes, slot_kmax;
 };
 
 struct SolverWork {
