@@ -26,9 +26,11 @@ static std::mutex g_pool_mu;
 static DevPool g_pools[64];
 static std::atomic<int> g_handles[64];
 
-// What the pool keeps across synchronisations: up to 1 GiB while the device
-// has handles, up to 256 MiB otherwise.
-static constexpr uint64_t POOL_KEEP = 1024ull << 20, POOL_KEEP_IDLE = 256ull << 20;
+// What the pool holds across synchronisations, used and free together: up to
+// 4 GiB while the device has handles (a 2-million-row matrix with its solver
+// workspace takes 0.65 GB; mapping that anew costs 12 ms), up to 256 MiB
+// otherwise.
+static constexpr uint64_t POOL_KEEP = 4096ull << 20, POOL_KEEP_IDLE = 256ull << 20;
 
 static cudaError_t device_pool(int *dev, DevPool *out)
 {

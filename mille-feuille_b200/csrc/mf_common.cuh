@@ -19,7 +19,7 @@ void set_last_error(const char *fmt, ...);
 void note_launch(int k = 1);
 // Stream-ordered temporary allocation from the library's own memory pool of
 // the current device (created on first use; it keeps freed memory across
-// synchronisations instead of returning it each time -- up to 1 GiB while the
+// synchronisations instead of returning it each time -- up to 4 GiB while the
 // device has matrix handles, up to 256 MiB otherwise -- so the temporaries of
 // a solve's checkpoints cost no driver allocation).  Free with cudaFreeAsync.
 cudaError_t pool_malloc_async(void **p, size_t bytes, cudaStream_t s);
