@@ -250,7 +250,7 @@ mf_status mf_matrix_destroy(mf_matrix m)
     void *bufs[] = {m->tiles_mem, m->d_part, m->d_cta_chunk, m->d_chunks, m->work, m->host_io,
                     m->d_wcls, m->d_poff, m->d_pay, m->d_resid, m->d_pol, m->slots_mem,
                     m->d_shdr, m->d_spay, m->d_scta_chunk, m->d_schunks, m->d_spos, m->d_sdesc, m->mr_work,
-                    m->mr_io, m->d_tc_index, m->d_tc_dense};
+                    m->mr_io, m->tc_mem};
     for (void *p : bufs) handle_free(p);
     handle_count(m->device, -1);
     if (dev != m->device && dev >= 0) cudaSetDevice(dev);

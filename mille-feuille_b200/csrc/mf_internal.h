@@ -111,12 +111,16 @@ struct mf_matrix_s {
     size_t mr_work_bytes = 0;
     void *mr_io = nullptr;
     size_t mr_io_bytes = 0;
-    // tensor-core SpMM (spmm_tc.cu): dense FP16 copies of the tiles with at
-    // least tc_fill entries, and each tile's index among them (-1: sparse)
+    // tensor-core SpMM (spmm_tc.cu): per strip its dense tiles (at least
+    // tc_fill entries) and its other entries; one allocation
     int tc_fill = 0;
     int tc_ndense = 0;
-    int *d_tc_index = nullptr;
-    void *d_tc_dense = nullptr;
+    void *tc_mem = nullptr;
+    int *d_tc_dptr = nullptr;      // [tilem+1] first dense tile of each strip
+    int *d_tc_dcol = nullptr;      // tile column of each dense tile
+    int *d_tc_rptr = nullptr;      // [16*tilem+1] first other entry of each row
+    int2 *d_tc_sent = nullptr;     // column and FP32 value bits
+    void *d_tc_dense = nullptr;    // FP16 blocks in MMA fragment order
 };
 
 namespace mf {
