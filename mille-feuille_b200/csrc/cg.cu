@@ -233,8 +233,12 @@ __global__ void __launch_bounds__(NT, LAY == 0 ? MINB : LAY == 1 ? SMINB : stage
         }
         MF_MARK(2);
         double rho_new, rz_new = 0.0;
-        if constexpr (PC) grid_sum_pair(a, loc, locz, 3, gc, S, rho_new, rz_new);
-        else rho_new = grid_sum(a, loc, 3, gc, S);
+        if constexpr (PC) {
+            double d[2];
+            grid_sums<2>(a, {loc, locz}, 3, gc, S, d);
+            rho_new = d[0];
+            rz_new = d[1];
+        } else rho_new = grid_sum(a, loc, 3, gc, S);
         MF_MARK(3);
         if (!gc.ok) break;
         it++;
@@ -271,8 +275,12 @@ __global__ void __launch_bounds__(NT, LAY == 0 ? MINB : LAY == 1 ? SMINB : stage
             } else {
                 if (!spmv_any<0, LAY>(a, S, gc, cb, ce, sb0, se0, xsrc, rout, nullptr)) gc.ok = false;
             }
-            if constexpr (PC) grid_sum_pair(a, loc, locz, 0, gc, S, rho_new, rz_new);
-            else rho_new = grid_sum(a, loc, 1, gc, S);
+            if constexpr (PC) {
+                double d[2];
+                grid_sums<2>(a, {loc, locz}, 0, gc, S, d);
+                rho_new = d[0];
+                rz_new = d[1];
+            } else rho_new = grid_sum(a, loc, 1, gc, S);
             if (!gc.ok) break;
             rmax = sqrt(rho_new);
             relres_true = sqrt(rho_new) / nb;
@@ -397,7 +405,7 @@ __global__ void __launch_bounds__(NT, LAY == 0 ? MINB : SMINB) k_cg1(CgArgs a)
         double d[4];
         // two sets of partials in turn: a CTA that is ahead writes the next
         // ones while others still read these
-        grid_sum4(a, l, ((it + 1) & 1) ? 0 : 4, gc, S, d);
+        grid_sums<4>(a, l, ((it + 1) & 1) ? 0 : 4, gc, S, d);
         if (!gc.ok) break;
         it++;
         rr = d[3];

@@ -132,38 +132,20 @@ __device__ __forceinline__ double grid_sum(const CgArgs &a, double local, int sl
     return block_sum_partials<NT>(a.partials + slot * G, G, S.warp);
 }
 
-// Two sums at once (one barrier): slots slot and slot+1 of the partials;
-// every CTA gets the same two values.  Consecutive reductions must use
-// different slots (a CTA may write the next partials while another still
-// reads these).
-template <class SM>
-__device__ __forceinline__ void grid_sum_pair(const CgArgs &a, double l0, double l1, int slot, GridCtx &gc, SM &S,
-                                              double &o0, double &o1)
+// K sums at once (one barrier, one batch of partial loads, one exchange between
+// the warps on each side of it): slots slot..slot+K-1 of the partials; every CTA
+// gets the same values, each the one that grid_sum would give.  Consecutive
+// reductions must use different slots (a CTA may write the next partials while
+// another still reads these).
+template <int K, class SM>
+__device__ __forceinline__ void grid_sums(const CgArgs &a, const double (&l)[K], int slot, GridCtx &gc, SM &S,
+                                          double (&o)[K])
 {
     const int G = gridDim.x;
-    const double c0 = block_sum<NT>(l0, S.warp);
-    const double c1 = block_sum<NT>(l1, S.warp);
-    if (threadIdx.x == 0) {
-        a.partials[slot * G + blockIdx.x] = c0;
-        a.partials[(slot + 1) * G + blockIdx.x] = c1;
-    }
-    gc.epoch++;
-    gc.ok = gc.ok && MF_GRID_BARRIER(a.bar, gc.epoch, a.status, a.budget_ns);
-    o0 = block_sum_partials<NT>(a.partials + slot * G, G, S.warp);
-    o1 = block_sum_partials<NT>(a.partials + (slot + 1) * G, G, S.warp);
-}
-
-// Four sums at once (one barrier, one batch of partial loads): slots
-// slot..slot+3 of the partials; every CTA gets the same four values.
-template <class SM>
-__device__ __forceinline__ void grid_sum4(const CgArgs &a, const double (&l)[4], int slot, GridCtx &gc, SM &S,
-                                          double (&o)[4])
-{
-    const int G = gridDim.x;
-    __shared__ double s_w4[NT / 32][4];
-    double v[4];
+    __shared__ double s_w[NT / 32][K];
+    double v[K];
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
+    for (int k = 0; k < K; k++) {
         v[k] = l[k];
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], off);
@@ -172,37 +154,37 @@ __device__ __forceinline__ void grid_sum4(const CgArgs &a, const double (&l)[4],
     __syncthreads();
     if ((threadIdx.x & 31) == 0)
 #pragma unroll
-        for (int k = 0; k < 4; k++) s_w4[w][k] = v[k];
+        for (int k = 0; k < K; k++) s_w[w][k] = v[k];
     __syncthreads();
     if (threadIdx.x == 0) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
+        for (int k = 0; k < K; k++) {
             double c = 0.0;
-            for (int i = 0; i < NT / 32; i++) c += s_w4[i][k];
+            for (int i = 0; i < NT / 32; i++) c += s_w[i][k];
             a.partials[(slot + k) * G + blockIdx.x] = c;
         }
     }
     gc.epoch++;
     gc.ok = gc.ok && MF_GRID_BARRIER(a.bar, gc.epoch, a.status, a.budget_ns);
-    // every thread loads its share of all four partial arrays, then one tree
+    // every thread loads its share of all the partial arrays, then one tree
 #pragma unroll
-    for (int k = 0; k < 4; k++) v[k] = 0.0;
+    for (int k = 0; k < K; k++) v[k] = 0.0;
     for (int i = threadIdx.x; i < G; i += NT)
 #pragma unroll
-        for (int k = 0; k < 4; k++) v[k] += __ldcg(a.partials + (slot + k) * G + i);
+        for (int k = 0; k < K; k++) v[k] += __ldcg(a.partials + (slot + k) * G + i);
 #pragma unroll
-    for (int k = 0; k < 4; k++)
+    for (int k = 0; k < K; k++)
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], off);
     __syncthreads();
     if ((threadIdx.x & 31) == 0)
 #pragma unroll
-        for (int k = 0; k < 4; k++) s_w4[w][k] = v[k];
+        for (int k = 0; k < K; k++) s_w[w][k] = v[k];
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
+    for (int k = 0; k < K; k++) {
         double c = 0.0;
-        for (int i = 0; i < NT / 32; i++) c += s_w4[i][k];
+        for (int i = 0; i < NT / 32; i++) c += s_w[i][k];
         o[k] = c;
     }
 }
