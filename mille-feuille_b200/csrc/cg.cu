@@ -446,9 +446,9 @@ __global__ void __launch_bounds__(NT, LAY == 0 ? MINB : SMINB) k_cg1(CgArgs a)
 // buffered), so a pass is one round of gathers, the row's sum, one record
 // written, and the reduction.  The reduction's scalars (alpha, beta, the stop
 // test) are worked out by warp 0 alone before the CTA barrier that hands them
-// out.  Taken for rows of at most ROWS_K entries and at most as many rows as
-// threads are resident (2 CTAs per SM: 75,776); above, k_cg1 streams the slots
-// (13.7 us per iteration at 216,000 rows).  Bound by latency: gathers from L2,
+// out.  Taken for rows of at most ROWS_K entries, from 16,385 rows (below,
+// k_cg1_cluster) to as many as threads are resident (2 CTAs per SM: 75,776);
+// above, k_cg1 streams the slots (13.7 us per iteration at 216,000 rows).  Bound by latency: gathers from L2,
 // FP64 chains, the grid barrier.  Against k_cg1, us per iteration: 1,024 rows
 // (5-point) 6.9 -> 3.6, 16,384 rows 6.9 -> 4.0, 72,900 rows 8.4 -> 6.2, 74,046
 // rows (7-point) 9.4 -> 7.1.
@@ -655,6 +655,262 @@ __global__ void __launch_bounds__(NT, ROWS_MINB) k_cg1_rows(CgArgs a)
     }
 }
 static_assert(sizeof(RowRec) == 4 * sizeof(double), "two record buffers fit eight solver vectors");
+
+// The same again for at most CL_MAX * 1024 rows: one thread-block cluster, its
+// rows' r, q and p (double buffered), values and columns in shared memory, the
+// neighbours of other CTAs read over distributed shared memory, one hardware
+// cluster barrier per iteration instead of a barrier through L2.  A CTA's 4 sums
+// take one transposed warp sum (6 double shuffles instead of 20) on each side.
+// Bound by latency (the two levels of sums, the barrier, one FP64 square root
+// and two divisions) and, with 1,024 rows per CTA, by shared-memory reads.
+// Against k_cg1_rows, us per iteration: 1,024 rows 3.6 -> 1.9, 4,096 rows 3.7 ->
+// 2.1, 16,384 rows 4.0 -> 3.0.  (Values and columns in registers instead: 3.0,
+// with spills at 64 registers; the three quotients of the scalars in three
+// lanes at once: no difference.)
+constexpr int CL_MAX = 16;  // CTAs
+constexpr unsigned CL_NONE = 31u << 20;  // no entry: no such rank
+
+constexpr size_t cl_smem(int threads) { return (size_t)threads * (6 * 8 + ROWS_K * (8 + 4)); }
+
+__device__ __forceinline__ void cl_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ unsigned cl_map(unsigned addr, unsigned rank)
+{
+    unsigned r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ double cl_load(unsigned addr)
+{
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
+    return v;
+}
+
+// Four sums over a warp: lane l gets the sum of l[lane >> 3].
+__device__ __forceinline__ double cl_warp_sums(const double (&l)[4])
+{
+    const int lane = threadIdx.x & 31;
+    const bool hi = lane & 16, odd = lane & 8;
+    const double a = (hi ? l[2] : l[0]) + __shfl_xor_sync(0xffffffffu, hi ? l[0] : l[2], 16);
+    const double b = (hi ? l[3] : l[1]) + __shfl_xor_sync(0xffffffffu, hi ? l[1] : l[3], 16);
+    double c = (odd ? b : a) + __shfl_xor_sync(0xffffffffu, odd ? a : b, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    return c;
+}
+
+template <typename OT>
+__global__ void __launch_bounds__(1024, 1) k_cg1_cluster(CgArgs a)
+{
+    constexpr OT EMPTY = (OT)(sizeof(OT) == 2 ? INT16_MIN : INT32_MIN);
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double s_w[32][4];
+    __shared__ double s_part[2][4][CL_MAX];  // every CTA's sums, two sets in turn
+    __shared__ double s_out[3];              // alpha, beta, r.r
+    __shared__ int s_exit;                   // -1: go on, else the exit reason
+    const int T = blockDim.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5, C = gridDim.x;
+    const unsigned g = blockIdx.x;
+    const int i = g * T + tid;
+    const bool row = i < a.A.rows;
+    double *vec = (double *)smem_raw;              // [2][3][T]: r, q, p
+    double *val = vec + 6 * T;                     // [ROWS_K][T]
+    unsigned *at = (unsigned *)(val + ROWS_K * T);  // [ROWS_K][T]: rank << 20 | row in its CTA
+    unsigned first = 0;
+    bool far = false;
+    int n = 0;
+    {
+        const int s = i >> 4, k0 = row ? a.sslot[s] : 0, K = row ? a.sslot[s + 1] - k0 : 0;
+        const size_t e0 = (size_t)k0 * MF_TILE + (i & 15);
+        int prev = -1;
+#pragma unroll
+        for (int u = 0; u < ROWS_K; u++) {
+            const OT d = u < K ? ((const OT *)a.soff)[e0 + (size_t)u * MF_TILE] : EMPTY;
+            const int c = d != EMPTY ? i + (int)d : -1;
+            if (c >= 0 && (c >> 4) != prev) {
+                first |= 1u << u;
+                prev = c >> 4;
+            }
+            // columns past the rows meet zeros
+            const bool in = c >= 0 && c < a.A.rows;
+            val[u * T + tid] = d != EMPTY ? a.sval[e0 + (size_t)u * MF_TILE] : 0.0;
+            at[u * T + tid] = in ? (unsigned)(c / T) << 20 | (unsigned)(c % T) : CL_NONE;
+            if (in && c / T != (int)g) far = true;
+            if (in) n = u + 1;
+        }
+    }
+    far = __any_sync(0xffffffffu, far);
+    n = __reduce_max_sync(0xffffffffu, n);
+    double r = row ? a.b[i] : 0.0, q = 0.0, p = 0.0, x = 0.0;
+    unsigned epoch = 0;
+    // sums of l over the cluster in v (lanes of warp 0, every CTA the same
+    // bits), after this thread's records: a cluster barrier
+    auto exchange = [&](double (&l)[4], double (&v)[4]) {
+        const double c = cl_warp_sums(l);
+        if ((lane & 7) == 0) s_w[w][lane >> 3] = c;
+        __syncthreads();
+        epoch ^= 1;
+        if (w == 0) {
+            double t[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) t[k] = lane < T / 32 ? s_w[lane][k] : 0.0;
+            const double cs = cl_warp_sums(t);
+            // to every CTA: lane l writes sums 2 (l / 16) and the next one to rank l % 16
+            const int k = (lane >> 4) * 2;
+            const double c0 = __shfl_sync(0xffffffffu, cs, k * 8), c1 = __shfl_sync(0xffffffffu, cs, k * 8 + 8);
+            if ((lane & 15) < C) {
+                const unsigned d0 = cl_map((unsigned)__cvta_generic_to_shared(&s_part[epoch][k][g]), lane & 15);
+                const unsigned d1 = cl_map((unsigned)__cvta_generic_to_shared(&s_part[epoch][k + 1][g]), lane & 15);
+                asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(d0), "d"(c0) : "memory");
+                asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(d1), "d"(c1) : "memory");
+            }
+            __syncwarp();
+        }
+        cl_arrive();
+        cl_wait();
+        if (w == 0) {
+            const int k = lane >> 3, j = lane & 7;
+            double c = (j < C ? s_part[epoch][k][j] : 0.0) + (j + 8 < C ? s_part[epoch][k][j + 8] : 0.0);
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+#pragma unroll
+            for (int m = 0; m < 4; m++) v[m] = __shfl_sync(0xffffffffu, c, m * 8);
+        }
+    };
+    vec[tid] = r;
+    vec[T + tid] = 0.0;
+    vec[2 * T + tid] = 0.0;
+    // every CTA runs before its shared memory is written from another one
+    __syncthreads();
+    cl_arrive();
+    cl_wait();
+    double l[4] = {__dmul_rn(r, r), 0.0, 0.0, 0.0}, v[4] = {0.0, 0.0, 0.0, 0.0};
+    exchange(l, v);
+    double nb = 0.0, limit = 0.0;  // warp 0
+    if (w == 0) {
+        const double bb = v[0];
+        nb = sqrt(bb) > 0.0 ? sqrt(bb) : 1.0;
+        limit = a.tol * nb;
+        if (a.hist && g == 0 && lane == 0) a.hist[0] = sqrt(bb) / nb;
+    }
+    double al = 0.0, be = 0.0, rr = 0.0;
+    int it = -1, o = 0, reason = -1;  // it: updates done; pass 0 makes r_0
+    while (reason < 0) {
+        const double *old = vec + o * 3 * T;
+        double yd = 0.0, part = 0.0;
+        auto add = [&](int u, double gr, double gq, double gp) {
+            const double pu = fma(be, gp, fma(-al, gq, gr));
+            if ((first >> u) & 1u) {
+                yd = __dadd_rn(yd, part);
+                part = 0.0;
+            }
+            part = __dadd_rn(part, __dmul_rn(pu, val[u * T + tid]));
+        };
+        if (!far) {
+            // all neighbours of the warp's rows in this CTA
+#pragma unroll
+            for (int u = 0; u < ROWS_K; u++) {
+                if (u >= n) break;
+                const unsigned e = at[u * T + tid];
+                const bool in = e != CL_NONE;
+                const double *d = old + (in ? e & 0xFFFFFu : 0u);
+                const double gr = d[0], gq = d[T], gp = d[2 * T];
+                add(u, in ? gr : 0.0, in ? gq : 0.0, in ? gp : 0.0);
+            }
+        } else {
+            const unsigned base = (unsigned)__cvta_generic_to_shared(old);
+#pragma unroll
+            for (int h = 0; h < ROWS_K; h += 4) {
+                if (h >= n) break;
+                double gr[4], gq[4], gp[4];
+                bool in[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const unsigned e = at[(h + u) * T + tid];
+                    in[u] = e != CL_NONE;
+                    const unsigned d = cl_map(base + 8 * (in[u] ? e & 0xFFFFFu : 0u), in[u] ? e >> 20 : g);
+                    gr[u] = cl_load(d);
+                    gq[u] = cl_load(d + 8 * T);
+                    gp[u] = cl_load(d + 16 * T);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u++) add(h + u, in[u] ? gr[u] : 0.0, in[u] ? gq[u] : 0.0, in[u] ? gp[u] : 0.0);
+            }
+        }
+        const double y = __dadd_rn(yd, part);
+        const double pn = fma(be, p, fma(-al, q, r));
+        r = fma(-al, q, r);
+        x = fma(al, p, x);
+        p = pn;
+        q = y;
+        o ^= 1;
+        double *to = vec + o * 3 * T + tid;
+        to[0] = r;
+        to[T] = q;
+        to[2 * T] = p;
+        l[0] = __dmul_rn(p, q);
+        l[1] = __dmul_rn(r, q);
+        l[2] = __dmul_rn(q, q);
+        l[3] = __dmul_rn(r, r);
+        exchange(l, v);
+        it++;
+        if (w == 0) {
+            const double s = v[3];
+            int ex = -1;
+            double na = 0.0, nbe = 0.0;
+            const bool done = (!a.fixed && sqrt(s) <= limit) || s == 0.0;
+            if (done) {
+                ex = EXIT_CONVERGED;
+            } else if (it >= a.maxiter) {
+                ex = EXIT_MAXITER;
+            } else if (!(v[0] != 0.0) || !isfinite(v[0])) {
+                if (g == 0 && lane == 0) atomicCAS(a.status, DEV_OK, DEV_BREAKDOWN);
+                ex = EXIT_BREAKDOWN;
+            } else {
+                na = s / v[0];
+                nbe = (s - 2.0 * na * v[1] + na * na * v[2]) / s;
+            }
+            if (lane == 0) {
+                s_out[0] = na;
+                s_out[1] = nbe;
+                s_out[2] = s;
+                s_exit = ex;
+                if (a.hist && g == 0) a.hist[it] = sqrt(s) / nb;
+            }
+        }
+        __syncthreads();
+        al = s_out[0];
+        be = s_out[1];
+        rr = s_out[2];
+        reason = s_exit;
+    }
+    if (row) a.xhi[i] = x;
+    if (g == 0 && tid == 0) {
+        double *st = a.state;
+        st[S_RHO] = rr;
+        st[S_BETA] = be;
+        st[S_NB] = nb;
+        st[S_RMAX] = sqrt(rr);
+        st[S_ITERS] = (double)(it < 0 ? 0 : it);
+        st[S_REFS] = 0.0;
+        st[S_EXIT] = (double)reason;
+        st[S_RELRES] = sqrt(rr) / nb;
+    }
+}
+
+// Threads per CTA and CTAs of the cluster for `rows` rows: few rows per SM (FP64
+// issue), at most CL_MAX CTAs.  Whether the device takes the cluster, checked
+// once per shape.
+struct ClShape {
+    int threads, ctas;
+};
+ClShape cl_shape(int rows)
+{
+    ClShape s{256, 1};
+    while (s.threads < 1024 && rows > s.threads * CL_MAX) s.threads *= 2;
+    while (s.ctas < CL_MAX && rows > s.threads * s.ctas) s.ctas *= 2;
+    return s;
+}
 
 // Jacobi: 1 / a_ii of every row from the tile format (the diagonal tile of
 // the row's strip, the row's entry in its column), 1 where the diagonal is
@@ -878,6 +1134,36 @@ mf_status launch_cg(bool mixed, CgArgs &a, int G, cudaStream_t s)
             }
             return MF_OK;
         };
+        if (rows && a.A.rows <= CL_MAX * 1024) {
+            const ClShape cs = cl_shape(a.A.rows);
+            const void *cf = li == 3 ? (const void *)k_cg1_cluster<int32_t> : (const void *)k_cg1_cluster<int16_t>;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = cs.ctas;
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(cs.ctas);
+            cfg.blockDim = dim3(cs.threads);
+            cfg.dynamicSmemBytes = cl_smem(cs.threads);
+            cfg.stream = s;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            // resident clusters of this shape (-1: not asked yet)
+            static int clusters[2][3][5] = {{{-1, -1, -1, -1, -1}, {-1, -1, -1, -1, -1}, {-1, -1, -1, -1, -1}},
+                                            {{-1, -1, -1, -1, -1}, {-1, -1, -1, -1, -1}, {-1, -1, -1, -1, -1}}};
+            int &fit = clusters[li - 2][cs.threads / 512][__builtin_ctz(cs.ctas)];
+            MF_CUDA(cudaFuncSetAttribute(cf, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cl_smem(1024)));
+            MF_CUDA(cudaFuncSetAttribute(cf, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            if (fit < 0) {
+                int most = 0;
+                if (cudaOccupancyMaxActiveClusters(&most, cf, &cfg) != cudaSuccess) cudaGetLastError();
+                fit = most;
+            }
+            if (fit >= 1) {
+                MF_CUDA(cudaLaunchKernelExC(&cfg, cf, args));
+                return MF_OK;
+            }
+        }
         MF_TRY(fits());
         if (G > resident[li] && li >= 2) {  // more rows than resident threads: the chunked kernel
             li = 1;
