@@ -157,6 +157,12 @@ __global__ void __launch_bounds__(NT, LAY == 0 ? MINB : LAY == 1 ? SMINB : MF_ST
         };
         if constexpr (LAY == 2) {
             if (!spmv_staged<PK, true, VT, 2>(a, S, gc, cb, ce, rr, pold, bt, aout, nullptr)) gc.ok = false;
+        } else if constexpr (LAY == 1 && !MIX) {
+            if (a.direct) {
+                spmv_direct<4>(a, row0, row1, rr, pold, vold, -om, bt, aout);
+            } else {
+                if (!spmv_any<PK, LAY>(a, S, gc, cb, ce, sb0, se0, psrc, aout, nullptr)) gc.ok = false;
+            }
         } else {
             if (!spmv_any<PK, LAY>(a, S, gc, cb, ce, sb0, se0, psrc, aout, nullptr)) gc.ok = false;
         }
@@ -186,6 +192,12 @@ __global__ void __launch_bounds__(NT, LAY == 0 ? MINB : LAY == 1 ? SMINB : MF_ST
         };
         if constexpr (LAY == 2) {
             if (!spmv_staged<PK, true, VT, 2>(a, S, gc, cb, ce, rr, vn, (VT)-al, tout, nullptr)) gc.ok = false;
+        } else if constexpr (LAY == 1 && !MIX) {
+            if (a.direct) {
+                spmv_direct<2>(a, row0, row1, rr, vn, nullptr, -al, 0.0, tout);
+            } else {
+                if (!spmv_any<PK, LAY>(a, S, gc, cb, ce, sb0, se0, ssrc, tout, nullptr)) gc.ok = false;
+            }
         } else {
             if (!spmv_any<PK, LAY>(a, S, gc, cb, ce, sb0, se0, ssrc, tout, nullptr)) gc.ok = false;
         }

@@ -173,6 +173,12 @@ __global__ void __launch_bounds__(NT, LAY == 0 ? MINB : LAY == 1 ? SMINB : stage
         if constexpr (LAY == 2) {
             if (!spmv_staged<PK, true, VT, 2>(a, S, gc, cb, ce, rr, pold, bt, aout, timed ? tph : nullptr))
                 gc.ok = false;
+        } else if constexpr (LAY == 1 && !MIX) {
+            if (a.direct) {
+                spmv_direct<2>(a, row0, row1, rr, pold, nullptr, bt, 0.0, aout);
+            } else {
+                if (!spmv_any<PK, LAY>(a, S, gc, cb, ce, sb0, se0, psrc, aout, timed ? tph : nullptr)) gc.ok = false;
+            }
         } else {
             if (!spmv_any<PK, LAY>(a, S, gc, cb, ce, sb0, se0, psrc, aout, timed ? tph : nullptr)) gc.ok = false;
         }
@@ -401,7 +407,11 @@ __global__ void __launch_bounds__(NT, LAY == 0 ? MINB : SMINB) k_cg1(CgArgs a)
             l[2] = __dadd_rn(l[2], __dmul_rn(y, y));
             l[3] = __dadd_rn(l[3], __dmul_rn(rv, rv));
         };
-        if (!spmv_any<0, LAY>(a, S, gc, cb, ce, sb0, se0, psrc, aout, nullptr)) gc.ok = false;
+        if (LAY == 1 && a.direct) {
+            spmv_direct<3>(a, row0, row1, ro, po, qo, -al, be, aout);
+        } else if (!spmv_any<0, LAY>(a, S, gc, cb, ce, sb0, se0, psrc, aout, nullptr)) {
+            gc.ok = false;
+        }
         double d[4];
         // two sets of partials in turn: a CTA that is ahead writes the next
         // ones while others still read these
@@ -448,7 +458,7 @@ __global__ void __launch_bounds__(NT, LAY == 0 ? MINB : SMINB) k_cg1(CgArgs a)
 // test) are worked out by warp 0 alone before the CTA barrier that hands them
 // out.  Taken for rows of at most ROWS_K entries, from 16,385 rows (below,
 // k_cg1_cluster) to as many as threads are resident (2 CTAs per SM: 75,776);
-// above, k_cg1 streams the slots (13.7 us per iteration at 216,000 rows).  Bound by latency: gathers from L2,
+// above, k_cg1 streams the slots (10.4 us per iteration at 216,000 rows).  Bound by latency: gathers from L2,
 // FP64 chains, the grid barrier.  Against k_cg1, us per iteration: 1,024 rows
 // (5-point) 6.9 -> 3.6, 16,384 rows 6.9 -> 4.0, 72,900 rows 8.4 -> 6.2, 74,046
 // rows (7-point) 9.4 -> 7.1.

@@ -682,6 +682,92 @@ __device__ bool spmv_slots(const CgArgs &a, SlotSmem &S, GridCtx &gc, int cb, in
     return true;
 }
 
+// ---- rows straight from the slot arrays ----
+//
+// N entries of a row: distances and values, then the vectors at the entries'
+// columns, all in flight.  The entry of the multiplied vector is c b + a (NV 2),
+// e b + (c q + a) (NV 3) or e (c q + b) + a (NV 4).
+template <int N, int NV, typename OT>
+__device__ __forceinline__ void direct_sums(const OT *d0, const double *v0, const double *a, const double *b,
+                                            const double *q, double c, double e, int hl, int &prev, double &yd,
+                                            double &part)
+{
+    constexpr OT EMPTY = (OT)(sizeof(OT) == 2 ? INT16_MIN : INT32_MIN);
+    int d[N];
+    double v[N], av[N], bv[N], qv[N];
+#pragma unroll
+    for (int u = 0; u < N; u++) {
+        d[u] = (int)__ldcs(d0 + u * MF_TILE);
+        v[u] = __ldcs(v0 + u * MF_TILE);
+    }
+#pragma unroll
+    for (int u = 0; u < N; u++) {
+        av[u] = d[u] != (int)EMPTY ? a[d[u]] : 0.0;
+        bv[u] = d[u] != (int)EMPTY ? b[d[u]] : 0.0;
+        if (NV > 2) qv[u] = d[u] != (int)EMPTY ? q[d[u]] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < N; u++) {
+        const int t = (d[u] + hl) >> 4;  // tile column, counted from the strip's own
+        if (t != (u == 0 ? prev : (d[u - 1] + hl) >> 4)) {
+            yd = __dadd_rn(yd, part);
+            part = 0.0;
+        }
+        const double x = NV == 2   ? fma(c, bv[u], av[u])
+                         : NV == 3 ? fma(e, bv[u], fma(c, qv[u], av[u]))
+                                   : fma(e, fma(c, qv[u], bv[u]), av[u]);
+        part = __dadd_rn(part, __dmul_rn(x, v[u]));
+    }
+    prev = (d[N - 1] + hl) >> 4;
+}
+
+template <int NV, typename OT, class Out>
+__device__ __forceinline__ void spmv_direct_as(const CgArgs &g, int row0, int row1, const double *a, const double *b,
+                                               const double *q, double c, double e, Out &out)
+{
+    for (int i = row0 + threadIdx.x; i < row1; i += NT) {
+        const int s = i >> 4, hl = i & 15;
+        const int k0 = g.sslot[s];
+        int K = g.sslot[s + 1] - k0;
+        const OT *d = (const OT *)g.soff + (size_t)k0 * MF_TILE + hl;
+        const double *v = g.sval + (size_t)k0 * MF_TILE + hl;
+        const double *ai = a + i, *bi = b + i, *qi = NV > 2 ? q + i : nullptr;
+        double yd = 0.0, part = 0.0;
+        int prev = INT_MIN;
+        for (; K > 8; K -= 8, d += 8 * MF_TILE, v += 8 * MF_TILE)
+            direct_sums<8, NV>(d, v, ai, bi, qi, c, e, hl, prev, yd, part);
+        switch (K) {  // straight code for every remainder: no load is predicated
+        case 8: direct_sums<8, NV>(d, v, ai, bi, qi, c, e, hl, prev, yd, part); break;
+        case 7: direct_sums<7, NV>(d, v, ai, bi, qi, c, e, hl, prev, yd, part); break;
+        case 6: direct_sums<6, NV>(d, v, ai, bi, qi, c, e, hl, prev, yd, part); break;
+        case 5: direct_sums<5, NV>(d, v, ai, bi, qi, c, e, hl, prev, yd, part); break;
+        case 4: direct_sums<4, NV>(d, v, ai, bi, qi, c, e, hl, prev, yd, part); break;
+        case 3: direct_sums<3, NV>(d, v, ai, bi, qi, c, e, hl, prev, yd, part); break;
+        case 2: direct_sums<2, NV>(d, v, ai, bi, qi, c, e, hl, prev, yd, part); break;
+        case 1: direct_sums<1, NV>(d, v, ai, bi, qi, c, e, hl, prev, yd, part); break;
+        default: break;
+        }
+        out(s, hl, __dadd_rn(yd, part), 0.0, false);
+    }
+}
+
+// y = A x for rows [row0, row1), x made as above: a thread per row,
+// blockspmv_cpu's sums (FP64).  Bound by the L2 latency of two dependent
+// rounds (distances and values, then the gathers), hidden by 8 entries in flight
+// per thread and 24 warps per SM.  Against the staged slot chunks, whose rows
+// wait for a copy, a CTA barrier and a chain of tile-column look-ups, us per CG
+// iteration: 128^3 7-point 70.0 -> 58.8 with two reductions, 216,000 rows 12.9
+// -> 10.4 with one; BiCGSTAB 128^3 161 -> 138; 27-point 96^3 140 -> 74.  80
+// registers, 3 CTAs per SM (64 registers and 4: 128^3 71.8 ms a solve against
+// 51.8).
+template <int NV, class Out>
+__device__ __forceinline__ void spmv_direct(const CgArgs &g, int row0, int row1, const double *a, const double *b,
+                                            const double *q, double c, double e, Out &out)
+{
+    if (g.soff_bytes == 2) spmv_direct_as<NV, int16_t>(g, row0, row1, a, b, q, c, e, out);
+    else spmv_direct_as<NV, int32_t>(g, row0, row1, a, b, q, c, e, out);
+}
+
 // ---- staged slot chunks ----
 //
 // Stage layout: strip descriptors, slot positions, FP64 values or the mixed

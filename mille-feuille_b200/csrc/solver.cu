@@ -34,7 +34,8 @@ static mf_status persistent_solve(bool bicg, mf_matrix m, const double *b, doubl
     // cannot describe the matrix.  (The FP64 CG kernel stages two FP64
     // vectors, which leaves room for two CTAs per SM only; its plain row
     // slots run faster.)  MF_SOLVER_LAYOUT=tiles / slots restricts the
-    // choice, =staged also stages the FP64 CG kernel.
+    // choice, =staged also stages the FP64 CG kernel, =chunks keeps FP64 rows on
+    // the staged slot chunks.
     const char *lay = getenv("MF_SOLVER_LAYOUT");
     const bool want_slots = !(lay && !strcmp(lay, "tiles"));
     if (want_slots) MF_TRY(build_slots(m, s));
@@ -106,6 +107,19 @@ static mf_status persistent_solve(bool bicg, mf_matrix m, const double *b, doubl
         a.soff = m->d_soff;
         a.soff_bytes = m->soff_bytes;
         a.slot_kmax = m->slot_kmax;
+        // FP64 rows straight from the slot arrays, a thread per row, unless some
+        // rows are so long that their threads hold the others up; those are cut
+        // over half-warps from staged chunks.  us per CG iteration, staged and
+        // direct: rows of 7 (2.1 M rows) 70.0 / 58.8, of 27 (0.9 M) 140 / 74, of
+        // 33 (5,000) 11.6 / 9.5; of 65: 2,000 rows 10.9 / 11.7, 20,000 rows 16.6 /
+        // 15.2, 100,000 rows 47.6 / 25.9; random rows of 65, the longest 93, 118
+        // / 86; of 129 (40,000 rows) 35.6 / 41.1; rows of 7 with 20 of 36 among
+        // 600,000 28.0 / 29.2, with 20 of 132 29.9 / 48.5.
+        const long long avg = m->v.rows > 0 ? m->v.nnz / m->v.rows : 0;
+        const int kmax = m->slot_kmax;
+        a.direct = !(lay && !strcmp(lay, "chunks")) &&
+                   ((kmax <= 64 && kmax <= std::max(8ll, 4 * avg)) ||
+                    (kmax <= 96 && kmax <= 2 * avg && m->v.rows >= 65536));
         a.shdr = m->d_shdr;
         a.spay = m->d_spay;
         a.scta_chunk = m->d_scta_chunk;

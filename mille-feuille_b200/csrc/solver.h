@@ -113,6 +113,7 @@ struct CgArgs {
     // column - row of the slot entries (k_cg1_rows), and their size
     const void *soff;
     int soff_bytes, slot_kmax;
+    int direct;  // FP64: rows straight from the slot arrays (spmv_direct)
 };
 
 struct SolverWork {
