@@ -603,7 +603,7 @@ def workload_single(args, mf, world, local):
 
 
 def workload_spmv(args, mf, world, local):
-    """The standalone FP64 tiled SpMV (mf_spmv, k_spmv_fp64) on the
+    """The standalone FP64 tiled SpMV (mf_spmv, k_spmv_slots) on the
     poisson3d matrix; value = SpMVs per second.  Algorithmic bytes of one
     SpMV: nnz x (8-byte value + 1-byte in-tile column) + 24 bytes per tile
     (tile column, entry offset, 16 row pointers) + x read once and y written
@@ -663,7 +663,7 @@ def workload_spmv(args, mf, world, local):
     e2e_s = _max_over_ranks(e2e_s, world)
     result["e2e"] = {"value": args.steps * world / e2e_s, "unit": "spmv/s", "h2d_bytes_per_step": 8 * len(xs),
                      "d2h_bytes_per_step": 8 * n}
-    result["roofline_in"] = (bytes_spmv, ms / (reps * args.steps), "k_spmv_fp64", None)
+    result["roofline_in"] = (bytes_spmv, ms / (reps * args.steps), "k_spmv_slots", None)
     result["dtype"] = "f64"
     result["cpu"] = None
     M.close()

@@ -16,6 +16,9 @@
 //     (TMA, cp.async.bulk, completion on an mbarrier), two chunks in flight;
 //     the CTA then builds the chunk's x segments and computes its rows from
 //     shared memory, one half-warp per strip and one lane per row;
+//   * FP64 rows that are short or even are read straight from the row slots by a
+//     thread each (spmv_direct, persist.cuh); the smallest systems run from
+//     registers and shared memory (k_cg1_rows, k_cg1_cluster);
 //   * two grid-wide reductions per iteration and no third barrier: the new
 //     search direction p = r + beta p is formed while the SpMV builds its x
 //     segments (p is double-buffered), so no pass must write p before the
@@ -458,10 +461,10 @@ __global__ void __launch_bounds__(NT, LAY == 0 ? MINB : SMINB) k_cg1(CgArgs a)
 // test) are worked out by warp 0 alone before the CTA barrier that hands them
 // out.  Taken for rows of at most ROWS_K entries, from 16,385 rows (below,
 // k_cg1_cluster) to as many as threads are resident (2 CTAs per SM: 75,776);
-// above, k_cg1 streams the slots (10.4 us per iteration at 216,000 rows).  Bound by latency: gathers from L2,
-// FP64 chains, the grid barrier.  Against k_cg1, us per iteration: 1,024 rows
-// (5-point) 6.9 -> 3.6, 16,384 rows 6.9 -> 4.0, 72,900 rows 8.4 -> 6.2, 74,046
-// rows (7-point) 9.4 -> 7.1.
+// above, k_cg1 (10.4 us per iteration at 216,000 rows).  Bound by latency:
+// gathers from L2, FP64 chains, the grid barrier.  Against k_cg1 on slot chunks,
+// us per iteration: 1,024 rows (5-point) 6.9 -> 3.6, 16,384 rows 6.9 -> 4.0,
+// 72,900 rows 8.4 -> 6.2, 74,046 rows (7-point) 9.4 -> 7.1.
 constexpr int ROWS_K = 8;
 constexpr int ROWS_MINB = 2;  // CTAs per SM: 128 registers
 

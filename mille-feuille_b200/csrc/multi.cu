@@ -30,7 +30,7 @@
 // 96^3).  Measured against the earlier form (16-bit tile words looked up
 // per entry, x updated with r: 11 vector streams, always swept upwards): 16
 // right-hand sides of the 96^3 Poisson matrix 278 -> 218 ms, mf_spmm with 5
-// columns of a 290,177-row matrix 47.1 -> 28.6 us (its result is written
+// columns of a 290,177-row matrix 47.1 -> 30.5 us (its result is written
 // column-major by the SpMM itself).
 //
 // No tensor cores: FP64 has no tcgen05 kind, and the tiles of the stencil
