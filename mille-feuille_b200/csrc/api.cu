@@ -100,6 +100,9 @@ cudaError_t handle_malloc(void **p, size_t bytes)
     return e;
 }
 
+// Nothing on the device can still use a handle's memory when this returns.
+void handle_wait() { cudaDeviceSynchronize(); }
+
 // Back to the pool; the caller has waited for everything that uses it.
 void handle_free(void *p)
 {
@@ -133,8 +136,7 @@ void set_last_error(const char *fmt, ...)
 mf_status ensure_work(mf_matrix m, size_t bytes)
 {
     if (m->work_bytes >= bytes) return MF_OK;
-    if (m->work) cudaFree(m->work);
-    m->work = nullptr;
+    handle_release(m->work);
     m->work_bytes = 0;
     MF_CUDA(handle_malloc(&m->work, bytes));
     m->work_bytes = bytes;
@@ -246,7 +248,7 @@ mf_status mf_matrix_destroy(mf_matrix m)
     int dev = -1;
     cudaGetDevice(&dev);
     if (dev != m->device) cudaSetDevice(m->device);
-    cudaDeviceSynchronize();  // nothing on the device can still use the handle's memory
+    handle_wait();
     void *bufs[] = {m->tiles_mem, m->d_part, m->d_cta_chunk, m->d_chunks, m->work, m->host_io,
                     m->d_wcls, m->d_poff, m->d_pay, m->d_resid, m->d_pol, m->slots_mem,
                     m->d_shdr, m->d_spay, m->d_scta_chunk, m->d_schunks, m->d_spos, m->d_sdesc, m->mr_work,
@@ -437,8 +439,7 @@ static mf_status solve_host_common(bool bicg, mf_matrix m, const double *b_host,
     if (!m || !b_host || !x_host) return MF_ERR_INVALID_ARG;
     const size_t n = m->v.rows;
     if (m->host_io_n < n) {
-        if (m->host_io) cudaFree(m->host_io);
-        m->host_io = nullptr;
+        handle_release(m->host_io);
         m->host_io_n = 0;
         MF_CUDA(handle_malloc(&m->host_io, sizeof(double) * (2 * n + 2)));
         m->host_io_n = n;
@@ -543,8 +544,7 @@ mf_status mf_cg_solve_multi_host(mf_matrix m, int k, const double *B_host, doubl
     if (n == 0) return mf_cg_solve_multi(m, k, nullptr, 0, nullptr, 0, opts, reports, nullptr);
     cudaStream_t s = 0;
     if (m->mr_io_bytes < 2 * bytes) {
-        if (m->mr_io) cudaFree(m->mr_io);
-        m->mr_io = nullptr;
+        handle_release(m->mr_io);
         m->mr_io_bytes = 0;
         MF_CUDA(handle_malloc(&m->mr_io, 2 * bytes));
         m->mr_io_bytes = 2 * bytes;

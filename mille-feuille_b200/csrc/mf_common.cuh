@@ -25,10 +25,23 @@ void note_launch(int k = 1);
 cudaError_t pool_malloc_async(void **p, size_t bytes, cudaStream_t s);
 // Memory kept on a handle, from the same pool (a driver allocation costs 0.1
 // to 1 ms, a matrix has up to twenty): usable on every stream at once.
-// handle_free returns it; nothing may still use it.  handle_count(device, +1 /
-// -1): a matrix handle was made / destroyed.
+// handle_free returns it; nothing may still use it.  handle_release is for a
+// buffer that a larger one replaces: it waits for the device first, since an
+// earlier call may still run on any stream and neither cudaFree nor
+// cudaFreeAsync of a pool's memory waits for it -- the block could be handed
+// out again at once.  handle_count(device, +1 / -1): a matrix handle was made /
+// destroyed.
 cudaError_t handle_malloc(void **p, size_t bytes);
 void handle_free(void *p);
+void handle_wait();
+template <typename T>
+inline void handle_release(T *&p)
+{
+    if (!p) return;
+    handle_wait();
+    handle_free((void *)p);
+    p = nullptr;
+}
 void handle_count(int device, int d);
 template <typename T>
 inline cudaError_t handle_malloc(T **p, size_t bytes)

@@ -509,8 +509,7 @@ mf_status cg_multi_kp(mf_matrix m, int k, const double *B, int ldb, double *X, i
     const size_t part_bytes = (sizeof(double) * (size_t)MR_GRID * KP + 255) / 256 * 256;
     const size_t need = vec_bytes + part_bytes + sizeof(MrState);
     if (m->mr_work_bytes < need) {
-        if (m->mr_work) cudaFree(m->mr_work);
-        m->mr_work = nullptr;
+        handle_release(m->mr_work);
         m->mr_work_bytes = 0;
         if (handle_malloc(&m->mr_work, need) != cudaSuccess) {
             cudaGetLastError();

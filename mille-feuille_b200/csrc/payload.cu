@@ -105,8 +105,7 @@ mf_status pack_payload(mf_matrix m, const unsigned char *d_wcls, cudaStream_t s)
     }
     const size_t need = (size_t)total + 32;
     if (m->pay_bytes < need) {
-        if (m->d_pay) cudaFree(m->d_pay);
-        m->d_pay = nullptr;
+        handle_release(m->d_pay);
         m->pay_bytes = 0;
         // the largest packing (every tile FP32) bounds all later ones
         const size_t cap = (size_t)m->v.nnz * 4 + (size_t)T * 4 + 32;

@@ -378,8 +378,7 @@ static mf_status policy_work(mf_matrix m, PolicyWork &pw, cudaStream_t s)
     const int T = m->v.tilenum, ns = m->v.tilen > m->v.tilem ? m->v.tilen : m->v.tilem;
     const size_t need = sizeof(float) * ((size_t)2 * T + 6 * (size_t)ns + 64) + 64;
     if (m->pol_bytes < need) {
-        if (m->d_pol) cudaFree(m->d_pol);
-        m->d_pol = nullptr;
+        handle_release(m->d_pol);
         m->pol_bytes = 0;
         MF_CUDA(handle_malloc(&m->d_pol, need));
         m->pol_bytes = need;

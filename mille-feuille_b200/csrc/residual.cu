@@ -94,8 +94,7 @@ extern "C" mf_status mf_residual_norm(mf_matrix m, const double *b, const double
     }
     const size_t need = sizeof(double) * 2 * (size_t)(m->v.tilem > 0 ? m->v.tilem : 1);
     if (m->resid_bytes < need) {
-        if (m->d_resid) cudaFree(m->d_resid);
-        m->d_resid = nullptr;
+        handle_release(m->d_resid);
         m->resid_bytes = 0;
         MF_CUDA(handle_malloc(&m->d_resid, need));
         m->resid_bytes = need;

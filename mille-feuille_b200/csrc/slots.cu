@@ -424,10 +424,8 @@ mf_status build_slot_chunks(mf_matrix m, int G, bool staged, cudaStream_t s)
 {
     const int mode = staged ? 2 : 1;
     if (m->schunk_ctas == G && m->d_schunks && m->schunk_mode == mode) return MF_OK;
-    if (m->d_scta_chunk) cudaFree(m->d_scta_chunk);
-    if (m->d_schunks) cudaFree(m->d_schunks);
-    m->d_scta_chunk = nullptr;
-    m->d_schunks = nullptr;
+    handle_release(m->d_scta_chunk);
+    handle_release(m->d_schunks);
     m->schunk_ctas = 0;
     m->schunk_mode = 0;
     m->schunk_staged = 0;

@@ -400,8 +400,7 @@ mf_status tc_prepare(mf_matrix m, int fill, cudaStream_t s)
 {
     if (m->tc_mem && m->tc_fill == fill) return MF_OK;
     const int T = m->v.tilenum, tilem = m->v.tilem;
-    if (m->tc_mem) cudaFree(m->tc_mem);
-    m->tc_mem = nullptr;
+    handle_release(m->tc_mem);
     m->tc_fill = 0;
     m->tc_ndense = 0;
     // temporaries: flags and block index per tile; dense tiles per strip and

@@ -844,8 +844,7 @@ mf_status build_tiles(mf_matrix m, int rowA, int colA, const int *d_rowptr, cons
 mf_status strip_partition(mf_matrix m, int ctas, cudaStream_t s)
 {
     if (m->part_ctas == ctas && m->d_part) return MF_OK;
-    if (m->d_part) cudaFree(m->d_part);
-    m->d_part = nullptr;
+    handle_release(m->d_part);
     m->part_ctas = 0;
     const int tilem = m->v.tilem;
     MF_CUDA(handle_malloc(&m->d_part, sizeof(int) * (ctas + 1)));

@@ -1,0 +1,72 @@
+"""Memory kept on a handle, where calls on several streams and threads meet
+(needs a B200)."""
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SLEEP = 200_000_000  # clock cycles: about 0.1 s
+
+
+def _spmm_f16(mf, M, X, Y, fill, stream=None):
+    k, n = X.shape
+    mf.check(mf.lib().mf_spmm_f16(M.h, k, X.data_ptr(), n, Y.data_ptr(), n, fill, None, stream))
+
+
+def test_new_dense_threshold_waits_for_the_last_call(mf):
+    """mf_spmm_f16 with another dense_fill replaces the handle's lists; a call
+    still running on another stream reads the old ones."""
+    A = mf.synth_block_dense(1000, 3, 4, 7)
+    n = A.n_rows
+    X = torch.from_numpy(np.random.default_rng(1).normal(size=(16, n))).cuda()
+    want = {}
+    for fill in (1, 256):
+        M = mf.Matrix(A)
+        want[fill] = torch.zeros_like(X)
+        _spmm_f16(mf, M, X, want[fill], fill)
+        torch.cuda.synchronize()
+        M.close()
+    M = mf.Matrix(A)
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    Y = [torch.zeros_like(X) for _ in range(3)]
+    _spmm_f16(mf, M, X, Y[0], 1, a.cuda_stream)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(a):
+        torch.cuda._sleep(SLEEP)
+    _spmm_f16(mf, M, X, Y[1], 1, a.cuda_stream)
+    _spmm_f16(mf, M, X, Y[2], 256, b.cuda_stream)
+    torch.cuda.synchronize()
+    assert torch.equal(Y[0], want[1]) and torch.equal(Y[1], want[1]) and torch.equal(Y[2], want[256])
+    M.close()
+
+
+def test_unstageable_matrices_from_two_threads(mf):
+    """A mixed solve of a matrix whose chunks cannot be staged replaces its
+    chunk table twice; another thread's handle draws from the same pool."""
+    mats = [mf.synth_random_spd(s, 3000 + 500 * s) for s in (1, 2)]
+    xs = [mf.synth_xstar(s, A.n_rows) for s, A in enumerate(mats)]
+    rhs = [A.matvec(x) for A, x in zip(mats, xs)]
+
+    def solve(A, b, M=None):
+        M = M or mf.Matrix(A)
+        return M.solve_host(b, tol=1e-10, maxiter=5000, policy="static")
+
+    want = [solve(A, b) for A, b in zip(mats, rhs)]
+    assert all(r.status == 0 and r.layout == 1 for _, r in want)  # plain slots: not staged
+    bad = []
+
+    def work(k):
+        M = mf.Matrix(mats[k])
+        for _ in range(20):
+            x, r = solve(mats[k], rhs[k], M)
+            if r.iterations != want[k][1].iterations or not np.array_equal(x, want[k][0]):
+                bad.append((k, r.iterations))
+        M.close()
+
+    th = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    [t.start() for t in th]
+    [t.join() for t in th]
+    assert not bad
