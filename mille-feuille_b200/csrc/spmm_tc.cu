@@ -449,7 +449,10 @@ mf_status tc_prepare(mf_matrix m, int fill, cudaStream_t s)
                                                                            (__half *)m->d_tc_dense);
             note_launch();
         }
-        const cudaError_t e = cudaGetLastError();
+        // waited for before anything tells that they are there: the next call
+        // may come on another stream
+        cudaError_t e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) {
             set_last_error("mf_spmm_f16: %s", cudaGetErrorString(e));
             st = MF_ERR_CUDA;

@@ -43,6 +43,25 @@ def test_new_dense_threshold_waits_for_the_last_call(mf):
     M.close()
 
 
+def test_first_call_is_complete_for_every_stream(mf):
+    """The lists that mf_spmm_f16's first call builds are read by a call on
+    another stream that follows at once."""
+    A = mf.synth_block_dense(4000, 3, 4, 8)
+    X = torch.from_numpy(np.random.default_rng(2).normal(size=(16, A.n_rows))).cuda()
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    for fill in (1, 100, 256):
+        M = mf.Matrix(A)
+        Y = [torch.zeros_like(X) for _ in range(3)]
+        torch.cuda.synchronize()
+        _spmm_f16(mf, M, X, Y[0], fill, a.cuda_stream)
+        _spmm_f16(mf, M, X, Y[1], fill, b.cuda_stream)
+        torch.cuda.synchronize()
+        _spmm_f16(mf, M, X, Y[2], fill)
+        torch.cuda.synchronize()
+        assert torch.equal(Y[0], Y[2]) and torch.equal(Y[1], Y[2])
+        M.close()
+
+
 def test_unstageable_matrices_from_two_threads(mf):
     """A mixed solve of a matrix whose chunks cannot be staged replaces its
     chunk table twice; another thread's handle draws from the same pool."""
