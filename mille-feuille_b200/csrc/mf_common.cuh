@@ -23,6 +23,14 @@ void note_launch(int k = 1);
 // device has matrix handles, up to 256 MiB otherwise -- so the temporaries of
 // a solve's checkpoints cost no driver allocation).  Free with cudaFreeAsync.
 cudaError_t pool_malloc_async(void **p, size_t bytes, cudaStream_t s);
+// While it lives, a stream capture of the calling thread does not mind calls
+// that allocate, free or wait (other threads' captures never do).
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    RelaxedCapture(const RelaxedCapture &) = delete;
+};
 // Memory kept on a handle, from the same pool (a driver allocation costs 0.1
 // to 1 ms, a matrix has up to twenty): usable on every stream at once.
 // handle_free returns it; nothing may still use it.  handle_release is for a

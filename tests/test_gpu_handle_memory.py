@@ -89,3 +89,41 @@ def test_unstageable_matrices_from_two_threads(mf):
     [t.start() for t in th]
     [t.join() for t in th]
     assert not bad
+
+
+@pytest.mark.parametrize("mode,other", [("thread_local", True), ("relaxed", True), ("relaxed", False)])
+def test_destroy_leaves_a_capture_valid(mf, mode, other):
+    """A handle destroyed on another thread than the capturing one (or under a
+    relaxed capture): the graph is complete."""
+    M = mf.Matrix(mf.synth_laplace2d(40, 30))
+    x = torch.ones(1000, device="cuda")
+    y = torch.zeros_like(x)
+    g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(s):
+        g.capture_begin(capture_error_mode=mode)
+        y.add_(x)
+        if other:
+            t = threading.Thread(target=M.close)
+            t.start()
+            t.join()
+        else:
+            M.close()
+        y.add_(x)
+        g.capture_end()
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.all(y == 2.0)
+
+
+def test_destroy_waits_for_the_device(mf):
+    M = mf.Matrix(mf.synth_laplace2d(40, 30))
+    a = torch.cuda.Stream()
+    done = torch.cuda.Event()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(a):
+        torch.cuda._sleep(SLEEP)
+        done.record()
+    assert not done.query()
+    M.close()
+    assert done.query()
