@@ -5,8 +5,9 @@
 //
 // A handle's first product runs from the tiles; from the second on it runs
 // from the row slots (slots.cu), built then: a strip's slots are read
-// coalesced and a row's entries load eight at a time, where the tiles cost
-// two X#include <climits>
+// coalesced and a row's entries load eight at a time, where the tiles cost a
+// chain of dependent loads per tile (128^3 Poisson 62.4 -> 37.9 us).
+#include <climits>
 
 #include "solver.h"
 #include "spmv_core.cuh"
