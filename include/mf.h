@@ -83,7 +83,7 @@ typedef struct mf_matrix_info {
     int rowblkblock;    /* entries of the blockspmv_cpu schedule */
     int class_tiles[5]; /* tiles per static class, indexed by MF_CLASS_* */
     int max_tile_nnz;
-    size_t device_bytes;
+    size_t device_bytes; /* the tile arrays and, once built, the row slots */
 } mf_matrix_info;
 
 /*
@@ -127,7 +127,17 @@ mf_status mf_encode_column_index(mf_matrix m, void *stream);
 
 /* y = A x in FP64 (device pointers; x has tilen*16 entries readable, y has
  * rows entries).  Row sums follow blockspmv_cpu's order: per tile a
- * sequential sum over the row's entries, tiles added in column order. */
+ * sequential sum over the row's entries, tiles added in column order.
+ * Asynchronous: no call waits for the GPU.  A handle's first product runs from
+ * the tiles.  The second allocates the row slots (12 or 14 bytes per entry and
+ * padding, kept until the handle is destroyed, counted in device_bytes) and
+ * queues their kernels on its stream; from then on products on any stream run
+ * from them, with the same bits.  Matrices whose slots would be more than half
+ * padding, or whose slots find no memory, stay with the tiles.  A capture
+ * never allocates: products captured before the slots are complete run from
+ * the tiles in every replay.  (The solvers and mf_spmm build the slots too; the
+ * one matrix whose slots they first have to count, with a wait, has a tile of
+ * 256 entries with duplicates and an empty last row.) */
 mf_status mf_spmv(mf_matrix m, const double *x, double *y, void *stream);
 
 /* FP64 true relative residual ||b - A x|| / ||b|| of a square system (the

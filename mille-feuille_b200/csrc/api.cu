@@ -274,6 +274,7 @@ mf_status mf_matrix_destroy(mf_matrix m)
                     m->d_shdr, m->d_spay, m->d_scta_chunk, m->d_schunks, m->d_spos, m->d_sdesc, m->mr_work,
                     m->mr_io, m->tc_mem};
     for (void *p : bufs) handle_free(p);
+    if (m->slots_done) cudaEventDestroy(m->slots_done);
     handle_count(m->device, -1);
     if (dev != m->device && dev >= 0) cudaSetDevice(dev);
     delete m;

@@ -35,7 +35,7 @@ struct mf_matrix_s {
     int nonzero_rows;          // cnt_non_new
     int last_tile_begin;       // tile_ptr[tilem-1]
     int rowblkblock;
-    size_t device_bytes;
+    std::atomic<size_t> device_bytes{0};  // the tile arrays and, once built, the row slots
 
     // the tile arrays below live in one allocation of the library's pool
     void *tiles_mem = nullptr;
@@ -76,10 +76,12 @@ struct mf_matrix_s {
     int pol_static_ready = 0, pol_have_prev = 0;
     float pol_prev_relres = 0.f;
     // row-slot execution layout of the persistent solvers (slots.cu)
-    std::mutex slots_mu;           // held while they are built
-    std::atomic<int> slots_state{0};  // 0 not built, 1 built, -1 not describable
+    std::mutex slots_mu;           // held while they are queued
+    std::atomic<int> slots_state{0};  // 0 not built, 1 queued, -1 not describable
+    std::atomic<bool> slots_pending{false};  // queued and not seen complete yet
+    cudaEvent_t slots_done = nullptr;        // recorded behind their last kernel
     std::atomic<int> spmv_calls{0};   // products from the tiles so far (mf_spmv)
-    long long nslots = 0;
+    std::atomic<long long> nslots{-1};  // -1: the build of the tiles cannot tell
     void *slots_mem = nullptr;     // the four arrays below live in it
     int *d_sslot = nullptr;
     uint16_t *d_smeta = nullptr;
@@ -130,6 +132,11 @@ mf_status exclusive_scan_i32(const int *in, int *out, int n, cudaStream_t s, int
 mf_status build_tiles(mf_matrix m, int rowA, int colA, const int *d_rowptr, const int *d_colidx,
                       const double *d_val, const float *d_val_low, cudaStream_t s);
 mf_status strip_partition(mf_matrix m, int ctas, cudaStream_t s);
+// slots.cu: what the build of the tiles knows of the row slots: their number
+// (-1: a strip has too many tiles), the most tile columns between a tile and
+// its strip, the entries of the longest row
+constexpr int SLOT_MAX_TILES = 4096;
+void set_slot_sizes(mf_matrix m, long long total, int far, int kmax);
 // spmv.cu
 mf_status spmv_fp64(const MfTiles &A, const double *x, double *y, cudaStream_t s);
 mf_status spmv(mf_matrix m, const double *x, double *y, cudaStream_t s);

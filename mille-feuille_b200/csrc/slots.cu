@@ -38,8 +38,6 @@
 namespace mf {
 namespace {
 
-constexpr int SLOT_MAX_TILES = 4096;
-
 int grid_for3(long long work, int nt)
 {
     long long g = (work + nt - 1) / nt;
@@ -474,70 +472,143 @@ mf_status build_slot_chunks(mf_matrix m, int G, bool staged, cudaStream_t s)
     return MF_OK;
 }
 
-// Builds the slots once (any thread; they do not change afterwards, and the
-// stream is waited for, so every stream may read them).  most > 0: not built
-// when they would hold more entries than that.
-mf_status build_slots(mf_matrix m, cudaStream_t s, long long most)
+// The slots' sizes where the build of the tiles could not tell them (a tile of
+// 256 entries whose last row is empty wraps its row pointers, and a row then
+// has other entries than its CSR row): counted, the stream waited for.
+static mf_status measure_slots(mf_matrix m, cudaStream_t s)
 {
-    if (m->slots_state.load(std::memory_order_acquire) != 0) return MF_OK;
-    std::lock_guard<std::mutex> lk(m->slots_mu);
-    if (m->slots_state.load(std::memory_order_relaxed) != 0) return MF_OK;
+    const int tilem = m->v.tilem;
+    int *d_K = nullptr;
+    MF_CUDA(pool_malloc_async(&d_K, sizeof(int) * ((size_t)tilem + 4), s));
+    int *d_flag = d_K + tilem + 1, total = 0, h[3] = {0, 0, 0};  // too many tiles, farthest tile, largest K
+    mf_status st = MF_OK;
+    cudaError_t e = cudaMemsetAsync(d_flag, 0, 3 * sizeof(int), s);
+    if (e == cudaSuccess) {
+        k_slot_count<<<grid_for3((long long)(tilem + 1) * 16, 256), 256, 0, s>>>(m->v, d_K, d_flag, d_flag + 1, d_flag + 2);
+        note_launch();
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) st = exclusive_scan_i32(d_K, d_K, tilem + 1, s, &total);
+    if (e == cudaSuccess && st == MF_OK) e = cudaMemcpyAsync(h, d_flag, sizeof(h), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess && st == MF_OK) e = cudaStreamSynchronize(s);
+    cudaFreeAsync(d_K, s);
+    MF_TRY(st);
+    MF_CUDA(e);
+    set_slot_sizes(m, h[0] || total < 0 ? -1 : total, h[1], h[2]);
+    return MF_OK;
+}
+
+// Queues the slots on s (sizes known); nothing here waits.
+static mf_status queue_slots(mf_matrix m, cudaStream_t s)
+{
     const MfTiles &A = m->v;
-    const int tilem = A.tilem;
-    int *d_K = nullptr, *d_flag = nullptr;
-    // one temporary: slots per strip; flag, farthest tile, largest K; their scan
-    MF_CUDA(pool_malloc_async(&d_K, sizeof(int) * 2 * ((size_t)tilem + 3), s));
-    d_flag = d_K + tilem + 1;
-    int *d_at = d_flag + 3;
-    MF_CUDA(cudaMemsetAsync(d_flag, 0, 3 * sizeof(int), s));
-    k_slot_count<<<grid_for3((long long)(tilem + 1) * 16, 256), 256, 0, s>>>(A, d_K, d_flag, d_flag + 1, d_flag + 2);
-    note_launch();
-    MF_CUDA(cudaGetLastError());
-    int total = 0, h_flag[3] = {0, 0, 0};
-    MF_TRY(exclusive_scan_i32(d_K, d_at, tilem + 1, s, &total));
-    MF_CUDA(cudaMemcpyAsync(h_flag, d_flag, sizeof(h_flag), cudaMemcpyDeviceToHost, s));
-    MF_CUDA(cudaStreamSynchronize(s));
-    const size_t E = (size_t)total * MF_TILE;
-    // tiles within 2,046 tile columns of the strip: every entry within 32,751 columns
-    const int ob = h_flag[1] <= 2046 ? 2 : 4;
-    if (h_flag[0] || total < 0 || (long long)E > (1ll << 40)) {
-        cudaFreeAsync(d_K, s);
-        m->slots_state.store(-1, std::memory_order_release);  // chunked tile path
-        return MF_OK;
-    }
-    if (most > 0 && (long long)E > most) {
-        cudaFreeAsync(d_K, s);
-        return MF_OK;
-    }
+    const int tilem = A.tilem, ob = m->soff_bytes;
+    const size_t E = (size_t)m->nslots * MF_TILE;
     // slack: 16-byte bulk-copy rounding
     const size_t o_val = (sizeof(int) * ((size_t)tilem + 1) + 32 + 255) / 256 * 256,
                  o_off = o_val + (sizeof(double) * E + 32 + 255) / 256 * 256,
-                 o_meta = o_off + (ob * E + 32 + 255) / 256 * 256;
-    if (handle_malloc(&m->slots_mem, o_meta + sizeof(uint16_t) * E + 32) != cudaSuccess) {
+                 o_meta = o_off + (ob * E + 32 + 255) / 256 * 256, bytes = o_meta + sizeof(uint16_t) * E + 32;
+    void *mem = nullptr;
+    int *flag = nullptr;
+    if (pool_malloc_async(&mem, bytes, s) != cudaSuccess) {
         cudaGetLastError();
-        cudaFreeAsync(d_K, s);
         set_last_error("no device memory for the row slots (%zu entries)", E);
         return MF_ERR_NO_MEMORY;
     }
-    m->d_sslot = (int *)m->slots_mem;
-    m->d_sval = (double *)((char *)m->slots_mem + o_val);
-    m->d_soff = (char *)m->slots_mem + o_off;
-    m->d_smeta = (uint16_t *)((char *)m->slots_mem + o_meta);
-    MF_CUDA(cudaMemcpyAsync(m->d_sslot, d_at, sizeof(int) * (tilem + 1), cudaMemcpyDeviceToDevice, s));
-    cudaFreeAsync(d_K, s);
-    if (tilem > 0) {
+    m->d_sslot = (int *)mem;
+    m->d_sval = (double *)((char *)mem + o_val);
+    m->d_soff = (char *)mem + o_off;
+    m->d_smeta = (uint16_t *)((char *)mem + o_meta);
+    mf_status st = MF_OK;
+    cudaError_t e = pool_malloc_async(&flag, 3 * sizeof(int), s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(flag, 0, 3 * sizeof(int), s);
+    if (e == cudaSuccess) {
+        k_slot_count<<<grid_for3((long long)(tilem + 1) * 16, 256), 256, 0, s>>>(A, m->d_sslot, flag, flag + 1, flag + 2);
+        note_launch();
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) st = exclusive_scan_i32(m->d_sslot, m->d_sslot, tilem + 1, s, nullptr);
+    if (e == cudaSuccess && st == MF_OK && tilem > 0) {
         const int grid = grid_for3((long long)tilem * 16, 256);
         if (ob == 2) k_slot_fill<<<grid, 256, 0, s>>>(A, m->d_sslot, m->d_smeta, m->d_sval, (int16_t *)m->d_soff);
         else k_slot_fill<<<grid, 256, 0, s>>>(A, m->d_sslot, m->d_smeta, m->d_sval, (int32_t *)m->d_soff);
         note_launch();
-        MF_CUDA(cudaGetLastError());
+        e = cudaGetLastError();
     }
-    MF_CUDA(cudaStreamSynchronize(s));
-    m->nslots = total;
-    m->soff_bytes = ob;
-    m->slot_kmax = h_flag[2];
+    if (flag) cudaFreeAsync(flag, s);
+    if (e == cudaSuccess && st == MF_OK && !m->slots_done)
+        e = cudaEventCreateWithFlags(&m->slots_done, cudaEventDisableTiming);
+    if (e == cudaSuccess && st == MF_OK) e = cudaEventRecord(m->slots_done, s);
+    if (e != cudaSuccess || st != MF_OK) {
+        cudaFreeAsync(mem, s);
+        MF_TRY(st);
+        MF_CUDA(e);
+    }
+    m->slots_mem = mem;
+    m->device_bytes += bytes;
     m->slot_policy = -1;
-    m->slots_state.store(1, std::memory_order_release);
+    return MF_OK;
+}
+
+void set_slot_sizes(mf_matrix m, long long total, int far, int kmax)
+{
+    if (total < 0 || total > INT_MAX) {
+        m->slots_state.store(-1, std::memory_order_release);  // chunked tile path
+        return;
+    }
+    m->nslots = total;
+    // tiles within 2,046 tile columns of the strip: every entry within 32,751 columns
+    m->soff_bytes = far <= 2046 ? 2 : 4;
+    m->slot_kmax = kmax;
+}
+
+bool slots_ready(mf_matrix m, bool &done)
+{
+    done = true;
+    if (!m->slots_pending.load(std::memory_order_acquire)) return true;
+    RelaxedCapture relaxed;
+    const cudaError_t e = cudaEventQuery(m->slots_done);
+    if (e == cudaSuccess) {
+        m->slots_pending.store(false, std::memory_order_release);
+        return true;
+    }
+    cudaGetLastError();
+    done = false;
+    return e == cudaErrorNotReady;
+}
+
+// The slots for work on s: built once, by whichever call comes first, in the
+// order of its stream; a call on another stream makes its stream wait for
+// them.  The host waits for nothing, except under a capture (whose graph cannot
+// depend on work outside it) and to measure the few matrices above.  now = false:
+// not built while another thread is at it.
+mf_status build_slots(mf_matrix m, cudaStream_t s, bool now)
+{
+    if (m->slots_state.load(std::memory_order_acquire) == 0) {
+        std::unique_lock<std::mutex> lk(m->slots_mu, std::defer_lock);
+        if (now) lk.lock();
+        else if (!lk.try_lock()) return MF_OK;
+        if (m->slots_state.load(std::memory_order_relaxed) == 0) {
+            if (m->nslots < 0) MF_TRY(measure_slots(m, s));
+            if (m->slots_state.load(std::memory_order_relaxed) != 0) return MF_OK;
+            MF_TRY(queue_slots(m, s));
+            m->slots_pending.store(true, std::memory_order_relaxed);
+            m->slots_state.store(1, std::memory_order_release);
+            return MF_OK;
+        }
+    }
+    if (m->slots_state.load(std::memory_order_acquire) != 1) return MF_OK;
+    bool done;
+    if (!slots_ready(m, done)) MF_CUDA(cudaEventSynchronize(m->slots_done));
+    if (done) return MF_OK;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    RelaxedCapture relaxed;
+    if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+        MF_CUDA(cudaStreamWaitEvent(s, m->slots_done, 0));
+    } else {
+        cudaGetLastError();
+        MF_CUDA(cudaEventSynchronize(m->slots_done));
+    }
     return MF_OK;
 }
 

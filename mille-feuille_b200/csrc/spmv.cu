@@ -155,28 +155,38 @@ static bool may_build(cudaStream_t s)
     return st == cudaStreamCaptureStatusNone;
 }
 
-// y = A x.  Building the slots costs as much as ~30 products (128^3 Poisson: 1
-// ms, mostly allocation, against 28 us saved by each later one), so the first
-// product of a handle, which may be its only one, does not; a matrix whose slots would be more than half padding, or that they
-// cannot describe, stays with the tiles.
+// y = A x.  Building the slots costs as much as several products, so the first
+// product of a handle, which may be its only one, does not; the second queues
+// them in front of its own kernel.  Their sizes are known from the build of the
+// tiles, so no call waits for the GPU.  A matrix whose slots would be more than
+// half padding, or that they cannot describe, stays with the tiles, and so does a
+// captured product while they are still on their way.
 mf_status spmv(mf_matrix m, const double *x, double *y, cudaStream_t s)
 {
     const MfTiles &A = m->v;
     if (A.tilem == 0) return MF_OK;
-    if (m->slots_state.load(std::memory_order_acquire) == 0 && m->spmv_calls.load(std::memory_order_relaxed) >= 0) {
+    const long long most = 2LL * A.nnz + 4096;
+    bool slots = m->slots_state.load(std::memory_order_acquire) == 1, done = true;
+    if (!slots && m->spmv_calls.load(std::memory_order_relaxed) >= 0) {
         const int calls = m->spmv_calls.fetch_add(1, std::memory_order_relaxed);
-        if (calls >= 1 && may_build(s)) {
-            // another thread's capture does not mind the allocations here
-            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-            cudaThreadExchangeStreamCaptureMode(&mode);
-            const mf_status st = build_slots(m, s, 2LL * A.nnz + 4096);
-            cudaThreadExchangeStreamCaptureMode(&mode);
-            if (st != MF_OK) cudaGetLastError();  // no memory for them: the tiles serve
-            if (st != MF_OK || m->slots_state.load() != 1) m->spmv_calls.store(-1);  // do not try again
+        if (m->slots_state.load() < 0 || m->nslots < 0 || m->nslots * MF_TILE > most) {
+            m->spmv_calls.store(-1);  // never from slots that this call would have to build
+        } else if (calls >= 1 && may_build(s)) {
+            RelaxedCapture relaxed;  // another thread's capture does not mind the allocations here
+            mf_status st = build_slots(m, s, false);
+            slots = m->slots_state.load(std::memory_order_acquire) == 1;
+            if (st == MF_OK && slots) st = build_slots(m, s);  // another thread's: s waits for them
+            if (st != MF_OK) {  // no memory for them: the tiles serve
+                cudaGetLastError();
+                m->spmv_calls.store(-1);
+                slots = false;
+            }
         }
+    } else if (slots && !(slots_ready(m, done) && done)) {
+        if (may_build(s)) MF_TRY(build_slots(m, s));
+        else slots = false;
     }
-    if (m->slots_state.load(std::memory_order_acquire) != 1 || m->nslots * MF_TILE > 2LL * A.nnz + 4096)
-        return spmv_fp64(A, x, y, s);
+    if (!slots || m->nslots * MF_TILE > most) return spmv_fp64(A, x, y, s);
     const int grid = ceil_div(A.rows, SPMV_NT);
     if (m->soff_bytes == 2)
         k_spmv_slots<<<grid, SPMV_NT, 0, s>>>(A.rows, m->d_sslot, (const int16_t *)m->d_soff, m->d_sval, x, y);

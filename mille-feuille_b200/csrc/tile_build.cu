@@ -29,6 +29,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cstring>
 #include <type_traits>
 
 #include "mf_internal.h"
@@ -188,6 +189,12 @@ struct TileOut {
     uint16_t *f16;
     int8_t *i8;
     int *err, *class_count, *max_nz;
+    // the row slots (slots.cu): the sum over the strips of their longest row,
+    // the longest of all, the most tile columns between a tile and its strip;
+    // odd: 1 a tile's row pointers wrap (its rows are not the CSR's), 2 a strip
+    // has more tiles than a slot's word can name
+    unsigned long long *slots;
+    int *slot_kmax, *slot_far, *slot_odd;
 };
 
 // Pass 2 for tile-rows of at most `most` entries, a warp each.
@@ -200,11 +207,15 @@ k_fill_warps(int tilem, int rowA, int T, int most, const int *__restrict__ rowpt
     __shared__ int s_rp[NW][MF_TILE + 1];
     __shared__ unsigned s_cnt[NW][WARP_CAP][MF_TILE / 2];  // entries per tile and row, 16 bits each
     __shared__ unsigned s_flag[NW][WARP_CAP];
-    __shared__ int s_class[5], s_max;
+    __shared__ int s_class[5], s_max, s_kmax, s_far;
+    __shared__ unsigned long long s_slots;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (threadIdx.x < 5) s_class[threadIdx.x] = 0;
-    if (threadIdx.x == 5) s_max = 0;
+    if (threadIdx.x == 5) s_max = s_kmax = s_far = 0;
+    if (threadIdx.x == 6) s_slots = 0;
     __syncthreads();
+    int kmax = 0, far = 0;          // of this warp's tile-rows; this lane's entries
+    unsigned long long slots = 0;
     const int rp0 = rowptr[0];
     const int last_begin = tile_ptr[tilem - 1], rowlen_last = rowA - (tilem - 1) * MF_TILE;
     for (int bi = blockIdx.x * NW + w; bi < tilem; bi += gridDim.x * NW) {
@@ -216,6 +227,9 @@ k_fill_warps(int tilem, int rowA, int T, int most, const int *__restrict__ rowpt
         for (int k = lane; k < nt * (MF_TILE / 2); k += 32) s_cnt[w][k / (MF_TILE / 2)][k % (MF_TILE / 2)] = 0;
         for (int k = lane; k < nt; k += 32) s_flag[w][k] = FL_ALL;
         __syncwarp();
+        const int K = __reduce_max_sync(0xffffffffu, lane < rows ? s_rp[w][lane + 1] - s_rp[w][lane] : 0);
+        slots += K;
+        kmax = max(kmax, K);
         int carry = -1, last = -1;  // tile ordinal and tile column before this group of 32 entries
         for (int c0 = 0; c0 < m; c0 += 32) {
             const int k = c0 + lane;
@@ -238,6 +252,7 @@ k_fill_warps(int tilem, int rowA, int T, int most, const int *__restrict__ rowpt
             carry += __popc(heads);
             if (in) {
                 const int dst = d0 + k;
+                far = max(far, abs(bi - jc));
                 if (head) {
                     o.tile_columnidx[t0 + ord] = jc;
                     o.tile_nnz[t0 + ord] = dst;
@@ -272,6 +287,8 @@ k_fill_warps(int tilem, int rowA, int T, int most, const int *__restrict__ rowpt
             }
             const int nz = at;
             if (nz > 256) atomicExch(o.err, (int)MF_ERR_UNSUPPORTED);
+            if (nz == 256 && ((s_cnt[w][k][(rows - 1) >> 1] >> (16 * ((rows - 1) & 1))) & 0xffffu) == 0)
+                atomicOr(o.slot_odd, 1);
             const int po = t < last_begin ? t * MF_TILE : last_begin * MF_TILE + (t - last_begin) * rowlen_last;
             int nonempty = 0;
             if (rows == MF_TILE) {
@@ -302,9 +319,18 @@ k_fill_warps(int tilem, int rowA, int T, int most, const int *__restrict__ rowpt
         }
         __syncwarp();
     }
+    far = __reduce_max_sync(0xffffffffu, far);
+    if (lane == 0) {
+        atomicAdd(&s_slots, slots);
+        atomicMax(&s_kmax, kmax);
+        atomicMax(&s_far, far);
+    }
     __syncthreads();
     if (threadIdx.x < 5 && s_class[threadIdx.x]) atomicAdd(&o.class_count[threadIdx.x], s_class[threadIdx.x]);
     if (threadIdx.x == 5 && s_max) atomicMax(o.max_nz, s_max);
+    if (threadIdx.x == 6 && s_slots) atomicAdd(o.slots, s_slots);
+    if (threadIdx.x == 7 && s_kmax) atomicMax(o.slot_kmax, s_kmax);
+    if (threadIdx.x == 8 && s_far) atomicMax(o.slot_far, s_far);
 }
 
 // The ends of the arrays with one entry more than tiles.
@@ -368,7 +394,7 @@ k_fill_tilerows(int tilem, int rowA, int most, int rp0, const int *__restrict__ 
                 const double *__restrict__ val, const float *__restrict__ val_low, const int *__restrict__ perm,
                 const int *__restrict__ tile_ptr, int *__restrict__ tile_columnidx, int *__restrict__ tile_nnz,
                 int *__restrict__ tile_rowidx, int *__restrict__ run_start, double *__restrict__ out_val,
-                float *__restrict__ out_low, unsigned char *__restrict__ out_col)
+                float *__restrict__ out_low, unsigned char *__restrict__ out_col, TileOut o)
 {
     __shared__ int s_rp[MF_TILE + 1];
     __shared__ int s_warp[BUILD_NT / 32];
@@ -384,6 +410,15 @@ k_fill_tilerows(int tilem, int rowA, int most, int rp0, const int *__restrict__ 
             continue;
         }
         const int t0 = tile_ptr[bi];
+        if (threadIdx.x == 0 && m > 0) {
+            int K = 0;
+            for (int r = 0; r < rows; r++) K = max(K, s_rp[r + 1] - s_rp[r]);
+            const int first = colidx[base + perm[base]] >> 4, last = colidx[base + perm[base + m - 1]] >> 4;
+            atomicAdd(o.slots, (unsigned long long)K);
+            atomicMax(o.slot_kmax, K);
+            atomicMax(o.slot_far, max(abs(bi - first), abs(bi - last)));
+            if (tile_ptr[bi + 1] - t0 > SLOT_MAX_TILES) atomicOr(o.slot_odd, 2);
+        }
         for (int c0 = 0; c0 < m; c0 += BUILD_NT) {
             const int k = c0 + threadIdx.x;
             int src = 0, jc = -1, row = 0, head = 0, rowhead = 0;
@@ -469,6 +504,7 @@ __global__ void k_tile_finish(int tilem, int rowA, int T, int most, const int *_
         const int nz = o.tile_nnz[t + 1] - off;
         if (nz > 256) atomicExch(o.err, (int)MF_ERR_UNSUPPORTED);
         const int rowlen = (bi == tilem - 1) ? rowlen_last : MF_TILE;
+        if (nz == 256 && run_start[(size_t)t * MF_TILE + rowlen - 1] < 0) atomicOr(o.slot_odd, 1);
         const int po = (t < last_row_tiles_begin) ? t * MF_TILE
                                                    : last_row_tiles_begin * MF_TILE + (t - last_row_tiles_begin) * rowlen_last;
         o.csrptr_offset[t] = po;
@@ -663,10 +699,13 @@ mf_status build_tiles(mf_matrix m, int rowA, int colA, const int *d_rowptr, cons
         }
     } tmp;
     tmp.s = s;
-    // status words: [0] err, [1..5] tiles per class, [6] largest tile, [7] long tile-rows
+    // status words: [0] err, [1..5] tiles per class, [6] largest tile, [7] long
+    // tile-rows, of the row slots [8, 9] number, [10] longest row, [11] farthest
+    // tile, [12] odd
+    constexpr int NSTAT = 16;
     int *d_err = nullptr;
-    MF_TRY(tmp.take((void **)&d_err, sizeof(int) * 8));
-    MF_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int) * 8, s));
+    MF_TRY(tmp.take((void **)&d_err, sizeof(int) * NSTAT));
+    MF_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int) * NSTAT, s));
     if (rowA > 0) {
         k_validate<<<std::min(grid_for(rowA, 64), 148 * 16), 256, 0, s>>>(rowA, colA, most, d_rowptr, d_colidx, d_err,
                                                                          d_err + 7);
@@ -759,7 +798,7 @@ mf_status build_tiles(mf_matrix m, int rowA, int colA, const int *d_rowptr, cons
     MF_CUDA(cudaMemsetAsync(m->d_cidx, 0, (size_t)(nnz + 1) / 2 + 1, s));
     TileOut o{m->d_tile_columnidx, m->d_tile_nnz, m->d_tile_rowidx, m->d_csrptr_offset, m->d_nonzero_row_new,
               m->d_ptr, m->d_blknnznnz, m->d_col, m->d_class, m->d_f16ok, m->d_val, m->d_val_low, m->d_f16, m->d_i8,
-              d_err, d_err + 1, d_err + 6};
+              d_err, d_err + 1, d_err + 6, (unsigned long long *)(d_err + 8), d_err + 10, d_err + 11, d_err + 12};
     k_tile_ends<<<1, 1, 0, s>>>(tilem, rowA, T, nnz, m->d_tile_ptr, o);
     note_launch();
     if (tilem > 0) {
@@ -772,7 +811,7 @@ mf_status build_tiles(mf_matrix m, int rowA, int colA, const int *d_rowptr, cons
             MF_CUDA(cudaMemsetAsync(d_run, 0xff, sizeof(int) * (size_t)T * MF_TILE + 16, s));
             k_fill_tilerows<<<grid_for(tilem, 1), BUILD_NT, 0, s>>>(
                 tilem, rowA, most, rp0, d_rowptr, d_colidx, d_val, d_val_low, d_perm, m->d_tile_ptr, m->d_tile_columnidx,
-                m->d_tile_nnz, m->d_tile_rowidx, d_run, m->d_val, m->d_val_low, m->d_col);
+                m->d_tile_nnz, m->d_tile_rowidx, d_run, m->d_val, m->d_val_low, m->d_col, o);
             k_tile_finish<<<grid_for(T, 256), 256, 0, s>>>(tilem, rowA, T, most, d_rowptr, m->d_tile_ptr, d_run, o);
             k_payloads<<<grid_for(T, 256), 256, 0, s>>>(T, rowA, most, d_rowptr, o);
             note_launch(3);
@@ -803,10 +842,10 @@ mf_status build_tiles(mf_matrix m, int rowA, int colA, const int *d_rowptr, cons
     }
     MF_CUDA(cudaGetLastError());
 
-    int cnt_non = 0, rbb = 0, host_counts[8] = {0};
+    int cnt_non = 0, rbb = 0, host_counts[NSTAT] = {0};
     MF_CUDA(cudaMemcpyAsync(&cnt_non, m->d_nonzero_row_new + T, sizeof(int), cudaMemcpyDeviceToHost, s));
     MF_CUDA(cudaMemcpyAsync(&rbb, d_cnt + tilem, sizeof(int), cudaMemcpyDeviceToHost, s));
-    MF_CUDA(cudaMemcpyAsync(host_counts, d_err, sizeof(int) * 8, cudaMemcpyDeviceToHost, s));
+    MF_CUDA(cudaMemcpyAsync(host_counts, d_err, sizeof(host_counts), cudaMemcpyDeviceToHost, s));
     MF_CUDA(cudaStreamSynchronize(s));
     if (host_counts[0]) {
         set_last_error("a 16x16 tile holds more than 256 entries (duplicate entries); u8 row pointers cannot describe it");
@@ -838,6 +877,10 @@ mf_status build_tiles(mf_matrix m, int rowA, int colA, const int *d_rowptr, cons
     m->last_tile_begin = last_begin;
     m->rowblkblock = rbb;
     m->device_bytes = total;
+    unsigned long long slots = 0;
+    memcpy(&slots, host_counts + 8, sizeof(slots));
+    if (!(host_counts[12] & 1))  // else measured when the slots are built
+        set_slot_sizes(m, host_counts[12] & 2 ? -1 : (long long)slots, host_counts[11], host_counts[10]);
     return MF_OK;
 }
 
