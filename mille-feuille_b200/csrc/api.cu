@@ -25,11 +25,11 @@ struct DevPool {
 };
 static std::mutex g_pool_mu;
 static DevPool g_pools[64];
-static std::atomic<int> g_handles[64];
+static int g_handles[64];  // matrix handles of each device
 
 // What the pool holds across synchronisations, used and free together: up to
-// 4 GiB while the device has handles (a 2-million-row matrix with its solver
-// workspace takes 0.65 GB; mapping that anew costs 12 ms), up to 256 MiB
+// 4 GiB while the device has matrix handles (a 2-million-row matrix with its
+// solver workspace takes 0.65 GB; mapping that anew costs 12 ms), up to 256 MiB
 // otherwise.
 static constexpr uint64_t POOL_KEEP = 4096ull << 20, POOL_KEEP_IDLE = 256ull << 20;
 
@@ -56,7 +56,7 @@ static cudaError_t device_pool(int *dev, DevPool *out)
             cudaGetLastError();
             d.anchor = nullptr;
         }
-        uint64_t keep = POOL_KEEP;
+        uint64_t keep = g_handles[*dev] > 0 ? POOL_KEEP : POOL_KEEP_IDLE;
         cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
     }
     *out = d;
@@ -136,12 +136,15 @@ void handle_free(void *p)
 void handle_count(int device, int d)
 {
     if (device < 0 || device >= 64) return;
-    if (g_handles[device].fetch_add(d) + d == 0 && d < 0) {
-        cudaStream_t hs = nullptr;
-        if (handle_stream(&hs) == cudaSuccess) cudaStreamSynchronize(hs);
-        std::lock_guard<std::mutex> lk(g_pool_mu);
-        if (g_pools[device].pool) cudaMemPoolTrimTo(g_pools[device].pool, POOL_KEEP_IDLE);
-    }
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    const int n = g_handles[device] += d;
+    const DevPool &p = g_pools[device];
+    if (!p.pool || n != (d > 0 ? 1 : 0)) return;
+    uint64_t keep = n > 0 ? POOL_KEEP : POOL_KEEP_IDLE;
+    cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (n > 0) return;
+    if (p.stream) cudaStreamSynchronize(p.stream);  // the last handle's frees
+    cudaMemPoolTrimTo(p.pool, POOL_KEEP_IDLE);
 }
 
 void set_last_error(const char *fmt, ...)

@@ -127,3 +127,40 @@ def test_destroy_waits_for_the_device(mf):
     assert not done.query()
     M.close()
     assert done.query()
+
+
+POOL_SCRIPT = """
+import sys
+sys.path.insert(0, {root!r})
+import numpy as np, torch
+import __graft_entry__ as ge
+mf = ge.load_package()
+n = 50000
+one = mf.HostCsr(n, n, np.arange(n + 1), np.arange(n), np.ones(n))
+def batch():  # 16 million rows: 320 MiB of temporaries
+    B = mf.Batch([one] * 320)
+    B.close()
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+M = mf.Matrix(mf.synth_laplace2d(40, 30))
+held = batch()
+M.close()
+torch.cuda.synchronize()
+idle = torch.cuda.mem_get_info()[0]
+print(held, idle, batch())
+"""
+
+
+def test_pool_without_handles_keeps_256_mib():
+    """What the pool keeps of a batch's temporaries: more while a matrix handle
+    lives; without one 256 MiB, whatever handles there were before."""
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    root = str(Path(__file__).resolve().parent.parent)
+    out = subprocess.run([sys.executable, "-c", POOL_SCRIPT.format(root=root)], capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stderr[-2000:]
+    held, idle, after = (int(v) / 2**20 for v in out.stdout.split()[-3:])
+    assert idle - held >= 32  # the handle's pool had kept more than 256 MiB
+    assert idle - after <= 32, (held, idle, after)
