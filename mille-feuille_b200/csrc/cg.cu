@@ -558,6 +558,7 @@ __global__ void __launch_bounds__(NT, ROWS_MINB) k_cg1_rows(CgArgs a)
             }
             fence_acq_rel_gpu();  // with the relaxed load that saw the target: acquire
         }
+        __syncwarp();  // the other lanes' loads come after lane 0's fence
         ok = __shfl_sync(0xffffffffu, ok, 0);
 #pragma unroll
         for (int k = 0; k < 4; k++) v[k] = 0.0;
