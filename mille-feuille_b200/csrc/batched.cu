@@ -100,6 +100,24 @@ constexpr int BCR = MF_BATCH_BCR;   // rows of a chunk
 }  // namespace
 }  // namespace mf
 
+// What a captured solve has fixed: two solves share a graph when all of it
+// agrees.
+struct BatchGraphKey {
+    const double *b;
+    double *x;
+    int lanes, cluster, policy, maxiter;
+    double tol, delta;
+    const void *weights;  // LEARNED
+    unsigned long long budget_ns;
+    unsigned backoff_ns;
+    bool operator==(const BatchGraphKey &o) const
+    {
+        return b == o.b && x == o.x && lanes == o.lanes && cluster == o.cluster && policy == o.policy &&
+               maxiter == o.maxiter && tol == o.tol && delta == o.delta && weights == o.weights &&
+               budget_ns == o.budget_ns && backoff_ns == o.backoff_ns;
+    }
+};
+
 struct mf_batch_s {
     int count = 0;
     long long rows_total = 0, nnz_total = 0;
@@ -145,9 +163,7 @@ struct mf_batch_s {
     uint16_t *d_sc16 = nullptr;
     // CUDA graph of the last solve configuration
     cudaGraphExec_t graph = nullptr;
-    const void *graph_b = nullptr;
-    void *graph_x = nullptr;
-    int graph_key[7] = {0, 0, 0, 0, 0, 0, 0};
+    BatchGraphKey graph_key = {};
     int tuned_lanes = 0, tuned_cluster = 0;
     int static_fp16_chunks = 0, fp16_allowed_chunks = 0;
     struct mf_policy_s *policy = nullptr;     // LEARNED solves
@@ -2394,11 +2410,11 @@ mf_status mf_batch_cg_solve(mf_batch bt, const double *b, double *x, const mf_so
     MF_CUDA(cudaEventCreate(&e0));
     MF_CUDA(cudaEventCreate(&e1));
     MF_CUDA(cudaEventRecord(e0, s));
-    const int key[7] = {lanes, cluster, o.policy, (int)(o.tol * 1e15), o.maxiter,
-                        (int)(a.delta * 1e6), (int)(uintptr_t)a.mlp_w};
+    const BatchGraphKey key = {b,     x,       lanes,   cluster,     o.policy,    o.maxiter,
+                               o.tol, a.delta, a.mlp_w, a.budget_ns, a.backoff_ns};
     if (use_graph) {
         // one graph per (buffers, configuration): replayed on later calls
-        if (!bt->graph || bt->graph_b != b || bt->graph_x != x || memcmp(key, bt->graph_key, sizeof(key))) {
+        if (!bt->graph || !(bt->graph_key == key)) {
             if (bt->graph) cudaGraphExecDestroy(bt->graph);
             bt->graph = nullptr;
             cudaStream_t cs;
@@ -2416,9 +2432,7 @@ mf_status mf_batch_cg_solve(mf_batch bt, const double *b, double *x, const mf_so
             }
             MF_CUDA(cudaGraphInstantiate(&bt->graph, g, 0));
             cudaGraphDestroy(g);
-            bt->graph_b = b;
-            bt->graph_x = x;
-            memcpy(bt->graph_key, key, sizeof(key));
+            bt->graph_key = key;
         }
         MF_CUDA(cudaGraphLaunch(bt->graph, s));
         note_launch(2);  // the graph's kernels: the batched CG and the residual check
