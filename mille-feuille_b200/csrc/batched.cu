@@ -2239,7 +2239,8 @@ mf_status mf_batch_info(mf_batch bt, long long *rows_total, long long *nnz_total
 // per system (the mixed kernel starts every system on a 16-byte boundary)
 static size_t batch_vec_len(mf_batch bt) { return ((size_t)bt->rows_total + 4 * (size_t)bt->count + PW + 16 + 3) & ~(size_t)3; }
 
-static mf_status batch_work(mf_batch bt)
+// The workspace, zeroed in the order of the stream that uses it first.
+static mf_status batch_work(mf_batch bt, cudaStream_t s)
 {
     const size_t need = batch_vec_len(bt) * 8 * 5 + 1024;
     if (bt->work_bytes >= need) return MF_OK;
@@ -2247,7 +2248,7 @@ static mf_status batch_work(mf_batch bt)
     bt->work = nullptr;
     bt->work_bytes = 0;
     MF_CUDA(cudaMalloc(&bt->work, need));
-    MF_CUDA(cudaMemset(bt->work, 0, need));
+    MF_CUDA(cudaMemsetAsync(bt->work, 0, need, s));
     bt->work_bytes = need;
     return MF_OK;
 }
@@ -2403,7 +2404,7 @@ mf_status mf_batch_cg_solve(mf_batch bt, const double *b, double *x, const mf_so
     int lanes, cluster;
     const bool mixed = o.policy != MF_POLICY_FP64;
     batch_schedule(bt, mixed, lanes, cluster);
-    MF_TRY(batch_work(bt));
+    MF_TRY(batch_work(bt, s));
     const int ctas = batch_ctas(bt, mixed, lanes, cluster);
     const BatchArgs a = batch_args(bt, b, x, o);
     cudaEvent_t e0, e1;
@@ -2602,7 +2603,7 @@ mf_status mf_batch_policy_collect(mf_learned p, mf_batch bt, const double *b, in
     unsigned char *cy = nullptr;
     long long have = 0;
     MF_TRY(policy_sample_buffers(p, max_samples, &cx, &cy, &have));
-    MF_TRY(batch_work(bt));
+    MF_TRY(batch_work(bt, 0));
     double *x = nullptr;
     unsigned long long *cnt = nullptr;
     MF_CUDA(cudaMalloc(&x, sizeof(double) * (bt->rows_total + 1)));
@@ -2658,7 +2659,7 @@ mf_status mf_batch_tune(mf_batch bt, const double *b, double *x, const mf_solve_
     int bl = 8, bc = 2;
     cudaStream_t s = (cudaStream_t)stream;
     const bool mixed = o.policy != MF_POLICY_FP64;
-    MF_TRY(batch_work(bt));
+    MF_TRY(batch_work(bt, s));
     const BatchArgs a = batch_args(bt, b, x, o);
     for (int li : lanes_c)
         for (int ci : clus_c) {
