@@ -141,10 +141,13 @@ void handle_count(int device, int d)
     const DevPool &p = g_pools[device];
     if (!p.pool || n != (d > 0 ? 1 : 0)) return;
     uint64_t keep = n > 0 ? POOL_KEEP : POOL_KEEP_IDLE;
+    if (n == 0) {
+        // trimmed under the higher threshold: a wait under the lower one would
+        // give back more than the excess
+        if (p.stream) cudaStreamSynchronize(p.stream);  // the last handle's frees
+        cudaMemPoolTrimTo(p.pool, POOL_KEEP_IDLE);
+    }
     cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    if (n > 0) return;
-    if (p.stream) cudaStreamSynchronize(p.stream);  // the last handle's frees
-    cudaMemPoolTrimTo(p.pool, POOL_KEEP_IDLE);
 }
 
 void set_last_error(const char *fmt, ...)
