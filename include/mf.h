@@ -214,7 +214,9 @@ typedef struct mf_solve_report {
      * largest per-CTA SpMV-phase time; inside the SpMV phase: [6] waiting
      * for staged chunks, then for tile chunks [7] building x segments and
      * [8] computing rows, for row slots [7] computing rows and [8] the
-     * closing barrier and refill */
+     * closing barrier and refill.  [6] to [8] are 0 where FP64 rows are read
+     * straight from the slot arrays, all of them in the one-reduction CG of
+     * small FP64 systems */
     double phase_us[9];
     int layout;            /* execution layout of the solve: 0 tile chunks,
                               1 row slots, 2 staged row slots (the chunk's

@@ -20,6 +20,12 @@
 // to SELL_BINS gets equal shares: bit reversal spreads the bins with one slice
 // more evenly over every such split.
 //
+// A row is summed in the order its entries are stored in: another rounding
+// than the matrix's own order (FP32 in the products, FP64 in the refinement).
+// Error of solves to 1e-14 against 64 bits, CSR order and this one: 24 systems
+// of 1,000-4,000 rows 1.9e-12 and 2.5e-12, 256 of 1,000-32,000 rows 2.44e-12 and
+// 2.42e-12.
+//
 // Four arrays share that geometry: cv (FP16 value bits << 16 | column in the
 // window), v32 and v64 (FP32 and FP64 values) and c16 (column in the window).  Diagonal
 // entries are left out: a row's FP32 diagonal and FP16 scale are part of its

@@ -19,10 +19,11 @@
 // gathers hit shared memory.  Systems whose window and vectors fit (up to
 // ~22,000 rows with 2 CTAs) keep p, r, q and the correction on the chip, p
 // and q going to the cluster's other CTAs by distributed shared memory.
-// What bounds it: the L1 data pipe (a warp's slot of 32 entries takes ~5
-// wavefronts -- 2 for its words, ~2 for the gather, the rest for the row
-// ends; 6.4 cycles measured), then the three cluster barriers of an
-// iteration.  The earlier form -- bulk copies into three shared-memory
+// What bounds it: in the product the L1 data pipe (a warp's slot of 32 entries
+// takes 5.1 wavefronts -- 2 for its words, ~2 for the gather, the rest for the
+// row ends -- and 6.4 cycles); over a whole launch that pipe is busy 48 % of the
+// time, the rest goes to the words' latency, the vectors and the three cluster
+// barriers of an iteration.  The earlier form -- bulk copies into three shared-memory
 // stages, products written back to shared memory, one lane per row adding
 // them, vectors in global memory -- moved every entry through shared memory
 // four times.  Measured on one B200: the 512-system benchmark batch (1,000 to

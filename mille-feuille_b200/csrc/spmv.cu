@@ -155,7 +155,8 @@ static bool may_build(cudaStream_t s)
     return st == cudaStreamCaptureStatusNone;
 }
 
-// y = A x.  Building the slots costs as much as several products, so the first
+// y = A x.  Building the slots costs as much as five products (128^3 Poisson: 0.18
+// ms of kernels, against 25 us saved by each later product), so the first
 // product of a handle, which may be its only one, does not; the second queues
 // them in front of its own kernel.  Their sizes are known from the build of the
 // tiles, so no call waits for the GPU.  A matrix whose slots would be more than

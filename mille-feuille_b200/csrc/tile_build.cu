@@ -23,9 +23,11 @@
 //
 // All arrays live in one allocation of the library's memory pool, sized by
 // bounds known once the tiles are counted, so a build waits for the GPU three
-// times and allocates once.  Measured on a 96^3 Poisson matrix (6.1 M
-// entries), create, one product, destroy: 11.3 -> 0.43 ms (create 6.3 -> 0.40,
-// of which kernels ~0.2; destroy 4.2 -> 0.01).
+// times and allocates once.  What the row slots (slots.cu) need to be allocated
+// without another wait -- their number, the longest row, the farthest tile -- is
+// summed up beside it.  Measured on a 96^3 Poisson matrix (6.1 M entries),
+// create, one product, destroy: 11.3 -> 0.44 ms (create 6.3 -> 0.40, of which
+// kernels 0.25 run one by one and cold; destroy 4.2 -> 0.01).
 #include <cuda_fp16.h>
 
 #include <algorithm>
