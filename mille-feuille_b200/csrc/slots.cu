@@ -562,6 +562,14 @@ void set_slot_sizes(mf_matrix m, long long total, int far, int kmax)
     m->slot_kmax = kmax;
 }
 
+bool capturing(cudaStream_t s)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
 bool slots_ready(mf_matrix m, bool &done)
 {
     done = true;
@@ -585,6 +593,10 @@ bool slots_ready(mf_matrix m, bool &done)
 mf_status build_slots(mf_matrix m, cudaStream_t s, bool now)
 {
     if (m->slots_state.load(std::memory_order_acquire) == 0) {
+        if (capturing(s)) {
+            set_last_error("a matrix's row slots cannot be built under a stream capture: make one call before it");
+            return MF_ERR_CUDA;
+        }
         std::unique_lock<std::mutex> lk(m->slots_mu, std::defer_lock);
         if (now) lk.lock();
         else if (!lk.try_lock()) return MF_OK;
@@ -601,14 +613,9 @@ mf_status build_slots(mf_matrix m, cudaStream_t s, bool now)
     bool done;
     if (!slots_ready(m, done)) MF_CUDA(cudaEventSynchronize(m->slots_done));
     if (done) return MF_OK;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     RelaxedCapture relaxed;
-    if (cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
-        MF_CUDA(cudaStreamWaitEvent(s, m->slots_done, 0));
-    } else {
-        cudaGetLastError();
-        MF_CUDA(cudaEventSynchronize(m->slots_done));
-    }
+    if (capturing(s)) MF_CUDA(cudaEventSynchronize(m->slots_done));
+    else MF_CUDA(cudaStreamWaitEvent(s, m->slots_done, 0));
     return MF_OK;
 }
 

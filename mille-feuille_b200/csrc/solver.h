@@ -146,6 +146,9 @@ mf_status launch_bicgstab(bool mixed, CgArgs &a, int G, cudaStream_t s);
 int bicgstab_grid(mf_matrix m, bool mixed, int layout);  // layout as solver_grid (2: mixed only)
 // slots.cu: the row-slot layout (built once; state -1 = not describable)
 mf_status build_slots(mf_matrix m, cudaStream_t s, bool now = true);
+// whether s (or, s being the legacy stream, any blocking stream) is captured:
+// memory allocated on it would belong to the graph
+bool capturing(cudaStream_t s);
 // whether the slots' kernels are through (done), without waiting; false: the
 // query failed
 bool slots_ready(mf_matrix m, bool &done);

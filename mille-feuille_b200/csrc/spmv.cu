@@ -143,18 +143,6 @@ mf_status spmv_fp64(const MfTiles &A, const double *x, double *y, cudaStream_t s
     return MF_OK;
 }
 
-// Whether the slots may be built on this call: not while the stream (or, on
-// the legacy stream, any blocking stream) is being captured.
-static bool may_build(cudaStream_t s)
-{
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return st == cudaStreamCaptureStatusNone;
-}
-
 // y = A x.  Building the slots costs as much as five products (128^3 Poisson: 0.18
 // ms of kernels, against 25 us saved by each later product), so the first
 // product of a handle, which may be its only one, does not; the second queues
@@ -172,7 +160,7 @@ mf_status spmv(mf_matrix m, const double *x, double *y, cudaStream_t s)
         const int calls = m->spmv_calls.fetch_add(1, std::memory_order_relaxed);
         if (m->slots_state.load() < 0 || m->nslots < 0 || m->nslots * MF_TILE > most) {
             m->spmv_calls.store(-1);  // never from slots that this call would have to build
-        } else if (calls >= 1 && may_build(s)) {
+        } else if (calls >= 1 && !capturing(s)) {
             RelaxedCapture relaxed;  // another thread's capture does not mind the allocations here
             mf_status st = build_slots(m, s, false);
             slots = m->slots_state.load(std::memory_order_acquire) == 1;
@@ -184,7 +172,7 @@ mf_status spmv(mf_matrix m, const double *x, double *y, cudaStream_t s)
             }
         }
     } else if (slots && !(slots_ready(m, done) && done)) {
-        if (may_build(s)) MF_TRY(build_slots(m, s));
+        if (!capturing(s)) MF_TRY(build_slots(m, s));
         else slots = false;
     }
     if (!slots || m->nslots * MF_TILE > most) return spmv_fp64(A, x, y, s);

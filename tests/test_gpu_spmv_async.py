@@ -128,3 +128,31 @@ def test_device_bytes_count_the_slots(mf):
     torch.cuda.synchronize()
     assert M.info().device_bytes >= before + 12 * A.nnz
     M.close()
+
+
+def test_slots_are_not_built_under_a_capture(mf):
+    """mf_spmm's first call needs the slots: refused while its stream is captured
+    (their memory would belong to the graph), and nothing of it stays."""
+    A = mf.synth_poisson3d_scaled(12, 3)
+    n = A.n_rows
+    M, T = mf.Matrix(A), mf.Matrix(A)
+    L = mf.lib()
+    X = torch.from_numpy(np.random.default_rng(3).normal(size=(2, n))).cuda()
+    Y, want = torch.zeros_like(X), torch.zeros_like(X)
+    mf.check(L.mf_spmm(T.h, 2, X.data_ptr(), n, want.data_ptr(), n, None))
+    torch.cuda.synchronize()
+    g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        g.capture_begin(capture_error_mode="thread_local")
+        st = L.mf_spmm(M.h, 2, X.data_ptr(), n, Y.data_ptr(), n, s.cuda_stream)
+        Y.add_(1.0)
+        g.capture_end()
+    assert st == 2  # MF_ERR_CUDA
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.all(Y == 1.0)
+    mf.check(L.mf_spmm(M.h, 2, X.data_ptr(), n, Y.data_ptr(), n, None))
+    torch.cuda.synchronize()
+    assert torch.equal(Y, want)
+    M.close()
+    T.close()
