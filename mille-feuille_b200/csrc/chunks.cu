@@ -100,8 +100,7 @@ int grid_for3(long long work, int nt)
 mf_status build_chunks(mf_matrix m, cudaStream_t s)
 {
     const int G = m->part_ctas;
-    handle_release(m->d_cta_chunk);
-    handle_release(m->d_chunks);
+    handle_release(m->d_cta_chunk, m->d_chunks);
     MF_CUDA(handle_malloc(&m->d_cta_chunk, sizeof(int) * (G + 1)));
     k_chunk_count<<<grid_for3(G + 1, 128), 128, 0, s>>>(G, m->d_part, m->d_tile_ptr, m->d_tile_nnz, m->d_cta_chunk);
     note_launch();

@@ -33,8 +33,8 @@ struct RelaxedCapture {
 };
 // Memory kept on a handle, from the same pool (a driver allocation costs 0.1
 // to 1 ms, a matrix has up to twenty): usable on every stream at once.
-// handle_free returns it; nothing may still use it.  handle_release is for a
-// buffer that a larger one replaces: it waits for the device first, since an
+// handle_free returns it; nothing may still use it.  handle_release is for
+// buffers that others replace: it waits for the device first, since an
 // earlier call may still run on any stream and neither cudaFree nor
 // cudaFreeAsync of a pool's memory waits for it -- the block could be handed
 // out again at once.  handle_count(device, +1 / -1): a matrix handle was made /
@@ -42,13 +42,13 @@ struct RelaxedCapture {
 cudaError_t handle_malloc(void **p, size_t bytes);
 void handle_free(void *p);
 void handle_wait();
-template <typename T>
-inline void handle_release(T *&p)
+template <typename... T>
+inline void handle_release(T *&...p)
 {
-    if (!p) return;
+    if (!(p || ...)) return;
     handle_wait();
-    handle_free((void *)p);
-    p = nullptr;
+    (handle_free((void *)p), ...);
+    ((p = nullptr), ...);
 }
 void handle_count(int device, int d);
 template <typename T>

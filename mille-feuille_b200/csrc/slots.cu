@@ -422,8 +422,7 @@ mf_status build_slot_chunks(mf_matrix m, int G, bool staged, cudaStream_t s)
 {
     const int mode = staged ? 2 : 1;
     if (m->schunk_ctas == G && m->d_schunks && m->schunk_mode == mode) return MF_OK;
-    handle_release(m->d_scta_chunk);
-    handle_release(m->d_schunks);
+    handle_release(m->d_scta_chunk, m->d_schunks);
     m->schunk_ctas = 0;
     m->schunk_mode = 0;
     m->schunk_staged = 0;
