@@ -2018,7 +2018,8 @@ cudaError_t batch_slices(mf_batch bt)
     } while (false);
     if (tmp) cudaFreeAsync(tmp, 0);
     if (quads) cudaFreeAsync(quads, 0);
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    // (not the device: that is not permitted while another thread captures)
+    if (e == cudaSuccess) e = cudaStreamSynchronize(0);
     return e;
 }
 
@@ -2586,7 +2587,7 @@ mf_status mf_batch_policy_classify(mf_batch bt, const double *r, const double *p
                                                          classes, features);
     note_launch();
     MF_CUDA(cudaGetLastError());
-    MF_CUDA(cudaDeviceSynchronize());
+    MF_CUDA(cudaStreamSynchronize(0));
     return MF_OK;
 }
 
