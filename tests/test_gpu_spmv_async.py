@@ -156,3 +156,30 @@ def test_slots_are_not_built_under_a_capture(mf):
     assert torch.equal(Y, want)
     M.close()
     T.close()
+
+
+@pytest.mark.parametrize("tiles", [4096, 4097])
+def test_strip_of_many_tiles(mf, tiles):
+    """A strip of 4,096 tiles has slots, one more has none (a slot's word cannot
+    name the tile): products from the tiles, mf_spmm refused."""
+    n = 16 * tiles
+    ci = 16 * np.arange(tiles) + np.arange(tiles) % 16
+    rp = np.zeros(n + 1, np.int32)
+    rp[6:] = tiles
+    A = mf.HostCsr(n, n, rp, ci, np.random.default_rng(2).normal(size=tiles))
+    M = mf.Matrix(A)
+    L = mf.lib()
+    x = torch.from_numpy(np.cos(0.1 * np.arange(n))).cuda()
+    ys = [torch.full((n,), 9.0, dtype=torch.float64, device="cuda") for _ in range(3)]
+    for y in ys:
+        mf.check(L.mf_spmv(M.h, x.data_ptr(), y.data_ptr(), None))
+    X = torch.stack([x, x])
+    Y = torch.zeros_like(X)
+    st = L.mf_spmm(M.h, 2, X.data_ptr(), n, Y.data_ptr(), n, None)
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, ys[0]) for y in ys[1:])
+    assert abs(ys[0][5].item() - float(A.val @ np.cos(0.1 * ci))) <= 1e-10 * tiles
+    assert st == (0 if tiles <= 4096 else 8)  # MF_ERR_UNSUPPORTED
+    if st == 0:
+        assert torch.equal(Y[0], ys[0]) and torch.equal(Y[1], ys[0])
+    M.close()
