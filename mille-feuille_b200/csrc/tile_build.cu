@@ -191,12 +191,7 @@ struct TileOut {
     uint16_t *f16;
     int8_t *i8;
     int *err, *class_count, *max_nz;
-    // the row slots (slots.cu): the sum over the strips of their longest row,
-    // the longest of all, the most tile columns between a tile and its strip;
-    // odd: 1 a tile's row pointers wrap (its rows are not the CSR's), 2 a strip
-    // has more tiles than a slot's word can name
-    unsigned long long *slots;
-    int *slot_kmax, *slot_far, *slot_odd;
+    int *slot_odd;  // bit 0: a tile's row pointers wrap (its rows are not the CSR's)
 };
 
 // Pass 2 for tile-rows of at most `most` entries, a warp each.
@@ -209,17 +204,19 @@ k_fill_warps(int tilem, int rowA, int T, int most, const int *__restrict__ rowpt
     __shared__ int s_rp[NW][MF_TILE + 1];
     __shared__ unsigned s_cnt[NW][WARP_CAP][MF_TILE / 2];  // entries per tile and row, 16 bits each
     __shared__ unsigned s_flag[NW][WARP_CAP];
-    __shared__ int s_class[5], s_max, s_kmax, s_far;
-    __shared__ unsigned long long s_slots;
+    __shared__ int s_class[5], s_max;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (threadIdx.x < 5) s_class[threadIdx.x] = 0;
-    if (threadIdx.x == 5) s_max = s_kmax = s_far = 0;
-    if (threadIdx.x == 6) s_slots = 0;
+    if (threadIdx.x == 5) s_max = 0;
     __syncthreads();
-    int kmax = 0, far = 0;          // of this warp's tile-rows; this lane's entries
-    unsigned long long slots = 0;
     const int rp0 = rowptr[0];
     const int last_begin = tile_ptr[tilem - 1], rowlen_last = rowA - (tilem - 1) * MF_TILE;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {  // the ends of the arrays with one entry more than tiles
+        o.tile_nnz[T] = rowptr[rowA] - rp0;
+        o.csrptr_offset[T] = T > last_begin ? last_begin * MF_TILE + (T - last_begin) * rowlen_last : T * MF_TILE;
+        o.blknnznnz[T] = 0;
+        o.nz_rows[T] = 0;
+    }
     for (int bi = blockIdx.x * NW + w; bi < tilem; bi += gridDim.x * NW) {
         const int rs = bi * MF_TILE, rows = min(rowA - rs, MF_TILE);
         const int base = rowptr[rs], m = rowptr[rs + rows] - base;
@@ -229,9 +226,6 @@ k_fill_warps(int tilem, int rowA, int T, int most, const int *__restrict__ rowpt
         for (int k = lane; k < nt * (MF_TILE / 2); k += 32) s_cnt[w][k / (MF_TILE / 2)][k % (MF_TILE / 2)] = 0;
         for (int k = lane; k < nt; k += 32) s_flag[w][k] = FL_ALL;
         __syncwarp();
-        const int K = __reduce_max_sync(0xffffffffu, lane < rows ? s_rp[w][lane + 1] - s_rp[w][lane] : 0);
-        slots += K;
-        kmax = max(kmax, K);
         int carry = -1, last = -1;  // tile ordinal and tile column before this group of 32 entries
         for (int c0 = 0; c0 < m; c0 += 32) {
             const int k = c0 + lane;
@@ -254,7 +248,6 @@ k_fill_warps(int tilem, int rowA, int T, int most, const int *__restrict__ rowpt
             carry += __popc(heads);
             if (in) {
                 const int dst = d0 + k;
-                far = max(far, abs(bi - jc));
                 if (head) {
                     o.tile_columnidx[t0 + ord] = jc;
                     o.tile_nnz[t0 + ord] = dst;
@@ -321,28 +314,9 @@ k_fill_warps(int tilem, int rowA, int T, int most, const int *__restrict__ rowpt
         }
         __syncwarp();
     }
-    far = __reduce_max_sync(0xffffffffu, far);
-    if (lane == 0) {
-        atomicAdd(&s_slots, slots);
-        atomicMax(&s_kmax, kmax);
-        atomicMax(&s_far, far);
-    }
     __syncthreads();
     if (threadIdx.x < 5 && s_class[threadIdx.x]) atomicAdd(&o.class_count[threadIdx.x], s_class[threadIdx.x]);
     if (threadIdx.x == 5 && s_max) atomicMax(o.max_nz, s_max);
-    if (threadIdx.x == 6 && s_slots) atomicAdd(o.slots, s_slots);
-    if (threadIdx.x == 7 && s_kmax) atomicMax(o.slot_kmax, s_kmax);
-    if (threadIdx.x == 8 && s_far) atomicMax(o.slot_far, s_far);
-}
-
-// The ends of the arrays with one entry more than tiles.
-__global__ void k_tile_ends(int tilem, int rowA, int T, int nnz, const int *__restrict__ tile_ptr, TileOut o)
-{
-    const int lb = tilem > 0 ? tile_ptr[tilem - 1] : 0, rowlen_last = rowA - (tilem - 1) * MF_TILE;
-    o.tile_nnz[T] = nnz;
-    o.csrptr_offset[T] = (T > lb) ? lb * MF_TILE + (T - lb) * rowlen_last : T * MF_TILE;
-    o.blknnznnz[T] = 0;
-    o.nz_rows[T] = 0;
 }
 
 // Pass 1 for tile-rows above `most` entries: sort by (tile column, CSR
@@ -396,7 +370,7 @@ k_fill_tilerows(int tilem, int rowA, int most, int rp0, const int *__restrict__ 
                 const double *__restrict__ val, const float *__restrict__ val_low, const int *__restrict__ perm,
                 const int *__restrict__ tile_ptr, int *__restrict__ tile_columnidx, int *__restrict__ tile_nnz,
                 int *__restrict__ tile_rowidx, int *__restrict__ run_start, double *__restrict__ out_val,
-                float *__restrict__ out_low, unsigned char *__restrict__ out_col, TileOut o)
+                float *__restrict__ out_low, unsigned char *__restrict__ out_col)
 {
     __shared__ int s_rp[MF_TILE + 1];
     __shared__ int s_warp[BUILD_NT / 32];
@@ -412,15 +386,6 @@ k_fill_tilerows(int tilem, int rowA, int most, int rp0, const int *__restrict__ 
             continue;
         }
         const int t0 = tile_ptr[bi];
-        if (threadIdx.x == 0 && m > 0) {
-            int K = 0;
-            for (int r = 0; r < rows; r++) K = max(K, s_rp[r + 1] - s_rp[r]);
-            const int first = colidx[base + perm[base]] >> 4, last = colidx[base + perm[base + m - 1]] >> 4;
-            atomicAdd(o.slots, (unsigned long long)K);
-            atomicMax(o.slot_kmax, K);
-            atomicMax(o.slot_far, max(abs(bi - first), abs(bi - last)));
-            if (tile_ptr[bi + 1] - t0 > SLOT_MAX_TILES) atomicOr(o.slot_odd, 2);
-        }
         for (int c0 = 0; c0 < m; c0 += BUILD_NT) {
             const int k = c0 + threadIdx.x;
             int src = 0, jc = -1, row = 0, head = 0, rowhead = 0;
@@ -555,20 +520,62 @@ __global__ void k_nonzero_lists(int tilem, int rowA, int T, const int *__restric
     }
 }
 
-// Row-block schedule of blockspmv_cpu (src/blockspmv_cpu.h:35-83).
-__global__ void k_rbb_count(int tilem, const int *__restrict__ tile_ptr, int *__restrict__ cnt,
-                            int *__restrict__ block_signal)
+// What the row slots (slots.cu) need: the sum over the strips of their longest
+// row, the longest of all, the most tile columns between a tile and its strip;
+// bit 1 of odd: a strip has more tiles than a slot's word can name.
+struct SlotSizes {
+    unsigned long long *total;
+    int *kmax, *far, *odd;
+};
+
+// Row-block schedule of blockspmv_cpu (src/blockspmv_cpu.h:35-83), and the row
+// slots' sizes.
+__global__ void __launch_bounds__(BUILD_NT)
+k_rbb_count(int tilem, int rowA, const int *__restrict__ rowptr, const int *__restrict__ tile_ptr,
+            const int *__restrict__ tile_columnidx, int *__restrict__ cnt, int *__restrict__ block_signal, SlotSizes o)
 {
-    for (int bi = blockIdx.x * blockDim.x + threadIdx.x; bi <= tilem; bi += gridDim.x * blockDim.x) {
+    __shared__ int s_total[BUILD_NT / 32], s_kmax[BUILD_NT / 32], s_far[BUILD_NT / 32];
+    int total = 0, kmax = 0, far = 0;  // a thread's few strips: far below 2^31
+    for (int bi = blockIdx.x * BUILD_NT + threadIdx.x; bi <= tilem; bi += gridDim.x * BUILD_NT) {
         if (bi == tilem) {
             cnt[bi] = 0;
             block_signal[bi] = 0;
             continue;
         }
-        int k = tile_ptr[bi + 1] - tile_ptr[bi];
+        const int t0 = tile_ptr[bi], t1 = tile_ptr[bi + 1], k = t1 - t0;
+        int at[MF_TILE + 1], K = 0;  // all in flight together (rows past the last: empty)
+#pragma unroll
+        for (int r = 0; r <= MF_TILE; r++) at[r] = rowptr[min(bi * MF_TILE + r, rowA)];
         cnt[bi] = (k <= 4) ? 1 : (k + 3) / 4;
         block_signal[bi] = k;
+#pragma unroll
+        for (int r = 0; r < MF_TILE; r++) K = max(K, at[r + 1] - at[r]);
+        total += K;
+        kmax = max(kmax, K);
+        if (k > 0) far = max(far, max(bi - tile_columnidx[t0], tile_columnidx[t1 - 1] - bi));
+        if (k > SLOT_MAX_TILES) atomicOr(o.odd, 2);
     }
+    const int w = threadIdx.x >> 5;
+    unsigned long long sum = 0;
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) total += __shfl_xor_sync(0xffffffffu, total, d);
+    kmax = __reduce_max_sync(0xffffffffu, kmax);
+    far = __reduce_max_sync(0xffffffffu, far);
+    if ((threadIdx.x & 31) == 0) {
+        s_total[w] = total;
+        s_kmax[w] = kmax;
+        s_far[w] = far;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int v = 0; v < BUILD_NT / 32; v++) {
+        sum += s_total[v];
+        kmax = max(kmax, s_kmax[v]);
+        far = max(far, s_far[v]);
+    }
+    if (sum) atomicAdd(o.total, sum);
+    if (kmax > *(volatile int *)o.kmax) atomicMax(o.kmax, kmax);
+    if (far > *(volatile int *)o.far) atomicMax(o.far, far);
 }
 
 __global__ void k_rbb_fill(int tilem, const int *__restrict__ tile_ptr, const int *__restrict__ off,
@@ -800,9 +807,8 @@ mf_status build_tiles(mf_matrix m, int rowA, int colA, const int *d_rowptr, cons
     MF_CUDA(cudaMemsetAsync(m->d_cidx, 0, (size_t)(nnz + 1) / 2 + 1, s));
     TileOut o{m->d_tile_columnidx, m->d_tile_nnz, m->d_tile_rowidx, m->d_csrptr_offset, m->d_nonzero_row_new,
               m->d_ptr, m->d_blknnznnz, m->d_col, m->d_class, m->d_f16ok, m->d_val, m->d_val_low, m->d_f16, m->d_i8,
-              d_err, d_err + 1, d_err + 6, (unsigned long long *)(d_err + 8), d_err + 10, d_err + 11, d_err + 12};
-    k_tile_ends<<<1, 1, 0, s>>>(tilem, rowA, T, nnz, m->d_tile_ptr, o);
-    note_launch();
+              d_err, d_err + 1, d_err + 6, d_err + 12};
+    if (tilem == 0) MF_CUDA(cudaMemsetAsync(m->tiles_mem, 0, total, s));  // no tiles: every array ends at 0
     if (tilem > 0) {
         k_fill_warps<<<grid_for((long long)tilem * 32, WF_NT), WF_NT, 0, s>>>(
             tilem, rowA, T, most, d_rowptr, d_colidx, d_val, d_val_low, d_perm8, m->d_tile_ptr, o);
@@ -813,7 +819,7 @@ mf_status build_tiles(mf_matrix m, int rowA, int colA, const int *d_rowptr, cons
             MF_CUDA(cudaMemsetAsync(d_run, 0xff, sizeof(int) * (size_t)T * MF_TILE + 16, s));
             k_fill_tilerows<<<grid_for(tilem, 1), BUILD_NT, 0, s>>>(
                 tilem, rowA, most, rp0, d_rowptr, d_colidx, d_val, d_val_low, d_perm, m->d_tile_ptr, m->d_tile_columnidx,
-                m->d_tile_nnz, m->d_tile_rowidx, d_run, m->d_val, m->d_val_low, m->d_col, o);
+                m->d_tile_nnz, m->d_tile_rowidx, d_run, m->d_val, m->d_val_low, m->d_col);
             k_tile_finish<<<grid_for(T, 256), 256, 0, s>>>(tilem, rowA, T, most, d_rowptr, m->d_tile_ptr, d_run, o);
             k_payloads<<<grid_for(T, 256), 256, 0, s>>>(T, rowA, most, d_rowptr, o);
             note_launch(3);
@@ -834,7 +840,10 @@ mf_status build_tiles(mf_matrix m, int rowA, int colA, const int *d_rowptr, cons
     }
 
     // row-block schedule (d_cnt is free again)
-    k_rbb_count<<<grid_for(tilem + 1, 256), 256, 0, s>>>(tilem, m->d_tile_ptr, d_cnt, m->d_block_signal);
+    const SlotSizes slot_sizes{(unsigned long long *)(d_err + 8), d_err + 10, d_err + 11, d_err + 12};
+    k_rbb_count<<<grid_for(tilem + 1, BUILD_NT), BUILD_NT, 0, s>>>(tilem, rowA, d_rowptr, m->d_tile_ptr,
+                                                                    m->d_tile_columnidx, d_cnt, m->d_block_signal,
+                                                                    slot_sizes);
     note_launch();
     MF_TRY(exclusive_scan_i32(d_cnt, d_cnt, tilem + 1, s, nullptr));
     if (tilem > 0) {

@@ -183,3 +183,13 @@ def test_strip_of_many_tiles(mf, tiles):
     if st == 0:
         assert torch.equal(Y[0], ys[0]) and torch.equal(Y[1], ys[0])
     M.close()
+
+
+def test_matrix_without_rows(mf):
+    """No tile-row: every array with an end entry ends at 0."""
+    M = mf.Matrix(mf.HostCsr(0, 40, [0], [], []))
+    i = M.info()
+    assert (i.rows, i.nnz, i.tilem, i.tilenum, i.csrptrlen, i.nonzero_rows) == (0, 0, 0, 0, 0, 0)
+    for name in ("tile_nnz", "csrptr_offset", "blknnznnz", "nonzero_row_new"):
+        assert not np.any(M.export(name))
+    M.close()
